@@ -67,63 +67,6 @@ struct Acc<float> {
 };
 
 // ===========================================================================
-// init_tracers_AB: valuesAB and the valuesold shift (src/oce_tracer_mod.F90:46-123)
-// ===========================================================================
-template <typename R>
-__global__ void k_ab(DTracers<R> tr, size_t n, int ab) {
-    const R ca = R(0.5 + kABEpsilon), cb = R(1.5 + kABEpsilon);
-    for (int t = 0; t < tr.ntr; t++) {
-        R *T = tr.T + t * tr.sN, *TAB = tr.TAB + t * tr.sN;
-        R *O = tr.Told + t * tr.sN * (ab - 1);
-        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-            R v = T[i];
-            if (ab == 2) {
-                TAB[i] = -(ca * O[i]) + cb * v;
-                O[i] = v;
-            } else {
-                R o1 = O[2 * i], o2 = O[2 * i + 1];
-                R x = R(5.0) * o2 - R(16.0) * o1 + R(23.0) * v;
-                TAB[i] = x / R(12.0);
-                O[2 * i + 1] = o1;
-                O[2 * i] = v;
-            }
-        }
-    }
-}
-
-// ===========================================================================
-// tracer_gradient_elements (src/oce_tracer_mod.F90:147-188): warp per element
-// ===========================================================================
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_trxy(DTopo tp, DGeom<R> g, DTracers<R> tr) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L1 = tp.L1;
-    for (int el = blockIdx.x * kWarpsPerBlock + warp; el < tp.T2; el += gridDim.x * kWarpsPerBlock) {
-        const int a = tp.t_n[3 * el], b = tp.t_n[3 * el + 1], c = tp.t_n[3 * el + 2];
-        const R *gs = g.gs + 6 * (size_t)el;
-        const R g0 = gs[0], g1 = gs[1], g2 = gs[2], g3 = gs[3], g4 = gs[4], g5 = gs[5];
-        const int nzmin = tp.t_ulev[el], nzmax = tp.t_nlev[el];
-        for (int t = 0; t < tr.ntr; t++) {
-            const R *T = tr.T + t * tr.sN;
-            R *out = tr.trxy + t * tr.sT;
-            for (int nz = nzmin + lane; nz <= nzmax - 1; nz += 32) {
-                R ta = T[ix1(nz, a, L1)], tb = T[ix1(nz, b, L1)], tc = T[ix1(nz, c, L1)];
-                R s = R(0);
-                s = s + g0 * ta;
-                s = s + g1 * tb;
-                s = s + g2 * tc;
-                R s2 = R(0);
-                s2 = s2 + g3 * ta;
-                s2 = s2 + g4 * tb;
-                s2 = s2 + g5 * tc;
-                out[2 * ix1(nz, el, L1)] = s;
-                out[2 * ix1(nz, el, L1) + 1] = s2;
-            }
-        }
-    }
-}
-
-// ===========================================================================
 // tracer_gradient_z (src/oce_tracer_mod.F90:192-232): warp per node, lanes over levels;
 // tr_z(nz) = (T(nz-1) - T(nz)) / (0.5 (hnode(nz-1) + hnode(nz))) inside the column, zero at
 // the first and last interface; the interfaces outside [nzmin, nzmax] are left as they are
@@ -162,112 +105,6 @@ __device__ __forceinline__ void node_mean_grad(const DTopo &tp, const DGeom<R> &
     }
     gx = tx / tvol;
     gy = ty / tvol;
-}
-
-// ===========================================================================
-// Edge fluxes: adv_tra_hor_upw1 (LO, values) and adv_tra_hor_muscl / _mfct /
-// _upw1 (HO, valuesAB) with fill_up_dn_grad inlined
-// (src/oce_adv_tra_hor.F90:64-834, src/oce_muscl_adv.F90:356-525).
-// Writes FLO (FCT only) and ADh = HO - LO (FCT) or HO (no limiter).
-// ===========================================================================
-template <typename R>
-__global__ void __launch_bounds__(kThreads)
-k_edge_flux(DTopo tp, DGeom<R> g, DForcing<R> f, DTracers<R> tr) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L1 = tp.L1;
-    const R RE = R(kREarth);
-    for (int e = blockIdx.x * kWarpsPerBlock + warp; e < tp.E2; e += gridDim.x * kWarpsPerBlock) {
-        const int n1 = tp.e_n1[e], n2 = tp.e_n2[e];
-        const int el1 = tp.e_t1[e], el2 = tp.e_t2[e];
-        const int nl1 = tp.t_nlev[el1] - 1, nu1 = tp.t_ulev[el1];
-        const R dX1 = g.ecd[4 * (size_t)e], dY1 = g.ecd[4 * (size_t)e + 1];
-        R a = RE * g.elem_cos[el1];
-        int nl2 = 0, nu2 = 0;
-        R dX2 = R(0), dY2 = R(0);
-        if (el2 >= 0) {
-            dX2 = g.ecd[4 * (size_t)e + 2];
-            dY2 = g.ecd[4 * (size_t)e + 3];
-            nl2 = tp.t_nlev[el2] - 1;
-            nu2 = tp.t_ulev[el2];
-            a = R(0.5) * (a + RE * g.elem_cos[el2]);
-        }
-        const int fnl12 = nl1 < nl2 ? nl1 : nl2;
-        const int fnu12 = nu1 > nu2 ? nu1 : nu2;
-        const int lo = tp.e_lo[e], hi = tp.e_hi[e];
-        const R ex = g.edxy[2 * (size_t)e], ey = g.edxy[2 * (size_t)e + 1];
-        const int up = tp.e_up[e], dn = tp.e_dn[e];
-        const bool inner = (up >= 0) && (dn >= 0);
-        int gzmin = 0, gzmax = 0;
-        if (inner) {
-            gzmin = max(tp.n_ulevmax[n1], tp.n_ulevmax[n2]);
-            gzmax = min(tp.n_nlevmin[n1], tp.n_nlevmin[n2]);
-        }
-        const int nbl1 = tp.n_nbl[n1], nbl2 = tp.n_nbl[n2];
-        for (int nz = lo + lane; nz <= hi; nz += 32) {
-            // segment rule of the reference's five loops (A..E)
-            int seg = 0;
-            if (nz >= nu1 && nz <= fnu12 - 1) seg = 1;
-            else if (nu2 > 0 && nz >= nu2 && nz <= fnu12 - 1) seg = 2;
-            else if (nz >= fnu12 && nz <= fnl12) seg = 3;
-            else if (nz >= fnl12 + 1 && nz <= nl1) seg = 1;
-            else if (nz >= fnl12 + 1 && nz <= nl2) seg = 2;
-            R vf = R(0);
-            if (seg & 1) {
-                const R u = f.uv[2 * ix1(nz, el1, L1)], v = f.uv[2 * ix1(nz, el1, L1) + 1];
-                vf = (-(v * dX1) + u * dY1) * g.helem[ix1(nz, el1, L1)];
-            }
-            if (seg & 2) {
-                const R u = f.uv[2 * ix1(nz, el2, L1)], v = f.uv[2 * ix1(nz, el2, L1) + 1];
-                const R v2 = (v * dX2 - u * dY2) * g.helem[ix1(nz, el2, L1)];
-                vf = (seg == 3) ? vf + v2 : v2;
-            }
-            const R avf = rabs(vf);
-            for (int t = 0; t < tr.ntr; t++) {
-                const DCfg c = tr.cfg[t];
-                const int fct = c.lim;
-                const R *T = tr.T + t * tr.sN;
-                const R *TA = tr.TAB + t * tr.sN;
-                R flo = R(0);
-                if (fct && seg)
-                    flo = -(R(0.5) * (T[ix1(nz, n1, L1)] * (vf + avf) + T[ix1(nz, n2, L1)] * (vf - avf))) - R(0);
-                const R fin = fct ? flo : R(0);
-                R ad = fin;
-                if (seg) {
-                    const R t1 = TA[ix1(nz, n1, L1)], t2 = TA[ix1(nz, n2, L1)];
-                    if (c.hor == 2) {
-                        ad = -(R(0.5) * (t1 * (vf + avf) + t2 * (vf - avf))) - fin;
-                    } else {
-                        const R *txy = tr.trxy + t * tr.sT;
-                        R g1, g2, g3, g4;
-                        if (inner && nz >= gzmin && nz <= gzmax - 1) {
-                            g1 = txy[2 * ix1(nz, up, L1)];
-                            g3 = txy[2 * ix1(nz, up, L1) + 1];
-                            g2 = txy[2 * ix1(nz, dn, L1)];
-                            g4 = txy[2 * ix1(nz, dn, L1) + 1];
-                        } else {
-                            node_mean_grad(tp, g, txy, n1, nz, g1, g3);
-                            node_mean_grad(tp, g, txy, n2, nz, g2, g4);
-                        }
-                        R Tm2, Tm1;
-                        if (c.hor == 0) {
-                            const R clo1 = (nbl1 - nz) >= 0 ? R(1) : R(0);
-                            const R clo2 = (nbl2 - nz) >= 0 ? R(1) : R(0);
-                            Tm2 = t2 - (R(2.0) * (t2 - t1) + ex * a * g2 + ey * RE * g4) / R(6.0) * clo2;
-                            Tm1 = t1 + (R(2.0) * (t2 - t1) + ex * a * g1 + ey * RE * g3) / R(6.0) * clo1;
-                        } else {
-                            Tm2 = t2 - (R(2.0) * (t2 - t1) + ex * a * g2 + ey * RE * g4) / R(6.0);
-                            Tm1 = t1 + (R(2.0) * (t2 - t1) + ex * a * g1 + ey * RE * g3) / R(6.0);
-                        }
-                        const R no = R(c.ph);
-                        const R cHO = (vf + avf) * Tm1 + (vf - avf) * Tm2;
-                        ad = -(R(0.5) * (R(1.0) - no) * cHO) - vf * no * R(0.5) * (Tm1 + Tm2) - fin;
-                    }
-                }
-                if (fct) tr.FLO[t * tr.sE + ix1(nz, e, L1)] = flo;
-                tr.ADh[t * tr.sE + ix1(nz, e, L1)] = ad;
-            }
-        }
-    }
 }
 
 // ===========================================================================
@@ -1077,25 +914,8 @@ static inline int grid_for(int nent, int per_block) {
 }
 
 template <typename R>
-void Launch<R>::ab(const DTopo &tp, DTracers<R> &tr, int ab, cudaStream_t s) {
-    const size_t n = (size_t)tp.L1 * tp.N2;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 152 * 16) blocks = 152 * 16;
-    k_ab<R><<<blocks, 256, 0, s>>>(tr, n, ab);
-}
-template <typename R>
-void Launch<R>::trxy(const DTopo &tp, const DGeom<R> &g, DTracers<R> &tr, cudaStream_t s) {
-    k_trxy<R><<<grid_for(tp.T2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, tr);
-}
-template <typename R>
 void Launch<R>::trz(const DTopo &tp, const DGeom<R> &g, const R *T, R *trz, cudaStream_t s) {
     k_trz<R><<<grid_for(tp.N2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, T, trz);
-}
-template <typename R>
-void Launch<R>::edge_flux(const DTopo &tp, const DGeom<R> &g, const DForcing<R> &f, DTracers<R> &tr, int fct,
-                          cudaStream_t s) {
-    (void)fct;
-    k_edge_flux<R><<<grid_for(tp.E2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, f, tr);
 }
 template <typename R>
 void Launch<R>::node_lo(const DTopo &tp, const DGeom<R> &g, const DForcing<R> &f, DTracers<R> &tr, double dt, int fct,

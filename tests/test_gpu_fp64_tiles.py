@@ -1,0 +1,48 @@
+"""The FP64 form's tiled kernels at the sizes where they can go wrong: entity counts that leave a
+partial tile, tiles of 4 and of 8, columns around a warp's 32 levels, and the general expressions
+behind the short ones (adv_ph /= 0, adv_pv /= 1); bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from fesom2_gb300 import gpu as G
+from fesom2_gb300 import mesh as M
+from oracle import oracle as O
+from tests.conftest import perturbed_old
+
+pytestmark = pytest.mark.gpu
+
+# nx, ny, layers, partial cells, tracers: (horizontal, vertical, limiter, adv_ph, adv_pv), ab
+CASES = [
+    (5, 7, 4, False, [("MUSCL", "QR4C", "FCT", 0.0, 1.0)], 2),
+    (5, 7, 5, False, [("MFCT", "QR4C", "FCT", 0.4, 0.3), ("UPW1", "CDIFF", "FCT", 0.0, 1.0)], 3),
+    (7, 11, 31, True, [("MUSCL", "QR4C", "FCT", 0.0, 1.0)] * 2, 2),
+    (9, 13, 32, True, [("MFCT", "CDIFF", "NON", 0.0, 1.0), ("MUSCL", "UPW1", "FCT", 1.0, 0.0)], 2),
+    (9, 13, 33, True, [("MUSCL", "QR4C", "FCT", 0.25, 0.5)] * 3, 3),
+    (11, 17, 65, True, [("MUSCL", "QR4C", "FCT", 0.0, 1.0), ("MFCT", "PPM", "FCT", 0.0, 1.0)], 2),
+    (101, 97, 21, True, [("MUSCL", "QR4C", "FCT", 0.0, 1.0)] * 2, 2),
+]
+
+
+@pytest.mark.parametrize("nx,ny,layers,partial,schemes,ab", CASES)
+def test_step_bitwise(nx, ny, layers, partial, schemes, ab):
+    mesh = M.channel_mesh(nx, ny, 5000.0, M.stretched_zbar(layers, 10.0, 200.0), seamounts=2 if partial else 0, seed=5,
+                          partial_cells=partial)
+    f = O.ensure_f64(M.make_forcing(mesh, "channel", seed=3, dt=600.0))
+    n = len(schemes)
+    tr = M.make_tracers(mesh, "channel", ntr=n, seed=4)
+    om = O.OracleMesh(mesh)
+    ctx = G.Context(mesh, G.PREC_FP64, max_tracers=n)
+    rng = np.random.default_rng(2)
+    To = [np.array(t, copy=True) for t in tr]
+    Oo = [np.ascontiguousarray(np.stack([perturbed_old(t, rng) for _ in range(ab - 1)], axis=-1)) for t in To]
+    Tg, Og = [t.copy() for t in To], [o.copy() for o in Oo]
+    gcfg = [G.tra_cfg(h, v, l, ph, pv, ab, True, k + 1) for k, (h, v, l, ph, pv) in enumerate(schemes)]
+    ocfg = [O.cfg_struct(h, v, l, ph, pv, ab) for h, v, l, ph, pv in schemes]
+    for step in range(2):
+        for k in range(n):
+            om.tracer_step(f, ocfg[k], To[k], np.zeros_like(To[k]), Oo[k])
+        ctx.tracer_step(f, gcfg, Tg, Og)
+        for k in range(n):
+            assert np.array_equal(Tg[k], To[k]), f"step {step} tracer {k}"
+            assert np.array_equal(Og[k], Oo[k]), f"step {step} tracer {k}: previous levels"
+    assert ctx.status() == 0
