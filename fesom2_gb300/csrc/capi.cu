@@ -827,8 +827,7 @@ int enqueue_step(fesom_gpu_ctx *ctx, double dt, StageTimer *tm = nullptr) {
         if (any_ex) STAGE(7, Launch<R>::vexpl(ctx->tp, g, f, tr, dt, tr.VX, 0, 0, ctx->stream));
         if (redi) STAGE(7, Launch<R>::redi_v(ctx->tp, g, tr, dt, 0, ctx->stream));
         if (any_fct) {
-            STAGE(4, Launch<R>::bounds(ctx->tp, g, tr, ctx->stream));
-            STAGE(5, Launch<R>::rpm(ctx->tp, g, tr, dt, ctx->stream));
+            STAGE(4, Launch<R>::bounds_rpm(ctx->tp, g, tr, dt, ctx->stream));
         }
         STAGE(6, Launch<R>::update(ctx->tp, g, tr, dt, any_fct, 1, ctx->stream));
         if (any_vd) {
@@ -969,7 +968,7 @@ int launches_per_step(fesom_gpu_ctx *ctx) {
         }
         bool any_ex = false;
         for (int t = t0; t < t0 + nt; t++) any_ex |= ctx->cfgs[t].i_vert_diff == 0;
-        n += 4 + ((any_ho || ctx->Ki) ? 1 : 0) + (any_fct ? 2 : 0) + (any_vd ? 1 : 0) + (ctx->Ki ? 1 : 0) +
+        n += 4 + ((any_ho || ctx->Ki) ? 1 : 0) + (any_fct ? 1 : 0) + (any_vd ? 1 : 0) + (ctx->Ki ? 1 : 0) +
              (any_ex ? 1 : 0) + ((ctx->wsplit && any_fct) ? 1 : 0) + (redi_on(ctx) ? 1 : 0);
     }
     return n;
@@ -1094,6 +1093,7 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
     int rc;
     const HostTopo &h = ctx->ht;
     DTopo &tp = ctx->tp;
+    tp.ring_ok = h.ring_ok;
     tp.N2 = ctx->N2; tp.E2 = ctx->E2; tp.T2 = ctx->T2; tp.nl = ctx->nl; tp.L1 = ctx->L1;
     if ((rc = upload_int(ctx, &tp.e_n1, h.e_n1)) || (rc = upload_int(ctx, &tp.e_n2, h.e_n2)) ||
         (rc = upload_int(ctx, &tp.e_t1, h.e_t1)) || (rc = upload_int(ctx, &tp.e_t2, h.e_t2)) ||
@@ -1120,6 +1120,15 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
     if (precision == FESOM_PREC_FP32) rc = init_geom<float>(ctx, mesh, ctx->g32);
     else rc = init_geom<double>(ctx, mesh, ctx->g64);
     if (rc) return rc;
+    if (precision == FESOM_PREC_FP64) {
+        const size_t n = (size_t)ctx->nl * ctx->N2, m = (size_t)ctx->L1 * ctx->N2;
+        if ((rc = dalloc(ctx, (void **)&ctx->g64.rav, n * sizeof(double2))) ||
+            (rc = dalloc(ctx, (void **)&ctx->g64.rhn, m * sizeof(double2))))
+            return rc;
+        recip_table(ctx->g64.areasvol, (double2 *)ctx->g64.rav, n, ctx->stream);
+        recip_table(ctx->g64.hnode_new, (double2 *)ctx->g64.rhn, m, ctx->stream);
+        CK(cudaGetLastError());
+    }
     if (precision == FESOM_PREC_FP32 && (rc = init_muscl_weights(ctx, mesh))) return rc;
     {
         std::vector<double> y(ctx->N2);
@@ -1228,6 +1237,8 @@ int fesom_gpu_update_thickness(fesom_gpu_ctx *ctx, const double *hnode, const do
             (rc = put(ctx, (void *)g.helem, helem, L1 * T2)) || (rc = put(ctx, (void *)g.Z3, Z_3d_n, L1 * N2)) ||
             (rc = put(ctx, (void *)g.zbar3, zbar_3d_n, nl * N2)))
             return rc;
+        if (hnode_new) recip_table(g.hnode_new, (double2 *)g.rhn, L1 * N2, ctx->stream);
+        CK(cudaGetLastError());
     }
     return wait_stream(ctx, -1);
 }
@@ -1299,8 +1310,7 @@ int fesom_gpu_adv_tra(fesom_gpu_ctx *ctx, double dt, const double *vel, const do
     Launch<double>::node_lo(ctx->tp, ctx->g64, f, tr, dt, fct, ctx->stream);
     if (fct && ctx->wsplit) Launch<double>::lo_impl(ctx->tp, ctx->g64, f, tr, dt, ctx->scratch, ctx->stream);
     if (fct) {
-        Launch<double>::bounds(ctx->tp, ctx->g64, tr, ctx->stream);
-        Launch<double>::rpm(ctx->tp, ctx->g64, tr, dt, ctx->stream);
+        Launch<double>::bounds_rpm(ctx->tp, ctx->g64, tr, dt, ctx->stream);
     }
     Launch<double>::update(ctx->tp, ctx->g64, tr, dt, fct, 0, ctx->stream);
     CK(cudaGetLastError());

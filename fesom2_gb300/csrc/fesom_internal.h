@@ -33,6 +33,8 @@ struct DTopo {
     const int *nie_ptr, *nie_idx;  // node -> element, ascending element order
     int n_wide;                    // nodes of more than 8 edges (FP32 form: their own launch)
     const int *wide_nodes;
+    // every element lies on exactly three edges and in the element lists of exactly its three nodes
+    int ring_ok;
 };
 
 template <typename R>
@@ -44,6 +46,9 @@ struct DGeom {
     const R *helem;                      // nl-1 per element
     const R *Z3, *zbar3;                 // nl-1 / nl per node
     const R *zbar_n_bot;                 // per node
+    // FP64 form: 1/areasvol and 1/hnode_new as sums of two FP64 numbers (recip64), for the
+    // divisions of every tracer and step by them
+    const double2 *rav, *rhn;
 };
 
 template <typename R>
@@ -73,7 +78,7 @@ struct DTracers {
     R *trxy;
     R *FLO, *ADh;        // low-order / antidiffusive edge fluxes
     R *LO, *ADv;         // low-order solution / antidiffusive vertical flux
-    R *bmax, *bmin;      // FCT bound increments, then R+ / R- in place
+    R *bmax, *bmin;      // R+ / R-
     R *dttf_h, *dttf_v;  // advective increments (drop-in outputs)
     const DCfg *cfg;
     unsigned *status;
@@ -247,6 +252,9 @@ void bm32_update(const Inst32 *, const MultiIdx &, bool wide, cudaStream_t);
 void bm32_hdiff(const Inst32 *, const MultiIdx &edges, cudaStream_t);
 void bm32_diff(const Inst32 *, const MultiIdx &nodes, bool wide, cudaStream_t);
 
+// reciprocals of a divisor array for DGeom::rav / rhn (kernels_fp64.cu)
+void recip_table(const double *y, double2 *out, size_t n, cudaStream_t);
+
 // tail of the tracer loop (kernels_tail.cu): one tracer's decay, relaxation and clamp
 struct TailArgs {
     int decay;            // multiply the whole field by decay_f
@@ -270,8 +278,8 @@ struct Launch {
     static void edge_flux(const DTopo &, const DGeom<R> &, const DForcing<R> &, DTracers<R> &, int fct, cudaStream_t);
     static void node_lo(const DTopo &, const DGeom<R> &, const DForcing<R> &, DTracers<R> &, double dt, int fct,
                         cudaStream_t);
-    static void bounds(const DTopo &, const DGeom<R> &, DTracers<R> &, cudaStream_t);
-    static void rpm(const DTopo &, const DGeom<R> &, DTracers<R> &, double dt, cudaStream_t);
+    // FCT bounds and the ratios R+ / R- (into bmax / bmin)
+    static void bounds_rpm(const DTopo &, const DGeom<R> &, DTracers<R> &, double dt, cudaStream_t);
     // mode 0: write dttf_h/dttf_v only; mode 1: del_ttf sum + T* update into T
     static void update(const DTopo &, const DGeom<R> &, DTracers<R> &, double dt, int fct, int mode, cudaStream_t);
     static void vdiff(const DTopo &, const DGeom<R> &, const DForcing<R> &, DTracers<R> &, double dt,

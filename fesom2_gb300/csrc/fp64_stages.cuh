@@ -285,6 +285,338 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
 }
 
 // ===========================================================================
+// Node columns, stage 1: LO solution (edge gather of the upwind fluxes,
+// adv_tra_ver_upw1 with w_e, src/oce_adv_tra_driver.F90:122-250) and the
+// vertical high-order flux minus the LO flux (adv_tra_ver_qr4c / _upw1 / _cdiff / _ppm with w,
+// src/oce_adv_tra_ver.F90:244-695).  Without a limiter only the HO vertical
+// flux (with w_e) is formed.
+//
+// Two passes over a tile of nodes: the upwind flux and the gradient quotient
+// (T(nz-1) - T(nz)) / (Z(nz-1) - Z(nz)) of every interface once into shared memory, then the
+// layers, which read both neighbours' (the quotient was formed three times, the flux twice).
+// Every centred or surface flux is -(0.5 (A + B) W area) - fin with A, B chosen per interface;
+// the factor 0.5 is exact, so it is applied in the last, fused operation.
+// ===========================================================================
+// the upwind flux of adv_tra_ver_upw1 through interface nz above layer nz (top: the surface)
+__device__ __forceinline__ double ver_upw64(double T0, double Tu, double W, double ar, bool top) {
+    if (top) return -(W * T0 * ar);
+    const bool neg = neg64(W);
+    const double x = neg ? Tu : T0, y = neg ? T0 : Tu;
+    if (nonfinite64(y) || nonfinite64(W)) {
+        const double aW = fabs(W);
+        return -(0.5 * (T0 * (W + aW) + Tu * (W - aW)) * ar);
+    }
+    return -(x * W * ar);
+}
+
+static __global__ void __launch_bounds__(kTileThreads)
+k_node_lo(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, double dt, int tile) {
+    extern __shared__ __align__(16) double sm64[];
+    __shared__ Tile S;
+    const int L1 = tp.L1, nl = tp.nl, n0 = blockIdx.x * tile;
+    double *fl = sm64, *qc = sm64 + (size_t)tile * L1;
+    if (threadIdx.x < 32) {
+        const int n = n0 + threadIdx.x;
+        const bool ok = threadIdx.x < tile && n < tp.N2;
+        S.fill(threadIdx.x, ok ? tp.n_ulev[n] : 1, ok ? tp.n_nlev[n] - tp.n_ulev[n] : 0);
+    }
+    for (int t = 0; t < tr.ntr; t++) {
+        const DCfg c = tr.cfg[t];
+        const bool fct = c.lim != 0;
+        const double *T = tr.T + t * tr.sN, *TA = tr.TAB + t * tr.sN, *FLO = tr.FLO + t * tr.sE;
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+            const int j = S.find(i), n = n0 + j, nz = S.top[j] + i - S.pre[j];
+            const bool top = i == S.pre[j];
+            const size_t k = ix1(nz, n, L1), kv = ixn(nz, n, nl);
+            if (fct) fl[i] = ver_upw64(T[k], top ? 0.0 : T[k - 1], f.we[kv], g.area[kv], top);
+            if (c.ver == 0 && !top) qc[i] = (TA[k - 1] - TA[k]) / (g.Z3[k - 1] - g.Z3[k]);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+            const int j = S.find(i), n = n0 + j, nz = S.top[j] + i - S.pre[j];
+            const int nzmin = S.top[j], nzmax = nzmin + S.pre[j + 1] - S.pre[j];
+            const bool top = nz == nzmin, bot = nz == nzmax - 1;
+            const size_t k = ix1(nz, n, L1), kv = ixn(nz, n, nl);
+            double fin = 0.0;
+            if (fct) {
+                fin = fl[i];
+                const double f1 = bot ? 0.0 : fl[i + 1];
+                double acc = 0.0;
+                for (int q = tp.ne_ptr[n]; q < tp.ne_ptr[n + 1]; q++) {
+                    const int code = tp.ne_idx[q], e = code >= 0 ? code : ~code;
+                    if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
+                    const double x = FLO[ix1(nz, e, L1)];
+                    acc = acc + (code >= 0 ? x : -x);
+                }
+                const double h = T[k] * g.hnode[k];
+                tr.LO[t * tr.sN + k] = sdiv64(h + sdiv64((acc + (fin - f1)) * dt, g.areasvol[kv], g.rav[kv]),
+                                              g.hnode_new[k], g.rhn[k]);
+                // with the split vertical velocity the LO part of the antidiffusive flux is the
+                // upwind flux of the full w (oce_adv_tra_driver.F90:323-334)
+                if (f.wsplit) fin = ver_upw64(T[k], top ? 0.0 : T[k - 1], f.w[kv], g.area[kv], top);
+            }
+            const double *pw = fct ? f.w : f.we;
+            double v;
+            if (c.ver == 3) {
+                v = ver_ppm_flux(TA, pw, g.area, g.hnode_new, g.hnode, dt, nz, n, nzmin, nzmax, L1, nl, fin);
+            } else {
+                const double W = pw[kv], ar = g.area[kv], t0 = TA[k];
+                if (c.ver == 1) {
+                    v = ver_upw64(t0, top ? 0.0 : TA[k - 1], W, ar, top) - fin;
+                } else {
+                    double A = top ? t0 : TA[k - 1], B = t0;
+                    const bool inner = c.ver == 0 && nz >= nzmin + 2 && !bot;
+                    if (inner) {
+                        const double zb = g.zbar3[kv], q0 = qc[i];
+                        // 2 qc is exact: one rounding in the fused sum, as in the reference's
+                        A = A + div_3x2k<3>(__fma_rn(2.0, q0, qc[i - 1]) * (zb - g.Z3[k - 1]));
+                        B = B + div_3x2k<3>(__fma_rn(2.0, q0, qc[i + 1]) * (zb - g.Z3[k]));
+                    }
+                    if (inner && (c.pv != 1.0 || nonfinite64(W) || nonfinite64(A) || nonfinite64(B))) {
+                        const double no = c.pv, aW = fabs(W);
+                        const double Tmean = (W + aW) * B + (W - aW) * A;
+                        v = (-(0.5 * (1.0 - no) * Tmean) - no * (0.5 * (B + A)) * W) * ar - fin;
+                    } else {
+                        const double P = (A + B) * W * ar;
+                        v = __fma_rn(-0.5, P, -fin);
+                        // a two-layer column writes its middle interface twice (nzmin+1, nzmax-1)
+                        if (c.ver == 0 && bot && nz == nzmin + 1) v = -(0.5 * P) - v;
+                    }
+                }
+            }
+            tr.ADv[t * tr.sNI + kv] = v;
+            if (bot) tr.ADv[t * tr.sNI + kv + 1] = 0.0;
+        }
+    }
+}
+
+// ===========================================================================
+// FCT bounds a1-a3 and b1 + b2: the bounds of a node-layer over the node's elements and the
+// adjacent layers, the sums of positive / negative antidiffusive fluxes (vertical, then edges in
+// ascending order) and the ratios R+ / R- (src/oce_adv_tra_fct.F90:124-405), in one kernel.
+//
+// The maximum over the node's wet elements is the maximum over the node and the neighbours whose
+// edge is wet (each wet element is the wet side of two of the node's edges), plus -bignumber
+// where an element of the node is dry: 7 values instead of 18.  Maxima run on integer keys in
+// shared memory; only the sums and quotients are FP64 instructions (about 45 per node-layer and
+// tracer, 165 in two kernels before).  A mesh whose edges do not cover its elements' sides, or a
+// value that is not a number, takes the elements themselves with the FP64 comparisons.
+// ===========================================================================
+// max / min over the elements of node n at layer nz in the order of the reference's loop
+static __device__ __noinline__ void bounds_elements(const DTopo &tp, const double *T, const double *LO, int n, int nz,
+                                                    double &mx, double &mn) {
+    const int L1 = tp.L1, k0 = tp.nie_ptr[n], k1 = tp.nie_ptr[n + 1];
+    mx = mn = 0.0;
+    for (int k = k0; k < k1; k++) {
+        const int el = tp.nie_idx[k];
+        double amx = -kBigNumber, amn = kBigNumber;
+        if (nz >= tp.t_ulev[el] && nz <= tp.t_nlev[el] - 1) {
+            const size_t a = ix1(nz, tp.t_n[3 * el], L1), b = ix1(nz, tp.t_n[3 * el + 1], L1),
+                         c = ix1(nz, tp.t_n[3 * el + 2], L1);
+            amx = rmax(rmax(rmax(LO[a], T[a]), rmax(LO[b], T[b])), rmax(LO[c], T[c]));
+            amn = rmin(rmin(rmin(LO[a], T[a]), rmin(LO[b], T[b])), rmin(LO[c], T[c]));
+        }
+        mx = k == k0 ? amx : rmax(mx, amx);
+        mn = k == k0 ? amn : rmin(mn, amn);
+    }
+}
+
+// rmin(1, b / fl); b and fl of one sign, |b| >= |fl|: the quotient rounds to 1 or more
+__device__ __forceinline__ double ratio1(double b, double fl) {
+    const unsigned long long ub = (unsigned long long)__double_as_longlong(b),
+                             uf = (unsigned long long)__double_as_longlong(fl);
+    if ((long long)(ub ^ uf) >= 0 && (ub << 1) >= (uf << 1) && !nonfinite64(b) && !zero64(fl)) return 1.0;
+    return rmin(1.0, b / fl);
+}
+
+static __global__ void __launch_bounds__(kTileThreads)
+k_bounds_rpm(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int tile) {
+    extern __shared__ __align__(16) long long smk[];
+    __shared__ Tile S;
+    __shared__ int wlo[kTileMax], whi[kTileMax];  // the levels at which every element of the node is wet
+    const int L1 = tp.L1, nl = tp.nl, n0 = blockIdx.x * tile;
+    long long *kmx = smk, *kmn = smk + (size_t)tile * L1;
+    if (threadIdx.x < 32) {
+        const int j = threadIdx.x, n = n0 + j;
+        const bool ok = j < tile && n < tp.N2;
+        if (ok) {
+            int lo = 1, hi = nl;
+            for (int k = tp.nie_ptr[n]; k < tp.nie_ptr[n + 1]; k++) {
+                const int el = tp.nie_idx[k];
+                lo = max(lo, tp.t_ulev[el]);
+                hi = min(hi, tp.t_nlev[el] - 1);
+            }
+            wlo[j] = lo;
+            whi[j] = hi;
+        }
+        S.fill(j, ok ? tp.n_ulev[n] : 1, ok ? tp.n_nlev[n] - tp.n_ulev[n] : 0);
+    }
+    for (int t = 0; t < tr.ntr; t++) {
+        if (!tr.cfg[t].lim) continue;
+        const double *T = tr.T + t * tr.sN, *LO = tr.LO + t * tr.sN;
+        const double *ADv = tr.ADv + t * tr.sNI, *ADh = tr.ADh + t * tr.sE;
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+            const int j = S.find(i), n = n0 + j, nz = S.top[j] + i - S.pre[j];
+            const bool dry = nz < wlo[j] || nz > whi[j];
+            const size_t k = ix1(nz, n, L1);
+            const double lo0 = LO[k], t0 = T[k];
+            bool bad = nan64(lo0) || nan64(t0), wet = false;
+            const long long a = key64(lo0), b = key64(t0);
+            long long mx = max(a, b), mn = min(a, b);
+            for (int q = tp.ne_ptr[n]; q < tp.ne_ptr[n + 1]; q++) {
+                const int code = tp.ne_idx[q], e = code >= 0 ? code : ~code;
+                if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
+                wet = true;
+                const size_t m = ix1(nz, code >= 0 ? tp.e_n2[e] : tp.e_n1[e], L1);
+                const double lm = LO[m], tm = T[m];
+                bad = bad || nan64(lm) || nan64(tm);
+                const long long ka = key64(lm), kb = key64(tm);
+                mx = max(mx, max(ka, kb));
+                mn = min(mn, min(ka, kb));
+            }
+            if (dry) {
+                const long long big = __double_as_longlong(kBigNumber), nbig = key64(-kBigNumber);
+                mx = wet ? max(mx, nbig) : nbig;
+                mn = wet ? min(mn, big) : big;
+            }
+            if (bad || !tp.ring_ok) {
+                double x, y;
+                bounds_elements(tp, T, LO, n, nz, x, y);
+                mx = key64(x);
+                mn = key64(y);
+            }
+            kmx[i] = mx;
+            kmn[i] = mn;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+            const int j = S.find(i), n = n0 + j, nz = S.top[j] + i - S.pre[j];
+            const bool end = i == S.pre[j] || i == S.pre[j + 1] - 1;
+            const size_t k = ix1(nz, n, L1), kv = ixn(nz, n, nl);
+            long long mx = kmx[i], mn = kmn[i];
+            if (!end) {
+                const long long xu = kmx[i - 1], xd = kmx[i + 1], yu = kmn[i - 1], yd = kmn[i + 1];
+                if (nan64(unkey64(xu)) || nan64(unkey64(mx)) || nan64(unkey64(xd)) || nan64(unkey64(yu)) ||
+                    nan64(unkey64(mn)) || nan64(unkey64(yd))) {
+                    mx = key64(rmax(rmax(unkey64(xu), unkey64(mx)), unkey64(xd)));
+                    mn = key64(rmin(rmin(unkey64(yu), unkey64(mn)), unkey64(yd)));
+                } else {
+                    mx = max(max(xu, mx), xd);
+                    mn = min(min(yu, mn), yd);
+                }
+            }
+            const double lo = LO[k], bx = unkey64(mx) - lo, bn = unkey64(mn) - lo;
+            // sums of the fluxes into (P) and out of (M) the layer; a flux adds to one of them
+            double P = 0.0, M = 0.0;
+            bool bad = false;
+            auto add = [&](double x) {
+                bad = bad || nan64(x);
+                const bool neg = neg64(x);
+                const double s = (neg ? M : P) + x;
+                P = neg ? P : s;
+                M = neg ? s : M;
+            };
+            add(ADv[kv]);
+            add(-ADv[kv + 1]);
+            for (int q = tp.ne_ptr[n]; q < tp.ne_ptr[n + 1]; q++) {
+                const int code = tp.ne_idx[q], e = code >= 0 ? code : ~code;
+                if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
+                const double x = ADh[ix1(nz, e, L1)];
+                add(code >= 0 ? x : -x);
+            }
+            if (bad) P = M = __longlong_as_double(0x7ff8000000000000ll);  // both sums take a NaN flux
+            const double av = g.areasvol[kv], hn = g.hnode_new[k];
+            const double2 ra = g.rav[kv], rh = g.rhn[k];
+            const double fp = sdiv64(sdiv64(P * dt, av, ra), hn, rh) + kFluxEps;
+            const double fm = sdiv64(sdiv64(M * dt, av, ra), hn, rh) - kFluxEps;
+            tr.bmax[t * tr.sN + k] = ratio1(bx, fp);
+            tr.bmin[t * tr.sN + k] = ratio1(bn, fm);
+        }
+    }
+}
+
+// ===========================================================================
+// FCT b3 limiting + oce_tra_adv_flux2dtracer (src/oce_adv_tra_fct.F90:425-500,
+// src/oce_adv_tra_driver.F90:494-646) + (mode 1) the del_ttf sum and the T*
+// update of diff_tracers_ale (src/oce_ale_tracer.F90:319-321, 743-754).
+// The limited edge flux is formed at each end node from R+/R- of both ends; a limited interface
+// flux once, in a first pass over the tile.  About 60 FP64 instructions per node-layer and
+// tracer (118 before: six of its divisions are by areasvol, at 4 instead of 8 each).
+// ===========================================================================
+static __global__ void __launch_bounds__(kTileThreads)
+k_update(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int mode, int tile) {
+    extern __shared__ __align__(16) double sm64[];
+    __shared__ Tile S;
+    const int L1 = tp.L1, nl = tp.nl, n0 = blockIdx.x * tile;
+    if (threadIdx.x < 32) {
+        const int n = n0 + threadIdx.x;
+        const bool ok = threadIdx.x < tile && n < tp.N2;
+        S.fill(threadIdx.x, ok ? tp.n_ulev[n] : 1, ok ? tp.n_nlev[n] - tp.n_ulev[n] : 0);
+    }
+    for (int t = 0; t < tr.ntr; t++) {
+        const bool fct = tr.cfg[t].lim != 0;
+        double *T = tr.T + t * tr.sN;
+        const double *ADv = tr.ADv + t * tr.sNI, *ADh = tr.ADh + t * tr.sE;
+        const double *Rp = tr.bmax + t * tr.sN, *Rm = tr.bmin + t * tr.sN;
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+            const int j = S.find(i), n = n0 + j, nz = S.top[j] + i - S.pre[j];
+            double x = ADv[ixn(nz, n, nl)];
+            if (fct) {
+                const size_t k = ix1(nz, n, L1);
+                const bool in = !neg64(x) || zero64(x);  // x >= 0 (a NaN stays one under any factor)
+                double ae = in ? Rp[k] : Rm[k];
+                if (i != S.pre[j]) ae = min64(in ? Rm[k - 1] : Rp[k - 1], ae);
+                x = ae * x;
+            }
+            sm64[i] = x;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+            const int j = S.find(i), n = n0 + j, nz = S.top[j] + i - S.pre[j];
+            const size_t k = ix1(nz, n, L1), kv = ixn(nz, n, nl);
+            const double av = g.areasvol[kv], h = g.hnode[k], hn = g.hnode_new[k], t0 = T[k];
+            const double2 ra = g.rav[kv];
+            const double f0 = sm64[i], f1 = i + 1 < S.pre[j + 1] ? sm64[i + 1] : ADv[kv + 1];
+            double dv = sdiv64((f0 - f1) * dt, av, ra);
+            if (fct) dv = (-(t0 * h) + tr.LO[t * tr.sN + k] * hn) + dv;
+            double dh = 0.0;
+            for (int q = tp.ne_ptr[n]; q < tp.ne_ptr[n + 1]; q++) {
+                const int code = tp.ne_idx[q], e = code >= 0 ? code : ~code;
+                if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
+                double x = ADh[ix1(nz, e, L1)];
+                if (fct) {
+                    const bool in = !neg64(x) || zero64(x), own = code >= 0;
+                    const size_t m = ix1(nz, own ? tp.e_n2[e] : tp.e_n1[e], L1);
+                    // x >= 0: R+ of edges(1,e), R- of edges(2,e); x < 0 the other way round
+                    const double rn = in == own ? Rp[k] : Rm[k], rm = in == own ? Rm[m] : Rp[m];
+                    x = min64(own ? rn : rm, own ? rm : rn) * x;
+                }
+                x = sdiv64(x * dt, av, ra);
+                dh = dh + (code >= 0 ? x : -x);
+            }
+            if (mode == 0) {
+                tr.dttf_h[t * tr.sN + k] = dh;
+                tr.dttf_v[t * tr.sN + k] = dv;
+            } else {
+                double del = dh + dv;
+                // diff_tracers_ale: horizontal, then explicit vertical diffusion
+                if (tr.HD) del = hdiff_add(tp, tr.HD + t * tr.sE, del, n, nz, L1, dt, av);
+                if (tr.VX && !tr.cfg[t].ivd) del = del + tr.VX[t * tr.sN + k];
+                // Redi: diff_ver_part_redi_expl (:623)
+                if (tr.RV) del = del + tr.RV[t * tr.sN + k];
+                del = del + t0 * (h - hn);
+                const double tn = t0 + sdiv64(del, hn, g.rhn[k]);
+                T[k] = tn;
+                if (nonfinite64(tn)) atomicOr(tr.status, 1u);
+            }
+        }
+    }
+}
+
+// ===========================================================================
 // launches
 // ===========================================================================
 template <>
@@ -302,6 +634,35 @@ void Launch<double>::edge_flux(const DTopo &tp, const DGeom<double> &g, const DF
                                int, cudaStream_t s) {
     const int t = tile_size(tp.E2, 0);
     k_edge_flux<<<(tp.E2 + t - 1) / t, kTileThreads, 0, s>>>(tp, g, f, tr, t);
+}
+template <>
+void Launch<double>::node_lo(const DTopo &tp, const DGeom<double> &g, const DForcing<double> &f, DTracers<double> &tr,
+                             double dt, int, cudaStream_t s) {
+    const size_t b = 2 * sizeof(double) * tp.L1;
+    const int t = tile_size(tp.N2, b);
+    k_node_lo<<<(tp.N2 + t - 1) / t, kTileThreads, t * b, s>>>(tp, g, f, tr, dt, t);
+}
+template <>
+void Launch<double>::bounds_rpm(const DTopo &tp, const DGeom<double> &g, DTracers<double> &tr, double dt,
+                                cudaStream_t s) {
+    const size_t b = 2 * sizeof(double) * tp.L1;
+    const int t = tile_size(tp.N2, b);
+    k_bounds_rpm<<<(tp.N2 + t - 1) / t, kTileThreads, t * b, s>>>(tp, g, tr, dt, t);
+}
+template <>
+void Launch<double>::update(const DTopo &tp, const DGeom<double> &g, DTracers<double> &tr, double dt, int, int mode,
+                            cudaStream_t s) {
+    const size_t b = sizeof(double) * tp.L1;
+    const int t = tile_size(tp.N2, b);
+    k_update<<<(tp.N2 + t - 1) / t, kTileThreads, t * b, s>>>(tp, g, tr, dt, mode, t);
+}
+// reciprocals of a divisor array (DGeom::rav, rhn)
+static __global__ void k_recip(const double *y, double2 *out, size_t n) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        out[i] = recip64(y[i]);
+}
+void recip_table(const double *y, double2 *out, size_t n, cudaStream_t s) {
+    k_recip<<<(int)std::min<size_t>((n + 255) / 256, 152 * 16), 256, 0, s>>>(y, out, n);
 }
 
 }  // namespace fesom

@@ -113,6 +113,34 @@ bool prepare_mesh(const fesom_mesh_desc &d, HostTopo &h, std::string &err) {
         h.ne_idx[pos[h.e_n1[e]]++] = e;
         h.ne_idx[pos[h.e_n2[e]]++] = ~e;
     }
+    // whether a node's neighbours over its edges are the nodes of its elements: every element on
+    // three edges that join different pairs of its nodes, and listed once by each of its nodes
+    {
+        std::vector<unsigned char> sides(T2, 0), lists(T2, 0);
+        h.ring_ok = 1;
+        for (int e = 0; e < E2; e++) {
+            for (int t : {h.e_t1[e], h.e_t2[e]}) {
+                if (t < 0) continue;
+                int m = 0;
+                for (int k = 0; k < 3; k++) {
+                    const int v = h.t_n[3 * (size_t)t + k];
+                    if (v == h.e_n1[e] || v == h.e_n2[e]) m |= 1 << k;
+                }
+                const unsigned char bit = m == 3 ? 1 : m == 5 ? 2 : m == 6 ? 4 : 0;
+                if (!bit || (sides[t] & bit)) h.ring_ok = 0;
+                sides[t] |= bit;
+            }
+        }
+        for (int n = 0; n < N2; n++)
+            for (int k = h.nie_ptr[n]; k < h.nie_ptr[n + 1]; k++) {
+                const int *tn = &h.t_n[3 * (size_t)h.nie_idx[k]];
+                const unsigned char bit = tn[0] == n ? 1 : tn[1] == n ? 2 : 4;
+                if (lists[h.nie_idx[k]] & bit) h.ring_ok = 0;
+                lists[h.nie_idx[k]] |= bit;
+            }
+        for (int t = 0; t < T2; t++)
+            if (sides[t] != 7 || lists[t] != 7) h.ring_ok = 0;
+    }
     // MUSCL init arrays
     h.n_nbl.resize(N2);
     if (d.nboundary_lay) {

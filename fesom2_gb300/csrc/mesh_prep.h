@@ -13,6 +13,7 @@ struct HostTopo {
     std::vector<int> t_n, t_nlev, t_ulev;
     std::vector<int> n_nlev, n_ulev, n_nlevmin, n_ulevmax, n_nbl;
     std::vector<int> ne_ptr, ne_idx, nie_ptr, nie_idx;
+    int ring_ok = 0;  // see DTopo
 };
 
 bool prepare_mesh(const fesom_mesh_desc &d, HostTopo &h, std::string &err);

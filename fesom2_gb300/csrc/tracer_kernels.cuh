@@ -29,42 +29,8 @@ template <typename R> __device__ __forceinline__ R rmin(R a, R b) { return a < b
 template <typename R> __device__ __forceinline__ R rabs(R a) { return fabs(a); }
 template <> __device__ __forceinline__ float rabs<float>(float a) { return fabsf(a); }
 
-// The FP64 form keeps the reference's statements and evaluation order.  The FP32
-// form keeps LO's increment (the low-order flux divergence times dt/areasvol)
-// in the LO buffer instead of LO itself, so the final update is a compensated
-// sum of flux terms rather than the difference LO*hnode_new - T*hnode of two
-// nearly equal products (which loses most FP32 bits); LO is rebuilt where the
-// FCT bounds need it.
-template <typename R> struct Exact { static constexpr bool value = false; };
-template <> struct Exact<double> { static constexpr bool value = true; };
-
 __device__ __forceinline__ size_t ix1(int nz, int n, int L1) { return (size_t)n * L1 + (nz - 1); }
 __device__ __forceinline__ size_t ixn(int nz, int n, int nl) { return (size_t)n * nl + (nz - 1); }
-
-// ---------------------------------------------------------------------------
-// Node-sum accumulator: plain for FP64 (the reference's order and rounding),
-// Neumaier-compensated for FP32.
-// ---------------------------------------------------------------------------
-template <typename R>
-struct Acc {
-    R s;
-    __device__ __forceinline__ Acc() : s(R(0)) {}
-    __device__ __forceinline__ void add(R x) { s = s + x; }
-    __device__ __forceinline__ void sub(R x) { s = s - x; }
-    __device__ __forceinline__ R get() const { return s; }
-};
-template <>
-struct Acc<float> {
-    float s, c;
-    __device__ __forceinline__ Acc() : s(0.f), c(0.f) {}
-    __device__ __forceinline__ void add(float x) {
-        float t = s + x;
-        c += (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
-        s = t;
-    }
-    __device__ __forceinline__ void sub(float x) { add(-x); }
-    __device__ __forceinline__ float get() const { return s + c; }
-};
 
 // ===========================================================================
 // tracer_gradient_z (src/oce_tracer_mod.F90:192-232): warp per node, lanes over levels;
@@ -105,66 +71,6 @@ __device__ __forceinline__ void node_mean_grad(const DTopo &tp, const DGeom<R> &
     }
     gx = tx / tvol;
     gy = ty / tvol;
-}
-
-// ===========================================================================
-// Node columns, stage 1: LO solution (edge gather of the upwind fluxes,
-// adv_tra_ver_upw1 with w_e, src/oce_adv_tra_driver.F90:122-250) and the
-// vertical high-order flux minus the LO flux (adv_tra_ver_qr4c / _upw1 with w,
-// src/oce_adv_tra_ver.F90:244-434).  Without a limiter only the HO vertical
-// flux (with w_e) is formed.
-// ===========================================================================
-template <typename R>
-__device__ __forceinline__ R ver_upw1_flux(const R *T, const R *W, const R *area, int nz, int n, int nzmin, int nzmax,
-                                           int L1, int nl, R fin) {
-    // statement order of the reference: surface, bottom, interior
-    R v = fin;
-    if (nz == nzmin) v = -(W[ixn(nz, n, nl)] * T[ix1(nz, n, L1)] * area[ixn(nz, n, nl)]) - v;
-    if (nz == nzmax) v = R(0.0) - v;
-    if (nz >= nzmin + 1 && nz <= nzmax - 1) {
-        const R Wv = W[ixn(nz, n, nl)], aW = rabs(Wv);
-        v = -(R(0.5) * (T[ix1(nz, n, L1)] * (Wv + aW) + T[ix1(nz - 1, n, L1)] * (Wv - aW)) * area[ixn(nz, n, nl)]) - v;
-    }
-    return v;
-}
-
-template <typename R>
-__device__ __forceinline__ R ver_qr4c_flux(const R *T, const R *W, const R *area, const R *Z3, const R *zb3, int nz,
-                                           int n, int nzmin, int nzmax, int L1, int nl, R no, R fin) {
-    // statement order of the reference: nzmin, nzmin+1, nzmax-1, nzmax, interior
-    R v = fin;
-    if (nz == nzmin) v = -(T[ix1(nz, n, L1)] * W[ixn(nz, n, nl)] * area[ixn(nz, n, nl)]) - v;
-    if (nz == nzmin + 1)
-        v = -(R(0.5) * (T[ix1(nz - 1, n, L1)] + T[ix1(nz, n, L1)]) * W[ixn(nz, n, nl)] * area[ixn(nz, n, nl)]) - v;
-    if (nz == nzmax - 1)
-        v = -(R(0.5) * (T[ix1(nz - 1, n, L1)] + T[ix1(nz, n, L1)]) * W[ixn(nz, n, nl)] * area[ixn(nz, n, nl)]) - v;
-    if (nz == nzmax) v = R(0.0) - v;
-    if (nz >= nzmin + 2 && nz <= nzmax - 2) {
-        const R tm2 = T[ix1(nz - 2, n, L1)], tm1 = T[ix1(nz - 1, n, L1)], t0 = T[ix1(nz, n, L1)],
-                tp1 = T[ix1(nz + 1, n, L1)];
-        const R zm2 = Z3[ix1(nz - 2, n, L1)], zm1 = Z3[ix1(nz - 1, n, L1)], z0 = Z3[ix1(nz, n, L1)],
-                zp1 = Z3[ix1(nz + 1, n, L1)];
-        const R qc = (tm1 - t0) / (zm1 - z0);
-        const R qu = (t0 - tp1) / (z0 - zp1);
-        const R qd = (tm2 - tm1) / (zm2 - zm1);
-        const R zb = zb3[ixn(nz, n, nl)];
-        const R Tm1 = t0 + (R(2.0) * qc + qu) * (zb - z0) / R(3.0);
-        const R Tm2 = tm1 + (R(2.0) * qc + qd) * (zb - zm1) / R(3.0);
-        const R Wv = W[ixn(nz, n, nl)], aW = rabs(Wv);
-        const R Tmean = (Wv + aW) * Tm1 + (Wv - aW) * Tm2;
-        v = (-(R(0.5) * (R(1.0) - no) * Tmean) - no * (R(0.5) * (Tm1 + Tm2)) * Wv) * area[ixn(nz, n, nl)] - v;
-    }
-    return v;
-}
-
-// adv_tra_ver_cdiff (src/oce_adv_tra_ver.F90:635-695): the bottom interface keeps its input
-template <typename R>
-__device__ __forceinline__ R ver_cdiff_flux(const R *T, const R *W, const R *area, int nz, int n, int nzmin, int nzmax,
-                                            int L1, int nl, R fin) {
-    if (nz == nzmin) return -(W[ixn(nz, n, nl)] * T[ix1(nz, n, L1)] * area[ixn(nz, n, nl)]) - fin;
-    if (nz == nzmax) return fin;
-    const R tv = R(0.5) * (T[ix1(nz - 1, n, L1)] + T[ix1(nz, n, L1)]);
-    return -(tv * W[ixn(nz, n, nl)] * area[ixn(nz, n, nl)]) - fin;
 }
 
 template <typename R>
@@ -238,283 +144,6 @@ __device__ R ver_ppm_flux(const R *T, const R *W, const R *area, const R *hn, co
         v = -aR + R(0.5) * x * (aR - aL - (R(1.0) - R(2.0) / R(3.0) * x) * aj);
     }
     return v * ac[nz] * w - fin;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kThreads)
-k_node_lo(DTopo tp, DGeom<R> g, DForcing<R> f, DTracers<R> tr, R dt) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L1 = tp.L1, nl = tp.nl;
-    for (int n = blockIdx.x * kWarpsPerBlock + warp; n < tp.N2; n += gridDim.x * kWarpsPerBlock) {
-        const int nzmin = tp.n_ulev[n], nzmax = tp.n_nlev[n];
-        const int k0 = tp.ne_ptr[n], k1 = tp.ne_ptr[n + 1];
-        for (int t = 0; t < tr.ntr; t++) {
-            const DCfg c = tr.cfg[t];
-            const int fct = c.lim;
-            const R *T = tr.T + t * tr.sN;
-            const R *TA = tr.TAB + t * tr.sN;
-            const R *FLO = tr.FLO + t * tr.sE;
-            for (int nz = nzmin + lane; nz <= nzmax; nz += 32) {
-                R fv0 = R(0);
-                if (fct) {
-                    fv0 = ver_upw1_flux(T, f.we, g.area, nz, n, nzmin, nzmax, L1, nl, R(0));
-                    if (nz <= nzmax - 1) {
-                        const R fv1 = ver_upw1_flux(T, f.we, g.area, nz + 1, n, nzmin, nzmax, L1, nl, R(0));
-                        Acc<R> acc;
-                        for (int k = k0; k < k1; k++) {
-                            const int code = tp.ne_idx[k];
-                            const int e = code >= 0 ? code : ~code;
-                            if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
-                            const R x = FLO[ix1(nz, e, L1)];
-                            if (code >= 0) acc.add(x);
-                            else acc.sub(x);
-                        }
-                        const size_t i = ix1(nz, n, L1);
-                        if (Exact<R>::value) {
-                            tr.LO[t * tr.sN + i] = (T[i] * g.hnode[i] + (acc.get() + (fv0 - fv1)) * dt /
-                                                    g.areasvol[ixn(nz, n, nl)]) / g.hnode_new[i];
-                        } else {
-                            acc.add(fv0);
-                            acc.sub(fv1);
-                            tr.LO[t * tr.sN + i] = acc.get() * dt / g.areasvol[ixn(nz, n, nl)];
-                        }
-                    }
-                }
-                const R *pw = fct ? f.w : f.we;
-                // with the split vertical velocity the LO part of the antidiffusive flux is the
-                // upwind flux of the full w (oce_adv_tra_driver.F90:323-334)
-                const R fin = (fct && f.wsplit) ? ver_upw1_flux(T, f.w, g.area, nz, n, nzmin, nzmax, L1, nl, R(0)) : fv0;
-                R v;
-                if (c.ver == 0)
-                    v = ver_qr4c_flux(TA, pw, g.area, g.Z3, g.zbar3, nz, n, nzmin, nzmax, L1, nl, R(c.pv), fin);
-                else if (c.ver == 2)
-                    v = ver_cdiff_flux(TA, pw, g.area, nz, n, nzmin, nzmax, L1, nl, fin);
-                else if (c.ver == 3)
-                    v = ver_ppm_flux(TA, pw, g.area, g.hnode_new, g.hnode, dt, nz, n, nzmin, nzmax, L1, nl, fin);
-                else
-                    v = ver_upw1_flux(TA, pw, g.area, nz, n, nzmin, nzmax, L1, nl, fin);
-                tr.ADv[t * tr.sNI + ixn(nz, n, nl)] = v;
-            }
-        }
-    }
-}
-
-// ===========================================================================
-// FCT bounds a1-a3 and bound increments (src/oce_adv_tra_fct.F90:124-248).
-// The element max/min (AUX) is recomputed per node from the element's three
-// nodes (max/min are exact, so this equals the reference's two passes).
-// ===========================================================================
-// LO of node x at layer nz (the FP32 form stores the increment, see Exact)
-template <typename R>
-__device__ __forceinline__ R lo_value(const R *LO, const R *T, const DGeom<R> &g, int nz, int x, int L1) {
-    const size_t i = ix1(nz, x, L1);
-    if (Exact<R>::value) return LO[i];
-    return (T[i] * g.hnode[i] + LO[i]) / g.hnode_new[i];
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_bounds(DTopo tp, DGeom<R> g, DTracers<R> tr) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    R *sm = reinterpret_cast<R *>(smem_raw);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L1 = tp.L1;
-    R *tvmax = sm + (size_t)warp * 2 * (L1 + 2);
-    R *tvmin = tvmax + (L1 + 2);
-    const R big = R(kBigNumber);
-    for (int n = blockIdx.x * kWarpsPerBlock + warp; n < tp.N2; n += gridDim.x * kWarpsPerBlock) {
-        const int nzmin = tp.n_ulev[n], nzmax = tp.n_nlev[n];
-        const int k0 = tp.nie_ptr[n], k1 = tp.nie_ptr[n + 1];
-        for (int t = 0; t < tr.ntr; t++) {
-            if (!tr.cfg[t].lim) continue;
-            const R *T = tr.T + t * tr.sN;
-            const R *LO = tr.LO + t * tr.sN;
-            for (int nz = nzmin + lane; nz <= nzmax - 1; nz += 32) {
-                R mx = R(0), mn = R(0);
-                for (int k = k0; k < k1; k++) {
-                    const int el = tp.nie_idx[k];
-                    R amx, amn;
-                    if (nz >= tp.t_ulev[el] && nz <= tp.t_nlev[el] - 1) {
-                        const int a = tp.t_n[3 * el], b = tp.t_n[3 * el + 1], cc = tp.t_n[3 * el + 2];
-                        const R la = lo_value(LO, T, g, nz, a, L1), ta = T[ix1(nz, a, L1)];
-                        const R lb = lo_value(LO, T, g, nz, b, L1), tb = T[ix1(nz, b, L1)];
-                        const R lc = lo_value(LO, T, g, nz, cc, L1), tc = T[ix1(nz, cc, L1)];
-                        amx = rmax(rmax(rmax(la, ta), rmax(lb, tb)), rmax(lc, tc));
-                        amn = rmin(rmin(rmin(la, ta), rmin(lb, tb)), rmin(lc, tc));
-                    } else {
-                        amx = -big;
-                        amn = big;
-                    }
-                    if (k == k0) { mx = amx; mn = amn; }
-                    else { mx = rmax(mx, amx); mn = rmin(mn, amn); }
-                }
-                tvmax[nz] = mx;
-                tvmin[nz] = mn;
-            }
-            __syncwarp();
-            R *bmx = tr.bmax + t * tr.sN, *bmn = tr.bmin + t * tr.sN;
-            for (int nz = nzmin + lane; nz <= nzmax - 1; nz += 32) {
-                const R lo = lo_value(LO, T, g, nz, n, L1);
-                R vmx, vmn;
-                if (nz == nzmin || nz == nzmax - 1) {
-                    vmx = tvmax[nz] - lo;
-                    vmn = tvmin[nz] - lo;
-                } else {
-                    vmx = rmax(rmax(tvmax[nz - 1], tvmax[nz]), tvmax[nz + 1]) - lo;
-                    vmn = rmin(rmin(tvmin[nz - 1], tvmin[nz]), tvmin[nz + 1]) - lo;
-                }
-                bmx[ix1(nz, n, L1)] = vmx;
-                bmn[ix1(nz, n, L1)] = vmn;
-            }
-            __syncwarp();
-        }
-    }
-}
-
-// ===========================================================================
-// FCT b1 + b2: sums of positive / negative antidiffusive fluxes into each
-// node-layer (vertical, then edges in ascending order) and the ratios R+ / R-
-// (src/oce_adv_tra_fct.F90:265-405).  R+ / R- overwrite bmax / bmin.
-// ===========================================================================
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_rpm(DTopo tp, DGeom<R> g, DTracers<R> tr, R dt) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L1 = tp.L1, nl = tp.nl;
-    const R eps = R(kFluxEps);
-    for (int n = blockIdx.x * kWarpsPerBlock + warp; n < tp.N2; n += gridDim.x * kWarpsPerBlock) {
-        const int nzmin = tp.n_ulev[n], nzmax = tp.n_nlev[n];
-        const int k0 = tp.ne_ptr[n], k1 = tp.ne_ptr[n + 1];
-        for (int t = 0; t < tr.ntr; t++) {
-            if (!tr.cfg[t].lim) continue;
-            const R *ADv = tr.ADv + t * tr.sNI;
-            const R *ADh = tr.ADh + t * tr.sE;
-            for (int nz = nzmin + lane; nz <= nzmax - 1; nz += 32) {
-                const R v0 = ADv[ixn(nz, n, nl)], v1 = ADv[ixn(nz + 1, n, nl)];
-                Acc<R> P, M;
-                P.add(rmax(R(0), v0) + rmax(R(0), -v1));
-                M.add(rmin(R(0), v0) + rmin(R(0), -v1));
-                for (int k = k0; k < k1; k++) {
-                    const int code = tp.ne_idx[k];
-                    const int e = code >= 0 ? code : ~code;
-                    if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
-                    const R x = ADh[ix1(nz, e, L1)];
-                    if (code >= 0) { P.add(rmax(R(0), x)); M.add(rmin(R(0), x)); }
-                    else { P.add(rmax(R(0), -x)); M.add(rmin(R(0), -x)); }
-                }
-                const size_t i = ix1(nz, n, L1);
-                const R av = g.areasvol[ixn(nz, n, nl)], hn = g.hnode_new[i];
-                R fl = P.get() * dt / av / hn + eps;
-                const R rp = rmin(R(1.0), tr.bmax[t * tr.sN + i] / fl);
-                fl = M.get() * dt / av / hn - eps;
-                const R rm = rmin(R(1.0), tr.bmin[t * tr.sN + i] / fl);
-                tr.bmax[t * tr.sN + i] = rp;
-                tr.bmin[t * tr.sN + i] = rm;
-            }
-        }
-    }
-}
-
-// ===========================================================================
-// FCT b3 limiting + oce_tra_adv_flux2dtracer (src/oce_adv_tra_fct.F90:425-500,
-// src/oce_adv_tra_driver.F90:494-646) + (mode 1) the del_ttf sum and the T*
-// update of diff_tracers_ale (src/oce_ale_tracer.F90:319-321, 743-754).
-// The limited edge flux is formed at each end node from R+/R- of both ends.
-// ===========================================================================
-template <typename R>
-__device__ __forceinline__ R limited_adv(const R *ADv, const R *Rp, const R *Rm, int nz, int n, int nzmin, int nzmax,
-                                         int L1, int nl) {
-    const R x = ADv[ixn(nz, n, nl)];
-    if (nz == nzmax) return x;
-    R ae = R(1.0);
-    if (nz == nzmin) {
-        ae = x >= R(0) ? rmin(ae, Rp[ix1(nz, n, L1)]) : rmin(ae, Rm[ix1(nz, n, L1)]);
-    } else if (x >= R(0)) {
-        ae = rmin(ae, Rm[ix1(nz - 1, n, L1)]);
-        ae = rmin(ae, Rp[ix1(nz, n, L1)]);
-    } else {
-        ae = rmin(ae, Rp[ix1(nz - 1, n, L1)]);
-        ae = rmin(ae, Rm[ix1(nz, n, L1)]);
-    }
-    return ae * x;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kThreads) k_update(DTopo tp, DGeom<R> g, DTracers<R> tr, R dt, int mode) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int L1 = tp.L1, nl = tp.nl;
-    for (int n = blockIdx.x * kWarpsPerBlock + warp; n < tp.N2; n += gridDim.x * kWarpsPerBlock) {
-        const int nzmin = tp.n_ulev[n], nzmax = tp.n_nlev[n];
-        const int k0 = tp.ne_ptr[n], k1 = tp.ne_ptr[n + 1];
-        for (int t = 0; t < tr.ntr; t++) {
-            const int fct = tr.cfg[t].lim;
-            R *T = tr.T + t * tr.sN;
-            const R *ADv = tr.ADv + t * tr.sNI;
-            const R *ADh = tr.ADh + t * tr.sE;
-            const R *Rp = tr.bmax + t * tr.sN, *Rm = tr.bmin + t * tr.sN;
-            for (int nz = nzmin + lane; nz <= nzmax - 1; nz += 32) {
-                const size_t i = ix1(nz, n, L1);
-                const R av = g.areasvol[ixn(nz, n, nl)];
-                R dv = R(0.0);
-                R f0, f1;
-                if (fct) {
-                    if (Exact<R>::value) dv = dv - T[i] * g.hnode[i] + tr.LO[t * tr.sN + i] * g.hnode_new[i];
-                    f0 = limited_adv(ADv, Rp, Rm, nz, n, nzmin, nzmax, L1, nl);
-                    f1 = limited_adv(ADv, Rp, Rm, nz + 1, n, nzmin, nzmax, L1, nl);
-                } else {
-                    f0 = ADv[ixn(nz, n, nl)];
-                    f1 = ADv[ixn(nz + 1, n, nl)];
-                }
-                Acc<R> dh;
-                if (!Exact<R>::value) {
-                    // FP32: one compensated sum of LO increment, vertical and horizontal terms
-                    if (fct) dh.add(tr.LO[t * tr.sN + i]);
-                    dh.add(f0 * dt / av);
-                    dh.sub(f1 * dt / av);
-                } else {
-                    dv = dv + (f0 - f1) * dt / av;
-                }
-                for (int k = k0; k < k1; k++) {
-                    const int code = tp.ne_idx[k];
-                    const int e = code >= 0 ? code : ~code;
-                    if (nz < tp.e_lo[e] || nz > tp.e_hi[e]) continue;
-                    R x = ADh[ix1(nz, e, L1)];
-                    if (fct) {
-                        const int a = tp.e_n1[e], b = tp.e_n2[e];
-                        R ae = R(1.0);
-                        if (x >= R(0)) {
-                            ae = rmin(ae, Rp[ix1(nz, a, L1)]);
-                            ae = rmin(ae, Rm[ix1(nz, b, L1)]);
-                        } else {
-                            ae = rmin(ae, Rm[ix1(nz, a, L1)]);
-                            ae = rmin(ae, Rp[ix1(nz, b, L1)]);
-                        }
-                        x = ae * x;
-                    }
-                    if (code >= 0) dh.add(x * dt / av);
-                    else dh.sub(x * dt / av);
-                }
-                if (!Exact<R>::value) dh.add(T[i] * (g.hnode[i] - g.hnode_new[i]));
-                const R dhv = dh.get();
-                if (mode == 0) {
-                    tr.dttf_h[t * tr.sN + i] = dhv;
-                    tr.dttf_v[t * tr.sN + i] = dv;
-                } else {
-                    R del = dhv;
-                    if (Exact<R>::value) {
-                        del = R(0.0) + dhv + dv;
-                        // diff_tracers_ale: horizontal, then explicit vertical diffusion
-                        if (tr.HD) del = hdiff_add(tp, tr.HD + t * tr.sE, del, n, nz, L1, dt, av);
-                        if (tr.VX && !tr.cfg[t].ivd) del = del + tr.VX[t * tr.sN + i];
-                        // Redi: diff_ver_part_redi_expl (:623)
-                        if (tr.RV) del = del + tr.RV[t * tr.sN + i];
-                        del = del + T[i] * (g.hnode[i] - g.hnode_new[i]);
-                    }
-                    const R tn = T[i] + del / g.hnode_new[i];
-                    T[i] = tn;
-                    if (!isfinite(tn)) atomicOr(tr.status, 1u);
-                }
-            }
-        }
-    }
 }
 
 // ===========================================================================
@@ -916,27 +545,6 @@ static inline int grid_for(int nent, int per_block) {
 template <typename R>
 void Launch<R>::trz(const DTopo &tp, const DGeom<R> &g, const R *T, R *trz, cudaStream_t s) {
     k_trz<R><<<grid_for(tp.N2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, T, trz);
-}
-template <typename R>
-void Launch<R>::node_lo(const DTopo &tp, const DGeom<R> &g, const DForcing<R> &f, DTracers<R> &tr, double dt, int fct,
-                        cudaStream_t s) {
-    (void)fct;
-    k_node_lo<R><<<grid_for(tp.N2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, f, tr, (R)dt);
-}
-template <typename R>
-void Launch<R>::bounds(const DTopo &tp, const DGeom<R> &g, DTracers<R> &tr, cudaStream_t s) {
-    const size_t sm = sizeof(R) * 2 * (tp.L1 + 2) * kWarpsPerBlock;
-    k_bounds<R><<<grid_for(tp.N2, kWarpsPerBlock), kThreads, sm, s>>>(tp, g, tr);
-}
-template <typename R>
-void Launch<R>::rpm(const DTopo &tp, const DGeom<R> &g, DTracers<R> &tr, double dt, cudaStream_t s) {
-    k_rpm<R><<<grid_for(tp.N2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, tr, (R)dt);
-}
-template <typename R>
-void Launch<R>::update(const DTopo &tp, const DGeom<R> &g, DTracers<R> &tr, double dt, int fct, int mode,
-                       cudaStream_t s) {
-    (void)fct;
-    k_update<R><<<grid_for(tp.N2, kWarpsPerBlock), kThreads, 0, s>>>(tp, g, tr, (R)dt, mode);
 }
 template <typename R>
 void Launch<R>::lo_impl(const DTopo &tp, const DGeom<R> &g, const DForcing<R> &f, DTracers<R> &tr, double dt,
