@@ -1121,6 +1121,7 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
     else rc = init_geom<double>(ctx, mesh, ctx->g64);
     if (rc) return rc;
     if (precision == FESOM_PREC_FP64) {
+        CK(fp64_prepare());
         const size_t n = (size_t)ctx->nl * ctx->N2, m = (size_t)ctx->L1 * ctx->N2;
         if ((rc = dalloc(ctx, (void **)&ctx->g64.rav, n * sizeof(double2))) ||
             (rc = dalloc(ctx, (void **)&ctx->g64.rhn, m * sizeof(double2))))

@@ -253,6 +253,8 @@ void bm32_hdiff(const Inst32 *, const MultiIdx &edges, cudaStream_t);
 void bm32_diff(const Inst32 *, const MultiIdx &nodes, bool wide, cudaStream_t);
 
 // reciprocals of a divisor array for DGeom::rav / rhn (kernels_fp64.cu)
+// shared-memory limits of the FP64 kernels, once per context (kernels_fp64.cu)
+cudaError_t fp64_prepare();
 void recip_table(const double *y, double2 *out, size_t n, cudaStream_t);
 
 // tail of the tracer loop (kernels_tail.cu): one tracer's decay, relaxation and clamp

@@ -617,6 +617,56 @@ k_update(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int mode, in
 }
 
 // ===========================================================================
+// diff_ver_part_impl_ale (src/oce_ale_tracer.F90:1071-1430): a tile of columns per block, the
+// tracers with implicit vertical diffusion NT at a time
+// ===========================================================================
+template <int NT>
+static __global__ void __launch_bounds__(kVThreads) k_vdiff_tile(VArgs P, DTracers<double> tr, const double *bc,
+                                                                 int wsplit) {
+    extern __shared__ __align__(16) double sm64[];
+    __shared__ VTile S;
+    const int n0 = blockIdx.x * kVCols;
+    if (threadIdx.x < 32) {
+        const int n = n0 + threadIdx.x;
+        const bool ok = n < P.N2;
+        S.fill(threadIdx.x, ok ? P.ulev[n] : 1, ok ? P.nlev[n] - P.ulev[n] : 0);
+    }
+    // the implicit part of a split vertical velocity joins the solve without a limiter (:961)
+    for (int w = 0; w <= (wsplit ? 1 : 0); w++) {
+        int t = 0;
+        while (t < tr.ntr) {
+            VTracer q[NT];
+            int nt = 0;
+#pragma unroll
+            for (int k = 0; k < NT; k++) {
+                while (t < tr.ntr && !(tr.cfg[t].ivd && (wsplit && !tr.cfg[t].lim) == (w != 0))) t++;
+                q[k] = VTracer{nullptr, nullptr};
+                if (t < tr.ntr) {
+                    q[k] = VTracer{tr.T + t * tr.sN, bc ? bc + (size_t)t * P.N2 : nullptr};
+                    nt = k + 1;
+                    t++;
+                }
+            }
+            if (!nt) break;
+            __syncthreads();
+            vdiff_tile<NT>(P, S, n0, sm64, q, nt, w != 0);
+        }
+    }
+}
+// shared-memory limits, once per context
+template <int NT>
+static cudaError_t vdiff_prepare() {
+    return cudaFuncSetAttribute(k_vdiff_tile<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmemMax);
+}
+cudaError_t fp64_prepare() {
+    cudaError_t e = vdiff_prepare<1>();
+    if (e == cudaSuccess) e = vdiff_prepare<2>();
+    if (e == cudaSuccess) e = vdiff_prepare<3>();
+    if (e == cudaSuccess) e = vdiff_prepare<4>();
+    return e;
+}
+
+// ===========================================================================
 // launches
 // ===========================================================================
 template <>
@@ -655,6 +705,24 @@ void Launch<double>::update(const DTopo &tp, const DGeom<double> &g, DTracers<do
     const size_t b = sizeof(double) * tp.L1;
     const int t = tile_size(tp.N2, b);
     k_update<<<(tp.N2 + t - 1) / t, kTileThreads, t * b, s>>>(tp, g, tr, dt, mode, t);
+}
+template <>
+void Launch<double>::vdiff(const DTopo &tp, const DGeom<double> &g, const DForcing<double> &f, DTracers<double> &tr,
+                           double dt, double *scratch, cudaStream_t s) {
+    if (vtile_smem(tp.L1, 1) > kVSmemMax) {
+        k_vdiff<double><<<(tp.N2 + 127) / 128, 128, 0, s>>>(tp, g, f, tr, dt, scratch);
+        return;
+    }
+    // as many tracers at a time as share the coefficients with two blocks resident per SM
+    int nt = std::min(tr.ntr, 4);
+    while (nt > 1 && vtile_smem(tp.L1, nt) > kVSmemMax / 2) nt--;
+    const VArgs P{tp.N2, tp.nl, tp.n_nlev, tp.n_ulev, g.zbar_n_bot, g.hnode_new, g.area, g.areasvol, f.Kv, f.wi, dt};
+    const int nb = (tp.N2 + kVCols - 1) / kVCols;
+    const size_t sm = vtile_smem(tp.L1, nt);
+    if (nt == 1) k_vdiff_tile<1><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);
+    else if (nt == 2) k_vdiff_tile<2><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);
+    else if (nt == 3) k_vdiff_tile<3><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);
+    else k_vdiff_tile<4><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);
 }
 // reciprocals of a divisor array (DGeom::rav, rhn)
 static __global__ void k_recip(const double *y, double2 *out, size_t n) {

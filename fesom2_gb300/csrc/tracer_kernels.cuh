@@ -552,12 +552,6 @@ void Launch<R>::lo_impl(const DTopo &tp, const DGeom<R> &g, const DForcing<R> &f
     k_lo_impl<R><<<(tp.N2 + 127) / 128, 128, 0, s>>>(tp, g, f, tr, dt, scratch);
 }
 template <typename R>
-void Launch<R>::vdiff(const DTopo &tp, const DGeom<R> &g, const DForcing<R> &f, DTracers<R> &tr, double dt,
-                      double *scratch, cudaStream_t s) {
-    int blocks = (tp.N2 + 127) / 128;
-    k_vdiff<R><<<blocks, 128, 0, s>>>(tp, g, f, tr, dt, scratch);
-}
-template <typename R>
 void Launch<R>::content(const DTopo &tp, const DGeom<R> &g, const DTracers<R> &tr, double *partials, int nblk,
                         double *out, cudaStream_t s) {
     k_content_partial<R><<<nblk, 256, 0, s>>>(tp, g, tr, partials);

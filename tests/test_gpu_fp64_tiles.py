@@ -46,3 +46,30 @@ def test_step_bitwise(nx, ny, layers, partial, schemes, ab):
             assert np.array_equal(Tg[k], To[k]), f"step {step} tracer {k}"
             assert np.array_equal(Og[k], Oo[k]), f"step {step} tracer {k}: previous levels"
     assert ctx.status() == 0
+
+
+@pytest.mark.parametrize("nx,ny,layers,ntr", [(5, 7, 4, 1), (8, 4, 32, 2), (7, 9, 33, 3), (11, 13, 65, 5),
+                                              (6, 7, 217, 2), (6, 7, 218, 2)])
+def test_vertical_diffusion_tiles_bitwise(nx, ny, layers, ntr):
+    """Tiles of 32 columns (a last one of fewer), up to four tracers to a pass, and the deepest
+    column a tile holds next to the first that takes a thread per column."""
+    mesh = M.channel_mesh(nx, ny, 5000.0, M.stretched_zbar(layers, 5.0, 20.0), seamounts=1, seed=5, partial_cells=True)
+    f = O.ensure_f64(M.make_forcing(mesh, "channel", seed=3, dt=600.0))
+    rng = np.random.default_rng(6)
+    tr = [np.ascontiguousarray(t) for t in M.make_tracers(mesh, "channel", ntr=ntr, seed=4)]
+    om = O.OracleMesh(mesh)
+    ctx = G.Context(mesh, G.PREC_FP64, max_tracers=ntr)
+    To, Tg = [t.copy() for t in tr], [t.copy() for t in tr]
+    Oo = [perturbed_old(t, rng) for t in To]
+    Og = [o.copy() for o in Oo]
+    for k in range(ntr):
+        om.tracer_step(f, O.cfg_struct(), To[k], np.zeros_like(To[k]), Oo[k])
+    ctx.tracer_step(f, [G.tra_cfg(id=k + 1) for k in range(ntr)], Tg, Og)
+    for k in range(ntr):
+        assert np.array_equal(Tg[k], To[k]), f"tracer {k}"
+    # the drop-ins, with a surface flux: one tracer through a context and without one
+    f.bc_surface = np.linspace(-1e-3, 1e-3, mesh.nod2D)
+    want, got = tr[0].copy(), tr[0].copy()
+    om.diff_ver_part_impl_ale(f, want)
+    ctx.vdiff_impl(f, G.tra_cfg(), got)
+    assert np.array_equal(got, want)
