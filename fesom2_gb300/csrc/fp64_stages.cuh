@@ -15,48 +15,10 @@
 #pragma once
 #include "fesom_internal.h"
 #include "fp64_arith.cuh"
+#include "tile.cuh"
 #include "tracer_kernels.cuh"
 
 namespace fesom {
-
-constexpr int kTileThreads = 128;
-constexpr int kTileMax = 8;  // entities per tile
-
-// the wet levels of a tile's entities as items 0 .. total-1: entity j holds the items
-// pre[j] .. pre[j+1]-1, levels top[j], top[j] + 1, ...
-struct Tile {
-    int total;
-    int pre[kTileMax + 1], top[kTileMax];
-    // one warp, lane j < kTileMax with the level count of entity j (0 past the tile's end)
-    __device__ __forceinline__ void fill(int lane, int first_level, int levels) {
-        int s = lane < kTileMax ? levels : 0;
-#pragma unroll
-        for (int o = 1; o < kTileMax; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += v;
-        }
-        if (lane < kTileMax) {
-            pre[lane + 1] = s;
-            top[lane] = first_level;
-            if (lane == 0) pre[0] = 0;
-            if (lane == kTileMax - 1) total = s;
-        }
-    }
-    __device__ __forceinline__ int find(int i) const {
-        int j = i >= pre[4] ? 4 : 0;
-        j += i >= pre[j + 2] ? 2 : 0;
-        return j + (i >= pre[j + 1] ? 1 : 0);
-    }
-};
-
-// entities per tile: 8, or 4 where 8 would leave less than eight blocks per SM (a mesh of 2.9k
-// nodes: 4.8 blocks per SM instead of 2.4, so the SMs finish together); fewer where the tile's
-// shared memory (`bytes` per entity) would pass 48 KB
-static inline int tile_size(int n, size_t bytes) {
-    int t = n >= 152 * 8 * kTileMax ? kTileMax : 4;
-    while (t > 1 && t * bytes > 46 * 1024) t >>= 1;
-    return t;
-}
 
 // -(0.5 (a (v + |v|) + b (v - |v|))), the upwind flux of a (v > 0) and b (v < 0)
 __device__ __forceinline__ double upwind64(double a, double b, double v) {

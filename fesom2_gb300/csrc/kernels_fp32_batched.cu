@@ -63,6 +63,7 @@
 #include <algorithm>
 
 #include "fesom_internal.h"
+#include "tile.cuh"
 
 namespace fesom {
 
@@ -99,10 +100,8 @@ struct MinB {
 #ifdef FESOM_MINB_HO
     static constexpr int ho = FESOM_MINB_HO;
 #else
-    static constexpr int ho = G == 4 ? 3 : 4;
+    static constexpr int ho = G == 4 ? 6 : 8;  // blocks of kTileThreads
 #endif
-    // the staged edge kernel: 80 KB (G = 4) of staging per block of eight warps
-    static constexpr int ho_stg = 2;
     // bounds and update: gathers in registers (three blocks of eight warps per SM measured
     // faster than two with more registers or one with the whole pass in flight), or staged in
     // shared memory (which holds one block of the G = 4 staging per SM)
@@ -137,46 +136,70 @@ __device__ __forceinline__ float sh_dn(float v, int d) { return __shfl_down_sync
 // ---------------------------------------------------------------------------
 // k32_vflux: volume flux of every edge-layer (shared by all tracers)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void vflux_edge(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, float *VF,
-                                           int e, int lane) {
-    const int L1 = tp.L1;
-    {
-        const int el1 = tp.e_t1[e], el2 = tp.e_t2[e];
-        const int nl1 = tp.t_nlev[el1] - 1, nu1 = tp.t_ulev[el1];
-        int nl2 = 0, nu2 = 0;
-        const float dX1 = g.ecd[4 * (size_t)e], dY1 = g.ecd[4 * (size_t)e + 1];
-        float dX2 = 0.f, dY2 = 0.f;
-        if (el2 >= 0) {
-            nl2 = tp.t_nlev[el2] - 1;
-            nu2 = tp.t_ulev[el2];
-            dX2 = g.ecd[4 * (size_t)e + 2];
-            dY2 = g.ecd[4 * (size_t)e + 3];
-        }
-        const int fnl12 = min(nl1, nl2), fnu12 = max(nu1, nu2);
-        for (int nz = tp.e_lo[e] + lane; nz <= tp.e_hi[e]; nz += 32) {
-            int seg = 0;
-            if (nz >= nu1 && nz <= fnu12 - 1) seg = 1;
-            else if (nu2 > 0 && nz >= nu2 && nz <= fnu12 - 1) seg = 2;
-            else if (nz >= fnu12 && nz <= fnl12) seg = 3;
-            else if (nz >= fnl12 + 1 && nz <= nl1) seg = 1;
-            else if (nz >= fnl12 + 1 && nz <= nl2) seg = 2;
-            float vf = 0.f;
-            if (seg & 1) {
-                const float u = f.uv[2 * i1(nz, el1, L1)], v = f.uv[2 * i1(nz, el1, L1) + 1];
-                vf = (-(v * dX1) + u * dY1) * g.helem[i1(nz, el1, L1)];
+struct EdgeV {
+    int el1, el2, nl1, nu1, nl2, nu2;
+    float dX1, dY1, dX2, dY2;
+};
+
+// tile ti of `tile` edges
+__device__ __forceinline__ void vflux_tile(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, float *VF,
+                                           int ti, int tile, Tile &S, EdgeV *Ed) {
+    const int L1 = tp.L1, e0 = ti * tile;
+    if (threadIdx.x < 32) {
+        const int j = threadIdx.x, e = e0 + j;
+        const bool in = j < tile && e < tp.E2;
+        if (in) {
+            EdgeV &E = Ed[j];
+            const int el1 = tp.e_t1[e], el2 = tp.e_t2[e];
+            E.el1 = el1;
+            E.el2 = el2;
+            E.nl1 = tp.t_nlev[el1] - 1;
+            E.nu1 = tp.t_ulev[el1];
+            const float4 d = reinterpret_cast<const float4 *>(g.ecd)[e];
+            E.dX1 = d.x;
+            E.dY1 = d.y;
+            E.nl2 = E.nu2 = 0;
+            E.dX2 = E.dY2 = 0.f;
+            if (el2 >= 0) {
+                E.nl2 = tp.t_nlev[el2] - 1;
+                E.nu2 = tp.t_ulev[el2];
+                E.dX2 = d.z;
+                E.dY2 = d.w;
             }
-            if (seg & 2) {
-                const float u = f.uv[2 * i1(nz, el2, L1)], v = f.uv[2 * i1(nz, el2, L1) + 1];
-                vf += (v * dX2 - u * dY2) * g.helem[i1(nz, el2, L1)];
-            }
-            VF[i1(nz, e, L1)] = vf;
         }
+        S.fill(j, in ? tp.e_lo[e] : 1, in ? tp.e_hi[e] - tp.e_lo[e] + 1 : 0);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+        const int j = S.find(i), nz = S.top[j] + i - S.pre[j];
+        const EdgeV &E = Ed[j];
+        const int fnl12 = min(E.nl1, E.nl2), fnu12 = max(E.nu1, E.nu2);
+        int seg = 0;
+        if (nz >= E.nu1 && nz <= fnu12 - 1) seg = 1;
+        else if (E.nu2 > 0 && nz >= E.nu2 && nz <= fnu12 - 1) seg = 2;
+        else if (nz >= fnu12 && nz <= fnl12) seg = 3;
+        else if (nz >= fnl12 + 1 && nz <= E.nl1) seg = 1;
+        else if (nz >= fnl12 + 1 && nz <= E.nl2) seg = 2;
+        float vf = 0.f;
+        if (seg & 1) {
+            const size_t k = i1(nz, E.el1, L1);
+            const float2 q = reinterpret_cast<const float2 *>(f.uv)[k];
+            vf = (-(q.y * E.dX1) + q.x * E.dY1) * g.helem[k];
+        }
+        if (seg & 2) {
+            const size_t k = i1(nz, E.el2, L1);
+            const float2 q = reinterpret_cast<const float2 *>(f.uv)[k];
+            vf += (q.y * E.dX2 - q.x * E.dY2) * g.helem[k];
+        }
+        VF[i1(nz, e0 + j, L1)] = vf;
     }
 }
 
-__global__ void __launch_bounds__(kTB) k32_vflux(DTopo tp, DGeom<float> g, DForcing<float> f, float *VF) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int e = blockIdx.x * kWB + warp; e < tp.E2; e += gridDim.x * kWB) vflux_edge(tp, g, f, VF, e, lane);
+__global__ void __launch_bounds__(kTileThreads)
+k32_vflux(DTopo tp, DGeom<float> g, DForcing<float> f, float *VF, int tile) {
+    __shared__ Tile S;
+    __shared__ EdgeV Ed[kTileMax];
+    vflux_tile(tp, g, f, VF, blockIdx.x, tile, S, Ed);
 }
 
 // ---------------------------------------------------------------------------
@@ -1055,158 +1078,78 @@ __device__ __forceinline__ Vec<G> ho_group(const B32View &B, int gq, int hor, co
     return out;
 }
 
-template <int G, bool PACK>
-__device__ __forceinline__ void ho_pass(const DTopo &tp, const B32View &B, const MusclW &mw,
-                                        const float *__restrict__ VF, int e, int nz0, int W, int P, int lane) {
-    const int L1 = tp.L1;
-    const int n1 = tp.e_n1[e], n2 = tp.e_n2[e];
-    const int ehi = tp.e_hi[e];
-    const int nbl1 = tp.n_nbl[n1], nbl2 = tp.n_nbl[n2];
-    const int4 un = mw.un[e], dn = mw.dn[e];
-    const float4 wu = mw.wu[e], wd = mw.wd[e];
-    const int gzmin = un.w & 0xffff, gzmax = un.w >> 16;
-    const int q = PACK ? lane / W : 0;
-    const int nz = nz0 + lane - q * W;
-    const bool tri = nz >= gzmin && nz <= gzmax - 1;
-    const bool ok = nz <= ehi && q < P;
-    if (!ok) return;
-    const int ie = e * L1 + nz - 1, ia = n1 * L1 + nz - 1, ib = n2 * L1 + nz - 1;
-    const float v = VF[ie];
-    const float cl1 = (nbl1 - nz) >= 0 ? 1.f : 0.f, cl2 = (nbl2 - nz) >= 0 ? 1.f : 0.f;
-    const int ua = un.y * L1 + nz - 1, ub = un.z * L1 + nz - 1;
-    const int da = dn.y * L1 + nz - 1, db = dn.z * L1 + nz - 1;
-#pragma unroll 1
-    for (int g0 = 0; g0 < B.ng; g0 += PACK ? P : 1) {
-        const int gq = g0 + q;
-        if (gq >= B.ng) break;
-        const int hor = B.hor[gq];
-        // MUSCL / MFCT levels outside the triangles' range: the node-mean launch
-        if (hor != 2 && !tri) continue;
-        const bool grad = hor != 2;
-        const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
-        const float *__restrict__ O1 = grp<G>(B.O1, gq, B.sN);
-        const float *__restrict__ O2 = B.ab == 3 ? grp<G>(B.O2, gq, B.sN) : O1;
-        const Vec<G> T1 = vld<G>(T, ia), T2 = vld<G>(T, ib);
-        const Vec<G> o1a = vld<G>(O1, ia), o1b = vld<G>(O1, ib);
-        const Vec<G> o2a = vldc<G>(B.ab == 3, O2, ia), o2b = vldc<G>(B.ab == 3, O2, ib);
-        const Vec<G> ga = vldc<G>(grad, T, ua), gb = vldc<G>(grad, T, ub);
-        const Vec<G> gc = vldc<G>(grad, T, da), gd = vldc<G>(grad, T, db);
-        vst<G>(grp<G>(B.ADh, gq, B.sE), ie,
-               ho_group<G>(B, gq, hor, T1, T2, o1a, o1b, o2a, o2b, ga, gb, gc, gd, wu, wd, v, cl1, cl2));
-    }
-}
+struct EdgeH {
+    int ia, ib, ua, ub, da, db;  // first entries of the columns of both ends and of the triangles' other nodes
+    int gmin, gmax, nbl1, nbl2;
+    float uy, uz, dy, dz;
+};
 
-// The same pass with each group's gathers (T and the previous levels at both ends, T at the
-// four triangle vertices) copied into shared memory by cp.async, double-buffered across the
-// groups: the next group's copies are in flight while the current one computes.  Each lane reads
-// back only its own copies, so the staging needs no barrier.  Staging of a warp:
-// [2 buffers][kNsHo entries][32 lanes][G floats].
-constexpr int kNsHo = 10;
+// tile ti of `tile` edges
 template <int G>
-__host__ __device__ constexpr int stage_bytes_ho() { return 2 * kNsHo * 32 * G * 4; }
-
-template <int G, bool PACK>
-__device__ __forceinline__ void ho_pass_pf(const DTopo &tp, const B32View &B, const MusclW &mw,
-                                           const float *__restrict__ VF, int e, int nz0, int W, int P, int lane,
-                                           float *sb) {
-    const int L1 = tp.L1;
-    const int n1 = tp.e_n1[e], n2 = tp.e_n2[e];
-    const int ehi = tp.e_hi[e];
-    const int nbl1 = tp.n_nbl[n1], nbl2 = tp.n_nbl[n2];
-    const int4 un = mw.un[e], dn = mw.dn[e];
-    const float4 wu = mw.wu[e], wd = mw.wd[e];
-    const int gzmin = un.w & 0xffff, gzmax = un.w >> 16;
-    const int q = PACK ? lane / W : 0;
-    const int nz = nz0 + lane - q * W;
-    const bool tri = nz >= gzmin && nz <= gzmax - 1;
-    const bool ok = nz <= ehi && q < P;
-    if (!ok) return;
-    const int ie = e * L1 + nz - 1, ia = n1 * L1 + nz - 1, ib = n2 * L1 + nz - 1;
-    const float v = VF[ie];
-    const float cl1 = (nbl1 - nz) >= 0 ? 1.f : 0.f, cl2 = (nbl2 - nz) >= 0 ? 1.f : 0.f;
-    // the triangle vertices' entries where the gradients apply (elsewhere the edge's own, unread)
-    const int ua = tri ? un.y * L1 + nz - 1 : ia, ub = tri ? un.z * L1 + nz - 1 : ia;
-    const int da = tri ? dn.y * L1 + nz - 1 : ib, db = tri ? dn.z * L1 + nz - 1 : ib;
-    const int npass = PACK ? (B.ng + P - 1) / P : B.ng;
-    auto issue = [&](int p, float *buf) {
-        const int gq = PACK ? p * P + q : p;
-        const bool on = gq < B.ng;
-        const int gi = on ? gq : 0;
-        const int hor = B.hor[gi];
-        const bool act = on && (hor == 2 || tri);
-        const bool grad = act && hor != 2;
-        const float *T = grp<G>(B.T, gi, B.sN), *O1 = grp<G>(B.O1, gi, B.sN);
-        const float *O2 = B.ab == 3 ? grp<G>(B.O2, gi, B.sN) : O1;
-        cpa<G>(stg<G>(buf, 0, lane), T + (size_t)ia * G, act);
-        cpa<G>(stg<G>(buf, 1, lane), T + (size_t)ib * G, act);
-        cpa<G>(stg<G>(buf, 2, lane), O1 + (size_t)ia * G, act);
-        cpa<G>(stg<G>(buf, 3, lane), O1 + (size_t)ib * G, act);
-        cpa<G>(stg<G>(buf, 4, lane), O2 + (size_t)ia * G, act && B.ab == 3);
-        cpa<G>(stg<G>(buf, 5, lane), O2 + (size_t)ib * G, act && B.ab == 3);
-        cpa<G>(stg<G>(buf, 6, lane), T + (size_t)ua * G, grad);
-        cpa<G>(stg<G>(buf, 7, lane), T + (size_t)ub * G, grad);
-        cpa<G>(stg<G>(buf, 8, lane), T + (size_t)da * G, grad);
-        cpa<G>(stg<G>(buf, 9, lane), T + (size_t)db * G, grad);
-        cpa_commit();
-    };
-    auto compute = [&](int p, const float *buf) {
-        const int gq = PACK ? p * P + q : p;
-        if (gq >= B.ng) return;
-        const int hor = B.hor[gq];
-        if (hor != 2 && !tri) return;  // MUSCL / MFCT outside the triangles' range: the node-mean launch
-        const Vec<G> r = ho_group<G>(B, gq, hor, lds<G>(stg<G>((float *)buf, 0, lane)),
-                                     lds<G>(stg<G>((float *)buf, 1, lane)), lds<G>(stg<G>((float *)buf, 2, lane)),
-                                     lds<G>(stg<G>((float *)buf, 3, lane)), lds<G>(stg<G>((float *)buf, 4, lane)),
-                                     lds<G>(stg<G>((float *)buf, 5, lane)), lds<G>(stg<G>((float *)buf, 6, lane)),
-                                     lds<G>(stg<G>((float *)buf, 7, lane)), lds<G>(stg<G>((float *)buf, 8, lane)),
-                                     lds<G>(stg<G>((float *)buf, 9, lane)), wu, wd, v, cl1, cl2);
-        vst<G>(grp<G>(B.ADh, gq, B.sE), ie, r);
-    };
-    issue(0, sb);
-    float *cur = sb, *nxt = sb + (size_t)kNsHo * 32 * G;
-    for (int p = 0; p < npass; p++) {
-        if (p + 1 < npass) {
-            issue(p + 1, nxt);
-            cpa_wait<1>();
-        } else {
-            cpa_wait<0>();
+__device__ __forceinline__ void ho_tile(const DTopo &tp, const B32View &B, const MusclW &mw,
+                                        const float *__restrict__ VF, int ti, int tile, Tile &S, EdgeH *Ed) {
+    const int L1 = tp.L1, e0 = ti * tile;
+    if (threadIdx.x < 32) {
+        const int j = threadIdx.x, e = e0 + j;
+        const bool in = j < tile && e < tp.E2;
+        if (in) {
+            EdgeH &E = Ed[j];
+            const int n1 = tp.e_n1[e], n2 = tp.e_n2[e];
+            const int4 un = mw.un[e], dn = mw.dn[e];
+            const float4 wu = mw.wu[e], wd = mw.wd[e];
+            E.ia = n1 * L1;
+            E.ib = n2 * L1;
+            E.ua = un.y * L1;
+            E.ub = un.z * L1;
+            E.da = dn.y * L1;
+            E.db = dn.z * L1;
+            E.gmin = un.w & 0xffff;
+            E.gmax = un.w >> 16;
+            E.nbl1 = tp.n_nbl[n1];
+            E.nbl2 = tp.n_nbl[n2];
+            E.uy = wu.y;
+            E.uz = wu.z;
+            E.dy = wd.y;
+            E.dz = wd.z;
         }
-        compute(p, cur);
-        float *t = cur;
-        cur = nxt;
-        nxt = t;
+        S.fill(j, in ? tp.e_lo[e] : 1, in ? tp.e_hi[e] - tp.e_lo[e] + 1 : 0);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+        const int j = S.find(i), nz = S.top[j] + i - S.pre[j], k = nz - 1;
+        const EdgeH &E = Ed[j];
+        const bool tri = nz >= E.gmin && nz <= E.gmax - 1;
+        const int ie = (e0 + j) * L1 + k, ia = E.ia + k, ib = E.ib + k;
+        const int ua = E.ua + k, ub = E.ub + k, da = E.da + k, db = E.db + k;
+        const float v = VF[ie];
+        const float cl1 = (E.nbl1 - nz) >= 0 ? 1.f : 0.f, cl2 = (E.nbl2 - nz) >= 0 ? 1.f : 0.f;
+        const float4 wu = make_float4(0.f, E.uy, E.uz, 0.f), wd = make_float4(0.f, E.dy, E.dz, 0.f);
+#pragma unroll 1
+        for (int gq = 0; gq < B.ng; gq++) {
+            const int hor = B.hor[gq];
+            // MUSCL / MFCT levels outside the triangles' range: the node-mean launch
+            if (hor != 2 && !tri) continue;
+            const bool grad = hor != 2;
+            const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
+            const float *__restrict__ O1 = grp<G>(B.O1, gq, B.sN);
+            const float *__restrict__ O2 = B.ab == 3 ? grp<G>(B.O2, gq, B.sN) : O1;
+            const Vec<G> T1 = vld<G>(T, ia), T2 = vld<G>(T, ib);
+            const Vec<G> o1a = vld<G>(O1, ia), o1b = vld<G>(O1, ib);
+            const Vec<G> o2a = vldc<G>(B.ab == 3, O2, ia), o2b = vldc<G>(B.ab == 3, O2, ib);
+            const Vec<G> ga = vldc<G>(grad, T, ua), gb = vldc<G>(grad, T, ub);
+            const Vec<G> gc = vldc<G>(grad, T, da), gd = vldc<G>(grad, T, db);
+            vst<G>(grp<G>(B.ADh, gq, B.sE), ie,
+                   ho_group<G>(B, gq, hor, T1, T2, o1a, o1b, o2a, o2b, ga, gb, gc, gd, wu, wd, v, cl1, cl2));
+        }
     }
 }
 
-template <int G, bool PK, bool STG>
-__device__ __forceinline__ void ho_unit(const DTopo &tp, const B32View &B, const MusclW &mw,
-                                        const float *__restrict__ VF, int e, float *sb) {
-    const int lane = threadIdx.x & 31;
-    if (e >= tp.E2) return;
-    const int elo = tp.e_lo[e], ehi = tp.e_hi[e];
-    int nz0 = elo;
-    for (; nz0 + 32 <= ehi; nz0 += 32) {
-        if (STG) ho_pass_pf<G, false>(tp, B, mw, VF, e, nz0, 32, 1, lane, sb);
-        else ho_pass<G, false>(tp, B, mw, VF, e, nz0, 32, 1, lane);
-    }
-    const int W = ehi - nz0 + 1;
-    if (W < 1) return;
-    const int P = 32 / W;
-    if (STG) {
-        if (PK && P > 1) ho_pass_pf<G, true>(tp, B, mw, VF, e, nz0, W, P, lane, sb);
-        else ho_pass_pf<G, false>(tp, B, mw, VF, e, nz0, 32, 1, lane, sb);
-    } else {
-        if (PK && P > 1) ho_pass<G, true>(tp, B, mw, VF, e, nz0, W, P, lane);
-        else ho_pass<G, false>(tp, B, mw, VF, e, nz0, 32, 1, lane);
-    }
-}
-
-template <int G, bool STG>
-__global__ void __launch_bounds__(kTB, STG ? MinB<G>::ho_stg : MinB<G>::ho)
-k32_ho(DTopo tp, B32View B, MusclW mw, const float *__restrict__ VF) {
-    extern __shared__ __align__(16) float dsm[];
-    float *sb = STG ? dsm + (size_t)(threadIdx.x >> 5) * (stage_bytes_ho<G>() / 4) : nullptr;
-    FOR_WARP_UNITS(e, tp.E2) ho_unit<G, true, STG>(tp, B, mw, VF, e, sb);
+template <int G>
+__global__ void __launch_bounds__(kTileThreads, MinB<G>::ho)
+k32_ho(DTopo tp, B32View B, MusclW mw, const float *__restrict__ VF, int tile) {
+    __shared__ Tile S;
+    __shared__ EdgeH Ed[kTileMax];
+    ho_tile<G>(tp, B, mw, VF, blockIdx.x, tile, S, Ed);
 }
 
 // The edge-layers of the node-mean gradients: one thread per (edge, level) item, every
@@ -2681,11 +2624,12 @@ __device__ __forceinline__ int find_inst(const MultiIdx &ix, int u) {
     return lo;
 }
 
-__global__ void __launch_bounds__(kTB) k32m_vflux(const Inst32 *__restrict__ I, MultiIdx ix) {
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        vflux_edge(I[i].tp, I[i].g, I[i].f, I[i].VF, u - ix.start[i], threadIdx.x & 31);
-    }
+// units: tiles of kTileMax edges, one block each
+__global__ void __launch_bounds__(kTileThreads) k32m_vflux(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ Tile S;
+    __shared__ EdgeV Ed[kTileMax];
+    const int i = find_inst(ix, blockIdx.x);
+    vflux_tile(I[i].tp, I[i].g, I[i].f, I[i].VF, blockIdx.x - ix.start[i], kTileMax, S, Ed);
 }
 __global__ void __launch_bounds__(kTB) k32m_vfactors(const Inst32 *__restrict__ I, MultiIdx ix) {
     FOR_WARP_UNITS(u, ix.start[ix.n]) {
@@ -2705,12 +2649,12 @@ __global__ void __launch_bounds__(kTB, WIDE ? 1 : MinB<4>::lo) k32m_lo_ad(const 
             lo_ad_unit<2, WIDE, WS, true>(I[i].tp, I[i].g, I[i].f, I[i].B, I[i].VF, I[i].dt, u - ix.start[i], Se, nullptr);
     }
 }
-__global__ void __launch_bounds__(kTB, MinB<4>::ho) k32m_ho(const Inst32 *__restrict__ I, MultiIdx ix) {
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        if (I[i].B.G == 4) ho_unit<4, true, false>(I[i].tp, I[i].B, I[i].mw, I[i].VF, u - ix.start[i], nullptr);
-        else ho_unit<2, true, false>(I[i].tp, I[i].B, I[i].mw, I[i].VF, u - ix.start[i], nullptr);
-    }
+__global__ void __launch_bounds__(kTileThreads, MinB<4>::ho) k32m_ho(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ Tile S;
+    __shared__ EdgeH Ed[kTileMax];
+    const int i = find_inst(ix, blockIdx.x), ti = blockIdx.x - ix.start[i];
+    if (I[i].B.G == 4) ho_tile<4>(I[i].tp, I[i].B, I[i].mw, I[i].VF, ti, kTileMax, S, Ed);
+    else ho_tile<2>(I[i].tp, I[i].B, I[i].mw, I[i].VF, ti, kTileMax, S, Ed);
 }
 __global__ void __launch_bounds__(256) k32m_ho_nodemean(const Inst32 *__restrict__ I, MultiIdx ix) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2793,11 +2737,6 @@ __global__ void __launch_bounds__(kTB) k32m_diff(const Inst32 *__restrict__ I, M
 // ---------------------------------------------------------------------------
 // launch wrappers
 // ---------------------------------------------------------------------------
-static int grid32(int nent, int per_block) {
-    int b = (nent + per_block - 1) / per_block;
-    const int cap = 152 * 48;
-    return b > cap ? cap : (b < 1 ? 1 : b);
-}
 // warp-per-unit kernels: one warp per unit, or at most blocks_per_sm blocks per SM looping
 static int grid_units(int units, const LaunchShape &sh) {
     int b = (units + kWB - 1) / kWB;
@@ -2808,7 +2747,8 @@ static int grid_nodes(int n) { return (n + kWB - 1) / kWB; }
 static int grid_flat(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 32); }
 
 void b32_vflux(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, float *VF, cudaStream_t s) {
-    k32_vflux<<<grid32(tp.E2, kWB), kTB, 0, s>>>(tp, g, f, VF);
+    const int t = tile_size(tp.E2, 0);
+    k32_vflux<<<(tp.E2 + t - 1) / t, kTileThreads, 0, s>>>(tp, g, f, VF, t);
 }
 void b32_vfactors(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, double dt, const VFactors &v,
                   cudaStream_t s) {
@@ -2822,8 +2762,6 @@ template <int G>
 constexpr int smem_bounds() { return kWB * stage_bytes_bounds<G>(); }
 template <int G>
 constexpr int smem_update() { return kWB * stage_bytes_update<G>(); }
-template <int G>
-constexpr int smem_ho() { return kWB * stage_bytes_ho<G>(); }
 
 template <int G>
 static cudaError_t prepare_g() {
@@ -2836,7 +2774,6 @@ static cudaError_t prepare_g() {
     set((const void *)k32_bounds<G, false, true>, smem_bounds<G>());
     set((const void *)k32_update<G, false, true, false>, smem_update<G>());
     set((const void *)k32_update<G, false, true, true>, smem_update<G>());
-    set((const void *)k32_ho<G, true>, smem_ho<G>());
     return e;
 }
 bool b32_fct_clamp() { return kFctClamp; }
@@ -2894,8 +2831,9 @@ void b32_lo_ad(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
 template <int G>
 static void ho_g(const DTopo &tp, const B32View &B, const MusclW &mw, const float *VF, const LaunchShape &sh,
                  cudaStream_t s) {
-    if (sh.staged) k32_ho<G, true><<<grid_units(tp.E2, sh), kTB, smem_ho<G>(), s>>>(tp, B, mw, VF);
-    else k32_ho<G, false><<<grid_units(tp.E2, sh), kTB, 0, s>>>(tp, B, mw, VF);
+    (void)sh;
+    const int t = tile_size(tp.E2, 0);
+    k32_ho<G><<<(tp.E2 + t - 1) / t, kTileThreads, 0, s>>>(tp, B, mw, VF, t);
     if (mw.n_items) {
         int blocks = (mw.n_items + 255) / 256;
         if (blocks > 152 * 8) blocks = 152 * 8;
@@ -3031,7 +2969,7 @@ template void b32_unpack_group<double>(const float *, int, size_t, const SlotDst
 // multi-instance launch wrappers: ix_* hold the per-instance unit offsets of each stage
 void bm32_vflux(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
-    if (u) k32m_vflux<<<grid_nodes(u), kTB, 0, s>>>(I, ix);
+    if (u) k32m_vflux<<<u, kTileThreads, 0, s>>>(I, ix);
 }
 void bm32_vfactors(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
@@ -3061,7 +2999,7 @@ void bm32_vdiff_w(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     if (u) k32m_vdiff_w<<<(u + 127) / 128, 128, 0, s>>>(I, ix);
 }
 void bm32_ho(const Inst32 *I, const MultiIdx &ix_e, const MultiIdx &ix_items, cudaStream_t s) {
-    if (ix_e.start[ix_e.n]) k32m_ho<<<grid_nodes(ix_e.start[ix_e.n]), kTB, 0, s>>>(I, ix_e);
+    if (ix_e.start[ix_e.n]) k32m_ho<<<ix_e.start[ix_e.n], kTileThreads, 0, s>>>(I, ix_e);
     const int u = ix_items.start[ix_items.n];
     if (u) k32m_ho_nodemean<<<(u + 255) / 256, 256, 0, s>>>(I, ix_items);
 }
