@@ -79,9 +79,8 @@ struct fesom_gpu_ctx {
     float *Rp32 = nullptr, *Rm32 = nullptr, *Bp32 = nullptr, *Bm32 = nullptr;
     float *pack_in = nullptr, *pack_out = nullptr;  // staging of the host-array step (FP32 columns)
     size_t pack_n = 0;                   // floats each staging buffer holds
-    // lo_ad, ho, bounds, update (the autotuner's choice); lo_ad stages its gathers in shared
-    // memory by default, bounds and update keep them in registers
-    LaunchShape shape[4] = {{0, true}, {0, false}, {0, false}, {0, false}};
+    // lo_ad, ho, bounds, update (the autotuner's choice)
+    LaunchShape shape[4] = {{0, 1}, {}, {}, {}};
     MusclW mw{};
     cudaGraphExec_t gexec32[3] = {nullptr, nullptr, nullptr};
     double g32_dt[3] = {0.0, 0.0, 0.0};
@@ -666,7 +665,6 @@ int alloc_state32(fesom_gpu_ctx *ctx, int ab) {
     if (clamp && (rc = dalloc(ctx, (void **)&ctx->Bm32, wg * sN))) return rc;
     if (ctx->Ki && (rc = dalloc(ctx, (void **)&ctx->HD32, wg * sE))) return rc;
     // created here, not on first use: a first step may run inside a stream capture
-    CK(b32_prepare());
     if (!ctx->side) {
         CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
@@ -943,11 +941,11 @@ int launches_per_step(fesom_gpu_ctx *ctx) {
         for (int g0 = 0; g0 < ctx->ngr; g0 += ctx->group) {
             const int ng = std::min(ctx->group, ctx->ngr - g0);
             const B32View B = view32(ctx, g0, ng);
-            // lo_ad, update (+ bounds), launched again for the wide nodes; ho (+ its node-mean
+            // lo_ad, update (+ bounds); diff, launched again for the wide nodes; ho (+ its node-mean
             // edge-layers); vdiff
             const int wide = ctx->tp.n_wide ? 2 : 1;
             auto passes = [&](int k) { return (ng + stage_group(ctx, k, ng) - 1) / stage_group(ctx, k, ng); };
-            n += wide * (passes(0) + passes(3) + (B.fct ? passes(2) : 0) + (B.diff ? 1 : 0)) +
+            n += passes(0) + passes(3) + (B.fct ? passes(2) : 0) + wide * (B.diff ? 1 : 0) +
                  passes(1) * (ctx->mw.n_items ? 2 : 1) + (((B.ivd & ~B.wimpl) && ctx->shape[3].vsep) ? 1 : 0) +
                  (ctx->Ki ? 1 : 0) +
                  (B.ppm ? 1 : 0) + ((ctx->wsplit && B.fct) ? 1 : 0) + (B.wimpl ? 1 : 0);
@@ -1115,6 +1113,23 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
         tp.n_wide = (int)wide.size();
         tp.wide_nodes = nullptr;
         if (!wide.empty() && (rc = upload_int(ctx, &tp.wide_nodes, wide))) return rc;
+    }
+    // tiles of consecutive nodes for the FP32 node kernels
+    tp.n_nt = 0;
+    tp.nt_ptr = nullptr;
+    if (precision == FESOM_PREC_FP32) {
+        std::vector<int> cut(1, 0);
+        for (int n = 0, lev = 0; n < ctx->N2; n++) {
+            const int m = h.n_nlev[n] - h.n_ulev[n];
+            if (n > cut.back() && (lev + m > kNodeTileLevels || n - cut.back() == kNodeTileNodes)) {
+                cut.push_back(n);
+                lev = 0;
+            }
+            lev += m;
+        }
+        cut.push_back(ctx->N2);
+        tp.n_nt = (int)cut.size() - 1;
+        if ((rc = upload_int(ctx, &tp.nt_ptr, cut))) return rc;
     }
     ctx->stage_n = std::min<size_t>((size_t)16 << 20, std::max<size_t>(2 * (size_t)ctx->L1 * ctx->T2, (size_t)ctx->nl * ctx->N2));
     if ((rc = dalloc(ctx, (void **)&ctx->stage, ctx->stage_n * sizeof(double)))) return rc;
@@ -1725,7 +1740,7 @@ int fesom_gpu_set_launch_shape(fesom_gpu_ctx *ctx, int32_t stage, int32_t blocks
 
 int fesom_gpu_set_stage_variant(fesom_gpu_ctx *ctx, int32_t stage, int32_t variant) {
     if (!ctx || stage < 0 || stage > 3 || variant < 0 || variant > (stage == 3 ? 3 : 1)) return FESOM_ERR_ARG;
-    ctx->shape[stage].staged = (variant & 1) != 0;
+    ctx->shape[stage].variant = variant & 1;
     ctx->shape[stage].vsep = (variant & 2) != 0;
     free_graphs32(ctx);
     return FESOM_OK;
@@ -1746,7 +1761,7 @@ struct TuneSetting {
     bool operator==(const TuneSetting &o) const {
         for (int k = 0; k < 4; k++)
             if (stage_tr[k] != o.stage_tr[k] || shape[k].blocks_per_sm != o.shape[k].blocks_per_sm ||
-                shape[k].staged != o.shape[k].staged || shape[k].vsep != o.shape[k].vsep)
+                shape[k].variant != o.shape[k].variant || shape[k].vsep != o.shape[k].vsep)
                 return false;
         return true;
     }
@@ -1805,7 +1820,7 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
     CK(cudaEventCreate(&e1));
     const TuneSetting start = get_setting(ctx);
     TuneSetting def{};
-    def.shape[0].staged = true;  // the library defaults: lo_ad staged, the rest in registers
+    def.shape[0].variant = 1;  // the library defaults
     int ncand = 0;
     float def_ms = 0.f, best_ms = 0.f;
     put_setting(ctx, def);
@@ -1825,14 +1840,13 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
     const int bps[] = {0, 2, 4};
     for (int k = 0; k < 4 && !rc; k++) {
         // the update: also with the vertical diffusion as its own launch
-        const int nvar = k == 3 ? 4 : 2;
+        const int nvar = k == 3 ? 2 : 1;
         const int ntrs = (k >= 2 && ntr_slots > 8) ? 2 : 1;
         for (int v = 0; v < nvar && !rc; v++)
             for (int b : bps)
                 for (int q = 0; q < ntrs && !rc; q++) {
                     TuneSetting c = best;
-                    c.shape[k].staged = (v & 1) != 0;
-                    c.shape[k].vsep = (v & 2) != 0;
+                    c.shape[k].vsep = v != 0;
                     c.shape[k].blocks_per_sm = b;
                     c.stage_tr[k] = q ? 8 : 0;
                     if (c == best) continue;
@@ -1858,7 +1872,7 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
     for (int k = 0; k < 4; k++) {
         res->stage_tracers[k] = best.stage_tr[k];
         res->blocks_per_sm[k] = best.shape[k].blocks_per_sm;
-        res->variant[k] = (best.shape[k].staged ? 1 : 0) | (best.shape[k].vsep ? 2 : 0);
+        res->variant[k] = best.shape[k].variant | (best.shape[k].vsep ? 2 : 0);
     }
     return FESOM_OK;
 }
@@ -2371,7 +2385,7 @@ struct fesom_gpu_batch {
     cudaStream_t stream = nullptr;
     Inst32 *d_inst = nullptr;  // ab descriptor sets (one per rotation phase), inst.size() each
     double d_dt = -1.0;
-    MultiIdx ix_e{}, ix_et{}, ix_n{}, ix_w{}, ix_it{};  // edges, edge tiles, nodes, wide nodes, node-mean items
+    MultiIdx ix_e{}, ix_et{}, ix_n{}, ix_nt{}, ix_w{}, ix_it{};  // edges, edge tiles, nodes, node tiles, wide nodes, node-mean items
     int maxL1 = 0;
     bool any_vd = false, any_fct = false, any_hd = false, any_diff = false;
     bool any_ws = false, any_ppm = false, any_lo_impl = false, any_wimpl = false;
@@ -2429,8 +2443,7 @@ void enqueue_batch_step(fesom_gpu_batch *b, cudaStream_t s) {
     const bool wide = b->ix_w.start[b->ix_w.n] > 0;
     bm32_vflux(I, b->ix_et, s);
     if (b->any_vd) bm32_vfactors(I, b->ix_n, s);
-    bm32_lo_ad(I, b->ix_n, false, b->any_ws, s);
-    if (wide) bm32_lo_ad(I, b->ix_w, true, b->any_ws, s);
+    bm32_lo_ad(I, b->ix_nt, b->any_ws, s);
     if (b->any_ppm) bm32_vppm(I, b->ix_n, s);
     if (b->any_lo_impl) bm32_lo_impl(I, b->ix_n, s);
     bm32_ho(I, b->ix_et, b->ix_it, s);
@@ -2439,13 +2452,9 @@ void enqueue_batch_step(fesom_gpu_batch *b, cudaStream_t s) {
         bm32_diff(I, b->ix_n, false, s);
         if (wide) bm32_diff(I, b->ix_w, true, s);
     }
-    if (b->any_fct) {
-        bm32_bounds(I, b->ix_n, false, s);
-        if (wide) bm32_bounds(I, b->ix_w, true, s);
-    }
-    // (the implicit vertical diffusion runs inside the update, per node)
-    bm32_update(I, b->ix_n, false, s);
-    if (wide) bm32_update(I, b->ix_w, true, s);
+    if (b->any_fct) bm32_bounds(I, b->ix_nt, s);
+    // (the implicit vertical diffusion runs inside the update, per tile)
+    bm32_update(I, b->ix_nt, s);
     if (b->any_wimpl) bm32_vdiff_w(I, b->ix_n, s);
 }
 
@@ -2462,7 +2471,7 @@ int fesom_gpu_batch_create(fesom_gpu_ctx *const *ctxs, int32_t n, fesom_gpu_batc
         b->err = "a batch holds 1 to 64 FP32 contexts";
         return FESOM_ERR_ARG;
     }
-    std::vector<int> ce, cet, cn, cw, cit;
+    std::vector<int> ce, cet, cn, cnt, cw, cit;
     for (int i = 0; i < n; i++) {
         fesom_gpu_ctx *c = ctxs[i];
         if (!c || c->prec != FESOM_PREC_FP32) { b->err = "batch instances must be FP32 contexts"; return FESOM_ERR_ARG; }
@@ -2497,12 +2506,14 @@ int fesom_gpu_batch_create(fesom_gpu_ctx *const *ctxs, int32_t n, fesom_gpu_batc
         ce.push_back(c->E2);
         cet.push_back((c->E2 + kTileMax - 1) / kTileMax);
         cn.push_back(c->N2);
+        cnt.push_back(c->tp.n_nt);
         cw.push_back(c->tp.n_wide);
         cit.push_back(c->mw.n_items);
     }
     set_prefix(b->ix_e, ce);
     set_prefix(b->ix_et, cet);
     set_prefix(b->ix_n, cn);
+    set_prefix(b->ix_nt, cnt);
     set_prefix(b->ix_w, cw);
     set_prefix(b->ix_it, cit);
     BCK(cudaMalloc((void **)&b->d_inst, sizeof(Inst32) * (size_t)n * b->ab));
@@ -2566,10 +2577,9 @@ int fesom_gpu_batch_run_steps(fesom_gpu_batch *b, double dt, int32_t nsteps, int
 int fesom_gpu_batch_launches_per_step(fesom_gpu_batch *b, int32_t *launches) {
     if (!b || !launches) return FESOM_ERR_ARG;
     const bool wide = b->ix_w.start[b->ix_w.n] > 0;
-    const int k = wide ? 2 : 1;
-    // vflux, vfactors (the diffusion itself runs inside the update), lo_ad and update (+ bounds,
-    // diff) per node range, ho (+ its node-mean items), the optional stages
-    int n = 1 + (b->any_vd ? 1 : 0) + k * (2 + (b->any_fct ? 1 : 0) + (b->any_diff ? 1 : 0)) + 1 +
+    // vflux, vfactors (the diffusion itself runs inside the update), lo_ad and update (+ bounds),
+    // diff per node range, ho (+ its node-mean items), the optional stages
+    int n = 1 + (b->any_vd ? 1 : 0) + 2 + (b->any_fct ? 1 : 0) + (b->any_diff ? (wide ? 2 : 1) : 0) + 1 +
             (b->ix_it.start[b->ix_it.n] ? 1 : 0) + (b->any_hd ? 1 : 0) + (b->any_ppm ? 1 : 0) +
             (b->any_lo_impl ? 1 : 0) + (b->any_wimpl ? 1 : 0);
     *launches = n;

@@ -33,6 +33,9 @@ struct DTopo {
     const int *nie_ptr, *nie_idx;  // node -> element, ascending element order
     int n_wide;                    // nodes of more than 8 edges (FP32 form: their own launch)
     const int *wide_nodes;
+    // FP32 form: node tile i holds the nodes nt_ptr[i] .. nt_ptr[i + 1] - 1 (tile.cuh)
+    int n_nt;
+    const int *nt_ptr;
     // every element lies on exactly three edges and in the element lists of exactly its three nodes
     int ring_ok;
 };
@@ -153,21 +156,17 @@ struct MusclW {
 struct VFactors {
     float *a, *c, *inv, *cp;
 };
-// once per process, before the first FP32 step (not inside a stream capture): the shared-memory
-// limits of the node kernels that stage their gathers
-cudaError_t b32_prepare();
 // whether the build clamps advected values into their stored FCT bounds (FESOM_FCT_CLAMP); the
 // bound arrays exist only then
 bool b32_fct_clamp();
 void b32_vflux(const DTopo &, const DGeom<float> &, const DForcing<float> &, float *VF, cudaStream_t);
 void b32_vfactors(const DTopo &, const DGeom<float> &, const DForcing<float> &, double dt, const VFactors &,
                   cudaStream_t);
-// launch shape of the node/edge stages (the autotuner's choices): blocks of 8 warps, at most
-// `blocks_per_sm` x 152 blocks (grid-stride loops over the units; 0: one warp per unit), and
-// for lo_ad, bounds and update the kernel variant
+// launch shape of the node stages (the autotuner's choices): at most `blocks_per_sm` x 152 blocks
+// looping over the tiles (0: one block per tile)
 struct LaunchShape {
     int blocks_per_sm = 0;
-    bool staged = false;  // node stages: gathers staged in shared memory (cp.async) instead of registers
+    int variant = 0;      // bit 0 of fesom_gpu_set_stage_variant (kept and reported; one kernel per stage)
     bool vsep = false;    // the update stage: the implicit vertical diffusion as its own kernel
 };
 void b32_lo_ad(const DTopo &, const DGeom<float> &, const DForcing<float> &, const B32View &, const float *VF,
@@ -240,15 +239,15 @@ struct MultiIdx {
     int n;
     int start[kMaxInst + 1];
 };
-void bm32_vflux(const Inst32 *, const MultiIdx &, cudaStream_t);
+void bm32_vflux(const Inst32 *, const MultiIdx &edge_tiles, cudaStream_t);
 void bm32_vfactors(const Inst32 *, const MultiIdx &, cudaStream_t);
-void bm32_lo_ad(const Inst32 *, const MultiIdx &nodes, bool wide, bool ws, cudaStream_t);
+void bm32_lo_ad(const Inst32 *, const MultiIdx &node_tiles, bool ws, cudaStream_t);
 void bm32_vppm(const Inst32 *, const MultiIdx &nodes, cudaStream_t);
 void bm32_lo_impl(const Inst32 *, const MultiIdx &nodes, cudaStream_t);
 void bm32_vdiff_w(const Inst32 *, const MultiIdx &nodes, cudaStream_t);
-void bm32_ho(const Inst32 *, const MultiIdx &edges, const MultiIdx &items, cudaStream_t);
-void bm32_bounds(const Inst32 *, const MultiIdx &, bool wide, cudaStream_t);
-void bm32_update(const Inst32 *, const MultiIdx &, bool wide, cudaStream_t);
+void bm32_ho(const Inst32 *, const MultiIdx &edge_tiles, const MultiIdx &items, cudaStream_t);
+void bm32_bounds(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
+void bm32_update(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 void bm32_hdiff(const Inst32 *, const MultiIdx &edges, cudaStream_t);
 void bm32_diff(const Inst32 *, const MultiIdx &nodes, bool wide, cudaStream_t);
 

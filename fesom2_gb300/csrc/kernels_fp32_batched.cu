@@ -87,36 +87,20 @@ constexpr int kWB = 8;                // warps (= nodes) per block
 constexpr int kTB = 32 * kWB;
 constexpr unsigned kFull = 0xffffffffu;
 
-// resident blocks per SM each group kernel is built for (registers: 65536 / (256 * blocks))
+// resident blocks per SM each group kernel is built for (registers: 65536 / (threads * blocks)),
+// and the edge slots whose gathers bounds (ub) and update (uu) keep in flight at once: the fastest
+// of sweeps over 2 to 6 blocks and 1 to 6 slots on the 640k-node seamount channel (G = 2), the
+// sphere of 8 subdivisions with 24 tracers and the one of 7 with 7 tracers (G = 4).  ms per step:
+//   ho     G=2: 1.62 (5 blocks) 1.00 (8) 0.94 (9) 1.04 (10) 1.20 (12); G=4: 4.00 (5) 4.02 (6) 4.70 (8)
+//   lo     G=2: 1.30 (4) 1.34 (5) 1.40 (6); G=4: 4.30 (2) 3.64 (3) 3.60 (4) 4.34 (5)
+//   bounds G=2: 1.15 (5 x 2 slots) 1.21 (4 x 3) 1.30 (4 x 6); G=4: 5.54 (4 x 3) 5.84 (3 x 3) 6.26 (4 x 2)
+//   update G=2: 1.70 (5 x 1) 1.76 (5 x 2) 1.98 (4 x 6); G=4: 7.16 (3 x 2) 7.55 (4 x 2) 8.17 (3 x 3)
 template <int G>
 struct MinB {
-    // the LO stage: three blocks per SM (the staged variant's double buffer fits 3 x 74 KB);
-    // two measured 1.3 ms slower per step on the 24-tracer sphere, though its own launch is faster
-#ifdef FESOM_MINB_LO
-    static constexpr int lo = FESOM_MINB_LO;
-#else
-    static constexpr int lo = 3;
-#endif
-#ifdef FESOM_MINB_HO
-    static constexpr int ho = FESOM_MINB_HO;
-#else
-    static constexpr int ho = G == 4 ? 6 : 8;  // blocks of kTileThreads
-#endif
-    // bounds and update: gathers in registers (three blocks of eight warps per SM measured
-    // faster than two with more registers or one with the whole pass in flight), or staged in
-    // shared memory (which holds one block of the G = 4 staging per SM)
-    static constexpr int node_reg = 3;
-    static constexpr int node_stg = G == 4 ? 1 : 2;
-#ifdef FESOM_MINB_UPDATE_REG
-    static constexpr int update_reg = FESOM_MINB_UPDATE_REG;
-#else
-    static constexpr int update_reg = node_reg;
-#endif
-#ifdef FESOM_MINB_BOUNDS_REG
-    static constexpr int bounds_reg = FESOM_MINB_BOUNDS_REG;
-#else
-    static constexpr int bounds_reg = node_reg;
-#endif
+    static constexpr int lo = 4;
+    static constexpr int ho = G == 4 ? 6 : 9;  // blocks of kTileThreads
+    static constexpr int bounds = G == 4 ? 4 : 5, ub = G == 4 ? 3 : 2;
+    static constexpr int update = G == 4 ? 3 : 5, uu = G == 4 ? 2 : 1;
 };
 
 __device__ __forceinline__ size_t i1(int nz, int n, int L1) { return (size_t)n * L1 + (nz - 1); }
@@ -443,46 +427,6 @@ __device__ __forceinline__ float *grp(float *base, int g, size_t count) {
     return base + (size_t)g * count * G;
 }
 
-// ---------------------------------------------------------------------------
-// per-lane asynchronous staging of a pass's gathers in shared memory
-// ---------------------------------------------------------------------------
-// The node stages gather, per pass (one chunk of a column for one tracer group), a few dozen
-// entries per lane: the node's own and every neighbour's.  Held in registers, only a part of
-// them can be in flight at once; staged with cp.async (one G-float copy per lane and entry,
-// zero-filled where the lane has nothing to gather) they all are, and the next pass's copies
-// run while the current pass computes.  Each lane reads back only what it copied, so the
-// staging needs no barrier: cp.async.wait_group orders a lane's copies before its reads.
-// Staging of a warp: [2 buffers][NS entries][32 lanes][G floats].
-template <int G>
-__device__ __forceinline__ void cpa(float *sdst, const float *gsrc, bool pred) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
-    const size_t a = __cvta_generic_to_global(gsrc);
-    if constexpr (G == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(a), "r"(pred ? 16 : 0) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(a), "r"(pred ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpa_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-// entry s of the lane in a staging buffer
-template <int G>
-__device__ __forceinline__ float *stg(float *buf, int s, int lane) {
-    return buf + ((size_t)s * 32 + lane) * G;
-}
-template <int G>
-__device__ __forceinline__ Vec<G> lds(const float *p) {
-    if constexpr (G == 4) {
-        const float4 q = *reinterpret_cast<const float4 *>(p);
-        return Vec<4>{{q.x, q.y, q.z, q.w}};
-    } else {
-        const float2 q = *reinterpret_cast<const float2 *>(p);
-        return Vec<2>{{q.x, q.y}};
-    }
-}
-
 // Adams-Bashforth value minus the current value: AB2 -(0.5+eps) T^{n-1} + (1.5+eps) T^n,
 // AB3 (23 T^n - 16 T^{n-1} + 5 T^{n-2}) / 12 (oce_tracer_mod.F90:53, 67-68), eps = 0.1
 __device__ __forceinline__ float ab_delta(int ab, float t, float o1, float o2) {
@@ -494,38 +438,6 @@ __device__ __forceinline__ float ab_delta(int ab, float t, float o1, float o2) {
 // summed: the rounding k32_lo_ad's node sums use for the same flux
 __device__ __forceinline__ float upw_flux(float T1, float T2, float v) {
     return -__fadd_rn(__fmul_rn(T1, fmaxf(v, 0.f)), __fmul_rn(T2, fminf(v, 0.f)));
-}
-
-// vertical high-order flux of interface nz on the AB values (QR4C / UPW1 / CDIFF,
-// oce_adv_tra_ver.F90:332-434, 635-695) minus the LO flux, for one slot
-__device__ __forceinline__ float ver_ad(int ver, bool lim, float pv, int nz, int nzmin, int nzmax, bool twolayer,
-                                        float tab, float tabu, float tabu2, float tabd, float pw, float ar0, float fv0,
-                                        float fw0, float idz0, float idzp, float idzm, float g1, float g2) {
-    float Cf;
-    if (nz == nzmin) {
-        Cf = -(tab * pw * ar0);
-    } else if (ver != 0 || nz == nzmin + 1 || nz == nzmax - 1) {
-        if (ver != 1) {  // QR4C next to the ends, CDIFF everywhere
-            Cf = -(0.5f * (tabu + tab) * pw * ar0);
-        } else {
-            const float aw = fabsf(pw);
-            Cf = -(0.5f * (tab * (pw + aw) + tabu * (pw - aw)) * ar0);
-        }
-    } else {
-        const float qc = (tabu - tab) * idz0;
-        const float qu = (tab - tabd) * idzp;
-        const float qd = (tabu2 - tabu) * idzm;
-        const float Tm1 = tab + (2.f * qc + qu) * g1;
-        const float Tm2 = tabu + (2.f * qc + qd) * g2;
-        const float aw = fabsf(pw);
-        const float Tmean = (pw + aw) * Tm1 + (pw - aw) * Tm2;
-        Cf = (-(0.5f * (1.f - pv) * Tmean) - pv * (0.5f * (Tm1 + Tm2)) * pw) * ar0;
-    }
-    // flux = C - flux_in; FCT passes the LO flux in, otherwise zero
-    float F = Cf - (lim ? fw0 : 0.f);
-    // a two-layer column writes its middle interface twice (statements nzmin+1, nzmax-1)
-    if (ver == 0 && twolayer && nz == nzmin + 1) F = Cf - F;
-    return lim ? F : F - fv0;
 }
 
 // Packed FP32 pairs: two slots of a group in one instruction (Blackwell's two-wide FP32 add,
@@ -541,401 +453,272 @@ __device__ __forceinline__ float2 pr(const Vec<G> &a, int j) {
     return make_float2(a.c[2 * j], a.c[2 * j + 1]);
 }
 
-// The per-group arithmetic of k32_lo_ad for two slots at once: the AB value, the upwind
-// vertical flux with w_e, LO from the edge-flux sum hs, and the vertical antidiffusive flux
-// (ver_ad's branches, taken per lane and group, so both slots of a pair share them).
+// The per-group arithmetic of k32_lo_ad for two slots at once, from the values of the column's
+// neighbouring layers: the upwind vertical flux with w_e, LO from the edge-flux sum hs, and the
+// vertical antidiffusive flux (QR4C / UPW1 / CDIFF, oce_adv_tra_ver.F90:332-434, 635-695; the
+// branches are taken per lane and group, so both slots of a pair share them).
+// adv_tra_ver_upw1's flux of an interface with velocity w and area ar
+__device__ __forceinline__ float2 upw_pair(float2 tn, float2 Tu, float w, float ar, bool top) {
+    if (top) return pmul(tn, pk(-(w * ar)));
+    const float aw = fabsf(w);
+    return pmul(pfma(tn, pk(w + aw), pmul(Tu, pk(w - aw))), pk(-0.5f * ar));
+}
+struct LoLane {  // tracer-independent data of a node-layer
+    int nz, nzmin, nzmax;
+    float ar0, we0, w0, ar1, we1, sdt, dhr, idz0, idzp, idzm, g1, g2;
+};
 template <bool WS>
-__device__ __forceinline__ void lo_ad_pair(const DForcing<float> &f, int ab, int ver, bool lim, bool lvt, float2 pv,
-                                           int nz, int nzmin, int nzmax, bool twolayer, float ar0, float we0, float w0,
-                                           float sdt, float dhr, float idz0, float idzp, float idzm, float g1,
-                                           float g2, float2 tn, float2 o1, float2 o2, float2 hs, float2 &lo,
-                                           float2 &ad) {
-    float2 tab = tn;
-    if (lvt)
-        tab = ab == 2 ? pfma(pk(0.6f), psub(tn, o1), tn)
-                      : pfma(pfma(pk(11.f), psub(tn, o1), pmul(pk(-5.f), psub(o1, o2))), pk(1.f / 12.f), tn);
-    const float2 Tu = make_float2(sh_up(tn.x, 1), sh_up(tn.y, 1));
-    const float2 tabu = make_float2(sh_up(tab.x, 1), sh_up(tab.y, 1));
-    const float2 tabu2 = make_float2(sh_up(tab.x, 2), sh_up(tab.y, 2));
-    const float2 tabd = make_float2(sh_dn(tab.x, 1), sh_dn(tab.y, 1));
-    float2 fv0 = pk(0.f);
-    if (lvt) {
-        if (nz == nzmin) {
-            fv0 = pmul(tn, pk(-(we0 * ar0)));
-        } else {
-            const float aw = fabsf(we0);
-            fv0 = pmul(pfma(tn, pk(we0 + aw), pmul(Tu, pk(we0 - aw))), pk(-0.5f * ar0));
-        }
-    }
-    float2 fv1 = make_float2(sh_dn(fv0.x, 1), sh_dn(fv0.y, 1));
-    if (nz == nzmax - 1) fv1 = pk(0.f);
-    lo = padd(tn, pfma(tn, pk(dhr), pmul(padd(hs, psub(fv0, fv1)), pk(sdt))));
+__device__ __forceinline__ void lo_ad_pair(const DForcing<float> &f, int ver, bool lim, float2 pv, const LoLane &k,
+                                           float2 tn, float2 Tu, float2 Td, float2 tab, float2 tabu, float2 tabu2,
+                                           float2 tabd, float2 hs, float2 &lo, float2 &ad) {
+    const int nz = k.nz;
+    const bool top = nz == k.nzmin;
+    const float2 fv0 = upw_pair(tn, Tu, k.we0, k.ar0, top);
+    const float2 fv1 = nz == k.nzmax - 1 ? pk(0.f) : upw_pair(Td, tn, k.we1, k.ar1, false);
+    lo = padd(tn, pfma(tn, pk(k.dhr), pmul(padd(hs, psub(fv0, fv1)), pk(k.sdt))));
     float2 fw0 = fv0;
-    if (WS && f.wsplit && lvt) {
-        if (nz == nzmin) {
-            fw0 = pmul(tn, pk(-(w0 * ar0)));
-        } else {
-            const float aw = fabsf(w0);
-            fw0 = pmul(pfma(tn, pk(w0 + aw), pmul(Tu, pk(w0 - aw))), pk(-0.5f * ar0));
-        }
-    }
-    const float pw = lim ? w0 : we0;
+    if (WS && f.wsplit) fw0 = upw_pair(tn, Tu, k.w0, k.ar0, top);
+    const float pw = lim ? k.w0 : k.we0;
     float2 Cf;
-    if (nz == nzmin) {
-        Cf = pmul(tab, pk(-(pw * ar0)));
-    } else if (ver != 0 || nz == nzmin + 1 || nz == nzmax - 1) {
+    if (top) {
+        Cf = pmul(tab, pk(-(pw * k.ar0)));
+    } else if (ver != 0 || nz == k.nzmin + 1 || nz == k.nzmax - 1) {
         if (ver != 1) {
-            Cf = pmul(padd(tabu, tab), pk(-0.5f * pw * ar0));
+            Cf = pmul(padd(tabu, tab), pk(-0.5f * pw * k.ar0));
         } else {
             const float aw = fabsf(pw);
-            Cf = pmul(pfma(tab, pk(pw + aw), pmul(tabu, pk(pw - aw))), pk(-0.5f * ar0));
+            Cf = pmul(pfma(tab, pk(pw + aw), pmul(tabu, pk(pw - aw))), pk(-0.5f * k.ar0));
         }
     } else {
-        const float2 qc = pmul(psub(tabu, tab), pk(idz0));
-        const float2 qu = pmul(psub(tab, tabd), pk(idzp));
-        const float2 qd = pmul(psub(tabu2, tabu), pk(idzm));
-        const float2 Tm1 = pfma(pfma(pk(2.f), qc, qu), pk(g1), tab);
-        const float2 Tm2 = pfma(pfma(pk(2.f), qc, qd), pk(g2), tabu);
+        const float2 qc = pmul(psub(tabu, tab), pk(k.idz0));
+        const float2 qu = pmul(psub(tab, tabd), pk(k.idzp));
+        const float2 qd = pmul(psub(tabu2, tabu), pk(k.idzm));
+        const float2 Tm1 = pfma(pfma(pk(2.f), qc, qu), pk(k.g1), tab);
+        const float2 Tm2 = pfma(pfma(pk(2.f), qc, qd), pk(k.g2), tabu);
         const float aw = fabsf(pw);
         const float2 Tmean = pfma(pk(pw + aw), Tm1, pmul(pk(pw - aw), Tm2));
         // (-(0.5 (1 - pv) Tmean) - pv (0.5 (Tm1 + Tm2)) pw) ar0
         const float2 a1 = pmul(pk(-0.5f), psub(pk(1.f), pv)), a2 = pmul(pk(-0.5f * pw), pv);
-        Cf = pmul(pfma(a1, Tmean, pmul(a2, padd(Tm1, Tm2))), pk(ar0));
+        Cf = pmul(pfma(a1, Tmean, pmul(a2, padd(Tm1, Tm2))), pk(k.ar0));
     }
+    // flux = C - flux_in; FCT passes the LO flux in, otherwise zero
     float2 F = lim ? psub(Cf, fw0) : Cf;
-    if (ver == 0 && twolayer && nz == nzmin + 1) F = psub(Cf, F);
+    // a two-layer column writes its middle interface twice (statements nzmin+1, nzmax-1)
+    if (ver == 0 && k.nzmin + 1 == k.nzmax - 1 && nz == k.nzmin + 1) F = psub(Cf, F);
     ad = lim ? F : psub(F, fv0);
 }
 
 // ---------------------------------------------------------------------------
+// tiles of nodes
+// ---------------------------------------------------------------------------
+// A block takes a tile of consecutive whole columns with at most 256 wet layers in all (tiles cut
+// once per mesh), one layer per thread, and keeps the layer's geometry, neighbour offsets and
+// volume fluxes in registers for every tracer group of the launch.  The layers above and below
+// sit in the neighbouring threads: they pass through shared memory, double-buffered over the
+// groups, so a group costs one barrier.  Nothing is computed twice (a warp per column needs 3 of
+// 32 lanes as halo and leaves the rest of a column's last chunk idle: 47 layers filled 73 % of
+// two chunks), and a node's edge list is read once per tile into shared memory.
+constexpr int kNT = kNodeTileLevels;  // threads
+constexpr int kND = 6;                // edge slots of a node that k32_lo_ad holds in registers
+constexpr int kSlots = kMaxDeg + 2;   // slots of a node in a tile: the last pass over ub or uu slots may run past kMaxDeg
+struct NodeTile {
+    int n0, cnt, total, degmax;
+    int pre[kNodeTileNodes + 1], top[kNodeTileNodes], deg[kNodeTileNodes];
+    // slot u of node j: first entry of the other end's column, of the edge's column, the edge's
+    // levels lo | hi << 16, and whether the node is edges(1, e)
+    int4 slot[kNodeTileNodes][kSlots];
+    __device__ __forceinline__ int find(int i) const {
+        int j = i >= pre[16] ? 16 : 0;
+        j += i >= pre[j + 8] ? 8 : 0;
+        j += i >= pre[j + 4] ? 4 : 0;
+        j += i >= pre[j + 2] ? 2 : 0;
+        return j + (i >= pre[j + 1] ? 1 : 0);
+    }
+};
+
+// every thread of the block; the tile's data are visible after it
+__device__ __forceinline__ void node_tile_load(const DTopo &tp, int ti, NodeTile &S) {
+    const int n0 = tp.nt_ptr[ti], cnt = tp.nt_ptr[ti + 1] - n0;
+    if (threadIdx.x < 32) {
+        const int j = threadIdx.x, n = n0 + j;
+        const bool in = j < cnt;
+        int s = in ? tp.n_nlev[n] - tp.n_ulev[n] : 0;
+        S.top[j] = in ? tp.n_ulev[n] : 1;
+        const int deg = in ? min(tp.ne_ptr[n + 1] - tp.ne_ptr[n], kMaxDeg) : 0;
+        S.deg[j] = deg;
+        const int dm = __reduce_max_sync(kFull, deg);
+        if (j == 0) S.degmax = dm;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, s, o);
+            if (j >= o) s += v;
+        }
+        S.pre[j + 1] = s;
+        if (j == 0) {
+            S.pre[0] = 0;
+            S.n0 = n0;
+            S.cnt = cnt;
+        }
+        if (j == 31) S.total = s;
+    }
+    for (int s = threadIdx.x; s < cnt * kMaxDeg; s += kNT) {
+        const int j = s / kMaxDeg, u = s % kMaxDeg;
+        const int k = tp.ne_ptr[n0 + j] + u;
+        if (k >= tp.ne_ptr[n0 + j + 1]) continue;
+        const int code = tp.ne_idx[k], e = code >= 0 ? code : ~code;
+        const int m = code >= 0 ? tp.e_n2[e] : tp.e_n1[e];
+        S.slot[j][u] = make_int4(m * tp.L1, e * tp.L1, tp.e_lo[e] | tp.e_hi[e] << 16, code >= 0);
+    }
+    __syncthreads();
+}
+
+// the thread's layer of a tile
+struct TileLane {
+    bool on;
+    int j, n, nz, nzmin, nzmax, i, iv;
+    __device__ __forceinline__ TileLane(const DTopo &tp, const NodeTile &S) {
+        on = threadIdx.x < S.total;
+        j = S.find(on ? threadIdx.x : 0);
+        n = S.n0 + j;
+        nzmin = S.top[j];
+        nzmax = nzmin + S.pre[j + 1] - S.pre[j];
+        nz = nzmin + (on ? (int)threadIdx.x - S.pre[j] : 0);
+        i = n * tp.L1 + nz - 1;
+        iv = n * tp.nl + nz - 1;
+    }
+};
+__device__ __forceinline__ bool slot_wet(const int4 &q, int nz) { return nz >= (q.z & 0xffff) && nz <= (q.z >> 16); }
+
+// loop of the blocks over the tiles (one launch may hold fewer blocks than tiles)
+#define FOR_NODE_TILES(ti, ntiles) for (int ti = blockIdx.x; ti < (ntiles); ti += gridDim.x)
+
+// ---------------------------------------------------------------------------
 // k32_lo_ad
 // ---------------------------------------------------------------------------
-// One chunk of a node's column for every group of the launch.  PACK: the column's last
-// chunk with P groups side by side in segments of W lanes; otherwise one group at a time
-// over the whole warp.
-template <int G, int KD, bool WS, bool PACK>
-__device__ __forceinline__ void lo_ad_chunk(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
-                                            const B32View &B, const float *__restrict__ VF, float dt, int n, int lane,
-                                            const WEdges &S, int ch, int W, int P) {
-    using C = Chunk<2, 1>;
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
-    const C k = PACK ? C(nzmin, nzmax, ch, lane, W, P) : C(nzmin, nzmax, ch, lane);
-    const int nz = k.nz;
-    const int i = n * L1 + nz - 1;   // layer nz of the node (valid where k.lvl)
-    const int iv = n * nl + nz - 1;  // interface nz
-    // ---- tracer-independent part of the chunk ----
-    // The node's share of edge slot u's upwind flux F = -(T1 v+ + T2 v-) (+F at edges(1,e),
-    // -F at edges(2,e)) is rn(rn(T_n p_u) + rn(T_m q_u)) with (p, q) = (-v+, -v-) at edges(1,e)
-    // and (v-, v+) at edges(2,e): the same two products and the same sum as at the other end,
-    // so the two ends add exactly opposite values.  A dry slot has p = q = 0 and gathers the
-    // node's own entry, so it adds zero without a per-tracer test.
-    int off[KD];
-    float pq[KD], qq[KD];
+// The node's share of an edge's upwind flux F = -(T1 v+ + T2 v-) (+F at edges(1,e), -F at
+// edges(2,e)) is rn(rn(T_n p) + rn(T_m q)) with (p, q) = (-v+, -v-) at edges(1,e) and (v-, v+) at
+// edges(2,e): the same two products and the same sum as at the other end, so the two ends add
+// exactly opposite values.
+__device__ __forceinline__ void edge_share(float v, bool own, float &p, float &q) {
+    const float vp = fmaxf(v, 0.f), vm = fminf(v, 0.f);
+    p = own ? -vp : vm;
+    q = own ? -vm : vp;
+}
+template <int G>
+using LoBuf = Vec<G>[2][2][kNT];  // [buffer][T, AB value][thread]
+
+template <int G, bool WS>
+__device__ __forceinline__ void lo_ad_tile(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
+                                           const B32View &B, const float *__restrict__ VF, float dt,
+                                           const NodeTile &S, LoBuf<G> &X) {
+    const TileLane k(tp, S);
+    const int x = threadIdx.x, i = k.i, iv = k.iv, nz = k.nz, deg = S.deg[k.j];
+    // dry and missing slots: offset -1, no flux
+    int off[kND];
+    float pq[kND], qq[kND];
 #pragma unroll
-    for (int u = 0; u < KD; u++) {
-        const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-        off[u] = ok ? S.m[u] * L1 + nz - 1 : i;
-        const float v = ok ? VF[S.e[u] * L1 + nz - 1] : 0.f;
-        const float vp = fmaxf(v, 0.f), vm = fminf(v, 0.f);
-        const bool ow = (own >> u) & 1u;
-        pq[u] = ow ? -vp : vm;
-        qq[u] = ow ? -vm : vp;
+    for (int u = 0; u < kND; u++) {
+        const int4 q = S.slot[k.j][u];
+        const bool ok = k.on && u < deg && slot_wet(q, nz);
+        off[u] = ok ? q.x + nz - 1 : -1;
+        edge_share(ok ? VF[q.y + nz - 1] : 0.f, q.w != 0, pq[u], qq[u]);
     }
-    float ar0 = 0.f, we0 = 0.f, w0 = 0.f, sdt = 0.f, Z0 = 0.f, dhr = 0.f;
-    if (k.lvl) {
-        ar0 = g.area[iv];
-        we0 = f.we[iv];
-        w0 = f.w[iv];
+    LoLane L{nz, k.nzmin, k.nzmax, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (k.on) {
+        L.ar0 = g.area[iv];
+        L.we0 = f.we[iv];
+        L.w0 = f.w[iv];
         const float hn = g.hnode_new[i];
-        sdt = qdiv(dt, g.areasvol[iv] * hn);
-        dhr = qdiv(g.hnode[i] - hn, hn);
-        Z0 = g.Z3[i];
+        L.sdt = qdiv(dt, g.areasvol[iv] * hn);
+        L.dhr = qdiv(g.hnode[i] - hn, hn);
+        if (nz < k.nzmax - 1) {
+            L.ar1 = g.area[iv + 1];
+            L.we1 = f.we[iv + 1];
+        }
+        // QR4C interior geometry, nzmin+2 <= nz <= nzmax-2 (oce_adv_tra_ver.F90:409-425)
+        if (nz >= k.nzmin + 2 && nz <= k.nzmax - 2) {
+            const float Z0 = g.Z3[i], Zm1 = g.Z3[i - 1], Zm2 = g.Z3[i - 2], Zp1 = g.Z3[i + 1], zb = g.zbar3[iv];
+            L.idz0 = qdiv(1.f, Zm1 - Z0);
+            L.idzp = qdiv(1.f, Z0 - Zp1);
+            L.idzm = qdiv(1.f, Zm2 - Zm1);
+            L.g1 = (zb - Z0) * (1.f / 3.f);
+            L.g2 = (zb - Zm1) * (1.f / 3.f);
+        }
     }
-    const float Zm1 = sh_up(Z0, 1), Zm2 = sh_up(Z0, 2), Zp1 = sh_dn(Z0, 1);
-    // QR4C interior geometry, nzmin+2 <= nz <= nzmax-2 (oce_adv_tra_ver.F90:409-425)
-    const bool qint = k.out && nz >= nzmin + 2 && nz <= nzmax - 2;
-    float idz0 = 0.f, idzp = 0.f, idzm = 0.f, g1 = 0.f, g2 = 0.f;
-    if (qint) {
-        const float zb = g.zbar3[iv];
-        idz0 = qdiv(1.f, Zm1 - Z0);
-        idzp = qdiv(1.f, Z0 - Zp1);
-        idzm = qdiv(1.f, Zm2 - Zm1);
-        g1 = (zb - Z0) * (1.f / 3.f);
-        g2 = (zb - Zm1) * (1.f / 3.f);
-    }
-    const bool twolayer = nzmin + 1 == nzmax - 1;
-    // ---- per group ----
 #pragma unroll 1
-    for (int g0 = 0; g0 < B.ng; g0 += PACK ? P : 1) {
-        // the lane's group (packed: the group of its segment; idle past the last)
-        const int gg = g0 + k.q;
-        const bool on = gg < B.ng;
-        const int gi = on ? gg : g0;
-        const bool lvt = k.lvl && on;
+    for (int gi = 0; gi < B.ng; gi++) {
         const bool lim = (B.fct >> gi) & 1ull;
         const int ver = B.ver[gi];
         const float *__restrict__ T = grp<G>(B.T, gi, B.sN);
-        const float *__restrict__ O1 = grp<G>(B.O1, gi, B.sN);
-        const float *__restrict__ O2 = B.ab == 3 ? grp<G>(B.O2, gi, B.sN) : O1;
-        // every load of the group's chunk first
-        const Vec<G> Tn = vldc<G>(lvt, T, i);
-        const Vec<G> o1 = vldc<G>(lvt, O1, i);
-        const Vec<G> o2 = vldc<G>(lvt && B.ab == 3, O2, i);
-        Vec<G> tm[KD];
+        // every load of the group first
+        const Vec<G> Tn = vldc<G>(k.on, T, i);
+        const Vec<G> o1 = vldc<G>(k.on, grp<G>(B.O1, gi, B.sN), i);
+        const Vec<G> o2 = vldc<G>(k.on && B.ab == 3, B.ab == 3 ? grp<G>(B.O2, gi, B.sN) : T, i);
+        Vec<G> tm[kND];
 #pragma unroll
-        for (int u = 0; u < KD; u++) tm[u] = vldc<G>(lvt, T, off[u]);
-        Vec<G> lo, ad;
-#if FESOM_PACKED_PAIRS
+        for (int u = 0; u < kND; u++) tm[u] = vldc<G>(off[u] >= 0, T, off[u]);
+        Vec<G> ta;
 #pragma unroll
         for (int j = 0; j < G / 2; j++) {
-            const float2 tn = pr(Tn, j);
-            float2 hs = pk(0.f);
+            const float2 tn = pr(Tn, j), p1 = pr(o1, j), p2 = pr(o2, j);
+            const float2 t = B.ab == 2 ? pfma(pk(0.6f), psub(tn, p1), tn)
+                                       : pfma(pfma(pk(11.f), psub(tn, p1), pmul(pk(-5.f), psub(p1, p2))),
+                                              pk(1.f / 12.f), tn);
+            ta.c[2 * j] = t.x;
+            ta.c[2 * j + 1] = t.y;
+        }
+        Vec<G>(&xt)[kNT] = X[gi & 1][0], (&xa)[kNT] = X[gi & 1][1];
+        xt[x] = Tn;
+        xa[x] = ta;
+        float2 hs[G / 2];
 #pragma unroll
-            for (int u = 0; u < KD; u++) hs = padd(hs, padd(pmul(tn, pk(pq[u])), pmul(pr(tm[u], j), pk(qq[u]))));
-            float2 l2, a2;
-            lo_ad_pair<WS>(f, B.ab, ver, lim, lvt, make_float2(B.pv[gi * G + 2 * j], B.pv[gi * G + 2 * j + 1]), nz,
-                           nzmin, nzmax, twolayer, ar0, we0, w0, sdt, dhr, idz0, idzp, idzm, g1, g2, tn, pr(o1, j),
-                           pr(o2, j), hs, l2, a2);
+        for (int j = 0; j < G / 2; j++) {
+            hs[j] = pk(0.f);
+#pragma unroll
+            for (int u = 0; u < kND; u++)
+                hs[j] = padd(hs[j], padd(pmul(pr(Tn, j), pk(pq[u])), pmul(pr(tm[u], j), pk(qq[u]))));
+        }
+        for (int u = kND; u < deg; u++) {  // nodes of more edges
+            const int4 q = S.slot[k.j][u];
+            if (!k.on || !slot_wet(q, nz)) continue;
+            float p, r;
+            edge_share(VF[q.y + nz - 1], q.w != 0, p, r);
+            const Vec<G> t = vld<G>(T, q.x + nz - 1);
+#pragma unroll
+            for (int j = 0; j < G / 2; j++) hs[j] = padd(hs[j], padd(pmul(pr(Tn, j), pk(p)), pmul(pr(t, j), pk(r))));
+        }
+        __syncthreads();
+        if (!k.on) continue;
+        // the layers above (up to two) and below; at the column's ends the thread's own entry (unused)
+        const int a1 = nz > k.nzmin ? x - 1 : x, a2 = nz > k.nzmin + 1 ? x - 2 : x, d1 = nz < k.nzmax - 1 ? x + 1 : x;
+        const Vec<G> Tu = xt[a1], Td = xt[d1], au = xa[a1], au2 = xa[a2], adn = xa[d1];
+        Vec<G> lo, ad;
+#pragma unroll
+        for (int j = 0; j < G / 2; j++) {
+            float2 l2, d2;
+            lo_ad_pair<WS>(f, ver, lim, make_float2(B.pv[gi * G + 2 * j], B.pv[gi * G + 2 * j + 1]), L, pr(Tn, j),
+                           pr(Tu, j), pr(Td, j), pr(ta, j), pr(au, j), pr(au2, j), pr(adn, j), hs[j], l2, d2);
             lo.c[2 * j] = l2.x;
             lo.c[2 * j + 1] = l2.y;
-            ad.c[2 * j] = a2.x;
-            ad.c[2 * j + 1] = a2.y;
+            ad.c[2 * j] = d2.x;
+            ad.c[2 * j + 1] = d2.y;
         }
-#else
-#pragma unroll
-        for (int c = 0; c < G; c++) {
-            const float tn = Tn.c[c];
-            const float tab = tn + (lvt ? ab_delta(B.ab, tn, o1.c[c], o2.c[c]) : 0.f);
-            const float Tu = sh_up(tn, 1);
-            const float tabu = sh_up(tab, 1), tabu2 = sh_up(tab, 2), tabd = sh_dn(tab, 1);
-            // LO: the upwind edge fluxes, + at edges(1,e), - at edges(2,e), in ascending edge
-            // order (oce_adv_tra_driver.F90:131-190)
-            float hs = 0.f;
-#pragma unroll
-            for (int u = 0; u < KD; u++) hs += __fadd_rn(__fmul_rn(tn, pq[u]), __fmul_rn(tm[u].c[c], qq[u]));
-            // upwind vertical flux with w_e at interface nz (adv_tra_ver_upw1)
-            float fv0 = 0.f;
-            if (lvt) {
-                if (nz == nzmin) {
-                    fv0 = -(we0 * tn * ar0);
-                } else {
-                    const float aw = fabsf(we0);
-                    fv0 = -(0.5f * (tn * (we0 + aw) + Tu * (we0 - aw)) * ar0);
-                }
-            }
-            float fv1 = sh_dn(fv0, 1);
-            if (nz == nzmax - 1) fv1 = 0.f;
-            // LO = (T hnode + flux divergence dt / areasvol) / hnode_new (oce_adv_tra_driver.F90:249),
-            // as T + T (hnode - hnode_new) / hnode_new + flux divergence dt / (areasvol hnode_new)
-            lo.c[c] = tn + fmaf(tn, dhr, (hs + (fv0 - fv1)) * sdt);
-            // with the split vertical velocity the LO part of the antidiffusive flux is the upwind
-            // flux of the full w (oce_adv_tra_driver.F90:323-334)
-            float fw0 = fv0;
-            if (WS && f.wsplit && lvt) {
-                if (nz == nzmin) {
-                    fw0 = -(w0 * tn * ar0);
-                } else {
-                    const float aw = fabsf(w0);
-                    fw0 = -(0.5f * (tn * (w0 + aw) + Tu * (w0 - aw)) * ar0);
-                }
-            }
-            ad.c[c] = ver_ad(ver, lim, B.pv[gi * G + c], nz, nzmin, nzmax, twolayer, tab, tabu, tabu2, tabd,
-                             lim ? w0 : we0, ar0, fv0, fw0, idz0, idzp, idzm, g1, g2);
-        }
-#endif
-        if (k.out && on) {
-            vst<G>(grp<G>(B.LO, gi, B.sN), i, lo);
-            // PPM fluxes come from k32_vppm
-            if (ver != 3) vst<G>(grp<G>(B.ADv, gi, B.sNI), iv, ad);
-        }
+        vst<G>(grp<G>(B.LO, gi, B.sN), i, lo);
+        // PPM fluxes come from k32_vppm
+        if (ver != 3) vst<G>(grp<G>(B.ADv, gi, B.sNI), iv, ad);
     }
 }
 
-// The same chunk with each pass's gathers staged in shared memory: entries T and the previous
-// levels of the node, then T of every edge slot (a dry slot stages the node's own T).
-constexpr int kNsLoAd = 3 + 6;
-template <int G, int KD, bool WS, bool PACK>
-__device__ __forceinline__ void lo_ad_chunk_pf(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
-                                               const B32View &B, const float *__restrict__ VF, float dt, int n,
-                                               int lane, const WEdges &S, int ch, int W, int P, float *sb) {
-    using C = Chunk<2, 1>;
-    constexpr int NS = 3 + KD;
-    static_assert(NS <= kNsLoAd, "staging sized for six edge slots");
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
-    const C k = PACK ? C(nzmin, nzmax, ch, lane, W, P) : C(nzmin, nzmax, ch, lane);
-    const int nz = k.nz;
-    const int i = n * L1 + nz - 1;
-    const int iv = n * nl + nz - 1;
-    // tracer-independent part of the chunk (as in lo_ad_chunk)
-    int off[KD];
-    float pq[KD], qq[KD];
-#pragma unroll
-    for (int u = 0; u < KD; u++) {
-        const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-        off[u] = ok ? S.m[u] * L1 + nz - 1 : (k.lvl ? i : 0);
-        const float v = ok ? VF[S.e[u] * L1 + nz - 1] : 0.f;
-        const float vp = fmaxf(v, 0.f), vm = fminf(v, 0.f);
-        const bool ow = (own >> u) & 1u;
-        pq[u] = ow ? -vp : vm;
-        qq[u] = ow ? -vm : vp;
+template <int G, bool WS>
+__global__ void __launch_bounds__(kNT, MinB<G>::lo)
+k32_lo_ad(DTopo tp, DGeom<float> g, DForcing<float> f, B32View B, const float *__restrict__ VF, float dt) {
+    __shared__ NodeTile S;
+    __shared__ LoBuf<G> X;
+    FOR_NODE_TILES(ti, tp.n_nt) {
+        node_tile_load(tp, ti, S);
+        lo_ad_tile<G, WS>(tp, g, f, B, VF, dt, S, X);
+        __syncthreads();
     }
-    float ar0 = 0.f, we0 = 0.f, w0 = 0.f, sdt = 0.f, Z0 = 0.f, dhr = 0.f;
-    if (k.lvl) {
-        ar0 = g.area[iv];
-        we0 = f.we[iv];
-        w0 = f.w[iv];
-        const float hn = g.hnode_new[i];
-        sdt = qdiv(dt, g.areasvol[iv] * hn);
-        dhr = qdiv(g.hnode[i] - hn, hn);
-        Z0 = g.Z3[i];
-    }
-    const float Zm1 = sh_up(Z0, 1), Zm2 = sh_up(Z0, 2), Zp1 = sh_dn(Z0, 1);
-    const bool qint = k.out && nz >= nzmin + 2 && nz <= nzmax - 2;
-    float idz0 = 0.f, idzp = 0.f, idzm = 0.f, g1 = 0.f, g2 = 0.f;
-    if (qint) {
-        const float zb = g.zbar3[iv];
-        idz0 = qdiv(1.f, Zm1 - Z0);
-        idzp = qdiv(1.f, Z0 - Zp1);
-        idzm = qdiv(1.f, Zm2 - Zm1);
-        g1 = (zb - Z0) * (1.f / 3.f);
-        g2 = (zb - Zm1) * (1.f / 3.f);
-    }
-    const bool twolayer = nzmin + 1 == nzmax - 1;
-    const int npass = PACK ? (B.ng + P - 1) / P : B.ng;
-    auto grp_of = [&](int p) { return PACK ? p * P + k.q : p; };
-    auto issue = [&](int p, float *buf) {
-        const int gg = grp_of(p);
-        const bool lvt = k.lvl && gg < B.ng;
-        const int gi = gg < B.ng ? gg : 0;
-        const float *T = grp<G>(B.T, gi, B.sN);
-        const int ii = lvt ? i : 0;
-        cpa<G>(stg<G>(buf, 0, lane), T + (size_t)ii * G, lvt);
-        cpa<G>(stg<G>(buf, 1, lane), grp<G>(B.O1, gi, B.sN) + (size_t)ii * G, lvt);
-        cpa<G>(stg<G>(buf, 2, lane), (B.ab == 3 ? grp<G>(B.O2, gi, B.sN) : T) + (size_t)ii * G, lvt && B.ab == 3);
-#pragma unroll
-        for (int u = 0; u < KD; u++) cpa<G>(stg<G>(buf, 3 + u, lane), T + (size_t)off[u] * G, lvt);
-        cpa_commit();
-    };
-    auto compute = [&](int p, float *buf) {
-        const int gg = grp_of(p);
-        const bool on = gg < B.ng;
-        const int gi = on ? gg : 0;
-        const bool lvt = k.lvl && on;
-        const bool lim = (B.fct >> gi) & 1ull;
-        const int ver = B.ver[gi];
-        const Vec<G> Tn = lds<G>(stg<G>(buf, 0, lane));
-        const Vec<G> o1 = lds<G>(stg<G>(buf, 1, lane));
-        const Vec<G> o2 = lds<G>(stg<G>(buf, 2, lane));
-#if FESOM_PACKED_PAIRS
-        Vec<G> lo, ad;
-        float2 hsp[G / 2];
-#pragma unroll
-        for (int j = 0; j < G / 2; j++) hsp[j] = pk(0.f);
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> tm = lds<G>(stg<G>(buf, 3 + u, lane));
-#pragma unroll
-            for (int j = 0; j < G / 2; j++)
-                hsp[j] = padd(hsp[j], padd(pmul(pr(Tn, j), pk(pq[u])), pmul(pr(tm, j), pk(qq[u]))));
-        }
-#pragma unroll
-        for (int j = 0; j < G / 2; j++) {
-            const float2 tn = pr(Tn, j), hs = hsp[j];
-            float2 l2, a2;
-            lo_ad_pair<WS>(f, B.ab, ver, lim, lvt, make_float2(B.pv[gi * G + 2 * j], B.pv[gi * G + 2 * j + 1]), nz,
-                           nzmin, nzmax, twolayer, ar0, we0, w0, sdt, dhr, idz0, idzp, idzm, g1, g2, tn, pr(o1, j),
-                           pr(o2, j), hs, l2, a2);
-            lo.c[2 * j] = l2.x;
-            lo.c[2 * j + 1] = l2.y;
-            ad.c[2 * j] = a2.x;
-            ad.c[2 * j + 1] = a2.y;
-        }
-#else
-        Vec<G> hs = vfill<G>(0.f);
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> tm = lds<G>(stg<G>(buf, 3 + u, lane));
-#pragma unroll
-            for (int c = 0; c < G; c++)
-                hs.c[c] += __fadd_rn(__fmul_rn(Tn.c[c], pq[u]), __fmul_rn(tm.c[c], qq[u]));
-        }
-        Vec<G> lo, ad;
-#pragma unroll
-        for (int c = 0; c < G; c++) {
-            const float tn = Tn.c[c];
-            const float tab = tn + (lvt ? ab_delta(B.ab, tn, o1.c[c], o2.c[c]) : 0.f);
-            const float Tu = sh_up(tn, 1);
-            const float tabu = sh_up(tab, 1), tabu2 = sh_up(tab, 2), tabd = sh_dn(tab, 1);
-            float fv0 = 0.f;
-            if (lvt) {
-                if (nz == nzmin) {
-                    fv0 = -(we0 * tn * ar0);
-                } else {
-                    const float aw = fabsf(we0);
-                    fv0 = -(0.5f * (tn * (we0 + aw) + Tu * (we0 - aw)) * ar0);
-                }
-            }
-            float fv1 = sh_dn(fv0, 1);
-            if (nz == nzmax - 1) fv1 = 0.f;
-            lo.c[c] = tn + fmaf(tn, dhr, (hs.c[c] + (fv0 - fv1)) * sdt);
-            float fw0 = fv0;
-            if (WS && f.wsplit && lvt) {
-                if (nz == nzmin) {
-                    fw0 = -(w0 * tn * ar0);
-                } else {
-                    const float aw = fabsf(w0);
-                    fw0 = -(0.5f * (tn * (w0 + aw) + Tu * (w0 - aw)) * ar0);
-                }
-            }
-            ad.c[c] = ver_ad(ver, lim, B.pv[gi * G + c], nz, nzmin, nzmax, twolayer, tab, tabu, tabu2, tabd,
-                             lim ? w0 : we0, ar0, fv0, fw0, idz0, idzp, idzm, g1, g2);
-        }
-#endif
-        if (k.out && on) {
-            vst<G>(grp<G>(B.LO, gi, B.sN), i, lo);
-            if (ver != 3) vst<G>(grp<G>(B.ADv, gi, B.sNI), iv, ad);
-        }
-    };
-    issue(0, sb);
-    float *cur = sb, *nxt = sb + (size_t)NS * 32 * G;
-    for (int p = 0; p < npass; p++) {
-        if (p + 1 < npass) {
-            issue(p + 1, nxt);
-            cpa_wait<1>();
-        } else {
-            cpa_wait<0>();
-        }
-        compute(p, cur);
-        float *t = cur;
-        cur = nxt;
-        nxt = t;
-    }
-}
-
-template <int G, int KD, bool WS, bool PK>
-__device__ __forceinline__ void lo_ad_node(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
-                                           const B32View &B, const float *__restrict__ VF, float dt, int n, int lane,
-                                           const WEdges &S, float *sb) {
-    using C = Chunk<2, 1>;
-    const int nch = C::count(S.nzmin, S.nzmax);
-    const int W = C::last_width(S.nzmin, S.nzmax), P = 32 / W;
-    if constexpr (KD == 6) {
-        if (sb) {
-            for (int ch = 0; ch < nch - 1; ch++)
-                lo_ad_chunk_pf<G, KD, WS, false>(tp, g, f, B, VF, dt, n, lane, S, ch, 32, 1, sb);
-            if (PK && P > 1) lo_ad_chunk_pf<G, KD, WS, true>(tp, g, f, B, VF, dt, n, lane, S, nch - 1, W, P, sb);
-            else lo_ad_chunk_pf<G, KD, WS, false>(tp, g, f, B, VF, dt, n, lane, S, nch - 1, 32, 1, sb);
-            return;
-        }
-    }
-    for (int ch = 0; ch < nch - 1; ch++) lo_ad_chunk<G, KD, WS, false>(tp, g, f, B, VF, dt, n, lane, S, ch, 32, 1);
-    // packed only for nodes of at most 6 edges (the wider packed bodies would spill)
-    if (PK && KD <= 6 && P > 1) lo_ad_chunk<G, KD, WS, true>(tp, g, f, B, VF, dt, n, lane, S, nch - 1, W, P);
-    else lo_ad_chunk<G, KD, WS, false>(tp, g, f, B, VF, dt, n, lane, S, nch - 1, 32, 1);
 }
 
 // the node of warp unit j: consecutive nodes, or (WIDE) the listed nodes of more than 8 edges
@@ -949,37 +732,9 @@ __device__ __forceinline__ int node_units(const DTopo &tp) {
     return WIDE ? tp.n_wide : tp.N2;
 }
 
-// WS: the split vertical velocity (a separate instantiation keeps the default path unchanged)
-template <int G, bool WIDE, bool WS, bool PK>
-__device__ __forceinline__ void lo_ad_unit(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
-                                           const B32View &B, const float *__restrict__ VF, float dt, int j, WEdges *Se,
-                                           float *sb) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = unit_node<WIDE>(tp, j);
-    if (n < 0) return;
-    WEdges &S = Se[warp];
-    stage_edges(tp, n, lane, S);
-    if ((S.deg > 8) != WIDE) return;
-    if (WIDE) lo_ad_node<G, kMaxDeg, WS, PK>(tp, g, f, B, VF, dt, n, lane, S, nullptr);
-    else if (S.deg <= 6) lo_ad_node<G, 6, WS, PK>(tp, g, f, B, VF, dt, n, lane, S, sb);
-    else lo_ad_node<G, 8, WS, PK>(tp, g, f, B, VF, dt, n, lane, S, nullptr);
-}
-
-template <int G>
-__host__ __device__ constexpr int stage_bytes_lo_ad() { return 2 * kNsLoAd * 32 * G * 4; }
-
 // grid-stride loop of the warps over the units (one launch may hold fewer blocks than units)
 #define FOR_WARP_UNITS(j, count)                                                               \
     for (int j = blockIdx.x * kWB + (threadIdx.x >> 5); j < (count); j += gridDim.x * kWB)
-
-template <int G, bool WIDE, bool WS, bool STG>
-__global__ void __launch_bounds__(kTB, WIDE ? 1 : MinB<G>::lo)
-k32_lo_ad(DTopo tp, DGeom<float> g, DForcing<float> f, B32View B, const float *__restrict__ VF, float dt) {
-    __shared__ WEdges Se[kWB];
-    extern __shared__ __align__(16) float dsm[];
-    float *sb = (WIDE || !STG) ? nullptr : dsm + (size_t)(threadIdx.x >> 5) * (stage_bytes_lo_ad<G>() / 4);
-    FOR_WARP_UNITS(j, node_units<WIDE>(tp)) lo_ad_unit<G, WIDE, WS, true>(tp, g, f, B, VF, dt, j, Se, sb);
-}
 
 // high-order minus low-order flux of one edge-layer from the two end values, their
 // previous time levels and the projected gradients s1 (up) / s2 (down)
@@ -1208,295 +963,106 @@ __global__ void __launch_bounds__(256) k32_ho_nodemean(DTopo tp, B32View B, Musc
 // One chunk of a node's column for the FCT groups of the launch.  PACK: the column's last
 // chunk with P groups side by side in segments of W lanes; otherwise one group at a time
 // over the whole warp.
-template <int G, int KD, bool PACK>
-__device__ __forceinline__ void bounds_chunk(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt, int n,
-                                             int lane, const WEdges &S, int ch, int W, int P) {
-    using C = Chunk<1, 1>;
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
-    const float eps = (float)kFluxEps;
-    const C k = PACK ? C(nzmin, nzmax, ch, lane, W, P) : C(nzmin, nzmax, ch, lane);
-    const int nz = k.nz;
-    const int i = n * L1 + nz - 1, iv = n * nl + nz - 1;
-    // a dry slot gathers the node's own T and LO (neutral for the bounds); its ADh is not loaded
-    int off[KD], eo[KD];
-    unsigned okx = 0;
-#pragma unroll
-    for (int u = 0; u < KD; u++) {
-        const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-        off[u] = ok ? S.m[u] * L1 + nz - 1 : i;
-        eo[u] = ok ? S.e[u] * L1 + nz - 1 : 0;
-        okx |= ok ? 1u << u : 0u;
-    }
-    const float s = k.lvl ? qdiv(dt, g.areasvol[iv] * g.hnode_new[i]) : 0.f;
-    unsigned long long todo = B.fct & (B.ng >= 64 ? ~0ull : ((1ull << B.ng) - 1));
-    int g0 = 0;
-    while (PACK ? g0 < B.ng : todo != 0ull) {
-        // the lane's group: the next FCT group, or (packed) group g0 + q of the segment, idle
-        // where that group has no FCT
-        int gq;
-        if (PACK) {
-            gq = g0 + k.q;
-            if (gq >= B.ng || !((B.fct >> gq) & 1ull)) gq = -1;
-            g0 += P;
-        } else {
-            gq = __ffsll((long long)todo) - 1;
-            todo &= todo - 1;
-        }
-        const bool lv = k.lvl && gq >= 0;
-        const int gs = gq < 0 ? 0 : gq;
-        const float *__restrict__ T = grp<G>(B.T, gs, B.sN);
-        const float *__restrict__ LO = grp<G>(B.LO, gs, B.sN);
-        const float *__restrict__ ADh = grp<G>(B.ADh, gs, B.sE);
-        const Vec<G> Tn = vldc<G>(lv, T, i);
-        const Vec<G> lo = vldc<G>(lv, LO, i);
-        const Vec<G> v0 = vldc<G>(lv, grp<G>(B.ADv, gs, B.sNI), iv);
-        // bounds over the node, its neighbours and the layers above and below
-        // (oce_adv_tra_fct.F90:124-248)
-        Vec<G> mx, mn;
-#pragma unroll
-        for (int c = 0; c < G; c++) {
-            mx.c[c] = fmaxf(lo.c[c], Tn.c[c]);
-            mn.c[c] = fminf(lo.c[c], Tn.c[c]);
-        }
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> tm = vldc<G>(lv, T, off[u]);
-            const Vec<G> lm = vldc<G>(lv, LO, off[u]);
-#pragma unroll
-            for (int c = 0; c < G; c++) {
-                mx.c[c] = fmaxf(mx.c[c], fmaxf(tm.c[c], lm.c[c]));
-                mn.c[c] = fminf(mn.c[c], fminf(tm.c[c], lm.c[c]));
-            }
-        }
-        // P / M: sums of the positive / negative antidiffusive fluxes into the node
-        Vec<G> Pp = vfill<G>(0.f), M = vfill<G>(0.f);
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> x = vldc<G>(lv && ((okx >> u) & 1u), ADh, eo[u]);
-            const bool ow = (own >> u) & 1u;
-#pragma unroll
-            for (int c = 0; c < G; c++) {
-                const float xv = ow ? x.c[c] : -x.c[c];
-                Pp.c[c] += fmaxf(0.f, xv);
-                M.c[c] += fminf(0.f, xv);
-            }
-        }
-        Vec<G> rp, rm, bp, bm;
-#pragma unroll
-        for (int c = 0; c < G; c++) {
-            const float mxu = sh_up(mx.c[c], 1), mxd = sh_dn(mx.c[c], 1);
-            const float mnu = sh_up(mn.c[c], 1), mnd = sh_dn(mn.c[c], 1);
-            float tup = mx.c[c], tlo = mn.c[c];
-            if (nz != nzmin && nz != nzmax - 1) {
-                tup = fmaxf(fmaxf(mxu, mx.c[c]), mxd);
-                tlo = fminf(fminf(mnu, mn.c[c]), mnd);
-            }
-            float v1 = sh_dn(v0.c[c], 1);
-            if (nz == nzmax - 1) v1 = 0.f;
-            const float pp = Pp.c[c] + (fmaxf(0.f, v0.c[c]) + fmaxf(0.f, -v1));
-            const float mm = M.c[c] + (fminf(0.f, v0.c[c]) + fminf(0.f, -v1));
-            const float bmx = tup - lo.c[c], bmn = tlo - lo.c[c];
-            rp.c[c] = fminf(1.f, qdiv(bmx, pp * s + eps));
-            rm.c[c] = fminf(1.f, qdiv(bmn, mm * s - eps));
-            // the bounds themselves: the update clamps the advected value into them, so FP32
-            // rounding in the limiter can never create a new extremum
-            bp.c[c] = tup;
-            bm.c[c] = tlo;
-        }
-        if (k.out && gq >= 0) {
-            vst<G>(grp<G>(B.Rp, gq, B.sN), i, rp);
-            vst<G>(grp<G>(B.Rm, gq, B.sN), i, rm);
-            if (kFctClamp) {
-                vst<G>(grp<G>(B.Bp, gq, B.sN), i, bp);
-                vst<G>(grp<G>(B.Bm, gq, B.sN), i, bm);
-            }
-        }
-    }
-}
+template <int G>
+using BoundsBuf = Vec<G>[2][2][kNT];  // [buffer][max, min][thread]
 
-// The same chunk with each pass's gathers staged in shared memory (sb: the warp's staging):
-// entries T, LO, ADv of the node, then T, LO, ADh of every edge slot.
-constexpr int kNsBounds = 3 + 3 * 6;
-template <int G, int KD, bool PACK>
-__device__ __forceinline__ void bounds_chunk_pf(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
-                                                int n, int lane, const WEdges &S, int ch, int W, int P, float *sb) {
-    using C = Chunk<1, 1>;
-    constexpr int NS = 3 + 3 * KD;
-    static_assert(NS <= kNsBounds, "staging sized for six edge slots");
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
+template <int G>
+__device__ __forceinline__ void bounds_tile(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
+                                            const NodeTile &S, BoundsBuf<G> &X) {
+    constexpr int kUB = MinB<G>::ub;
+    const TileLane k(tp, S);
+    const int x = threadIdx.x, i = k.i, iv = k.iv, nz = k.nz, deg = S.deg[k.j];
     const float eps = (float)kFluxEps;
-    const C k = PACK ? C(nzmin, nzmax, ch, lane, W, P) : C(nzmin, nzmax, ch, lane);
-    const int nz = k.nz;
-    const int i = n * L1 + nz - 1, iv = n * nl + nz - 1;
-    // a dry slot stages the node's own T and LO (neutral for the bounds) and zeros for ADh
-    int off[KD], eo[KD];
-    unsigned okx = 0;
-#pragma unroll
-    for (int u = 0; u < KD; u++) {
-        const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-        off[u] = ok ? S.m[u] * L1 + nz - 1 : (k.lvl ? i : 0);
-        eo[u] = ok ? S.e[u] * L1 + nz - 1 : 0;
-        okx |= ok ? 1u << u : 0u;
-    }
-    const float s = k.lvl ? qdiv(dt, g.areasvol[iv] * g.hnode_new[i]) : 0.f;
-    unsigned todo = (unsigned)(B.fct & (B.ng >= 32 ? 0xffffffffull : ((1ull << B.ng) - 1)));
-    int g0 = 0;
-    // the lane's group of the next pass (-1: idle); false when no pass is left
-    auto next = [&](int &gq) -> bool {
-        if (PACK) {
-            if (g0 >= B.ng) return false;
-            gq = g0 + k.q;
-            if (gq >= B.ng || !((B.fct >> gq) & 1ull)) gq = -1;
-            g0 += P;
-            return true;
-        }
-        if (!todo) return false;
-        gq = __ffs(todo) - 1;
-        todo &= todo - 1;
-        return true;
-    };
-    auto issue = [&](int gq, float *buf) {
-        const bool lv = k.lvl && gq >= 0;
-        const int gs = gq < 0 ? 0 : gq;
-        const float *T = grp<G>(B.T, gs, B.sN), *LO = grp<G>(B.LO, gs, B.sN);
-        const float *ADh = grp<G>(B.ADh, gs, B.sE), *ADv = grp<G>(B.ADv, gs, B.sNI);
-        cpa<G>(stg<G>(buf, 0, lane), T + (size_t)(lv ? i : 0) * G, lv);
-        cpa<G>(stg<G>(buf, 1, lane), LO + (size_t)(lv ? i : 0) * G, lv);
-        cpa<G>(stg<G>(buf, 2, lane), ADv + (size_t)(lv ? iv : 0) * G, lv);
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            cpa<G>(stg<G>(buf, 3 + 3 * u, lane), T + (size_t)off[u] * G, lv);
-            cpa<G>(stg<G>(buf, 4 + 3 * u, lane), LO + (size_t)off[u] * G, lv);
-            cpa<G>(stg<G>(buf, 5 + 3 * u, lane), ADh + (size_t)eo[u] * G, lv && ((okx >> u) & 1u));
-        }
-        cpa_commit();
-    };
-    auto compute = [&](int gq, float *buf) {
-        const Vec<G> Tn = lds<G>(stg<G>(buf, 0, lane));
-        const Vec<G> lo = lds<G>(stg<G>(buf, 1, lane));
-        const Vec<G> v0 = lds<G>(stg<G>(buf, 2, lane));
+    const float s = k.on ? qdiv(dt, g.areasvol[iv] * g.hnode_new[i]) : 0.f;
+    int b = 0;
+#pragma unroll 1
+    for (int gq = 0; gq < B.ng; gq++) {
+        if (!((B.fct >> gq) & 1ull)) continue;
+        const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
+        const float *__restrict__ LO = grp<G>(B.LO, gq, B.sN);
+        const float *__restrict__ ADh = grp<G>(B.ADh, gq, B.sE);
+        const Vec<G> Tn = vldc<G>(k.on, T, i);
+        const Vec<G> lo = vldc<G>(k.on, LO, i);
+        const Vec<G> v0 = vldc<G>(k.on, grp<G>(B.ADv, gq, B.sNI), iv);
+        const Vec<G> v1 = vldc<G>(k.on && nz < k.nzmax - 1, grp<G>(B.ADv, gq, B.sNI), iv + 1);
+        // bounds over the node, its neighbours and the layers above and below
+        // (oce_adv_tra_fct.F90:124-248); P / M: sums of the positive / negative antidiffusive
+        // fluxes into the node
         Vec<G> mx, mn, Pp = vfill<G>(0.f), M = vfill<G>(0.f);
 #pragma unroll
         for (int c = 0; c < G; c++) {
             mx.c[c] = fmaxf(lo.c[c], Tn.c[c]);
             mn.c[c] = fminf(lo.c[c], Tn.c[c]);
         }
+#pragma unroll 1
+        for (int u0 = 0; u0 < S.degmax; u0 += kUB) {
+            Vec<G> tm[kUB], lm[kUB], xe[kUB];
 #pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> tm = lds<G>(stg<G>(buf, 3 + 3 * u, lane));
-            const Vec<G> lm = lds<G>(stg<G>(buf, 4 + 3 * u, lane));
-            const Vec<G> x = lds<G>(stg<G>(buf, 5 + 3 * u, lane));
-            const bool ow = (own >> u) & 1u;
+            for (int u = 0; u < kUB; u++) {
+                const int4 q = S.slot[k.j][u0 + u];
+                const bool ok = k.on && u0 + u < deg && slot_wet(q, nz);
+                // a dry or missing slot: the node's own values (neutral for the bounds), no flux
+                tm[u] = Tn;
+                lm[u] = lo;
+                if (ok) tm[u] = vld<G>(T, q.x + nz - 1);
+                if (ok) lm[u] = vld<G>(LO, q.x + nz - 1);
+                xe[u] = vldc<G>(ok, ADh, q.y + nz - 1);
+            }
+#pragma unroll
+            for (int u = 0; u < kUB; u++) {
+                const bool ow = S.slot[k.j][u0 + u].w != 0;
+#pragma unroll
+                for (int c = 0; c < G; c++) {
+                    mx.c[c] = fmaxf(mx.c[c], fmaxf(tm[u].c[c], lm[u].c[c]));
+                    mn.c[c] = fminf(mn.c[c], fminf(tm[u].c[c], lm[u].c[c]));
+                    const float xv = ow ? xe[u].c[c] : -xe[u].c[c];
+                    Pp.c[c] += fmaxf(0.f, xv);
+                    M.c[c] += fminf(0.f, xv);
+                }
+            }
+        }
+        Vec<G>(&xmx)[kNT] = X[b][0], (&xmn)[kNT] = X[b][1];
+        xmx[x] = mx;
+        xmn[x] = mn;
+        b ^= 1;
+        __syncthreads();
+        if (!k.on) continue;
+        if (nz != k.nzmin && nz != k.nzmax - 1) {
+            const Vec<G> mxu = xmx[x - 1], mxd = xmx[x + 1], mnu = xmn[x - 1], mnd = xmn[x + 1];
 #pragma unroll
             for (int c = 0; c < G; c++) {
-                mx.c[c] = fmaxf(mx.c[c], fmaxf(tm.c[c], lm.c[c]));
-                mn.c[c] = fminf(mn.c[c], fminf(tm.c[c], lm.c[c]));
-                const float xv = ow ? x.c[c] : -x.c[c];
-                Pp.c[c] += fmaxf(0.f, xv);
-                M.c[c] += fminf(0.f, xv);
+                mx.c[c] = fmaxf(fmaxf(mxu.c[c], mx.c[c]), mxd.c[c]);
+                mn.c[c] = fminf(fminf(mnu.c[c], mn.c[c]), mnd.c[c]);
             }
         }
-        Vec<G> rp, rm, bp, bm;
+        Vec<G> rp, rm;
 #pragma unroll
         for (int c = 0; c < G; c++) {
-            const float mxu = sh_up(mx.c[c], 1), mxd = sh_dn(mx.c[c], 1);
-            const float mnu = sh_up(mn.c[c], 1), mnd = sh_dn(mn.c[c], 1);
-            float tup = mx.c[c], tlo = mn.c[c];
-            if (nz != nzmin && nz != nzmax - 1) {
-                tup = fmaxf(fmaxf(mxu, mx.c[c]), mxd);
-                tlo = fminf(fminf(mnu, mn.c[c]), mnd);
-            }
-            float v1 = sh_dn(v0.c[c], 1);
-            if (nz == nzmax - 1) v1 = 0.f;
-            const float pp = Pp.c[c] + (fmaxf(0.f, v0.c[c]) + fmaxf(0.f, -v1));
-            const float mm = M.c[c] + (fminf(0.f, v0.c[c]) + fminf(0.f, -v1));
-            const float bmx = tup - lo.c[c], bmn = tlo - lo.c[c];
-            rp.c[c] = fminf(1.f, qdiv(bmx, pp * s + eps));
-            rm.c[c] = fminf(1.f, qdiv(bmn, mm * s - eps));
-            bp.c[c] = tup;
-            bm.c[c] = tlo;
+            const float pp = Pp.c[c] + (fmaxf(0.f, v0.c[c]) + fmaxf(0.f, -v1.c[c]));
+            const float mm = M.c[c] + (fminf(0.f, v0.c[c]) + fminf(0.f, -v1.c[c]));
+            rp.c[c] = fminf(1.f, qdiv(mx.c[c] - lo.c[c], pp * s + eps));
+            rm.c[c] = fminf(1.f, qdiv(mn.c[c] - lo.c[c], mm * s - eps));
         }
-        if (k.out && gq >= 0) {
-            vst<G>(grp<G>(B.Rp, gq, B.sN), i, rp);
-            vst<G>(grp<G>(B.Rm, gq, B.sN), i, rm);
-            if (kFctClamp) {
-                vst<G>(grp<G>(B.Bp, gq, B.sN), i, bp);
-                vst<G>(grp<G>(B.Bm, gq, B.sN), i, bm);
-            }
-        }
-    };
-    int gq;
-    if (!next(gq)) return;
-    float *cur = sb, *nxt = sb + (size_t)NS * 32 * G;
-    issue(gq, cur);
-    for (;;) {
-        int gn;
-        const bool more = next(gn);
-        if (more) {
-            issue(gn, nxt);
-            cpa_wait<1>();
-        } else {
-            cpa_wait<0>();
-        }
-        compute(gq, cur);
-        if (!more) break;
-        float *t = cur;
-        cur = nxt;
-        nxt = t;
-        gq = gn;
-    }
-}
-
-template <int G, int KD, bool PK>
-__device__ __forceinline__ void bounds_node(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt, int n,
-                                            int lane, const WEdges &S, float *sb) {
-    using C = Chunk<1, 1>;
-    const int nch = C::count(S.nzmin, S.nzmax);
-    const int W = C::last_width(S.nzmin, S.nzmax), P = 32 / W;
-    if constexpr (KD == 6) {
-        if (sb) {
-            for (int ch = 0; ch < nch - 1; ch++) bounds_chunk_pf<G, KD, false>(tp, g, B, dt, n, lane, S, ch, 32, 1, sb);
-            if (PK && P > 1) bounds_chunk_pf<G, KD, true>(tp, g, B, dt, n, lane, S, nch - 1, W, P, sb);
-            else bounds_chunk_pf<G, KD, false>(tp, g, B, dt, n, lane, S, nch - 1, 32, 1, sb);
-            return;
+        vst<G>(grp<G>(B.Rp, gq, B.sN), i, rp);
+        vst<G>(grp<G>(B.Rm, gq, B.sN), i, rm);
+        if (kFctClamp) {
+            // the bounds themselves: the update clamps the advected value into them
+            vst<G>(grp<G>(B.Bp, gq, B.sN), i, mx);
+            vst<G>(grp<G>(B.Bm, gq, B.sN), i, mn);
         }
     }
-    for (int ch = 0; ch < nch - 1; ch++) bounds_chunk<G, KD, false>(tp, g, B, dt, n, lane, S, ch, 32, 1);
-    if (PK && KD <= 6 && P > 1) bounds_chunk<G, KD, true>(tp, g, B, dt, n, lane, S, nch - 1, W, P);
-    else bounds_chunk<G, KD, false>(tp, g, B, dt, n, lane, S, nch - 1, 32, 1);
 }
 
-// sb: the warp's shared-memory staging (null: the gathers go to registers)
-template <int G, bool WIDE, bool PK>
-__device__ __forceinline__ void bounds_unit(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt, int j,
-                                            WEdges *Se, float *sb) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = unit_node<WIDE>(tp, j);
-    if (n < 0) return;
-    WEdges &S = Se[warp];
-    stage_edges(tp, n, lane, S);
-    if ((S.deg > 8) != WIDE) return;
-    if (WIDE) bounds_node<G, kMaxDeg, PK>(tp, g, B, dt, n, lane, S, nullptr);
-    else if (S.deg <= 6) bounds_node<G, 6, PK>(tp, g, B, dt, n, lane, S, sb);
-    else bounds_node<G, 8, PK>(tp, g, B, dt, n, lane, S, nullptr);
-}
-
-// staging bytes per warp of the bounds kernel (two buffers of NS entries)
 template <int G>
-__host__ __device__ constexpr int stage_bytes_bounds() { return 2 * kNsBounds * 32 * G * 4; }
-
-// STG: each pass's gathers staged in shared memory (fewer resident warps) instead of registers
-template <int G, bool WIDE, bool STG>
-__global__ void __launch_bounds__(kTB, WIDE ? 1 : (STG ? MinB<G>::node_stg : MinB<G>::bounds_reg))
+__global__ void __launch_bounds__(kNT, MinB<G>::bounds)
 k32_bounds(DTopo tp, DGeom<float> g, B32View B, float dt) {
-    __shared__ WEdges Se[kWB];
-    extern __shared__ __align__(16) float dsm[];
-    float *sb = (WIDE || !STG) ? nullptr : dsm + (size_t)(threadIdx.x >> 5) * (stage_bytes_bounds<G>() / 4);
-    FOR_WARP_UNITS(j, node_units<WIDE>(tp)) bounds_unit<G, WIDE, true>(tp, g, B, dt, j, Se, sb);
+    __shared__ NodeTile S;
+    __shared__ BoundsBuf<G> X;
+    FOR_NODE_TILES(ti, tp.n_nt) {
+        node_tile_load(tp, ti, S);
+        bounds_tile<G>(tp, g, B, dt, S, X);
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1678,85 +1244,85 @@ __device__ __forceinline__ void vdiff_unit(const DTopo &tp, const B32View &B, co
 // ---------------------------------------------------------------------------
 // k32_update: limited update, T*
 // ---------------------------------------------------------------------------
-template <int G, int KD, bool PACK>
-__device__ __forceinline__ void update_chunk(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
-                                             int n, int lane, const WEdges &S, int ch, int W, int P) {
-    using C = Chunk<1, 1>;
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
-    const C k = PACK ? C(nzmin, nzmax, ch, lane, W, P) : C(nzmin, nzmax, ch, lane);
-    const int nz = k.nz;
-    const int i = n * L1 + nz - 1, iv = n * nl + nz - 1;
-    const float sdt = k.lvl ? qdiv(dt, g.areasvol[iv] * g.hnode_new[i]) : 0.f;
-    // a dry slot gathers the node's own R (finite); its ADh is not loaded (zero)
-    int off[KD], eo[KD];
-    unsigned okx = 0;
-#pragma unroll
-    for (int u = 0; u < KD; u++) {
-        const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-        off[u] = ok ? S.m[u] * L1 + nz - 1 : i;
-        eo[u] = ok ? S.e[u] * L1 + nz - 1 : 0;
-        okx |= ok ? 1u << u : 0u;
-    }
+template <int G>
+using UpdateBuf = Vec<G>[2][kNT];  // [buffer][thread]: limited interface fluxes
+
+template <int G>
+__device__ __forceinline__ void update_tile(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
+                                            const NodeTile &S, UpdateBuf<G> &X) {
+    constexpr int kUU = MinB<G>::uu;
+    const TileLane k(tp, S);
+    const int x = threadIdx.x, i = k.i, iv = k.iv, nz = k.nz, deg = S.deg[k.j];
+    const bool top = nz == k.nzmin;
+    const float sdt = k.on ? qdiv(dt, g.areasvol[iv] * g.hnode_new[i]) : 0.f;
 #pragma unroll 1
-    for (int g0 = 0; g0 < B.ng; g0 += PACK ? P : 1) {
-        // the lane's group (packed: the group of its segment)
-        const int gq = g0 + k.q;
-        const bool on = gq < B.ng;
-        const int gc = on ? gq : g0;
-        const bool fct = (B.fct >> gc) & 1ull;
-        const bool dif = (B.diff >> gc) & 1ull;
-        const bool lv = k.lvl && on;
-        const bool lf = lv && fct;
-        const float *__restrict__ Rp = grp<G>(B.Rp, gc, B.sN);
-        const float *__restrict__ Rm = grp<G>(B.Rm, gc, B.sN);
-        const float *__restrict__ ADh = grp<G>(B.ADh, gc, B.sE);
-        float *__restrict__ Tn = grp<G>(B.Tnew, gc, B.sN);
-        // every load of the group's chunk first
-        const Vec<G> lo = vldc<G>(lv, grp<G>(B.LO, gc, B.sN), i);
-        const Vec<G> f0 = vldc<G>(lv, grp<G>(B.ADv, gc, B.sNI), iv);
+    for (int gq = 0; gq < B.ng; gq++) {
+        const bool fct = (B.fct >> gq) & 1ull, dif = (B.diff >> gq) & 1ull;
+        const bool lf = k.on && fct;
+        const float *__restrict__ Rp = grp<G>(B.Rp, gq, B.sN);
+        const float *__restrict__ Rm = grp<G>(B.Rm, gq, B.sN);
+        const float *__restrict__ ADh = grp<G>(B.ADh, gq, B.sE);
+        float *__restrict__ Tn = grp<G>(B.Tnew, gq, B.sN);
+        const Vec<G> lo = vldc<G>(k.on, grp<G>(B.LO, gq, B.sN), i);
+        const Vec<G> f0 = vldc<G>(k.on, grp<G>(B.ADv, gq, B.sNI), iv);
         const Vec<G> r0p = lf ? vld<G>(Rp, i) : vfill<G>(1.f);
         const Vec<G> r0m = lf ? vld<G>(Rm, i) : vfill<G>(1.f);
-        const Vec<G> tbp = vldc<G>(lf && kFctClamp, grp<G>(B.Bp, gc, B.sN), i);
-        const Vec<G> tbm = vldc<G>(lf && kFctClamp, grp<G>(B.Bm, gc, B.sN), i);
+        const Vec<G> rup = lf && !top ? vld<G>(Rp, i - 1) : vfill<G>(1.f);
+        const Vec<G> rum = lf && !top ? vld<G>(Rm, i - 1) : vfill<G>(1.f);
+        const Vec<G> tbp = vldc<G>(lf && kFctClamp, grp<G>(B.Bp, gq, B.sN), i);
+        const Vec<G> tbm = vldc<G>(lf && kFctClamp, grp<G>(B.Bm, gq, B.sN), i);
         // the diffusion increment k32_diff parked in Tnew (the limiter acts on advection only)
-        const Vec<G> dd = vldc<G>(lv && dif, Tn, i);
+        const Vec<G> dd = vldc<G>(k.on && dif, Tn, i);
         Vec<G> hs = vfill<G>(0.f);
+        // horizontal limiting (oce_adv_tra_fct.F90:468-500) seen from the node: with G the
+        // antidiffusive flux into the node and m the other end, G >= 0 takes
+        // min(R+(n), R-(m)), G < 0 takes min(R-(n), R+(m))
+#pragma unroll 1
+        for (int u0 = 0; u0 < S.degmax; u0 += kUU) {
+            Vec<G> xe[kUU], rmp[kUU], rmm[kUU];
 #pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> x = vldc<G>(lv && ((okx >> u) & 1u), ADh, eo[u]);
-            const Vec<G> rmp = lf ? vld<G>(Rp, off[u]) : vfill<G>(1.f);
-            const Vec<G> rmm = lf ? vld<G>(Rm, off[u]) : vfill<G>(1.f);
-            const bool ow = (own >> u) & 1u;
-            // horizontal limiting (oce_adv_tra_fct.F90:468-500) seen from the node: with G the
-            // antidiffusive flux into the node and m the other end, G >= 0 takes
-            // min(R+(n), R-(m)), G < 0 takes min(R-(n), R+(m))
+            for (int u = 0; u < kUU; u++) {
+                const int4 q = S.slot[k.j][u0 + u];
+                const bool ok = k.on && u0 + u < deg && slot_wet(q, nz);
+                xe[u] = vldc<G>(ok, ADh, q.y + nz - 1);
+                rmp[u] = vldc<G>(ok && fct, Rp, q.x + nz - 1);
+                rmm[u] = vldc<G>(ok && fct, Rm, q.x + nz - 1);
+            }
 #pragma unroll
-            for (int c = 0; c < G; c++) {
-                float Gf = ow ? x.c[c] : -x.c[c];
-                if (fct) Gf *= Gf >= 0.f ? fminf(r0p.c[c], rmm.c[c]) : fminf(r0m.c[c], rmp.c[c]);
-                hs.c[c] += Gf;
+            for (int u = 0; u < kUU; u++) {
+                const bool ow = S.slot[k.j][u0 + u].w != 0;
+#pragma unroll
+                for (int c = 0; c < G; c++) {
+                    float Gf = ow ? xe[u].c[c] : -xe[u].c[c];
+                    if (fct) Gf *= Gf >= 0.f ? fminf(r0p.c[c], rmm[u].c[c]) : fminf(r0m.c[c], rmp[u].c[c]);
+                    hs.c[c] += Gf;
+                }
             }
         }
+        // vertical limiting (oce_adv_tra_fct.F90:425-456): interface nz by R of layers nz-1 and nz;
+        // the next interface is the next thread's
+        Vec<G> fz = f0;
+        if (fct) {
+#pragma unroll
+            for (int c = 0; c < G; c++) {
+                if (top) fz.c[c] *= fz.c[c] >= 0.f ? r0p.c[c] : r0m.c[c];
+                else fz.c[c] *= fz.c[c] >= 0.f ? fminf(rum.c[c], r0p.c[c]) : fminf(rup.c[c], r0m.c[c]);
+            }
+        }
+        Vec<G>(&xf)[kNT] = X[gq & 1];
+        xf[x] = fz;
+        __syncthreads();
+        if (!k.on) continue;
+        const Vec<G> f1 = nz == k.nzmax - 1 ? vfill<G>(0.f) : xf[x + 1];
         Vec<G> out;
+        bool fin = true;
 #pragma unroll
         for (int c = 0; c < G; c++) {
-            // vertical limiting (oce_adv_tra_fct.F90:425-456): interface nz by R of layers
-            // nz-1 and nz; the next interface is the lane below's
-            const float rux = sh_up(r0p.c[c], 1), ruy = sh_up(r0m.c[c], 1);
-            float fz = f0.c[c];
-            if (fct) {
-                if (nz == nzmin) fz *= fz >= 0.f ? r0p.c[c] : r0m.c[c];
-                else fz *= fz >= 0.f ? fminf(ruy, r0p.c[c]) : fminf(rux, r0m.c[c]);
-            }
-            float f1 = sh_dn(fz, 1);
-            if (nz == nzmax - 1) f1 = 0.f;
             // del_ttf = (LO hnode_new - T hnode) + limited flux divergence dt / areasvol;
             // T* = T + (del_ttf + T (hnode - hnode_new)) / hnode_new = LO + fluxes dt / areasvol / hnode_new
             // (oce_adv_tra_driver.F90:535-620, oce_ale_tracer.F90:319-321, 743-754)
-            float val = lo.c[c] + ((fz - f1) + hs.c[c]) * sdt;
-            if (kFctClamp && k.out && on && fct) {
+            float val = lo.c[c] + ((fz.c[c] - f1.c[c]) + hs.c[c]) * sdt;
+            if (kFctClamp && fct) {
                 const float vc = fminf(fmaxf(val, tbm.c[c]), tbp.c[c]);
                 // a clamp beyond round-off means the limiter itself failed
                 if (fabsf(vc - val) > 1e-5f * (tbp.c[c] - tbm.c[c]) + 1e-6f * fabsf(vc)) atomicOr(B.status, 2u);
@@ -1764,210 +1330,39 @@ __device__ __forceinline__ void update_chunk(const DTopo &tp, const DGeom<float>
             }
             if (dif) val += dd.c[c];
             out.c[c] = val;
+            fin = fin && isfinite(val);
         }
-        if (k.out && on) {
-            vst<G>(Tn, i, out);
-#pragma unroll
-            for (int c = 0; c < G; c++)
-                if (!isfinite(out.c[c])) atomicOr(B.status, 1u);
-        }
+        vst<G>(Tn, i, out);
+        if (!fin) atomicOr(B.status, 1u);
     }
 }
 
-// The same chunk with each pass's gathers staged in shared memory: entries LO, ADv, R+, R-, the
-// two bounds and the parked diffusion increment of the node, then ADh, R+, R- of every slot
-// (a dry slot stages zeros for ADh and the node's own R).
-constexpr int kNsUpdate = 7 + 3 * 6;
-template <int G, int KD, bool PACK>
-__device__ __forceinline__ void update_chunk_pf(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
-                                                int n, int lane, const WEdges &S, int ch, int W, int P, float *sb) {
-    using C = Chunk<1, 1>;
-    constexpr int NS = 7 + 3 * KD;
-    static_assert(NS <= kNsUpdate, "staging sized for six edge slots");
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
-    const C k = PACK ? C(nzmin, nzmax, ch, lane, W, P) : C(nzmin, nzmax, ch, lane);
-    const int nz = k.nz;
-    const int i = n * L1 + nz - 1, iv = n * nl + nz - 1;
-    const float sdt = k.lvl ? qdiv(dt, g.areasvol[iv] * g.hnode_new[i]) : 0.f;
-    int off[KD], eo[KD];
-    unsigned okx = 0;
-#pragma unroll
-    for (int u = 0; u < KD; u++) {
-        const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-        off[u] = ok ? S.m[u] * L1 + nz - 1 : (k.lvl ? i : 0);
-        eo[u] = ok ? S.e[u] * L1 + nz - 1 : 0;
-        okx |= ok ? 1u << u : 0u;
-    }
-    const int npass = PACK ? (B.ng + P - 1) / P : B.ng;
-    // the lane's group in pass p (packed: the group of its segment)
-    auto grp_of = [&](int p) { return PACK ? p * P + k.q : p; };
-    auto issue = [&](int p, float *buf) {
-        const int gq = grp_of(p);
-        const bool on = gq < B.ng;
-        const int gc = on ? gq : 0;
-        const bool lv = k.lvl && on;
-        const bool lf = lv && ((B.fct >> gc) & 1ull);
-        const bool ld = lv && ((B.diff >> gc) & 1ull);
-        const int ii = lv ? i : 0;
-        const float *Rp = grp<G>(B.Rp, gc, B.sN), *Rm = grp<G>(B.Rm, gc, B.sN);
-        const float *ADh = grp<G>(B.ADh, gc, B.sE);
-        cpa<G>(stg<G>(buf, 0, lane), grp<G>(B.LO, gc, B.sN) + (size_t)ii * G, lv);
-        cpa<G>(stg<G>(buf, 1, lane), grp<G>(B.ADv, gc, B.sNI) + (size_t)(lv ? iv : 0) * G, lv);
-        cpa<G>(stg<G>(buf, 2, lane), Rp + (size_t)ii * G, lf);
-        cpa<G>(stg<G>(buf, 3, lane), Rm + (size_t)ii * G, lf);
-        // (without the clamp the bounds are not allocated: the zero-filled copies name LO)
-        cpa<G>(stg<G>(buf, 4, lane), grp<G>(kFctClamp ? B.Bp : B.LO, gc, B.sN) + (size_t)ii * G, lf && kFctClamp);
-        cpa<G>(stg<G>(buf, 5, lane), grp<G>(kFctClamp ? B.Bm : B.LO, gc, B.sN) + (size_t)ii * G, lf && kFctClamp);
-        cpa<G>(stg<G>(buf, 6, lane), grp<G>(B.Tnew, gc, B.sN) + (size_t)ii * G, ld);
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            cpa<G>(stg<G>(buf, 7 + 3 * u, lane), ADh + (size_t)eo[u] * G, lv && ((okx >> u) & 1u));
-            cpa<G>(stg<G>(buf, 8 + 3 * u, lane), Rp + (size_t)off[u] * G, lf);
-            cpa<G>(stg<G>(buf, 9 + 3 * u, lane), Rm + (size_t)off[u] * G, lf);
-        }
-        cpa_commit();
-    };
-    auto compute = [&](int p, float *buf) {
-        const int gq = grp_of(p);
-        const bool on = gq < B.ng;
-        const int gc = on ? gq : 0;
-        const bool fct = (B.fct >> gc) & 1ull;
-        const bool dif = (B.diff >> gc) & 1ull;
-        const Vec<G> lo = lds<G>(stg<G>(buf, 0, lane));
-        const Vec<G> f0 = lds<G>(stg<G>(buf, 1, lane));
-        const Vec<G> r0p = lds<G>(stg<G>(buf, 2, lane));
-        const Vec<G> r0m = lds<G>(stg<G>(buf, 3, lane));
-        Vec<G> hs = vfill<G>(0.f);
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const Vec<G> x = lds<G>(stg<G>(buf, 7 + 3 * u, lane));
-            const bool ow = (own >> u) & 1u;
-            if (fct) {
-                const Vec<G> rmp = lds<G>(stg<G>(buf, 8 + 3 * u, lane));
-                const Vec<G> rmm = lds<G>(stg<G>(buf, 9 + 3 * u, lane));
-#pragma unroll
-                for (int c = 0; c < G; c++) {
-                    float Gf = ow ? x.c[c] : -x.c[c];
-                    Gf *= Gf >= 0.f ? fminf(r0p.c[c], rmm.c[c]) : fminf(r0m.c[c], rmp.c[c]);
-                    hs.c[c] += Gf;
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < G; c++) hs.c[c] += ow ? x.c[c] : -x.c[c];
-            }
-        }
-        const Vec<G> tbp = lds<G>(stg<G>(buf, 4, lane));
-        const Vec<G> tbm = lds<G>(stg<G>(buf, 5, lane));
-        const Vec<G> dd = lds<G>(stg<G>(buf, 6, lane));
-        Vec<G> out;
-#pragma unroll
-        for (int c = 0; c < G; c++) {
-            const float rux = sh_up(r0p.c[c], 1), ruy = sh_up(r0m.c[c], 1);
-            float fz = f0.c[c];
-            if (fct) {
-                if (nz == nzmin) fz *= fz >= 0.f ? r0p.c[c] : r0m.c[c];
-                else fz *= fz >= 0.f ? fminf(ruy, r0p.c[c]) : fminf(rux, r0m.c[c]);
-            }
-            float f1 = sh_dn(fz, 1);
-            if (nz == nzmax - 1) f1 = 0.f;
-            float val = lo.c[c] + ((fz - f1) + hs.c[c]) * sdt;
-            if (kFctClamp && k.out && on && fct) {
-                const float vc = fminf(fmaxf(val, tbm.c[c]), tbp.c[c]);
-                if (fabsf(vc - val) > 1e-5f * (tbp.c[c] - tbm.c[c]) + 1e-6f * fabsf(vc)) atomicOr(B.status, 2u);
-                val = vc;
-            }
-            if (dif) val += dd.c[c];
-            out.c[c] = val;
-        }
-        if (k.out && on) {
-            vst<G>(grp<G>(B.Tnew, gc, B.sN), i, out);
-#pragma unroll
-            for (int c = 0; c < G; c++)
-                if (!isfinite(out.c[c])) atomicOr(B.status, 1u);
-        }
-    };
-    issue(0, sb);
-    float *cur = sb, *nxt = sb + (size_t)NS * 32 * G;
-    for (int p = 0; p < npass; p++) {
-        if (p + 1 < npass) {
-            issue(p + 1, nxt);
-            cpa_wait<1>();
-        } else {
-            cpa_wait<0>();
-        }
-        compute(p, cur);
-        float *t = cur;
-        cur = nxt;
-        nxt = t;
-    }
-}
-
-template <int G, int KD, bool PK>
-__device__ __forceinline__ void update_node(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
-                                            int n, int lane, const WEdges &S, float *sb) {
-    using C = Chunk<1, 1>;
-    const int nch = C::count(S.nzmin, S.nzmax);
-    const int W = C::last_width(S.nzmin, S.nzmax), P = 32 / W;
-    if constexpr (KD == 6) {
-        if (sb) {
-            for (int ch = 0; ch < nch - 1; ch++) update_chunk_pf<G, KD, false>(tp, g, B, dt, n, lane, S, ch, 32, 1, sb);
-            if (PK && P > 1) update_chunk_pf<G, KD, true>(tp, g, B, dt, n, lane, S, nch - 1, W, P, sb);
-            else update_chunk_pf<G, KD, false>(tp, g, B, dt, n, lane, S, nch - 1, 32, 1, sb);
-            return;
-        }
-    }
-    for (int ch = 0; ch < nch - 1; ch++) update_chunk<G, KD, false>(tp, g, B, dt, n, lane, S, ch, 32, 1);
-    if (PK && KD <= 6 && P > 1) update_chunk<G, KD, true>(tp, g, B, dt, n, lane, S, nch - 1, W, P);
-    else update_chunk<G, KD, false>(tp, g, B, dt, n, lane, S, nch - 1, 32, 1);
-}
-
-// VD: the implicit vertical diffusion of the node's column follows its update in the same warp
-// (the diffusion is column-local: it reads only the column's own T*, which the warp has just
-// stored and reads back at L2), so T* is not written to and read back from HBM between two
-// launches.  Vw: the warp's diffusion workspace.
-template <int G, bool WIDE, bool PK, bool VD = false>
-__device__ __forceinline__ void update_unit(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt, int j,
-                                            WEdges *Se, float *sb, const VFactors *vf = nullptr,
-                                            VdiffWarp *Vw = nullptr) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = unit_node<WIDE>(tp, j);
-    if (n < 0) return;
-    WEdges &S = Se[warp];
-    stage_edges(tp, n, lane, S);
-    if ((S.deg > 8) != WIDE) return;
-    if (WIDE) update_node<G, kMaxDeg, PK>(tp, g, B, dt, n, lane, S, nullptr);
-    else if (S.deg <= 6) update_node<G, 6, PK>(tp, g, B, dt, n, lane, S, sb);
-    else update_node<G, 8, PK>(tp, g, B, dt, n, lane, S, nullptr);
-    // (vdiff_unit opens with a __syncwarp: every lane's T* stores are ordered before the reads)
-    if constexpr (VD) vdiff_unit<G, true>(tp, B, *vf, n, *Vw);
-}
-
+// the implicit vertical diffusion of the tile's columns, a warp per column (T* of the whole tile
+// is written before the block's barrier)
 template <int G>
-__host__ __device__ constexpr int stage_bytes_update() { return 2 * kNsUpdate * 32 * G * 4; }
+__device__ __forceinline__ void update_tile_vdiff(const DTopo &tp, const B32View &B, const VFactors &vf,
+                                                  const NodeTile &S, VdiffWarp *W) {
+    __syncthreads();
+    const int warp = threadIdx.x >> 5;
+    for (int j = warp; j < S.cnt; j += kNT / 32) vdiff_unit<G, true>(tp, B, vf, S.n0 + j, W[warp]);
+}
 
 // VD: with the implicit vertical diffusion of the groups in ivd & ~wimpl as the epilogue of each
-// node (factors vf); its workspace is the warp's staging buffer in the staged variant (idle once
-// the node's last pass has landed), static shared memory otherwise
-template <int G, bool WIDE, bool STG, bool VD>
-__global__ void __launch_bounds__(kTB, WIDE ? 1 : (STG ? MinB<G>::node_stg : MinB<G>::update_reg))
+// tile (factors vf)
+template <int G, bool VD>
+__global__ void __launch_bounds__(kNT, MinB<G>::update)
 k32_update(DTopo tp, DGeom<float> g, B32View B, float dt, VFactors vf) {
-    __shared__ WEdges Se[kWB];
-    extern __shared__ __align__(16) float dsm[];
-    constexpr bool kStaged = STG && !WIDE;
-    static_assert(sizeof(VdiffWarp) <= stage_bytes_update<G>(), "diffusion workspace inside the staging");
-    float *sb = kStaged ? dsm + (size_t)(threadIdx.x >> 5) * (stage_bytes_update<G>() / 4) : nullptr;
-    VdiffWarp *Vw = nullptr;
-    if constexpr (VD) {
-        if constexpr (kStaged) {
-            Vw = reinterpret_cast<VdiffWarp *>(sb);
-        } else {
-            __shared__ VdiffWarp Wsm[kWB];
-            Vw = &Wsm[threadIdx.x >> 5];
-        }
+    __shared__ NodeTile S;
+    __shared__ union {
+        UpdateBuf<G> X;
+        VdiffWarp W[VD ? kNT / 32 : 1];
+    } U;
+    FOR_NODE_TILES(ti, tp.n_nt) {
+        node_tile_load(tp, ti, S);
+        update_tile<G>(tp, g, B, dt, S, U.X);
+        if (VD) update_tile_vdiff<G>(tp, B, vf, S, U.W);
+        __syncthreads();
     }
-    FOR_WARP_UNITS(j, node_units<WIDE>(tp)) update_unit<G, WIDE, true, VD>(tp, g, B, dt, j, Se, sb, &vf, Vw);
 }
 
 // ---------------------------------------------------------------------------
@@ -2637,17 +2032,20 @@ __global__ void __launch_bounds__(kTB) k32m_vfactors(const Inst32 *__restrict__ 
         vfactors_col(I[i].tp, I[i].g, I[i].f, I[i].dt, I[i].vf, u - ix.start[i], threadIdx.x & 31);
     }
 }
-// WS: some instance has the split vertical velocity (each instance checks its own switch)
-template <bool WIDE, bool WS>
-__global__ void __launch_bounds__(kTB, WIDE ? 1 : MinB<4>::lo) k32m_lo_ad(const Inst32 *__restrict__ I, MultiIdx ix) {
-    __shared__ WEdges Se[kWB];
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        if (I[i].B.G == 4)
-            lo_ad_unit<4, WIDE, WS, true>(I[i].tp, I[i].g, I[i].f, I[i].B, I[i].VF, I[i].dt, u - ix.start[i], Se, nullptr);
-        else
-            lo_ad_unit<2, WIDE, WS, true>(I[i].tp, I[i].g, I[i].f, I[i].B, I[i].VF, I[i].dt, u - ix.start[i], Se, nullptr);
-    }
+// units: node tiles, one block each.  WS: some instance has the split vertical velocity (each
+// instance checks its own switch)
+template <bool WS>
+__global__ void __launch_bounds__(kNT, MinB<4>::lo) k32m_lo_ad(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ NodeTile S;
+    __shared__ union {
+        LoBuf<4> X4;
+        LoBuf<2> X2;
+    } U;
+    const int i = find_inst(ix, blockIdx.x);
+    const Inst32 &d = I[i];
+    node_tile_load(d.tp, blockIdx.x - ix.start[i], S);
+    if (d.B.G == 4) lo_ad_tile<4, WS>(d.tp, d.g, d.f, d.B, d.VF, d.dt, S, U.X4);
+    else lo_ad_tile<2, WS>(d.tp, d.g, d.f, d.B, d.VF, d.dt, S, U.X2);
 }
 __global__ void __launch_bounds__(kTileThreads, MinB<4>::ho) k32m_ho(const Inst32 *__restrict__ I, MultiIdx ix) {
     __shared__ Tile S;
@@ -2663,34 +2061,37 @@ __global__ void __launch_bounds__(256) k32m_ho_nodemean(const Inst32 *__restrict
     if (I[i].B.G == 4) nodemean_item<4>(I[i].tp, I[i].B, I[i].mw, I[i].VF, u - ix.start[i]);
     else nodemean_item<2>(I[i].tp, I[i].B, I[i].mw, I[i].VF, u - ix.start[i]);
 }
-template <bool WIDE>
-__global__ void __launch_bounds__(kTB, WIDE ? 1 : MinB<4>::node_reg) k32m_bounds(const Inst32 *__restrict__ I, MultiIdx ix) {
-    __shared__ WEdges Se[kWB];
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        if (I[i].B.G == 4) bounds_unit<4, WIDE, true>(I[i].tp, I[i].g, I[i].B, I[i].dt, u - ix.start[i], Se, nullptr);
-        else bounds_unit<2, WIDE, true>(I[i].tp, I[i].g, I[i].B, I[i].dt, u - ix.start[i], Se, nullptr);
-    }
+__global__ void __launch_bounds__(kNT, MinB<4>::bounds) k32m_bounds(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ NodeTile S;
+    __shared__ union {
+        BoundsBuf<4> X4;
+        BoundsBuf<2> X2;
+    } U;
+    const int i = find_inst(ix, blockIdx.x);
+    const Inst32 &d = I[i];
+    node_tile_load(d.tp, blockIdx.x - ix.start[i], S);
+    if (d.B.G == 4) bounds_tile<4>(d.tp, d.g, d.B, d.dt, S, U.X4);
+    else bounds_tile<2>(d.tp, d.g, d.B, d.dt, S, U.X2);
 }
-// each node's column is then diffused by the same warp where its instance has groups in
-// ivd & ~wimpl (as k32_update with the diffusion epilogue)
-template <bool WIDE>
-__global__ void __launch_bounds__(kTB, WIDE ? 1 : MinB<4>::node_reg) k32m_update(const Inst32 *__restrict__ I, MultiIdx ix) {
-    __shared__ WEdges Se[kWB];
-    __shared__ VdiffWarp Wsm[kWB];
-    VdiffWarp *Vw = &Wsm[threadIdx.x >> 5];
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        const Inst32 &d = I[i];
-        const bool vd = (d.B.ivd & ~d.B.wimpl) != 0;
-        const int j = u - ix.start[i];
-        if (d.B.G == 4) {
-            if (vd) update_unit<4, WIDE, true, true>(d.tp, d.g, d.B, d.dt, j, Se, nullptr, &d.vf, Vw);
-            else update_unit<4, WIDE, true>(d.tp, d.g, d.B, d.dt, j, Se, nullptr);
-        } else {
-            if (vd) update_unit<2, WIDE, true, true>(d.tp, d.g, d.B, d.dt, j, Se, nullptr, &d.vf, Vw);
-            else update_unit<2, WIDE, true>(d.tp, d.g, d.B, d.dt, j, Se, nullptr);
-        }
+// a tile's columns are then diffused where its instance has groups in ivd & ~wimpl (as k32_update
+// with the diffusion epilogue)
+__global__ void __launch_bounds__(kNT, MinB<4>::update) k32m_update(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ NodeTile S;
+    __shared__ union {
+        UpdateBuf<4> X4;
+        UpdateBuf<2> X2;
+        VdiffWarp W[kNT / 32];
+    } U;
+    const int i = find_inst(ix, blockIdx.x);
+    const Inst32 &d = I[i];
+    node_tile_load(d.tp, blockIdx.x - ix.start[i], S);
+    const bool vd = (d.B.ivd & ~d.B.wimpl) != 0;
+    if (d.B.G == 4) {
+        update_tile<4>(d.tp, d.g, d.B, d.dt, S, U.X4);
+        if (vd) update_tile_vdiff<4>(d.tp, d.B, d.vf, S, U.W);
+    } else {
+        update_tile<2>(d.tp, d.g, d.B, d.dt, S, U.X2);
+        if (vd) update_tile_vdiff<2>(d.tp, d.B, d.vf, S, U.W);
     }
 }
 __global__ void __launch_bounds__(kTB) k32m_vppm(const Inst32 *__restrict__ I, MultiIdx ix) {
@@ -2737,11 +2138,9 @@ __global__ void __launch_bounds__(kTB) k32m_diff(const Inst32 *__restrict__ I, M
 // ---------------------------------------------------------------------------
 // launch wrappers
 // ---------------------------------------------------------------------------
-// warp-per-unit kernels: one warp per unit, or at most blocks_per_sm blocks per SM looping
-static int grid_units(int units, const LaunchShape &sh) {
-    int b = (units + kWB - 1) / kWB;
-    if (sh.blocks_per_sm > 0 && b > 152 * sh.blocks_per_sm) b = 152 * sh.blocks_per_sm;
-    return b < 1 ? 1 : b;
+// node-tile kernels: one block per tile, or at most blocks_per_sm blocks per SM looping
+static int grid_tiles(int tiles, const LaunchShape &sh) {
+    return sh.blocks_per_sm > 0 ? std::min(tiles, 152 * sh.blocks_per_sm) : tiles;
 }
 static int grid_nodes(int n) { return (n + kWB - 1) / kWB; }
 static int grid_flat(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 32); }
@@ -2755,78 +2154,18 @@ void b32_vfactors(const DTopo &tp, const DGeom<float> &g, const DForcing<float> 
     k32_vfactors<<<grid_nodes(tp.N2), kTB, 0, s>>>(tp, g, f, (float)dt, v);
 }
 
-// dynamic shared memory of the staged node kernels: kWB warps' staging
-template <int G>
-constexpr int smem_lo_ad() { return kWB * stage_bytes_lo_ad<G>(); }
-template <int G>
-constexpr int smem_bounds() { return kWB * stage_bytes_bounds<G>(); }
-template <int G>
-constexpr int smem_update() { return kWB * stage_bytes_update<G>(); }
-
-template <int G>
-static cudaError_t prepare_g() {
-    cudaError_t e = cudaSuccess;
-    auto set = [&](const void *fn, int bytes) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    };
-    set((const void *)k32_lo_ad<G, false, false, true>, smem_lo_ad<G>());
-    set((const void *)k32_lo_ad<G, false, true, true>, smem_lo_ad<G>());
-    set((const void *)k32_bounds<G, false, true>, smem_bounds<G>());
-    set((const void *)k32_update<G, false, true, false>, smem_update<G>());
-    set((const void *)k32_update<G, false, true, true>, smem_update<G>());
-    return e;
-}
 bool b32_fct_clamp() { return kFctClamp; }
 
-cudaError_t b32_prepare() {
-    static cudaError_t done = cudaErrorNotReady;
-    if (done == cudaSuccess) return done;
-    cudaError_t e = prepare_g<4>();
-    if (e == cudaSuccess) e = prepare_g<2>();
-    done = e;
-    return e;
-}
-
-template <int G, bool WS>
-static void lo_ad_gw(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, const B32View &B,
-                     const float *VF, double dt, const LaunchShape &sh, cudaStream_t s) {
-    if (sh.staged)
-        k32_lo_ad<G, false, WS, true><<<grid_units(tp.N2, sh), kTB, smem_lo_ad<G>(), s>>>(tp, g, f, B, VF, (float)dt);
-    else
-        k32_lo_ad<G, false, WS, false><<<grid_units(tp.N2, sh), kTB, 0, s>>>(tp, g, f, B, VF, (float)dt);
-    if (tp.n_wide) k32_lo_ad<G, true, WS, false><<<grid_nodes(tp.n_wide), kTB, 0, s>>>(tp, g, f, B, VF, (float)dt);
-}
-template <int G>
-static void lo_ad_g(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, const B32View &B, const float *VF,
-                    double dt, const LaunchShape &sh, cudaStream_t s) {
-    if (f.wsplit) lo_ad_gw<G, true>(tp, g, f, B, VF, dt, sh, s);
-    else lo_ad_gw<G, false>(tp, g, f, B, VF, dt, sh, s);
-}
-template <int G>
-static void bounds_g(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, const LaunchShape &sh,
-                     cudaStream_t s) {
-    if (sh.staged) k32_bounds<G, false, true><<<grid_units(tp.N2, sh), kTB, smem_bounds<G>(), s>>>(tp, g, B, (float)dt);
-    else k32_bounds<G, false, false><<<grid_units(tp.N2, sh), kTB, 0, s>>>(tp, g, B, (float)dt);
-    if (tp.n_wide) k32_bounds<G, true, false><<<grid_nodes(tp.n_wide), kTB, 0, s>>>(tp, g, B, (float)dt);
-}
-template <int G, bool VD>
-static void update_gv(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, const LaunchShape &sh,
-                      const VFactors &vf, cudaStream_t s) {
-    const float d = (float)dt;
-    if (sh.staged) k32_update<G, false, true, VD><<<grid_units(tp.N2, sh), kTB, smem_update<G>(), s>>>(tp, g, B, d, vf);
-    else k32_update<G, false, false, VD><<<grid_units(tp.N2, sh), kTB, 0, s>>>(tp, g, B, d, vf);
-    if (tp.n_wide) k32_update<G, true, false, VD><<<grid_nodes(tp.n_wide), kTB, 0, s>>>(tp, g, B, d, vf);
-}
-template <int G>
-static void update_g(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, const LaunchShape &sh,
-                     const VFactors *vf, cudaStream_t s) {
-    if (vf) update_gv<G, true>(tp, g, B, dt, sh, *vf, s);
-    else update_gv<G, false>(tp, g, B, dt, sh, VFactors{}, s);
-}
 void b32_lo_ad(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f, const B32View &B, const float *VF,
                double dt, const LaunchShape &sh, cudaStream_t s) {
-    if (B.G == 4) lo_ad_g<4>(tp, g, f, B, VF, dt, sh, s);
-    else lo_ad_g<2>(tp, g, f, B, VF, dt, sh, s);
+    const int nb = grid_tiles(tp.n_nt, sh);
+    if (B.G == 4) {
+        if (f.wsplit) k32_lo_ad<4, true><<<nb, kNT, 0, s>>>(tp, g, f, B, VF, (float)dt);
+        else k32_lo_ad<4, false><<<nb, kNT, 0, s>>>(tp, g, f, B, VF, (float)dt);
+    } else {
+        if (f.wsplit) k32_lo_ad<2, true><<<nb, kNT, 0, s>>>(tp, g, f, B, VF, (float)dt);
+        else k32_lo_ad<2, false><<<nb, kNT, 0, s>>>(tp, g, f, B, VF, (float)dt);
+    }
 }
 template <int G>
 static void ho_g(const DTopo &tp, const B32View &B, const MusclW &mw, const float *VF, const LaunchShape &sh,
@@ -2847,13 +2186,21 @@ void b32_ho(const DTopo &tp, const DGeom<float> &, const B32View &B, const Muscl
 }
 void b32_bounds(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, const LaunchShape &sh,
                 cudaStream_t s) {
-    if (B.G == 4) bounds_g<4>(tp, g, B, dt, sh, s);
-    else bounds_g<2>(tp, g, B, dt, sh, s);
+    const int nb = grid_tiles(tp.n_nt, sh);
+    if (B.G == 4) k32_bounds<4><<<nb, kNT, 0, s>>>(tp, g, B, (float)dt);
+    else k32_bounds<2><<<nb, kNT, 0, s>>>(tp, g, B, (float)dt);
+}
+template <int G>
+static void update_g(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, int nb, const VFactors *vf,
+                     cudaStream_t s) {
+    if (vf) k32_update<G, true><<<nb, kNT, 0, s>>>(tp, g, B, (float)dt, *vf);
+    else k32_update<G, false><<<nb, kNT, 0, s>>>(tp, g, B, (float)dt, VFactors{});
 }
 void b32_update(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, const LaunchShape &sh,
                 const VFactors *vf, cudaStream_t s) {
-    if (B.G == 4) update_g<4>(tp, g, B, dt, sh, vf, s);
-    else update_g<2>(tp, g, B, dt, sh, vf, s);
+    const int nb = grid_tiles(tp.n_nt, sh);
+    if (B.G == 4) update_g<4>(tp, g, B, dt, nb, vf, s);
+    else update_g<2>(tp, g, B, dt, nb, vf, s);
 }
 void b32_vdiff(const DTopo &tp, const DForcing<float> &, const B32View &B, const VFactors &v, cudaStream_t s) {
     if (B.G == 4) k32_vdiff<4><<<(tp.N2 + kWV - 1) / kWV, 32 * kWV, 0, s>>>(tp, B, v);
@@ -2975,16 +2322,11 @@ void bm32_vfactors(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
     if (u) k32m_vfactors<<<grid_nodes(u), kTB, 0, s>>>(I, ix);
 }
-void bm32_lo_ad(const Inst32 *I, const MultiIdx &ix, bool wide, bool ws, cudaStream_t s) {
+void bm32_lo_ad(const Inst32 *I, const MultiIdx &ix, bool ws, cudaStream_t s) {
     const int u = ix.start[ix.n];
     if (!u) return;
-    if (ws) {
-        if (wide) k32m_lo_ad<true, true><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-        else k32m_lo_ad<false, true><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-    } else {
-        if (wide) k32m_lo_ad<true, false><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-        else k32m_lo_ad<false, false><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-    }
+    if (ws) k32m_lo_ad<true><<<u, kNT, 0, s>>>(I, ix);
+    else k32m_lo_ad<false><<<u, kNT, 0, s>>>(I, ix);
 }
 void bm32_vppm(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
@@ -3003,17 +2345,13 @@ void bm32_ho(const Inst32 *I, const MultiIdx &ix_e, const MultiIdx &ix_items, cu
     const int u = ix_items.start[ix_items.n];
     if (u) k32m_ho_nodemean<<<(u + 255) / 256, 256, 0, s>>>(I, ix_items);
 }
-void bm32_bounds(const Inst32 *I, const MultiIdx &ix, bool wide, cudaStream_t s) {
+void bm32_bounds(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
-    if (!u) return;
-    if (wide) k32m_bounds<true><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-    else k32m_bounds<false><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
+    if (u) k32m_bounds<<<u, kNT, 0, s>>>(I, ix);
 }
-void bm32_update(const Inst32 *I, const MultiIdx &ix, bool wide, cudaStream_t s) {
+void bm32_update(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
-    if (!u) return;
-    if (wide) k32m_update<true><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-    else k32m_update<false><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
+    if (u) k32m_update<<<u, kNT, 0, s>>>(I, ix);
 }
 void bm32_hdiff(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];

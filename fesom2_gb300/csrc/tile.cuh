@@ -15,6 +15,9 @@ namespace fesom {
 constexpr int kTileThreads = 128;
 constexpr int kTileMax = 8;  // entities per tile
 
+// tiles of nodes of the FP32 form, cut once per mesh: wet levels (= threads) and nodes of a tile
+constexpr int kNodeTileLevels = 256, kNodeTileNodes = 32;
+
 // the wet levels of a tile's entities as items 0 .. total-1: entity j holds the items
 // pre[j] .. pre[j+1]-1, levels top[j], top[j] + 1, ...
 struct Tile {

@@ -306,20 +306,19 @@ int fesom_gpu_set_wsplit(fesom_gpu_ctx *ctx, int32_t on);
 int fesom_gpu_set_stage_tracers(fesom_gpu_ctx *ctx, int32_t stage, int32_t tracers);
 /* Performance setting of the FP32 form (results do not change): grid of the node/edge stage
  * kernels (stages as in fesom_gpu_set_stage_tracers): blocks_per_sm > 0 launches at most
- * blocks_per_sm x 152 blocks whose warps loop over the units (nodes, edges); 0 (the default)
- * launches one warp per unit. */
+ * blocks_per_sm x 152 blocks looping over the tiles of nodes; 0 (the default) launches one block
+ * per tile.  The edge stage always launches one block per tile. */
 int fesom_gpu_set_launch_shape(fesom_gpu_ctx *ctx, int32_t stage, int32_t blocks_per_sm);
 /* Performance setting of the FP32 form: kernel variant of stage 0 (lo_ad), 1 (the edge fluxes),
- * 2 (bounds) or 3 (update): bit 0 clear gathers each pass's entries into registers, set stages
- * them in shared memory with asynchronous copies while the previous pass computes (fewer resident
- * warps, no register limit on the gathers in flight).  Stage 3 only, bit 1 (values 2, 3): the
- * implicit vertical diffusion runs as its own kernel after the update; clear (the default), each
- * node's column is diffused by the warp that has just updated it, in the same launch.  Defaults:
- * lo_ad 1, the others 0.  The variants are separate compilations and agree to FP32 round-off. */
+ * 2 (bounds) or 3 (update).  Bit 0 is kept and reported but selects nothing: each stage has one
+ * kernel.  Stage 3 only, bit 1 (values 2, 3): the implicit vertical diffusion runs as its own
+ * kernel after the update; clear (the default), the block that has updated a tile of nodes
+ * diffuses its columns in the same launch.  Results do not change.  Defaults: lo_ad 1, the
+ * others 0. */
 int fesom_gpu_set_stage_variant(fesom_gpu_ctx *ctx, int32_t stage, int32_t variant);
 /* Autotuner of the FP32 form's launch settings (results do not change): times the step of the
  * context's own state under the library defaults, then by coordinate descent over the four node/edge
- * stages under each kernel variant, blocks per SM (0, 2, 4) and, for bounds and update with more
+ * stages under blocks per SM (0, 2, 4), the place of the diffusion and, for bounds and update with more
  * than 8 tracer slots, 8 tracers per launch; a candidate is kept when it is more than 1 % faster.
  * Each candidate runs one untimed and `steps` timed steps (CUDA events on the context's stream).
  * The fastest settings stay on the context; the tracer state and its time levels are restored
