@@ -816,7 +816,7 @@ int enqueue_step(fesom_gpu_ctx *ctx, double dt, StageTimer *tm = nullptr) {
         // all tracers of a group share the valuesold depth of the context
         STAGE(0, Launch<R>::ab(ctx->tp, tr, ctx->ab_max, ctx->stream));
         if (any_ho || ctx->Ki) STAGE(1, Launch<R>::trxy(ctx->tp, g, tr, ctx->stream));
-        STAGE(2, Launch<R>::edge_flux(ctx->tp, g, f, tr, any_fct, ctx->stream));
+        STAGE(2, Launch<R>::edge_flux(ctx->tp, g, f, tr, any_ho, ctx->stream));
         STAGE(3, Launch<R>::node_lo(ctx->tp, g, f, tr, dt, any_fct, ctx->stream));
         // split vertical velocity: w_i advects the LO values implicitly (oce_adv_tra_driver.F90:323-334)
         if (ctx->wsplit && any_fct) STAGE(3, Launch<R>::lo_impl(ctx->tp, g, f, tr, dt, ctx->scratch, ctx->stream));
@@ -1323,7 +1323,7 @@ int fesom_gpu_adv_tra(fesom_gpu_ctx *ctx, double dt, const double *vel, const do
     DForcing<double> f = forcing_view<double>(ctx, 0);
     const int fct = cfg->adv_lim == FESOM_ADV_LIM_FCT;
     if (cfg->adv_hor != FESOM_ADV_HOR_UPW1) Launch<double>::trxy(ctx->tp, ctx->g64, tr, ctx->stream);
-    Launch<double>::edge_flux(ctx->tp, ctx->g64, f, tr, fct, ctx->stream);
+    Launch<double>::edge_flux(ctx->tp, ctx->g64, f, tr, cfg->adv_hor != FESOM_ADV_HOR_UPW1, ctx->stream);
     Launch<double>::node_lo(ctx->tp, ctx->g64, f, tr, dt, fct, ctx->stream);
     if (fct && ctx->wsplit) Launch<double>::lo_impl(ctx->tp, ctx->g64, f, tr, dt, ctx->scratch, ctx->stream);
     if (fct) {

@@ -276,7 +276,8 @@ struct Launch {
     static void trxy(const DTopo &, const DGeom<R> &, DTracers<R> &, cudaStream_t);
     // tracer_gradient_z of T into trz (nl per node)
     static void trz(const DTopo &, const DGeom<R> &, const R *T, R *trz, cudaStream_t);
-    static void edge_flux(const DTopo &, const DGeom<R> &, const DForcing<R> &, DTracers<R> &, int fct, cudaStream_t);
+    // any_ho: some tracer has a horizontal scheme other than UPW1
+    static void edge_flux(const DTopo &, const DGeom<R> &, const DForcing<R> &, DTracers<R> &, int any_ho, cudaStream_t);
     static void node_lo(const DTopo &, const DGeom<R> &, const DForcing<R> &, DTracers<R> &, double dt, int fct,
                         cudaStream_t);
     // FCT bounds and the ratios R+ / R- (into bmax / bmin)

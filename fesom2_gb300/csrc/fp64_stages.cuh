@@ -13,6 +13,8 @@
 //     (47 layers are 32 + 15 lanes), and an FP64 instruction costs its 16 cycles however many
 //     lanes take part.
 #pragma once
+#include <type_traits>
+
 #include "fesom_internal.h"
 #include "fp64_arith.cuh"
 #include "tile.cuh"
@@ -145,8 +147,13 @@ struct EdgeData {
     double dX1, dY1, dX2, dY2, ca, cb;  // ca = edge_dxdy(1) a, cb = edge_dxdy(2) r_earth
 };
 
+// The edge-layers whose gradients are node means (the last layers over a slope, every layer at a
+// coast: 2 % of a sphere's) cost five times the others' instructions, and lie in half of the
+// warps: they are set aside and take their own passes, full warps again.
 static __global__ void __launch_bounds__(kTileThreads)
-k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, int tile) {
+k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, int tile, int any_ho) {
+    extern __shared__ int aside[];
+    __shared__ int n_aside;
     __shared__ Tile S;
     __shared__ EdgeData Ed[kTileMax];
     const int L1 = tp.L1, e0 = blockIdx.x * tile;
@@ -186,10 +193,17 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
         }
         S.fill(j, ok ? tp.e_lo[e] : 1, ok ? tp.e_hi[e] - tp.e_lo[e] + 1 : 0);
     }
+    if (threadIdx.x == 32) n_aside = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+    auto layer = [&](int i, auto pass) {
+        constexpr bool means = decltype(pass)::value;
         const int j = S.find(i), nz = S.top[j] + i - S.pre[j];
         const EdgeData &E = Ed[j];
+        const bool tri = nz >= E.gmin && nz <= E.gmax;
+        if (!means && !tri && any_ho) {
+            aside[atomicAdd(&n_aside, 1)] = i;
+            return;
+        }
         const size_t ke = ix1(nz, e0 + j, L1), k1 = ix1(nz, E.n1, L1), k2 = ix1(nz, E.n2, L1);
         // segment rule of the reference's five loops (A..E)
         const int fnl12 = min(E.nl1, E.nl2), fnu12 = max(E.nu1, E.nu2);
@@ -212,7 +226,6 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
             vf = (seg == 3) ? vf + v2 : v2;
         }
         const bool neg = neg64(vf), vbad = nonfinite64(vf);
-        const bool tri = nz >= E.gmin && nz <= E.gmax;
         for (int t = 0; t < tr.ntr; t++) {
             const DCfg c = tr.cfg[t];
             double flo = 0.0, ad = 0.0;
@@ -225,17 +238,17 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
                 } else {
                     const double *txy = tr.trxy + t * tr.sT;
                     if (c.ph == 0.0 && !vbad && !nonfinite64(t1) && !nonfinite64(t2) &&
-                        !grad_bad(tp, txy, tri, neg ? E.up : E.dn, neg ? E.n1 : E.n2, nz)) {
+                        !grad_bad(tp, txy, !means, neg ? E.up : E.dn, neg ? E.n1 : E.n2, nz)) {
                         double2 gr;
-                        if (tri) gr = reinterpret_cast<const double2 *>(txy)[ix1(nz, neg ? E.dn : E.up, L1)];
-                        else node_mean_grad(tp, g, txy, neg ? E.n2 : E.n1, nz, gr.x, gr.y);
+                        if (means) node_mean_grad(tp, g, txy, neg ? E.n2 : E.n1, nz, gr.x, gr.y);
+                        else gr = reinterpret_cast<const double2 *>(txy)[ix1(nz, neg ? E.dn : E.up, L1)];
                         // 2 (t2 - t1) is exact: one rounding in the fused sum, as in the reference's
                         double q = div_3x2k<6>(__fma_rn(2.0, t2 - t1, E.ca * gr.x) + E.cb * gr.y);
                         if (c.hor == 0 && (neg ? E.nbl2 : E.nbl1) < nz) q = q * 0.0;
                         const double Tm = (neg ? t2 : t1) + (neg ? -q : q);
                         ad = -(Tm * vf) - flo;
                     } else {
-                        ad = edge_ho_full(tp, g, txy, c, tri, E.up, E.dn, E.n1, E.n2, nz, t1, t2, vf, E.ca, E.cb,
+                        ad = edge_ho_full(tp, g, txy, c, !means, E.up, E.dn, E.n1, E.n2, nz, t1, t2, vf, E.ca, E.cb,
                                           E.nbl1 >= nz, E.nbl2 >= nz, flo);
                     }
                 }
@@ -243,7 +256,10 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
             if (c.lim) tr.FLO[t * tr.sE + ke] = flo;
             tr.ADh[t * tr.sE + ke] = ad;
         }
-    }
+    };
+    for (int i = threadIdx.x; i < S.total; i += kTileThreads) layer(i, std::false_type{});
+    __syncthreads();
+    for (int q = threadIdx.x; q < n_aside; q += kTileThreads) layer(aside[q], std::true_type{});
 }
 
 // ===========================================================================
@@ -587,10 +603,10 @@ static __global__ void __launch_bounds__(kVThreads) k_vdiff_tile(VArgs P, DTrace
                                                                  int wsplit) {
     extern __shared__ __align__(16) double sm64[];
     __shared__ VTile S;
-    const int n0 = blockIdx.x * kVCols;
+    const int n0 = blockIdx.x * P.cols;
     if (threadIdx.x < 32) {
         const int n = n0 + threadIdx.x;
-        const bool ok = n < P.N2;
+        const bool ok = threadIdx.x < P.cols && n < P.N2;
         S.fill(threadIdx.x, ok ? P.ulev[n] : 1, ok ? P.nlev[n] - P.ulev[n] : 0);
     }
     // the implicit part of a split vertical velocity joins the solve without a limiter (:961)
@@ -643,9 +659,10 @@ void Launch<double>::trxy(const DTopo &tp, const DGeom<double> &g, DTracers<doub
 }
 template <>
 void Launch<double>::edge_flux(const DTopo &tp, const DGeom<double> &g, const DForcing<double> &f, DTracers<double> &tr,
-                               int, cudaStream_t s) {
-    const int t = tile_size(tp.E2, 0);
-    k_edge_flux<<<(tp.E2 + t - 1) / t, kTileThreads, 0, s>>>(tp, g, f, tr, t);
+                               int any_ho, cudaStream_t s) {
+    const size_t b = sizeof(int) * tp.L1;
+    const int t = tile_size(tp.E2, b);
+    k_edge_flux<<<(tp.E2 + t - 1) / t, kTileThreads, t * b, s>>>(tp, g, f, tr, t, any_ho);
 }
 template <>
 void Launch<double>::node_lo(const DTopo &tp, const DGeom<double> &g, const DForcing<double> &f, DTracers<double> &tr,
@@ -671,16 +688,18 @@ void Launch<double>::update(const DTopo &tp, const DGeom<double> &g, DTracers<do
 template <>
 void Launch<double>::vdiff(const DTopo &tp, const DGeom<double> &g, const DForcing<double> &f, DTracers<double> &tr,
                            double dt, double *scratch, cudaStream_t s) {
-    if (vtile_smem(tp.L1, 1) > kVSmemMax) {
+    if (vtile_smem(tp.L1, kVCols, 1) > kVSmemMax) {
         k_vdiff<double><<<(tp.N2 + 127) / 128, 128, 0, s>>>(tp, g, f, tr, dt, scratch);
         return;
     }
     // as many tracers at a time as share the coefficients with two blocks resident per SM
     int nt = std::min(tr.ntr, 4);
-    while (nt > 1 && vtile_smem(tp.L1, nt) > kVSmemMax / 2) nt--;
-    const VArgs P{tp.N2, tp.nl, tp.n_nlev, tp.n_ulev, g.zbar_n_bot, g.hnode_new, g.area, g.areasvol, f.Kv, f.wi, dt};
-    const int nb = (tp.N2 + kVCols - 1) / kVCols;
-    const size_t sm = vtile_smem(tp.L1, nt);
+    while (nt > 1 && vtile_smem(tp.L1, kVCols, nt) > kVSmemMax / 2) nt--;
+    const int cols = vtile_cols(tp.N2, nt);
+    const VArgs P{tp.N2, tp.nl,      cols, tp.n_nlev, tp.n_ulev, g.zbar_n_bot, g.hnode_new,
+                  g.area, g.areasvol, f.Kv, f.wi,      g.rav,     dt};
+    const int nb = (tp.N2 + cols - 1) / cols;
+    const size_t sm = vtile_smem(tp.L1, cols, nt);
     if (nt == 1) k_vdiff_tile<1><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);
     else if (nt == 2) k_vdiff_tile<2><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);
     else if (nt == 3) k_vdiff_tile<3><<<nb, kVThreads, sm, s>>>(P, tr, f.bc, f.wsplit);

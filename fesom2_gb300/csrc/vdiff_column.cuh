@@ -10,6 +10,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fp64_arith.cuh"
+
 namespace fesom {
 
 struct ColScratch {
@@ -118,21 +120,46 @@ __device__ __forceinline__ void vdiff_col_solve(const ColScratch &s, int nzmin, 
 // the same solve for a tile of 32 columns in shared memory
 // ---------------------------------------------------------------------------
 // A thread per column (above) reads every array with the stride of a column (32 lines per warp
-// load) and runs one chain of five divisions per level, four warps to an SM on a mesh of 20k
-// nodes.  Here only the recurrences themselves (mid-depths, pivots, substitutions) run a lane per
+// load) and runs one chain of five divisions per level.  Here only the recurrences run a lane per
 // column; coefficients and right-hand sides are formed by all 128 threads, the wet levels of the
-// tile dealt out one after another (coalesced, full warps).  Up to 4 tracers share the
-// coefficients and the pivots.  Entry (level, column) of a shared array sits at level * 33 +
-// column: both a lane per column and a lane per level touch 32 different bank pairs.
-// Deeper columns than the shared memory holds (217 layers) take the thread per column.
-constexpr int kVCols = 32, kVThreads = 128, kVPad = kVCols + 1;
+// tile dealt out one after another (coalesced, full warps), and up to 4 tracers share the
+// coefficients and the pivots.
+//
+// What bounds it is the FP64 unit: a warp issues a dependent or independent FP64 instruction every
+// 64 cycles whatever its active lanes, and an SM one every 19 (measured; a division is 9 of them).
+// A recurrence is one warp's work, so the pivots (11 instructions a level) and each tracer's
+// elimination (11) run on different warps, the tracers a chunk of 8 levels behind the pivots.
+//
+// Entry (level, column) of a shared array sits at level * pad + column with an odd pad: both a lane
+// per column and a lane per level touch different banks.  Deeper columns than the shared memory
+// holds (217 layers) take the thread per column.
+constexpr int kVCols = 32, kVThreads = 256, kVChunk = 8;
 constexpr size_t kVSmemMax = 224 * 1024;
-__host__ __device__ constexpr size_t vtile_smem(int L1, int nt) { return (size_t)(3 + nt) * L1 * kVPad * sizeof(double); }
+__host__ __device__ constexpr size_t vtile_smem(int L1, int cols, int nt) {
+    return (size_t)(3 + nt) * L1 * (cols | 1) * sizeof(double);
+}
+// columns per tile: the recurrences cost an SM 12 + 13 nt FP64 instructions per level and tile, the
+// rest 29 + 9 nt per 32 columns and level; the widest tile unless a narrower one shares the tiles
+// out better over the 152 SMs (2.9k columns: 20, one tile on each of 146 SMs)
+inline int vtile_cols(int n, int nt) {
+    int best = kVCols;
+    double cost = 0.0;
+    for (int c = kVCols; c >= 8; c--) {
+        const int waves = ((n + c - 1) / c + 151) / 152;
+        const double x = waves * (12.0 + 13.0 * nt + (29.0 + 9.0 * nt) * c / 32.0);
+        if (c == kVCols || x < 0.98 * cost) {
+            best = c;
+            cost = x;
+        }
+    }
+    return best;
+}
 
 struct VArgs {
-    int N2, nl;
+    int N2, nl, cols;
     const int *nlev, *ulev;
     const double *zbot, *hn, *ar, *av, *kv, *wi;
+    const double2 *rav;  // reciprocals of av (recip64), null: none at hand
     double dt;
 };
 struct VTracer {
@@ -141,7 +168,7 @@ struct VTracer {
 };
 
 struct VTile {
-    int total;
+    int total, lo, hi;  // items; first and last level of any column
     int pre[kVCols + 1], top[kVCols];
     __device__ __forceinline__ void fill(int lane, int first_level, int levels) {
         int s = levels;
@@ -153,7 +180,13 @@ struct VTile {
         pre[lane + 1] = s;
         top[lane] = first_level;
         if (lane == 0) pre[0] = 0;
-        if (lane == 31) total = s;
+        const int l0 = __reduce_min_sync(0xffffffffu, levels ? first_level : 1 << 20);
+        const int l1 = __reduce_max_sync(0xffffffffu, levels ? first_level + levels - 1 : 0);
+        if (lane == 31) {
+            total = s;
+            lo = l0;
+            hi = l1;
+        }
     }
     __device__ __forceinline__ int find(int i) const {
         int j = i >= pre[16] ? 16 : 0;
@@ -168,13 +201,13 @@ struct VTile {
 template <int NT>
 __device__ __forceinline__ void vdiff_tile(const VArgs &P, const VTile &S, int n0, double *sm, const VTracer *tr, int nt,
                                            bool wimpl) {
-    const int L1 = P.nl - 1, nl = P.nl;
-    const size_t sz = (size_t)L1 * kVPad;
+    const int L1 = P.nl - 1, nl = P.nl, pad = P.cols | 1;
+    const size_t sz = (size_t)L1 * pad;
     double *HB = sm, *ZR = sm + sz, *A = sm + 2 * sz, *C = sm + 3 * sz;  // h then b, Z then the first rhs, a, c
     auto R = [&](int t) { return t == 0 ? ZR : sm + (3 + t) * sz; };
 #define FOR_ITEMS                                                                                      \
-    for (int i = threadIdx.x; i < S.total; i += kVThreads) {                                           \
-        const int j = S.find(i), nz = S.top[j] + i - S.pre[j], x = (nz - 1) * kVPad + j;               \
+    _Pragma("unroll 2") for (int i = threadIdx.x; i < S.total; i += kVThreads) {                                           \
+        const int j = S.find(i), nz = S.top[j] + i - S.pre[j], x = (nz - 1) * pad + j;               \
         const bool top = i == S.pre[j], bot = i + 1 == S.pre[j + 1];                                   \
         const size_t k = (size_t)(n0 + j) * L1 + nz - 1, kv = (size_t)(n0 + j) * nl + nz - 1;          \
         (void)top; (void)bot; (void)k; (void)kv; (void)x;
@@ -182,30 +215,33 @@ __device__ __forceinline__ void vdiff_tile(const VArgs &P, const VTile &S, int n
         HB[x] = P.hn[k];
     }
     __syncthreads();
-    const int lane = threadIdx.x;
-    int lo = 0, hi = -1;  // shared-memory rows of the lane's column
-    if (lane < kVCols) {
-        lo = (S.top[lane] - 1) * kVPad + lane;
-        hi = lo + (S.pre[lane + 1] - S.pre[lane] - 1) * kVPad;
-        if (hi >= lo) {  // Z_n from the bottom up (src/oce_ale_tracer.F90:1088-1096)
-            double zb = P.zbot[n0 + lane];
-            for (int x = hi; x >= lo; x -= kVPad) {
-                const double h = HB[x];
-                ZR[x] = zb + h / 2.0;
-                zb = zb + h;
-            }
+    // warp 0: depths and pivots; warp 1 + t: tracer t
+    const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
+    const int r0 = S.top[lane] - 1, r1 = r0 + S.pre[lane + 1] - S.pre[lane] - 1;  // rows of the lane's column
+    if (role == 0) {  // bottom depth of every layer (src/oce_ale_tracer.F90:1088-1096)
+        double zb = r1 >= r0 ? P.zbot[n0 + lane] : 0.0;
+        for (int r = r1; r >= r0; r--) {
+            ZR[r * pad + lane] = zb;
+            zb = zb + HB[r * pad + lane];
         }
     }
     __syncthreads();
+    FOR_ITEMS
+        ZR[x] = ZR[x] + HB[x] / 2.0;  // Z_n
+    }
+    __syncthreads();
     // the interface above layer nz: a(nz) and c(nz - 1)
+    auto by_av = [&](double num, size_t i) {
+        return P.rav ? sdiv64(num, P.av[i], P.rav[i]) : num / P.av[i];
+    };
     FOR_ITEMS
         if (top) {
             A[x] = 0.0;
-            C[((S.top[j] - 1) + (S.pre[j + 1] - S.pre[j] - 1)) * kVPad + j] = 0.0;
+            C[((S.top[j] - 1) + (S.pre[j + 1] - S.pre[j] - 1)) * pad + j] = 0.0;
         } else {
-            const double q = P.kv[kv] * (1.0 / (ZR[x - kVPad] - ZR[x])) * P.dt, ar = P.ar[kv];
-            A[x] = -(q * (ar / P.av[kv]));
-            C[x - kVPad] = -(q * ar / P.av[kv - 1]);
+            const double q = P.kv[kv] * (1.0 / (ZR[x - pad] - ZR[x])) * P.dt, ar = P.ar[kv];
+            A[x] = -(q * by_av(ar, kv));
+            C[x - pad] = -by_av(q * ar, kv - 1);
         }
     }
     __syncthreads();
@@ -241,48 +277,44 @@ __device__ __forceinline__ void vdiff_tile(const VArgs &P, const VTile &S, int n
         }
     }
     __syncthreads();
-    if (lane < kVCols && hi >= lo) {
-        // forward elimination (:1406-1414), the next level's entries loaded a level ahead
-        double cp = 0.0, tp[NT], an = A[lo], bn = HB[lo], cn = C[lo], rn[NT];
-#pragma unroll
-        for (int t = 0; t < NT; t++) {
-            tp[t] = 0.0;
-            rn[t] = t < nt ? R(t)[lo] : 0.0;
-        }
-        for (int x = lo; x <= hi; x += kVPad) {
-            const double a = an, b = bn, c = cn;
-            double r[NT];
-#pragma unroll
-            for (int t = 0; t < NT; t++) r[t] = rn[t];
-            if (x < hi) {
-                an = A[x + kVPad];
-                bn = HB[x + kVPad];
-                cn = C[x + kVPad];
-#pragma unroll
-                for (int t = 0; t < NT; t++)
-                    if (t < nt) rn[t] = R(t)[x + kVPad];
+    // forward elimination (:1406-1414): the pivots m (into HB) and cp (into C), and the tracers a
+    // chunk of levels behind; at the top layer a = 0 and cp = tp = 0
+    {
+        double cp = 0.0, y = 0.0;
+        for (int c0 = S.lo - 1; c0 <= S.hi - 1 + kVChunk; c0 += kVChunk) {
+            if (role == 0) {
+                const int e = min(c0 + kVChunk - 1, r1);
+                for (int r = max(c0, r0); r <= e; r++) {
+                    const int x = r * pad + lane;
+                    const double m = HB[x] - cp * A[x];
+                    cp = C[x] / m;
+                    C[x] = cp;
+                    HB[x] = m;
+                }
             }
-            const double m = b - cp * a;
-            cp = c / m;
-            C[x] = cp;
 #pragma unroll
-            for (int t = 0; t < NT; t++)
-                if (t < nt) {
-                    tp[t] = (r[t] - tp[t] * a) / m;
-                    R(t)[x] = tp[t];
+            for (int t = 0; t < NT; t++) {
+                if (t >= nt || role != 1 + t) continue;
+                double *Rt = R(t);
+                const int e = min(c0 - 1, r1);
+                for (int r = max(c0 - kVChunk, r0); r <= e; r++) {
+                    const int x = r * pad + lane;
+                    y = (Rt[x] - y * A[x]) / HB[x];
+                    Rt[x] = y;
                 }
+            }
+            __syncthreads();
         }
-        // back substitution (:1417-1430); C is 0 at the bottom layer
+    }
+    // back substitution (:1417-1430); C is 0 at the bottom layer
 #pragma unroll
-        for (int t = 0; t < NT; t++) tp[t] = 0.0;
-        for (int x = hi; x >= lo; x -= kVPad) {
-            const double c = C[x];
-#pragma unroll
-            for (int t = 0; t < NT; t++)
-                if (t < nt) {
-                    tp[t] = R(t)[x] - c * tp[t];
-                    R(t)[x] = tp[t];
-                }
+    for (int t = 0; t < NT; t++) {
+        if (t >= nt || role != 1 + t) continue;
+        double *Rt = R(t), y = 0.0;
+        for (int r = r1; r >= r0; r--) {
+            const int x = r * pad + lane;
+            y = Rt[x] - C[x] * y;
+            Rt[x] = y;
         }
     }
     __syncthreads();

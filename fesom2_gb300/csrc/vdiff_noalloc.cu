@@ -99,11 +99,11 @@ k_vdiff_noalloc_tile(fesom::VArgs P, const double *__restrict__ bc_surf, double 
                      unsigned *status) {
     extern __shared__ __align__(16) double sm64[];
     __shared__ fesom::VTile S;
-    const int n0 = blockIdx.x * fesom::kVCols;
+    const int n0 = blockIdx.x * P.cols;
     if (threadIdx.x < 32) {
         const int n = n0 + threadIdx.x;
         int lo = 1, m = 0;
-        if (n < P.N2) {
+        if (threadIdx.x < P.cols && n < P.N2) {
             const int nzmax = P.nlev[n], nzmin = P.ulev[n];
             if (nzmin < 1 || nzmax > P.nl || nzmax - nzmin < 2) {
                 atomicOr(status, FESOM_STATUS_INDEX);
@@ -178,11 +178,11 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
     }
     // columns that fit a tile's shared memory leave the scratch alone (19.6k columns of 47 layers:
     // NOALLOC_NEW us against 217 us with a thread per column)
-    const size_t sm = fesom::vtile_smem(nl - 1, 1);
-    if (sm <= fesom::kVSmemMax) {
-        const fesom::VArgs P{nod2D, nl, nlevels_nod2D, ulevels_nod2D, zbar_n_bot, hnode_new, area, areasvol, Kv,
-                             nullptr, dt};
-        k_vdiff_noalloc_tile<<<(nod2D + fesom::kVCols - 1) / fesom::kVCols, fesom::kVThreads, sm, s>>>(
+    if (fesom::vtile_smem(nl - 1, fesom::kVCols, 1) <= fesom::kVSmemMax) {
+        const int cols = fesom::vtile_cols(nod2D, 1);
+        const fesom::VArgs P{nod2D,     nl,   cols, nlevels_nod2D, ulevels_nod2D, zbar_n_bot, hnode_new, area,
+                             areasvol, Kv,   nullptr, nullptr,     dt};
+        k_vdiff_noalloc_tile<<<(nod2D + cols - 1) / cols, fesom::kVThreads, fesom::vtile_smem(nl - 1, cols, 1), s>>>(
             P, bc_surf, values, st.status);
     } else {
         const int threads = 128;

@@ -73,3 +73,30 @@ def test_vertical_diffusion_tiles_bitwise(nx, ny, layers, ntr):
     om.diff_ver_part_impl_ale(f, want)
     ctx.vdiff_impl(f, G.tra_cfg(), got)
     assert np.array_equal(got, want)
+
+
+def test_element_lists_beside_the_edges_bitwise():
+    """A mesh whose nod_in_elem2D lists leave out an element of some nodes: the bounds of those nodes
+    come from the listed elements, not from the neighbours over the edges, as in the oracle."""
+    mesh = M.channel_mesh(9, 13, 5000.0, M.stretched_zbar(33, 10.0, 200.0), seamounts=2, seed=5, partial_cells=True)
+    ptr, keep = mesh.nod_in_elem2D_ptr, np.ones(mesh.nod_in_elem2D.size, dtype=bool)
+    short = [n for n in range(5, mesh.nod2D, 7) if ptr[n + 1] - ptr[n] == 6]
+    keep[[ptr[n + 1] - 1 for n in short]] = False
+    drop = np.zeros(mesh.nod2D, dtype=np.int64)
+    drop[short] = 1
+    mesh.nod_in_elem2D_ptr = (ptr - np.concatenate([[0], np.cumsum(drop)])).astype(np.int32)
+    mesh.nod_in_elem2D = np.ascontiguousarray(mesh.nod_in_elem2D[keep])
+    f = O.ensure_f64(M.make_forcing(mesh, "channel", seed=3, dt=600.0))
+    T = np.ascontiguousarray(M.make_tracers(mesh, "channel", ntr=1, seed=4)[0])
+    rng = np.random.default_rng(8)
+    T *= 1.0 + 0.05 * rng.standard_normal(T.shape)
+    TAB = np.ascontiguousarray(T * (1.0 + 1e-3 * rng.standard_normal(T.shape)))
+    om, cfg = O.OracleMesh(mesh), O.cfg_struct()
+    om.init_tracers_AB(cfg, T.copy(), np.zeros_like(T), T.copy())
+    om.do_oce_adv_tra(f, cfg, T, TAB)
+    ctx = G.Context(mesh, G.PREC_FP64)
+    dh, dv = ctx.adv_tra(f, G.tra_cfg(), T, TAB)
+    lev = np.arange(1, mesh.nl)[None, :]
+    wet = (lev >= mesh.ulevels_nod2D[:, None]) & (lev <= mesh.nlevels_nod2D[:, None] - 1)
+    assert np.array_equal(dh[wet], om.work["del_ttf_advhoriz"][wet])
+    assert np.array_equal(dv[wet], om.work["del_ttf_advvert"][wet])
