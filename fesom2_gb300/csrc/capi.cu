@@ -941,11 +941,10 @@ int launches_per_step(fesom_gpu_ctx *ctx) {
         for (int g0 = 0; g0 < ctx->ngr; g0 += ctx->group) {
             const int ng = std::min(ctx->group, ctx->ngr - g0);
             const B32View B = view32(ctx, g0, ng);
-            // lo_ad, update (+ bounds); diff, launched again for the wide nodes; ho (+ its node-mean
+            // lo_ad, update (+ bounds, diff); ho (+ its node-mean
             // edge-layers); vdiff
-            const int wide = ctx->tp.n_wide ? 2 : 1;
             auto passes = [&](int k) { return (ng + stage_group(ctx, k, ng) - 1) / stage_group(ctx, k, ng); };
-            n += passes(0) + passes(3) + (B.fct ? passes(2) : 0) + wide * (B.diff ? 1 : 0) +
+            n += passes(0) + passes(3) + (B.fct ? passes(2) : 0) + (B.diff ? 1 : 0) +
                  passes(1) * (ctx->mw.n_items ? 2 : 1) + (((B.ivd & ~B.wimpl) && ctx->shape[3].vsep) ? 1 : 0) +
                  (ctx->Ki ? 1 : 0) +
                  (B.ppm ? 1 : 0) + ((ctx->wsplit && B.fct) ? 1 : 0) + (B.wimpl ? 1 : 0);
@@ -1105,15 +1104,6 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
         (rc = upload_int(ctx, &tp.ne_ptr, h.ne_ptr)) || (rc = upload_int(ctx, &tp.ne_idx, h.ne_idx)) ||
         (rc = upload_int(ctx, &tp.nie_ptr, h.nie_ptr)) || (rc = upload_int(ctx, &tp.nie_idx, h.nie_idx)))
         return rc;
-    // nodes of more than 8 edges: the FP32 node kernels give them a launch of their own
-    {
-        std::vector<int> wide;
-        for (int n = 0; n < ctx->N2; n++)
-            if (h.ne_ptr[n + 1] - h.ne_ptr[n] > 8) wide.push_back(n);
-        tp.n_wide = (int)wide.size();
-        tp.wide_nodes = nullptr;
-        if (!wide.empty() && (rc = upload_int(ctx, &tp.wide_nodes, wide))) return rc;
-    }
     // tiles of consecutive nodes for the FP32 node kernels
     tp.n_nt = 0;
     tp.nt_ptr = nullptr;
@@ -2385,7 +2375,7 @@ struct fesom_gpu_batch {
     cudaStream_t stream = nullptr;
     Inst32 *d_inst = nullptr;  // ab descriptor sets (one per rotation phase), inst.size() each
     double d_dt = -1.0;
-    MultiIdx ix_e{}, ix_et{}, ix_n{}, ix_nt{}, ix_w{}, ix_it{};  // edges, edge tiles, nodes, node tiles, wide nodes, node-mean items
+    MultiIdx ix_et{}, ix_n{}, ix_nt{}, ix_it{};  // edge tiles, nodes, node tiles, node-mean items
     int maxL1 = 0;
     bool any_vd = false, any_fct = false, any_hd = false, any_diff = false;
     bool any_ws = false, any_ppm = false, any_lo_impl = false, any_wimpl = false;
@@ -2440,18 +2430,14 @@ int batch_descriptors(fesom_gpu_batch *b, double dt) {
 
 void enqueue_batch_step(fesom_gpu_batch *b, cudaStream_t s) {
     const Inst32 *I = b->d_inst + (size_t)b->phase * b->inst.size();
-    const bool wide = b->ix_w.start[b->ix_w.n] > 0;
     bm32_vflux(I, b->ix_et, s);
     if (b->any_vd) bm32_vfactors(I, b->ix_n, s);
     bm32_lo_ad(I, b->ix_nt, b->any_ws, s);
     if (b->any_ppm) bm32_vppm(I, b->ix_n, s);
     if (b->any_lo_impl) bm32_lo_impl(I, b->ix_n, s);
     bm32_ho(I, b->ix_et, b->ix_it, s);
-    if (b->any_hd) bm32_hdiff(I, b->ix_e, s);
-    if (b->any_diff) {
-        bm32_diff(I, b->ix_n, false, s);
-        if (wide) bm32_diff(I, b->ix_w, true, s);
-    }
+    if (b->any_hd) bm32_hdiff(I, b->ix_et, s);
+    if (b->any_diff) bm32_diff(I, b->ix_nt, s);
     if (b->any_fct) bm32_bounds(I, b->ix_nt, s);
     // (the implicit vertical diffusion runs inside the update, per tile)
     bm32_update(I, b->ix_nt, s);
@@ -2471,7 +2457,7 @@ int fesom_gpu_batch_create(fesom_gpu_ctx *const *ctxs, int32_t n, fesom_gpu_batc
         b->err = "a batch holds 1 to 64 FP32 contexts";
         return FESOM_ERR_ARG;
     }
-    std::vector<int> ce, cet, cn, cnt, cw, cit;
+    std::vector<int> cet, cn, cnt, cit;
     for (int i = 0; i < n; i++) {
         fesom_gpu_ctx *c = ctxs[i];
         if (!c || c->prec != FESOM_PREC_FP32) { b->err = "batch instances must be FP32 contexts"; return FESOM_ERR_ARG; }
@@ -2503,18 +2489,14 @@ int fesom_gpu_batch_create(fesom_gpu_ctx *const *ctxs, int32_t n, fesom_gpu_batc
         b->any_diff |= c->Ki != nullptr;
         b->maxL1 = std::max(b->maxL1, c->L1);
         b->inst.push_back(c);
-        ce.push_back(c->E2);
         cet.push_back((c->E2 + kTileMax - 1) / kTileMax);
         cn.push_back(c->N2);
         cnt.push_back(c->tp.n_nt);
-        cw.push_back(c->tp.n_wide);
         cit.push_back(c->mw.n_items);
     }
-    set_prefix(b->ix_e, ce);
     set_prefix(b->ix_et, cet);
     set_prefix(b->ix_n, cn);
     set_prefix(b->ix_nt, cnt);
-    set_prefix(b->ix_w, cw);
     set_prefix(b->ix_it, cit);
     BCK(cudaMalloc((void **)&b->d_inst, sizeof(Inst32) * (size_t)n * b->ab));
     return FESOM_OK;
@@ -2576,10 +2558,9 @@ int fesom_gpu_batch_run_steps(fesom_gpu_batch *b, double dt, int32_t nsteps, int
 
 int fesom_gpu_batch_launches_per_step(fesom_gpu_batch *b, int32_t *launches) {
     if (!b || !launches) return FESOM_ERR_ARG;
-    const bool wide = b->ix_w.start[b->ix_w.n] > 0;
     // vflux, vfactors (the diffusion itself runs inside the update), lo_ad and update (+ bounds),
-    // diff per node range, ho (+ its node-mean items), the optional stages
-    int n = 1 + (b->any_vd ? 1 : 0) + 2 + (b->any_fct ? 1 : 0) + (b->any_diff ? (wide ? 2 : 1) : 0) + 1 +
+    // diff, ho (+ its node-mean items), the optional stages
+    int n = 1 + (b->any_vd ? 1 : 0) + 2 + (b->any_fct ? 1 : 0) + (b->any_diff ? 1 : 0) + 1 +
             (b->ix_it.start[b->ix_it.n] ? 1 : 0) + (b->any_hd ? 1 : 0) + (b->any_ppm ? 1 : 0) +
             (b->any_lo_impl ? 1 : 0) + (b->any_wimpl ? 1 : 0);
     *launches = n;

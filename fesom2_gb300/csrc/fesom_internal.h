@@ -31,8 +31,6 @@ struct DTopo {
     const int *n_nlev, *n_ulev, *n_nlevmin, *n_ulevmax, *n_nbl;
     const int *ne_ptr, *ne_idx;    // node -> edge, idx >= 0: node is edges(1,e); ~e: node is edges(2,e)
     const int *nie_ptr, *nie_idx;  // node -> element, ascending element order
-    int n_wide;                    // nodes of more than 8 edges (FP32 form: their own launch)
-    const int *wide_nodes;
     // FP32 form: node tile i holds the nodes nt_ptr[i] .. nt_ptr[i + 1] - 1 (tile.cuh)
     int n_nt;
     const int *nt_ptr;
@@ -185,7 +183,7 @@ void b32_lo_impl(const DTopo &, const DGeom<float> &, const DForcing<float> &, c
 void b32_vdiff_w(const DTopo &, const DGeom<float> &, const DForcing<float> &, const B32View &, double dt,
                  double *scratch, cudaStream_t);
 void b32_hdiff(const DTopo &, const DGeom<float> &, const B32View &, cudaStream_t);
-// Redi: K33 (nl per node) = Kv + Kd s^2 of the implicit solve (FP64 arithmetic, FP32 result)
+// Redi: K33 (nl per node) = Kv + Kd s^2 of the implicit solve (two-FP32 arithmetic, rounded once)
 void b32_k33(const DTopo &, const DGeom<float> &, const float *Kv, const float *Ki, const float *slope, float *K33,
              cudaStream_t);
 void b32_diff(const DTopo &, const DGeom<float> &, const B32View &, double dt, cudaStream_t);
@@ -248,8 +246,8 @@ void bm32_vdiff_w(const Inst32 *, const MultiIdx &nodes, cudaStream_t);
 void bm32_ho(const Inst32 *, const MultiIdx &edge_tiles, const MultiIdx &items, cudaStream_t);
 void bm32_bounds(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 void bm32_update(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
-void bm32_hdiff(const Inst32 *, const MultiIdx &edges, cudaStream_t);
-void bm32_diff(const Inst32 *, const MultiIdx &nodes, bool wide, cudaStream_t);
+void bm32_hdiff(const Inst32 *, const MultiIdx &edge_tiles, cudaStream_t);
+void bm32_diff(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 
 // reciprocals of a divisor array for DGeom::rav / rhn (kernels_fp64.cu)
 // shared-memory limits of the FP64 kernels, once per context (kernels_fp64.cu)

@@ -94,6 +94,7 @@ constexpr unsigned kFull = 0xffffffffu;
 //   ho     G=2: 1.62 (5 blocks) 1.00 (8) 0.94 (9) 1.04 (10) 1.20 (12); G=4: 4.00 (5) 4.02 (6) 4.70 (8)
 //   lo     G=2: 1.30 (4) 1.34 (5) 1.40 (6); G=4: 4.30 (2) 3.64 (3) 3.60 (4) 4.34 (5)
 //   bounds G=2: 1.15 (5 x 2 slots) 1.21 (4 x 3) 1.30 (4 x 6); G=4: 5.54 (4 x 3) 5.84 (3 x 3) 6.26 (4 x 2)
+//   hdiff  G=4, Redi: 0.70 (6 to 8, with ho) 0.68 (9); diff 0.65 (2) 0.47 (3) 0.41 (4)
 //   update G=2: 1.70 (5 x 1) 1.76 (5 x 2) 1.98 (4 x 6); G=4: 7.16 (3 x 2) 7.55 (4 x 2) 8.17 (3 x 3)
 template <int G>
 struct MinB {
@@ -101,6 +102,8 @@ struct MinB {
     static constexpr int ho = G == 4 ? 6 : 9;  // blocks of kTileThreads
     static constexpr int bounds = G == 4 ? 4 : 5, ub = G == 4 ? 3 : 2;
     static constexpr int update = G == 4 ? 3 : 5, uu = G == 4 ? 2 : 1;
+    static constexpr int hdiff = 9;  // blocks of kTileThreads
+    static constexpr int diff = 4;
 };
 
 __device__ __forceinline__ size_t i1(int nz, int n, int L1) { return (size_t)n * L1 + (nz - 1); }
@@ -286,38 +289,6 @@ __global__ void __launch_bounds__(kTB) k32_vfactors(DTopo tp, DGeom<float> g, DF
                                                     VFactors vf) {
     for (int n = blockIdx.x * kWB + (threadIdx.x >> 5); n < tp.N2; n += gridDim.x * kWB)
         vfactors_col(tp, g, f, dt, vf, n, threadIdx.x & 31);
-}
-
-// ---------------------------------------------------------------------------
-// per-warp staging of the node's edge list (one warp per node)
-// ---------------------------------------------------------------------------
-struct WEdges {
-    int e[kMaxDeg], m[kMaxDeg], lo[kMaxDeg], hi[kMaxDeg];
-    unsigned own;  // bit j: the node is edges(1, e_j) (it owns the edge flux)
-    int deg, nzmin, nzmax;
-};
-
-__device__ __forceinline__ void stage_edges(const DTopo &tp, int n, int lane, WEdges &S) {
-    __syncwarp();  // every lane is done with the previous node's list (grid-stride loops)
-    const int k0 = tp.ne_ptr[n];
-    const int deg = min(tp.ne_ptr[n + 1] - k0, kMaxDeg);
-    int code = 0;
-    if (lane < deg) {
-        code = tp.ne_idx[k0 + lane];
-        const int e = code >= 0 ? code : ~code;
-        S.e[lane] = e;
-        S.m[lane] = code >= 0 ? tp.e_n2[e] : tp.e_n1[e];
-        S.lo[lane] = tp.e_lo[e];
-        S.hi[lane] = tp.e_hi[e];
-    }
-    const unsigned own = __ballot_sync(kFull, lane < deg && code >= 0);
-    if (lane == 0) {
-        S.own = own;
-        S.deg = deg;
-        S.nzmin = tp.n_ulev[n];
-        S.nzmax = tp.n_nlev[n];
-    }
-    __syncwarp();
 }
 
 // chunk ch of a column, HU halo levels above and HD below the stored levels
@@ -719,17 +690,6 @@ k32_lo_ad(DTopo tp, DGeom<float> g, DForcing<float> f, B32View B, const float *_
         lo_ad_tile<G, WS>(tp, g, f, B, VF, dt, S, X);
         __syncthreads();
     }
-}
-
-// the node of warp unit j: consecutive nodes, or (WIDE) the listed nodes of more than 8 edges
-template <bool WIDE>
-__device__ __forceinline__ int unit_node(const DTopo &tp, int j) {
-    if (WIDE) return j < tp.n_wide ? tp.wide_nodes[j] : -1;
-    return j < tp.N2 ? j : -1;
-}
-template <bool WIDE>
-__device__ __forceinline__ int node_units(const DTopo &tp) {
-    return WIDE ? tp.n_wide : tp.N2;
 }
 
 // grid-stride loop of the warps over the units (one launch may hold fewer blocks than units)
@@ -1659,123 +1619,142 @@ __global__ void __launch_bounds__(128) k32_vdiff_w(DTopo tp, DGeom<float> g, DFo
 // (tracer_gradient_z, 0 at the column's top and bottom interfaces), S_xy Tz = (Tz(n1) S(n1)
 // + Tz(n2) S(n2)) / 2 (:1583-1595)
 //
-// 1 / dz of the vertical gradient at interface nz of node n (0 where tr_z is 0)
-__device__ __forceinline__ float trz_rdz(const DTopo &tp, const DGeom<float> &g, int n, int nz) {
-    if (nz <= tp.n_ulev[n] || nz >= tp.n_nlev[n]) return 0.f;
-    const int i = n * tp.L1 + nz - 1;
-    return 2.f / (g.hnode[i - 1] + g.hnode[i]);
+// A tile of edges, as k32_ho.  The element gradients, projected on the edge's cross vectors, are
+// weights of the differences to T(edges(1,e)) formed once per edge: 4 + 4 gathers (the elements'
+// nodes, the layers next to both ends) per edge-layer and group where gradients of two elements and
+// vertical differences took 12, and a third of the arithmetic.  Latency of the gathers bounds it: 1.10
+// -> 0.39 ms on the sphere of 7 subdivisions, 47 layers, 7 tracers with Redi.
+struct EdgeD {
+    int ia, ib, xa, xb, l1, l2;          // first entries of the columns of both ends, the elements' third nodes, the elements
+    int nl1, ul1, nl2, ul2;              // levels of the elements
+    int top1, bot1, top2, bot2;          // ulevels / nlevels of the end nodes
+    float dX1, dY1, dX2, dY2;
+    float w1b, w1x, w2b, w2x, w3b, w3x, w3y;  // projected gradients as weights of T(node) - T(edges(1,e))
+};
+
+// gradient_sca of element el at node n: d/dx and d/dy weights
+__device__ __forceinline__ float2 gs_at(const DTopo &tp, const DGeom<float> &g, int el, int n) {
+    const int k = tp.t_n[3 * el] == n ? 0 : tp.t_n[3 * el + 1] == n ? 1 : 2;
+    const float *gs = g.gs + 6 * (size_t)el;
+    return make_float2(gs[k], gs[3 + k]);
 }
 
+// tile ti of `tile` edges
 template <int G>
-__device__ __forceinline__ void hdiff_edge32(const DTopo &tp, const DGeom<float> &g, const B32View &B, int e) {
-    const int lane = threadIdx.x & 31;
-    if (e >= tp.E2 || !B.Ki) return;
-    const int L1 = tp.L1;
-    const int el1 = tp.e_t1[e], el2 = tp.e_t2[e], n1 = tp.e_n1[e], n2 = tp.e_n2[e];
-    const int nl1 = tp.t_nlev[el1] - 1, ul1 = tp.t_ulev[el1];
-    int nl2 = 0, ul2 = 0;
-    const float dX1 = g.ecd[4 * (size_t)e], dY1 = g.ecd[4 * (size_t)e + 1];
-    float dX2 = 0.f, dY2 = 0.f;
-    const int a0 = tp.t_n[3 * el1], a1 = tp.t_n[3 * el1 + 1], a2 = tp.t_n[3 * el1 + 2];
-    const float *gs1 = g.gs + 6 * (size_t)el1;
-    int b0 = a0, b1 = a1, b2 = a2;
-    const float *gs2 = gs1;
-    if (el2 >= 0) {
-        nl2 = tp.t_nlev[el2] - 1;
-        ul2 = tp.t_ulev[el2];
-        dX2 = g.ecd[4 * (size_t)e + 2];
-        dY2 = g.ecd[4 * (size_t)e + 3];
-        b0 = tp.t_n[3 * el2];
-        b1 = tp.t_n[3 * el2 + 1];
-        b2 = tp.t_n[3 * el2 + 2];
-        gs2 = g.gs + 6 * (size_t)el2;
-    }
-    const float p0 = gs1[0], p1 = gs1[1], p2 = gs1[2], p3 = gs1[3], p4 = gs1[4], p5 = gs1[5];
-    const float q0 = gs2[0], q1 = gs2[1], q2 = gs2[2], q3 = gs2[3], q4 = gs2[4], q5 = gs2[5];
-    const int nl12 = min(nl1, nl2), ul12 = max(ul1, ul2);
-    const bool redi = B.slope != nullptr;
-    for (int nz0 = tp.e_lo[e]; nz0 <= tp.e_hi[e]; nz0 += 32) {
-        const int nz = nz0 + lane;
-        if (nz > tp.e_hi[e]) continue;
-        // Redi: 1/dz of the gradients above and below the layer at both nodes, the slopes
-        float ru1 = 0.f, rd1 = 0.f, ru2 = 0.f, rd2 = 0.f, sx1 = 0.f, sy1 = 0.f, sx2 = 0.f, sy2 = 0.f;
-        if (redi) {
-            ru1 = trz_rdz(tp, g, n1, nz);
-            rd1 = trz_rdz(tp, g, n1, nz + 1);
-            ru2 = trz_rdz(tp, g, n2, nz);
-            rd2 = trz_rdz(tp, g, n2, nz + 1);
-            const float *s1 = B.slope + 3 * (size_t)(n1 * L1 + nz - 1), *s2 = B.slope + 3 * (size_t)(n2 * L1 + nz - 1);
-            sx1 = s1[0];
-            sy1 = s1[1];
-            sx2 = s2[0];
-            sy2 = s2[1];
+__device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &g, const B32View &B, int ti, int tile,
+                                           Tile &S, EdgeD *Ed) {
+    const int L1 = tp.L1, e0 = ti * tile;
+    if (!B.Ki) return;
+    if (threadIdx.x < 32) {
+        const int j = threadIdx.x, e = e0 + j;
+        const bool in = j < tile && e < tp.E2;
+        if (in) {
+            EdgeD &E = Ed[j];
+            const int n1 = tp.e_n1[e], n2 = tp.e_n2[e], el1 = tp.e_t1[e], el2 = tp.e_t2[e];
+            const float4 d = reinterpret_cast<const float4 *>(g.ecd)[e];
+            auto third = [&](int el) { return tp.t_n[3 * el] + tp.t_n[3 * el + 1] + tp.t_n[3 * el + 2] - n1 - n2; };
+            const int x1 = third(el1);
+            const float2 b1 = gs_at(tp, g, el1, n2), c1 = gs_at(tp, g, el1, x1);
+            E.ia = n1 * L1;
+            E.ib = n2 * L1;
+            E.xa = x1 * L1;
+            E.l1 = el1 * L1;
+            E.nl1 = tp.t_nlev[el1] - 1;
+            E.ul1 = tp.t_ulev[el1];
+            E.dX1 = d.x;
+            E.dY1 = d.y;
+            E.w1b = d.y * b1.x - d.x * b1.y;
+            E.w1x = d.y * c1.x - d.x * c1.y;
+            E.xb = E.l2 = 0;
+            E.nl2 = E.ul2 = 0;
+            E.dX2 = E.dY2 = E.w2b = E.w2x = E.w3b = E.w3x = E.w3y = 0.f;
+            if (el2 >= 0) {
+                const int x2 = third(el2);
+                const float2 b2 = gs_at(tp, g, el2, n2), c2 = gs_at(tp, g, el2, x2);
+                const float X = d.z - d.x, Y = d.w - d.y;
+                E.xb = x2 * L1;
+                E.l2 = el2 * L1;
+                E.nl2 = tp.t_nlev[el2] - 1;
+                E.ul2 = tp.t_ulev[el2];
+                E.dX2 = d.z;
+                E.dY2 = d.w;
+                E.w2b = d.z * b2.y - d.w * b2.x;
+                E.w2x = d.z * c2.y - d.w * c2.x;
+                E.w3b = 0.5f * (X * (b1.y + b2.y) - Y * (b1.x + b2.x));
+                E.w3x = 0.5f * (X * c1.y - Y * c1.x);
+                E.w3y = 0.5f * (X * c2.y - Y * c2.x);
+            }
+            E.top1 = tp.n_ulev[n1];
+            E.bot1 = tp.n_nlev[n1];
+            E.top2 = tp.n_ulev[n2];
+            E.bot2 = tp.n_nlev[n2];
         }
+        S.fill(j, in ? tp.e_lo[e] : 1, in ? tp.e_hi[e] - tp.e_lo[e] + 1 : 0);
+    }
+    __syncthreads();
+    const bool redi = B.slope != nullptr;
+    for (int i = threadIdx.x; i < S.total; i += kTileThreads) {
+        const int j = S.find(i), nz = S.top[j] + i - S.pre[j], k = nz - 1;
+        const EdgeD &E = Ed[j];
+        const int i1 = E.ia + k, i2 = E.ib + k;
+        const int nl12 = min(E.nl1, E.nl2), ul12 = max(E.ul1, E.ul2);
         int seg = 0;
-        if (nz >= ul1 && nz <= ul12 - 1) seg = 1;
-        else if (ul2 > 0 && nz >= ul2 && nz <= ul12 - 1) seg = 2;
+        if (nz >= E.ul1 && nz <= ul12 - 1) seg = 1;
+        else if (E.ul2 > 0 && nz >= E.ul2 && nz <= ul12 - 1) seg = 2;
         else if (nz >= ul12 && nz <= nl12) seg = 3;
-        else if (nz >= nl12 + 1 && nz <= nl1) seg = 1;
-        else if (nz >= nl12 + 1 && nz <= nl2) seg = 2;
-        const float Kh = (B.Ki[n1 * L1 + nz - 1] + B.Ki[n2 * L1 + nz - 1]) * 0.5f;
-        const float h1 = g.helem[el1 * L1 + nz - 1], h2 = seg >= 2 ? g.helem[el2 * L1 + nz - 1] : 0.f;
-        const bool u1 = seg == 1 || seg == 3, u2 = seg >= 2;
+        else if (nz >= nl12 + 1 && nz <= E.nl1) seg = 1;
+        else if (nz >= nl12 + 1 && nz <= E.nl2) seg = 2;
+        const bool u1 = seg & 1, u2 = seg & 2;
+        // the flux is Kh h (weights . (T - T1) + dY S_x Tz - dX S_y Tz)
+        const float h = !seg ? 0.f : 0.5f * (B.Ki[i1] + B.Ki[i2]) *
+                        (seg == 3 ? 0.5f * (g.helem[E.l1 + k] + g.helem[E.l2 + k]) : g.helem[(u2 ? E.l2 : E.l1) + k]);
+        const float wb = h * (seg == 3 ? E.w3b : u1 ? E.w1b : u2 ? E.w2b : 0.f);
+        const float wx = u1 ? h * (seg == 3 ? E.w3x : E.w1x) : 0.f, wy = u2 ? h * (seg == 3 ? E.w3y : E.w2x) : 0.f;
+        // Redi: weights of the differences to the layers above and below at both ends (0 at the
+        // columns' ends)
+        float a1 = 0.f, b1 = 0.f, a2 = 0.f, b2 = 0.f;
+        if (redi && seg) {
+            const float dX = (u1 ? E.dX1 : 0.f) - (u2 ? E.dX2 : 0.f), dY = (u1 ? E.dY1 : 0.f) - (u2 ? E.dY2 : 0.f);
+            const float *s1 = B.slope + 3 * (size_t)i1, *s2 = B.slope + 3 * (size_t)i2;
+            const float q1 = 0.5f * h * (dY * s1[0] - dX * s1[1]), q2 = 0.5f * h * (dY * s2[0] - dX * s2[1]);
+            const float h1 = g.hnode[i1], h2 = g.hnode[i2];
+            if (nz > E.top1) a1 = q1 / (g.hnode[i1 - 1] + h1);
+            if (nz + 1 < E.bot1) b1 = q1 / (h1 + g.hnode[i1 + 1]);
+            if (nz > E.top2) a2 = q2 / (g.hnode[i2 - 1] + h2);
+            if (nz + 1 < E.bot2) b2 = q2 / (h2 + g.hnode[i2 + 1]);
+        }
+        const bool t1 = redi && nz > E.top1, d1 = redi && nz + 1 < E.bot1, t2 = redi && nz > E.top2,
+                   d2 = redi && nz + 1 < E.bot2;
 #pragma unroll 1
         for (int gq = 0; gq < B.ng; gq++) {
             const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
-            const Vec<G> va = vldc<G>(u1, T, a0 * L1 + nz - 1), vb = vldc<G>(u1, T, a1 * L1 + nz - 1),
-                         vc = vldc<G>(u1, T, a2 * L1 + nz - 1);
-            const Vec<G> wa = vldc<G>(u2, T, b0 * L1 + nz - 1), wb = vldc<G>(u2, T, b1 * L1 + nz - 1),
-                         wc = vldc<G>(u2, T, b2 * L1 + nz - 1);
-            Vec<G> tz1 = vfill<G>(0.f), tz2 = vfill<G>(0.f);
-            if (redi) {
-                // the column neighbours of both edge nodes (rd = 0 where nz + 1 is not a gradient
-                // interface, ru = 0 likewise, so the loads stay inside the columns)
-                const Vec<G> m0 = vldc<G>(ru1 != 0.f, T, n1 * L1 + nz - 2), m1 = vld<G>(T, n1 * L1 + nz - 1),
-                             m2 = vldc<G>(rd1 != 0.f, T, n1 * L1 + nz);
-                const Vec<G> o0 = vldc<G>(ru2 != 0.f, T, n2 * L1 + nz - 2), o1 = vld<G>(T, n2 * L1 + nz - 1),
-                             o2 = vldc<G>(rd2 != 0.f, T, n2 * L1 + nz);
-#pragma unroll
-                for (int c = 0; c < G; c++) {
-                    tz1.c[c] = 0.5f * ((m0.c[c] - m1.c[c]) * ru1 + (m1.c[c] - m2.c[c]) * rd1);
-                    tz2.c[c] = 0.5f * ((o0.c[c] - o1.c[c]) * ru2 + (o1.c[c] - o2.c[c]) * rd2);
-                }
-            }
+            const Vec<G> T1 = vld<G>(T, i1), T2 = vld<G>(T, i2);
+            const Vec<G> Tx = vldc<G>(u1, T, E.xa + k), Ty = vldc<G>(u2, T, E.xb + k);
+            const Vec<G> m1 = vldc<G>(t1, T, i1 - 1), p1 = vldc<G>(d1, T, i1 + 1);
+            const Vec<G> m2 = vldc<G>(t2, T, i2 - 1), p2 = vldc<G>(d2, T, i2 + 1);
             Vec<G> out;
 #pragma unroll
             for (int c = 0; c < G; c++) {
-                float tx1 = 0.f, ty1 = 0.f, tx2 = 0.f, ty2 = 0.f;
-                if (u1) {
-                    tx1 = p0 * va.c[c] + p1 * vb.c[c] + p2 * vc.c[c];
-                    ty1 = p3 * va.c[c] + p4 * vb.c[c] + p5 * vc.c[c];
-                }
-                if (u2) {
-                    tx2 = q0 * wa.c[c] + q1 * wb.c[c] + q2 * wc.c[c];
-                    ty2 = q3 * wa.c[c] + q4 * wb.c[c] + q5 * wc.c[c];
-                }
+                const float x1 = T1.c[c], x2 = T2.c[c];
+                float f = wb * (x2 - x1);
+                if (u1) f += wx * (Tx.c[c] - x1);
+                if (u2) f += wy * (Ty.c[c] - x1);
                 if (redi) {
-                    const float sx = 0.5f * (tz1.c[c] * sx1 + tz2.c[c] * sx2);
-                    const float sy = 0.5f * (tz1.c[c] * sy1 + tz2.c[c] * sy2);
-                    tx1 += sx;
-                    ty1 += sy;
-                    tx2 += sx;
-                    ty2 += sy;
+                    f += a1 * (m1.c[c] - x1) + b1 * (x1 - p1.c[c]);
+                    f += a2 * (m2.c[c] - x2) + b2 * (x2 - p2.c[c]);
                 }
-                float cf = 0.f;
-                if (seg == 1) cf = (-dX1 * (Kh * ty1) + dY1 * (Kh * tx1)) * h1;
-                else if (seg == 2) cf = (dX2 * (Kh * ty2) - dY2 * (Kh * tx2)) * h2;
-                else if (seg == 3)
-                    cf = ((dX2 - dX1) * (Kh * (0.5f * (ty1 + ty2))) - (dY2 - dY1) * (Kh * (0.5f * (tx1 + tx2)))) *
-                         ((h1 + h2) * 0.5f);
-                out.c[c] = cf;
+                out.c[c] = f;
             }
-            vst<G>(grp<G>(B.HD, gq, B.sE), e * L1 + nz - 1, out);
+            vst<G>(grp<G>(B.HD, gq, B.sE), (e0 + j) * L1 + k, out);
         }
     }
 }
 
 template <int G>
-__global__ void __launch_bounds__(kTB) k32_hdiff(DTopo tp, DGeom<float> g, B32View B) {
-    FOR_WARP_UNITS(e, tp.E2) hdiff_edge32<G>(tp, g, B, e);
+__global__ void __launch_bounds__(kTileThreads, MinB<G>::hdiff) k32_hdiff(DTopo tp, DGeom<float> g, B32View B, int tile) {
+    __shared__ Tile S;
+    __shared__ EdgeD Ed[kTileMax];
+    hdiff_tile<G>(tp, g, B, blockIdx.x, tile, S, Ed);
 }
 
 // k32_diff: the diffusion increment to T* of every group in the diff mask, parked in Tnew:
@@ -1788,119 +1767,166 @@ __global__ void __launch_bounds__(kTB) k32_hdiff(DTopo tp, DGeom<float> g, B32Vi
 // (h(nz-1) + h(nz)) area(nz) with h = hnode (the reference's depth differences z(nz-1) -
 // zbar(nz) = h(nz-1)/2 etc. in exact arithmetic), increment (vd(nz) - vd(nz+1)) dt / (areasvol
 // hnode_new)
-template <int G, int KD>
-__device__ __forceinline__ void diff_node32(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt, int n,
-                                            int lane, const WEdges &S) {
-    using C = Chunk<1, 1>;
-    const int L1 = tp.L1, nl = tp.nl;
-    const int nzmin = S.nzmin, nzmax = S.nzmax, deg = S.deg;
-    const unsigned own = S.own;
-    const int nch = C::count(nzmin, nzmax);
-    for (int ch = 0; ch < nch; ch++) {
-        const C k(nzmin, nzmax, ch, lane);
-        const int nz = k.nz;
-        const int i = n * L1 + nz - 1, iv = n * nl + nz - 1;
-        float sdt = 0.f, kz = 0.f, q = 0.f;
-        if (k.lvl) {
-            sdt = dt / (g.areasvol[iv] * g.hnode_new[i]);
-            if (nz > nzmin) kz = B.Kv[iv] / (g.Z3[i - 1] - g.Z3[i]) * g.area[iv];
-            q = sdt / (g.zbar3[iv] - g.zbar3[iv + 1]);
+//
+// A tile of nodes, as k32_lo_ad; the vertical neighbours of S_xy . g pass through shared memory.
+// With the weights below, 6 gathers of T per group instead of 18: 0.68 -> 0.41 ms on the sphere of 7
+// subdivisions, 47 layers, 7 tracers with Redi.
+//
+// Redi: the node gradient's weights per edge slot.  The gradients of the node's elements sum over
+// the neighbours: with weights of a triangle that add up to zero, sum_el ea grad T = sum_m w_m
+// (T_m - T_n), where w_m joins the node's two elements at edge (n, m), each where it is wet.
+struct DiffSlots {
+    float4 w[kNodeTileNodes][kSlots];  // elem_area * gradient_sca at m of the edge's two elements (x, y; x, y)
+    int2 r[kNodeTileNodes][kSlots];    // their levels lo | hi << 16 (0: no element)
+};
+__device__ __forceinline__ void diff_slots_load(const DTopo &tp, const DGeom<float> &g, const NodeTile &S,
+                                                DiffSlots &D) {
+    for (int s = threadIdx.x; s < S.cnt * kMaxDeg; s += kNT) {
+        const int j = s / kMaxDeg, u = s % kMaxDeg;
+        if (u >= S.deg[j]) continue;
+        const int4 q = S.slot[j][u];
+        const int e = q.y / tp.L1, m = q.x / tp.L1;
+        float2 w[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        int r[2] = {0, 0};
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int el = k ? tp.e_t2[e] : tp.e_t1[e];
+            if (el < 0) continue;
+            const float2 v = gs_at(tp, g, el, m);
+            const float ea = g.elem_area[el];
+            w[k] = make_float2(ea * v.x, ea * v.y);
+            r[k] = tp.t_ulev[el] | (tp.t_nlev[el] - 1) << 16;
         }
-        const float kzd = sh_dn(kz, 1);
-        // Redi: weights of p above and at the interface nz, 1 / (3 areasvol), the slopes
-        float cu = 0.f, cd = 0.f, r3 = 0.f, sx = 0.f, sy = 0.f;
-        if (B.slope && k.lvl) {
-            r3 = 1.f / (3.f * g.areasvol[iv]);
-            sx = B.slope[3 * (size_t)i];
-            sy = B.slope[3 * (size_t)i + 1];
-            if (nz > nzmin) {
-                const float hu = g.hnode[i - 1], hd = g.hnode[i];
-                const float w = g.area[iv] / (hu + hd);
+        D.w[j][u] = make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+        D.r[j][u] = make_int2(r[0], r[1]);
+    }
+    __syncthreads();
+}
+template <int G>
+using DiffBuf = Vec<G>[2][kNT];  // [buffer][thread]: S_xy . node gradient
+
+template <int G>
+__device__ __forceinline__ void diff_tile(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt,
+                                          const NodeTile &S, const DiffSlots &D, DiffBuf<G> &X) {
+    const TileLane k(tp, S);
+    const int x = threadIdx.x, i = k.i, iv = k.iv, nz = k.nz, deg = S.deg[k.j], nl = tp.nl;
+    const bool top = nz == k.nzmin, bot = nz == k.nzmax - 1;
+    float sdt = 0.f, q = 0.f, kz = 0.f, kzd = 0.f;
+    // Redi: weights of p above and at the interfaces nz and nz + 1, the slopes / (3 areasvol)
+    float cu = 0.f, cd = 0.f, cu1 = 0.f, cd1 = 0.f, sx = 0.f, sy = 0.f;
+    if (k.on) {
+        sdt = dt / (g.areasvol[iv] * g.hnode_new[i]);
+        if (!top) kz = B.Kv[iv] / (g.Z3[i - 1] - g.Z3[i]) * g.area[iv];
+        if (!bot) kzd = B.Kv[iv + 1] / (g.Z3[i] - g.Z3[i + 1]) * g.area[iv + 1];
+        q = sdt / (g.zbar3[iv] - g.zbar3[iv + 1]);
+        if (B.slope) {
+            const float r3 = 1.f / (3.f * g.areasvol[iv]), h = g.hnode[i], kh = h * B.Ki[i];
+            sx = B.slope[3 * (size_t)i] * r3;
+            sy = B.slope[3 * (size_t)i + 1] * r3;
+            if (!top) {
+                const float hu = g.hnode[i - 1], w = g.area[iv] / (hu + h);
                 cu = hu * B.Ki[i - 1] * w;
-                cd = hd * B.Ki[i] * w;
+                cd = kh * w;
+            }
+            if (!bot) {
+                const float hd = g.hnode[i + 1], w = g.area[iv + 1] / (h + hd);
+                cu1 = kh * w;
+                cd1 = hd * B.Ki[i + 1] * w;
             }
         }
-        unsigned okm = 0;
-#pragma unroll
-        for (int u = 0; u < KD; u++) {
-            const bool ok = u < deg && k.lvl && nz >= S.lo[u] && nz <= S.hi[u];
-            okm |= ok ? 1u << u : 0u;
-        }
+    }
+    (void)nl;
+    int b = 0;
 #pragma unroll 1
-        for (int gq = 0; gq < B.ng; gq++) {
-            if (!((B.diff >> gq) & 1ull)) continue;
-            Vec<G> d = vfill<G>(0.f);
-            if (B.Ki) {
-                const float *__restrict__ HD = grp<G>(B.HD, gq, B.sE);
+    for (int gq = 0; gq < B.ng; gq++) {
+        if (!((B.diff >> gq) & 1ull)) continue;
+        const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
+        const float *__restrict__ HD = grp<G>(B.HD, gq, B.sE);
+        const Vec<G> Tn = vldc<G>(k.on, T, i);
+        Vec<G> d = vfill<G>(0.f), p = vfill<G>(0.f);
+        if (B.Ki) {
+#pragma unroll 1
+            for (int u0 = 0; u0 < S.degmax; u0 += 3) {
+                Vec<G> xe[3], tm[3];
+                float w[3];
 #pragma unroll
-                for (int u = 0; u < KD; u++) {
-                    const Vec<G> x = vldc<G>((okm >> u) & 1u, HD, S.e[u] * L1 + nz - 1);
-                    const bool ow = (own >> u) & 1u;
-#pragma unroll
-                    for (int c = 0; c < G; c++) d.c[c] += ow ? x.c[c] : -x.c[c];
-                }
-#pragma unroll
-                for (int c = 0; c < G; c++) d.c[c] *= sdt;
-            }
-            if (!((B.ivd >> gq) & 1ull)) {
-                const Vec<G> Tv = vldc<G>(k.lvl, grp<G>(B.T, gq, B.sN), i);
-                const Vec<G> fs = B.fsurf ? vld<G>(B.fsurf, gq * tp.N2 + n) : vfill<G>(0.f);
-#pragma unroll
-                for (int c = 0; c < G; c++) {
-                    const float Tn = Tv.c[c];
-                    const float Tu = sh_up(Tn, 1), Td = sh_dn(Tn, 1);
-                    const float vd0 = nz == nzmin ? fs.c[c] : kz * (Tu - Tn);
-                    const float vd1 = nz == nzmax - 1 ? 0.f : kzd * (Tn - Td);
-                    d.c[c] += (vd0 - vd1) * q;
-                }
-            }
-            if (B.slope) {
-                const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
-                Vec<G> gx = vfill<G>(0.f), gy = vfill<G>(0.f);
-                for (int kk = tp.nie_ptr[n]; kk < tp.nie_ptr[n + 1]; kk++) {
-                    const int el = tp.nie_idx[kk];
-                    const bool wet = k.lvl && nz >= tp.t_ulev[el] && nz <= tp.t_nlev[el] - 1;
-                    const float *gs = g.gs + 6 * (size_t)el;
-                    const float ea = g.elem_area[el];
-                    const Vec<G> ta = vldc<G>(wet, T, tp.t_n[3 * el] * L1 + nz - 1),
-                                 tb = vldc<G>(wet, T, tp.t_n[3 * el + 1] * L1 + nz - 1),
-                                 tc = vldc<G>(wet, T, tp.t_n[3 * el + 2] * L1 + nz - 1);
-#pragma unroll
-                    for (int c = 0; c < G; c++) {
-                        gx.c[c] += (gs[0] * ta.c[c] + gs[1] * tb.c[c] + gs[2] * tc.c[c]) * ea;
-                        gy.c[c] += (gs[3] * ta.c[c] + gs[4] * tb.c[c] + gs[5] * tc.c[c]) * ea;
+                for (int u = 0; u < 3; u++) {
+                    const int4 s = S.slot[k.j][u0 + u];
+                    const bool ok = k.on && u0 + u < deg && slot_wet(s, nz);
+                    xe[u] = vldc<G>(ok, HD, s.y + nz - 1);
+                    w[u] = 0.f;
+                    tm[u] = Tn;
+                    if (B.slope && ok) {
+                        tm[u] = vld<G>(T, s.x + nz - 1);
+                        const float4 v = D.w[k.j][u0 + u];
+                        const int2 r = D.r[k.j][u0 + u];
+                        if (nz >= (r.x & 0xffff) && nz <= (r.x >> 16)) w[u] += sx * v.x + sy * v.y;
+                        if (nz >= (r.y & 0xffff) && nz <= (r.y >> 16)) w[u] += sx * v.z + sy * v.w;
                     }
                 }
 #pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    const bool ow = S.slot[k.j][u0 + u].w != 0;
+#pragma unroll
+                    for (int c = 0; c < G; c++) {
+                        d.c[c] += ow ? xe[u].c[c] : -xe[u].c[c];
+                        p.c[c] += w[u] * (tm[u].c[c] - Tn.c[c]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < G; c++) d.c[c] *= sdt;
+        }
+        if (!((B.ivd >> gq) & 1ull) && k.on) {
+            const Vec<G> Tu = vldc<G>(!top, T, i - 1), Td = vldc<G>(!bot, T, i + 1);
+            const Vec<G> fs = B.fsurf ? vld<G>(B.fsurf, gq * tp.N2 + k.n) : vfill<G>(0.f);
+#pragma unroll
+            for (int c = 0; c < G; c++) {
+                const float vd0 = top ? fs.c[c] : kz * (Tu.c[c] - Tn.c[c]);
+                const float vd1 = bot ? 0.f : kzd * (Tn.c[c] - Td.c[c]);
+                d.c[c] += (vd0 - vd1) * q;
+            }
+        }
+        if (B.slope) {
+            if (!tp.ring_ok && k.on) {  // edges that do not cover the elements' sides: the elements themselves
+                p = vfill<G>(0.f);
+                for (int kk = tp.nie_ptr[k.n]; kk < tp.nie_ptr[k.n + 1]; kk++) {
+                    const int el = tp.nie_idx[kk];
+                    if (nz < tp.t_ulev[el] || nz > tp.t_nlev[el] - 1) continue;
+                    const float ea = g.elem_area[el];
+                    for (int m = 0; m < 3; m++) {
+                        const Vec<G> t = vld<G>(T, tp.t_n[3 * el + m] * tp.L1 + nz - 1);
+                        const float w = (sx * g.gs[6 * (size_t)el + m] + sy * g.gs[6 * (size_t)el + 3 + m]) * ea;
+#pragma unroll
+                        for (int c = 0; c < G; c++) p.c[c] += w * (t.c[c] - Tn.c[c]);
+                    }
+                }
+            }
+            Vec<G>(&xp)[kNT] = X[b];
+            b ^= 1;
+            xp[x] = p;
+            __syncthreads();
+            if (k.on) {
+                const Vec<G> pu = xp[top ? x : x - 1], pd = xp[bot ? x : x + 1];
+#pragma unroll
                 for (int c = 0; c < G; c++) {
-                    const float pz = (sx * gx.c[c] + sy * gy.c[c]) * r3;
-                    const float vd = cu * sh_up(pz, 1) + cd * pz;
-                    const float vdn = sh_dn(vd, 1);
+                    const float vd = cu * pu.c[c] + cd * p.c[c], vdn = cu1 * p.c[c] + cd1 * pd.c[c];
                     d.c[c] += (vd - vdn) * sdt;
                 }
             }
-            if (k.out) vst<G>(grp<G>(B.Tnew, gq, B.sN), i, d);
         }
+        if (k.on) vst<G>(grp<G>(B.Tnew, gq, B.sN), i, d);
     }
 }
 
-template <int G, bool WIDE>
-__device__ __forceinline__ void diff_unit(const DTopo &tp, const DGeom<float> &g, const B32View &B, float dt, int j,
-                                          WEdges *Se) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = unit_node<WIDE>(tp, j);
-    if (n < 0 || !B.diff) return;
-    WEdges &S = Se[warp];
-    stage_edges(tp, n, lane, S);
-    if ((S.deg > 8) != WIDE) return;
-    if (WIDE) diff_node32<G, kMaxDeg>(tp, g, B, dt, n, lane, S);
-    else diff_node32<G, 8>(tp, g, B, dt, n, lane, S);
-}
-
-template <int G, bool WIDE>
-__global__ void __launch_bounds__(kTB) k32_diff(DTopo tp, DGeom<float> g, B32View B, float dt) {
-    __shared__ WEdges Se[kWB];
-    FOR_WARP_UNITS(j, node_units<WIDE>(tp)) diff_unit<G, WIDE>(tp, g, B, dt, j, Se);
+template <int G>
+__global__ void __launch_bounds__(kNT, MinB<G>::diff) k32_diff(DTopo tp, DGeom<float> g, B32View B, float dt) {
+    __shared__ NodeTile S;
+    __shared__ DiffSlots D;
+    __shared__ DiffBuf<G> X;
+    node_tile_load(tp, blockIdx.x, S);
+    if (B.slope && tp.ring_ok) diff_slots_load(tp, g, S, D);
+    diff_tile<G>(tp, g, B, dt, S, D, X);
 }
 
 template <int G>
@@ -2118,21 +2144,27 @@ __global__ void __launch_bounds__(128) k32m_vdiff_w(const Inst32 *__restrict__ I
     else vdiff_w_column<2>(I[i].tp, I[i].g, I[i].f, I[i].B, I[i].dtd, I[i].scratch, u - ix.start[i]);
 }
 
-__global__ void __launch_bounds__(kTB) k32m_hdiff(const Inst32 *__restrict__ I, MultiIdx ix) {
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        if (I[i].B.G == 4) hdiff_edge32<4>(I[i].tp, I[i].g, I[i].B, u - ix.start[i]);
-        else hdiff_edge32<2>(I[i].tp, I[i].g, I[i].B, u - ix.start[i]);
-    }
+__global__ void __launch_bounds__(kTileThreads, MinB<4>::hdiff) k32m_hdiff(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ Tile S;
+    __shared__ EdgeD Ed[kTileMax];
+    const int i = find_inst(ix, blockIdx.x), ti = blockIdx.x - ix.start[i];
+    if (I[i].B.G == 4) hdiff_tile<4>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
+    else hdiff_tile<2>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
 }
-template <bool WIDE>
-__global__ void __launch_bounds__(kTB) k32m_diff(const Inst32 *__restrict__ I, MultiIdx ix) {
-    __shared__ WEdges Se[kWB];
-    FOR_WARP_UNITS(u, ix.start[ix.n]) {
-        const int i = find_inst(ix, u);
-        if (I[i].B.G == 4) diff_unit<4, WIDE>(I[i].tp, I[i].g, I[i].B, I[i].dt, u - ix.start[i], Se);
-        else diff_unit<2, WIDE>(I[i].tp, I[i].g, I[i].B, I[i].dt, u - ix.start[i], Se);
-    }
+__global__ void __launch_bounds__(kNT, MinB<4>::diff) k32m_diff(const Inst32 *__restrict__ I, MultiIdx ix) {
+    __shared__ NodeTile S;
+    __shared__ DiffSlots D;
+    __shared__ union {
+        DiffBuf<4> X4;
+        DiffBuf<2> X2;
+    } U;
+    const int i = find_inst(ix, blockIdx.x);
+    const Inst32 &d = I[i];
+    if (!d.B.diff) return;
+    node_tile_load(d.tp, blockIdx.x - ix.start[i], S);
+    if (d.B.slope && d.tp.ring_ok) diff_slots_load(d.tp, d.g, S, D);
+    if (d.B.G == 4) diff_tile<4>(d.tp, d.g, d.B, d.dt, S, D, U.X4);
+    else diff_tile<2>(d.tp, d.g, d.B, d.dt, S, D, U.X2);
 }
 
 // ---------------------------------------------------------------------------
@@ -2222,50 +2254,70 @@ void b32_vdiff_w(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &
     else k32_vdiff_w<2><<<(tp.N2 + 127) / 128, 128, 0, s>>>(tp, g, f, B, dt, scratch);
 }
 // Redi K33 = Kv + Ty (oce_ale_tracer.F90:1099-1204) of every interface nzmin < nz < nzmax, one
-// thread per column, in FP64 from the FP32 inputs: Ty = (zbar(nz) - Z(nz)) / dZ s3(nz-1)^2
-// Ki(nz-1) + (Z(nz-1) - zbar(nz)) / dZ s3(nz)^2 Ki(nz), dZ = Z(nz-1) - Z(nz), zbar / Z of
-// hnode_new from zbar_n_bot upward; Kv elsewhere
-__global__ void __launch_bounds__(128) k32_k33(DTopo tp, DGeom<float> g, const float *Kv, const float *Ki,
-                                               const float *slope, float *K33) {
-    const int L1 = tp.L1, nl = tp.nl;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < tp.N2; n += gridDim.x * blockDim.x) {
-        const int nzmax = tp.n_nlev[n], nzmin = tp.n_ulev[n];
-        const size_t b = (size_t)n * nl, c = (size_t)n * L1;
-        for (int nz = 1; nz <= nl; nz++) K33[b + nz - 1] = Kv[b + nz - 1];
-        double zb = g.zbar_n_bot[n];
-        double Zc = zb + (double)g.hnode_new[c + nzmax - 2] / 2.0;
-        for (int nz = nzmax - 1; nz >= nzmin + 1; nz--) {
-            const double zbn = zb + (double)g.hnode_new[c + nz - 1];
-            const double Zu = zbn + (double)g.hnode_new[c + nz - 2] / 2.0;
-            const double zinv = 1.0 / (Zu - Zc);
-            const double sa = slope[3 * (c + nz - 2) + 2], sb = slope[3 * (c + nz - 1) + 2];
-            const double Ty = (zbn - Zc) * zinv * (sa * sa) * (double)Ki[c + nz - 2] +
-                              (Zu - zbn) * zinv * (sb * sb) * (double)Ki[c + nz - 1];
-            K33[b + nz - 1] = (float)((double)Kv[b + nz - 1] + Ty);
-            zb = zbn;
-            Zc = Zu;
+// K33 = Kv + Ty, Ty = (zbar(nz) - Z(nz)) / dZ s3(nz-1)^2 Ki(nz-1) + (Z(nz-1) - zbar(nz)) / dZ
+// s3(nz)^2 Ki(nz) with dZ = Z(nz-1) - Z(nz): the depth differences are half thicknesses, so Ty =
+// (h(nz) s3(nz-1)^2 Ki(nz-1) + h(nz-1) s3(nz)^2 Ki(nz)) / (h(nz-1) + h(nz)) with h = hnode_new; Kv
+// outside the column's inner interfaces.  A warp per column; the products, the sums and the quotient
+// as unevaluated sums of two FP32 numbers (errors of products and sums by fma and two-sum, T. J.
+// Dekker, Numer. Math. 18, 1971), rounded once: within 2^-24 of the exact value plus 2^-44, where
+// FP64 arithmetic along the column took 18 FP64 instructions per interface and strided reads: 293 ->
+// 60 us on the sphere of 7 subdivisions.
+struct F2 {
+    float h, l;
+};
+__device__ __forceinline__ F2 two_prod(float a, float b) {
+    const float p = __fmul_rn(a, b);
+    return {p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ F2 two_sum(float a, float b) {
+    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+    return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, float b) {
+    const F2 p = two_prod(a.h, b);
+    return {p.h, __fmaf_rn(a.l, b, p.l)};
+}
+__global__ void __launch_bounds__(kTB) k32_k33(DTopo tp, DGeom<float> g, const float *__restrict__ Kv,
+                                               const float *__restrict__ Ki, const float *__restrict__ slope,
+                                               float *__restrict__ K33) {
+    const int L1 = tp.L1, nl = tp.nl, lane = threadIdx.x & 31;
+    const int n = blockIdx.x * kWB + (threadIdx.x >> 5);
+    if (n >= tp.N2) return;
+    const int nzmax = tp.n_nlev[n], nzmin = tp.n_ulev[n];
+    for (int nz = 1 + lane; nz <= nl; nz += 32) {
+        const size_t b = (size_t)n * nl + nz - 1, c = (size_t)n * L1 + nz - 1;
+        float out = Kv[b];
+        if (nz > nzmin && nz < nzmax) {
+            const float hu = g.hnode_new[c - 1], hc = g.hnode_new[c];
+            const float sa = slope[3 * (c - 1) + 2], sb = slope[3 * c + 2];
+            const F2 x = f2_mul(f2_mul(two_prod(sa, sa), Ki[c - 1]), hc);
+            const F2 y = f2_mul(f2_mul(two_prod(sb, sb), Ki[c]), hu);
+            const F2 m = two_sum(x.h, y.h), d = two_sum(hu, hc);
+            const float ml = m.l + (x.l + y.l);
+            const float q = __fdiv_rn(m.h, d.h);
+            const float r = __fdiv_rn(__fmaf_rn(-q, d.l, __fadd_rn(__fmaf_rn(-q, d.h, m.h), ml)), d.h);
+            const F2 t = two_sum(out, q);
+            out = __fadd_rn(t.h, __fadd_rn(t.l, r));
         }
+        K33[b] = out;
     }
 }
 
 void b32_k33(const DTopo &tp, const DGeom<float> &g, const float *Kv, const float *Ki, const float *slope, float *K33,
              cudaStream_t s) {
-    k32_k33<<<(tp.N2 + 127) / 128, 128, 0, s>>>(tp, g, Kv, Ki, slope, K33);
+    k32_k33<<<grid_nodes(tp.N2), kTB, 0, s>>>(tp, g, Kv, Ki, slope, K33);
 }
 
 void b32_hdiff(const DTopo &tp, const DGeom<float> &g, const B32View &B, cudaStream_t s) {
-    if (B.G == 4) k32_hdiff<4><<<grid_nodes(tp.E2), kTB, 0, s>>>(tp, g, B);
-    else k32_hdiff<2><<<grid_nodes(tp.E2), kTB, 0, s>>>(tp, g, B);
+    const int t = tile_size(tp.E2, 0), nb = (tp.E2 + t - 1) / t;
+    if (B.G == 4) k32_hdiff<4><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+    else k32_hdiff<2><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
 }
 void b32_diff(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, cudaStream_t s) {
-    if (B.G == 4) {
-        k32_diff<4, false><<<grid_nodes(tp.N2), kTB, 0, s>>>(tp, g, B, (float)dt);
-        if (tp.n_wide) k32_diff<4, true><<<grid_nodes(tp.n_wide), kTB, 0, s>>>(tp, g, B, (float)dt);
-    } else {
-        k32_diff<2, false><<<grid_nodes(tp.N2), kTB, 0, s>>>(tp, g, B, (float)dt);
-        if (tp.n_wide) k32_diff<2, true><<<grid_nodes(tp.n_wide), kTB, 0, s>>>(tp, g, B, (float)dt);
-    }
+    if (B.G == 4) k32_diff<4><<<tp.n_nt, kNT, 0, s>>>(tp, g, B, (float)dt);
+    else k32_diff<2><<<tp.n_nt, kNT, 0, s>>>(tp, g, B, (float)dt);
 }
+
 void b32_content(const DTopo &tp, const DGeom<float> &g, const float *T, int ng, int G, double *partials, int nblk,
                  double *out, cudaStream_t s) {
     if (G == 4) k32_content_partial<4><<<nblk, 256, 0, s>>>(tp, g, T, ng, partials);
@@ -2355,13 +2407,11 @@ void bm32_update(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
 }
 void bm32_hdiff(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
-    if (u) k32m_hdiff<<<grid_nodes(u), kTB, 0, s>>>(I, ix);
+    if (u) k32m_hdiff<<<u, kTileThreads, 0, s>>>(I, ix);
 }
-void bm32_diff(const Inst32 *I, const MultiIdx &ix, bool wide, cudaStream_t s) {
+void bm32_diff(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
-    if (!u) return;
-    if (wide) k32m_diff<true><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
-    else k32m_diff<false><<<grid_nodes(u), kTB, 0, s>>>(I, ix);
+    if (u) k32m_diff<<<u, kNT, 0, s>>>(I, ix);
 }
 
 }  // namespace fesom
