@@ -1,8 +1,8 @@
 // fp64_arith.cuh -- FP64 helpers of the plain form: the reference's results with fewer
 // instructions on the FP64 pipe.
 //
-// sm_103a issues one FP64 warp instruction per SM every 16 cycles (2 lanes per cycle; measured:
-// 16.3 cycles per instruction with the pipe 86 % busy), so a compare, a maximum or a select done
+// sm_103a issues one FP64 warp instruction per SM every 19 cycles (measured over
+// the stages of the form; one warp alone, every 64), so a compare, a maximum or a select done
 // in integer instructions costs next to nothing beside one FP64 add, and a division (8 FP64
 // instructions) is the most expensive operation of the form.  Everything here returns the bits of
 // the plain expression it replaces (zeros may differ in sign; quotients below 2^-600 take the

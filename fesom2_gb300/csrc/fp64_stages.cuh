@@ -10,7 +10,7 @@
 //   * divisions by shared or constant divisors take 3 or 4 instructions instead of 8;
 //   * the wet levels of a tile of entities are dealt to the threads one after another (Tile), so
 //     every warp but a tile's last is full.  A warp per column left 27 to 50 % of the lanes idle
-//     (47 layers are 32 + 15 lanes), and an FP64 instruction costs its 16 cycles however many
+//     (47 layers are 32 + 15 lanes), and an FP64 instruction costs its 19 cycles however many
 //     lanes take part.
 #pragma once
 #include <type_traits>
@@ -150,7 +150,7 @@ struct EdgeData {
 // The edge-layers whose gradients are node means (the last layers over a slope, every layer at a
 // coast: 2 % of a sphere's) cost five times the others' instructions, and lie in half of the
 // warps: they are set aside and take their own passes, full warps again.
-static __global__ void __launch_bounds__(kTileThreads)
+static __global__ void __launch_bounds__(kTileThreads, 8)
 k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, int tile, int any_ho) {
     extern __shared__ int aside[];
     __shared__ int n_aside;
@@ -287,7 +287,7 @@ __device__ __forceinline__ double ver_upw64(double T0, double Tu, double W, doub
     return -(x * W * ar);
 }
 
-static __global__ void __launch_bounds__(kTileThreads)
+static __global__ void __launch_bounds__(kTileThreads, 7)
 k_node_lo(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, double dt, int tile) {
     extern __shared__ __align__(16) double sm64[];
     __shared__ Tile S;
@@ -408,7 +408,7 @@ __device__ __forceinline__ double ratio1(double b, double fl) {
     return rmin(1.0, b / fl);
 }
 
-static __global__ void __launch_bounds__(kTileThreads)
+static __global__ void __launch_bounds__(kTileThreads, 12)
 k_bounds_rpm(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int tile) {
     extern __shared__ __align__(16) long long smk[];
     __shared__ Tile S;
