@@ -7,16 +7,15 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/fesom_gpu.h"
 #include "fesom_internal.h"
+#include "host_wait.h"
 #include "mesh_prep.h"
 #include "tile.cuh"
 
@@ -50,6 +49,8 @@ struct fesom_gpu_ctx {
     double *scratch = nullptr, *partials = nullptr, *content_out = nullptr;
     int content_blocks = 0;
     unsigned *status = nullptr;
+    unsigned *h_status = nullptr;  // page-locked copy of the status word
+    cudaEvent_t ev_wait = nullptr;
     bool forcing_ready = false;
     bool state_ready = false;
     int wsplit = 0;            // dynamics%use_wsplit (fesom_gpu_set_wsplit)
@@ -91,7 +92,8 @@ struct fesom_gpu_ctx {
     // host-array step with overlapped transfers: copy-in and copy-out streams, an event per
     // tracer group for "resident" and "computed"
     cudaStream_t h2d = nullptr, d2h = nullptr;
-    cudaEvent_t ev_forcing = nullptr;
+    cudaEvent_t ev_forcing = nullptr, ev_vel = nullptr;
+    void *bc_stage = nullptr;            // surface fluxes of the host-array step (host type)
     std::vector<cudaEvent_t> ev_in, ev_done;
     // tail of the tracer loop: node y coordinates (relax_zonal_temp) and work arrays
     void *Ki = nullptr;        // horizontal diffusivity (context precision), null: none
@@ -619,12 +621,13 @@ int alloc_state32(fesom_gpu_ctx *ctx, int ab) {
     const int G = ctx->gw, ngr = ctx->ngr;
     void *old[] = {ctx->Bf[0], ctx->Bf[1], ctx->Bf[2], ctx->VF, ctx->vfac.a, ctx->vfac.c, ctx->vfac.inv, ctx->vfac.cp,
                    ctx->LO32, ctx->ADv32, ctx->ADh32, ctx->Rp32, ctx->Rm32, ctx->Bp32, ctx->Bm32, ctx->d_cfg, ctx->bc,
-                   ctx->HD32, ctx->partials, ctx->content_out, ctx->pack_in, ctx->pack_out};
+                   ctx->HD32, ctx->partials, ctx->content_out, ctx->pack_in, ctx->pack_out, ctx->bc_stage};
     for (void *b : old) { void *p = b; dfree(ctx, p); }
     ctx->Bf[0] = ctx->Bf[1] = ctx->Bf[2] = nullptr;
     ctx->VF = ctx->LO32 = ctx->ADv32 = ctx->ADh32 = ctx->HD32 = nullptr;
     ctx->Rp32 = ctx->Rm32 = ctx->Bp32 = ctx->Bm32 = nullptr;
     ctx->pack_in = ctx->pack_out = nullptr;
+    ctx->bc_stage = nullptr;
     ctx->pack_n = 0;
     ctx->partials = ctx->content_out = nullptr;
     ctx->vfac = VFactors{};
@@ -672,6 +675,7 @@ int alloc_state32(fesom_gpu_ctx *ctx, int ab) {
         CK(cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking));
         CK(cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&ctx->ev_forcing, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ctx->ev_vel, cudaEventDisableTiming));
     }
     ctx->rot = 0;
     ctx->ab_max = ab;
@@ -842,7 +846,8 @@ int enqueue_step(fesom_gpu_ctx *ctx, double dt, StageTimer *tm = nullptr) {
 
 // the tracer-independent stages of a step: edge volume fluxes, then the vertical-diffusion
 // factors (outside profiled steps on the side stream, joined before the first diffusion)
-int enqueue_shared32(fesom_gpu_ctx *ctx, double dt, StageTimer *tm, bool &fork) {
+// kv_ready: an event the factors wait for on the side stream (null: Kv is there)
+int enqueue_shared32(fesom_gpu_ctx *ctx, double dt, StageTimer *tm, bool &fork, cudaEvent_t kv_ready = nullptr) {
     const DGeom<float> &g = ctx->g32;
     DForcing<float> f = forcing_view<float>(ctx, 0);
     bool any_vd = false;
@@ -858,6 +863,7 @@ int enqueue_shared32(fesom_gpu_ctx *ctx, double dt, StageTimer *tm, bool &fork) 
     if (fork) {
         CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+        if (kv_ready) CK(cudaStreamWaitEvent(ctx->side, kv_ready, 0));
         b32_vfactors(ctx->tp, g, f, dt, ctx->vfac, ctx->side);
         CK(cudaEventRecord(ctx->ev_join, ctx->side));
     } else if (any_vd) {
@@ -977,28 +983,24 @@ int enqueue_step_any(fesom_gpu_ctx *ctx, double dt) {
 }
 
 int wait_stream(fesom_gpu_ctx *ctx, int timeout_ms) {
-    cudaEvent_t ev;
-    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    CK(cudaEventRecord(ev, ctx->stream));
-    auto t0 = std::chrono::steady_clock::now();
-    for (;;) {
-        cudaError_t q = cudaEventQuery(ev);
-        if (q == cudaSuccess) break;
-        if (q != cudaErrorNotReady) {
-            cudaEventDestroy(ev);
-            ctx->err = std::string("stream error: ") + cudaGetErrorString(q);
-            return FESOM_ERR_CUDA;
-        }
-        auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
-        if (timeout_ms >= 0 && ms > timeout_ms) {
-            cudaEventDestroy(ev);
-            ctx->err = "device work did not finish within the time limit";
-            return FESOM_ERR_TIMEOUT;
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(ms < 10 ? 20 : 500));
+    if (!ctx->ev_wait) CK(cudaEventCreateWithFlags(&ctx->ev_wait, cudaEventDisableTiming));
+    CK(cudaEventRecord(ctx->ev_wait, ctx->stream));
+    const cudaError_t q = wait_event(ctx->ev_wait, timeout_ms);
+    if (q == cudaSuccess) return FESOM_OK;
+    if (q == cudaErrorNotReady) {
+        ctx->err = "device work did not finish within the time limit";
+        return FESOM_ERR_TIMEOUT;
     }
-    cudaEventDestroy(ev);
-    return FESOM_OK;
+    ctx->err = std::string("stream error: ") + cudaGetErrorString(q);
+    return FESOM_ERR_CUDA;
+}
+
+// the same, with the status word read behind the stream's work
+int wait_status(fesom_gpu_ctx *ctx, unsigned *st) {
+    CK(cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    const int rc = wait_stream(ctx, -1);
+    *st = *ctx->h_status;
+    return rc;
 }
 
 int need_fp64(fesom_gpu_ctx *ctx) {
@@ -1155,6 +1157,7 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
     if ((rc = dalloc(ctx, (void **)&ctx->content_out, sizeof(double) * ctx->max_tr))) return rc;
     if ((rc = dalloc(ctx, (void **)&ctx->status, sizeof(unsigned)))) return rc;
     CK(cudaMemset(ctx->status, 0, sizeof(unsigned)));
+    CK(cudaHostAlloc((void **)&ctx->h_status, sizeof(unsigned), cudaHostAllocDefault));
     CK(cudaDeviceSynchronize());
     return FESOM_OK;
 }
@@ -1184,10 +1187,13 @@ int fesom_gpu_finalize(fesom_gpu_ctx *ctx) {
     if (!ctx) return FESOM_OK;
     if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
     free_graphs32(ctx);
+    if (ctx->h_status) cudaFreeHost(ctx->h_status);
+    if (ctx->ev_wait) cudaEventDestroy(ctx->ev_wait);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->ev_forcing) cudaEventDestroy(ctx->ev_forcing);
+    if (ctx->ev_vel) cudaEventDestroy(ctx->ev_vel);
     for (cudaEvent_t e : ctx->ev_in) cudaEventDestroy(e);
     for (cudaEvent_t e : ctx->ev_done) cudaEventDestroy(e);
     if (ctx->h2d) cudaStreamDestroy(ctx->h2d);
@@ -1611,10 +1617,8 @@ int fesom_gpu_tracer_step(fesom_gpu_ctx *ctx, int32_t ntr, const fesom_tra_cfg *
         if ((rc = get(ctx, valuesold[t], (char *)ctx->Told + rs * sN * (ctx->ab_max - 1) * t, sN * (ctx->ab_max - 1))))
             return rc;
     }
-    rc = wait_stream(ctx, -1);
-    if (rc) return rc;
     unsigned s = 0;
-    CK(cudaMemcpy(&s, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    if ((rc = wait_status(ctx, &s))) return rc;
     if (s & FESOM_STATUS_NAN) {
         CK(cudaMemset(ctx->status, 0, sizeof(unsigned)));
         ctx->err = "non-finite tracer value produced";
@@ -2158,7 +2162,6 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
     // staging per slot of the two rings: the largest stage's tracers, values and previous levels
     size_t need = 0;
     for (int k = 0; k < ns; k++) need = std::max(need, (size_t)(gs[k + 1] - gs[k]) * G * (1 + lv) * sN * sizeof(S));
-    need = std::max(need, sizeof(S) * (size_t)ctx->N2 * ctx->ntr);  // the surface fluxes pass through slot 0
     if (ctx->pack_n < need) {
         for (float **b : {&ctx->pack_in, &ctx->pack_out}) {
             void *p = *b;
@@ -2166,6 +2169,8 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
             *b = nullptr;
         }
         ctx->pack_n = 0;
+        dfree(ctx, ctx->bc_stage);
+        if ((rc = dalloc(ctx, &ctx->bc_stage, sizeof(double) * (size_t)ctx->N2 * ctx->ntr))) return rc;
         if ((rc = dalloc(ctx, (void **)&ctx->pack_in, 2 * need)) || (rc = dalloc(ctx, (void **)&ctx->pack_out, 2 * need)))
             return rc;
         ctx->pack_n = need;
@@ -2185,32 +2190,46 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
     CK(cudaEventRecord(ctx->ev_forcing, ctx->stream));
     CK(cudaStreamWaitEvent(ctx->h2d, ctx->ev_forcing, 0));
     if ((rc = put_on(ctx, ctx->h2d, (float *)ctx->uv, uv, 2 * (size_t)ctx->L1 * ctx->T2)) ||
-        (rc = put_on(ctx, ctx->h2d, (float *)ctx->w, w, sNI)) || (rc = put_on(ctx, ctx->h2d, (float *)ctx->we, we, sNI)) ||
-        (rc = put_on(ctx, ctx->h2d, (float *)ctx->Kv, Kv, sNI)))
+        (rc = put_on(ctx, ctx->h2d, (float *)ctx->w, w, sNI)))
         return rc;
+    // one array given as w and w_e crosses the host link once
+    if (we == w) CK(cudaMemcpyAsync(ctx->we, ctx->w, 4 * sNI, cudaMemcpyDeviceToDevice, ctx->h2d));
+    else if ((rc = put_on(ctx, ctx->h2d, (float *)ctx->we, we, sNI))) return rc;
     if (wi && (rc = put_on(ctx, ctx->h2d, (float *)ctx->wi, wi, sNI))) return rc;
-    CK(cudaMemsetAsync(ctx->bc, 0, 4 * (size_t)ctx->N2 * G * ctx->ngr, ctx->h2d));
-    if (bc_surf) {
-        // per tracer into its slot, through the first staging slot (free at this point)
-        S *st = (S *)ctx->pack_in;
-        CK(cudaMemcpyAsync(st, bc_surf, sizeof(S) * (size_t)ctx->N2 * ctx->ntr, cudaMemcpyDefault, ctx->h2d));
-        for (int g = 0; g < ctx->ngr; g++) {
-            SlotSrc<S> src{};
-            for (int c = 0; c < G; c++) {
-                const int t = ctx->slot_tr[(size_t)g * G + c];
-                src.p[c] = t >= 0 ? st + (size_t)t * ctx->N2 : nullptr;
+    CK(cudaEventRecord(ctx->ev_vel, ctx->h2d));
+    // the diffusivity and the surface fluxes are first read by the vertical-diffusion factors and
+    // the update, so they travel behind the first stage's tracers; explicit or horizontal
+    // diffusion reads them earlier
+    bool late = true;
+    for (int t = 0; t < ctx->ntr; t++) late = late && ctx->cfgs[t].i_vert_diff != 0;
+    late = late && !ctx->Ki && !ctx->wsplit;
+    auto put_rest = [&]() -> int {
+        if ((rc = put_on(ctx, ctx->h2d, (float *)ctx->Kv, Kv, sNI))) return rc;
+        CK(cudaMemsetAsync(ctx->bc, 0, 4 * (size_t)ctx->N2 * G * ctx->ngr, ctx->h2d));
+        if (bc_surf) {
+            // per tracer into its slot, through a staging buffer of their own
+            S *st = (S *)ctx->bc_stage;
+            CK(cudaMemcpyAsync(st, bc_surf, sizeof(S) * (size_t)ctx->N2 * ctx->ntr, cudaMemcpyDefault, ctx->h2d));
+            for (int g = 0; g < ctx->ngr; g++) {
+                SlotSrc<S> src{};
+                for (int c = 0; c < G; c++) {
+                    const int t = ctx->slot_tr[(size_t)g * G + c];
+                    src.p[c] = t >= 0 ? st + (size_t)t * ctx->N2 : nullptr;
+                }
+                b32_pack_group<S>(src, (float *)ctx->bc + (size_t)g * ctx->N2 * G, G, ctx->N2, 1, 0, ctx->h2d);
             }
-            b32_pack_group<S>(src, (float *)ctx->bc + (size_t)g * ctx->N2 * G, G, ctx->N2, 1, 0, ctx->h2d);
+            CK(cudaGetLastError());
         }
-        CK(cudaGetLastError());
-    }
+        CK(cudaEventRecord(ctx->ev_forcing, ctx->h2d));
+        return FESOM_OK;
+    };
+    if (!late && (rc = put_rest())) return rc;
     ctx->forcing_ready = true;
-    CK(cudaEventRecord(ctx->ev_forcing, ctx->h2d));
     float *L0 = level32(ctx, 0), *L1b = level32(ctx, 1), *L2b = ab == 3 ? level32(ctx, 2) : nullptr;
     float *Lnew = level32(ctx, ab - 1);
-    CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_forcing, 0));
+    CK(cudaStreamWaitEvent(ctx->stream, late ? ctx->ev_vel : ctx->ev_forcing, 0));
     bool fork = false, joined = false;
-    if ((rc = enqueue_shared32(ctx, dt, nullptr, fork))) return rc;
+    if (!late && (rc = enqueue_shared32(ctx, dt, nullptr, fork))) return rc;
     const size_t per_tr = (1 + lv) * sN;  // staged elements per tracer: values, then valuesold
     for (int k = 0; k < ns; k++) {
         S *in = (S *)((char *)ctx->pack_in + (k & 1) * need);
@@ -2227,6 +2246,9 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
                                    ctx->h2d));
             }
         CK(cudaEventRecord(ev_res[k], ctx->h2d));
+        if (late && k == 0) {
+            if ((rc = put_rest()) || (rc = enqueue_shared32(ctx, dt, nullptr, fork, ctx->ev_forcing))) return rc;
+        }
         // compute: pack into the time levels, the stages of the groups, unpack the results
         CK(cudaStreamWaitEvent(ctx->stream, ev_res[k], 0));
         q = 0;
@@ -2244,25 +2266,40 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev_pack[k], ctx->stream));
-        for (int g0 = gs[k]; g0 < gs[k + 1]; g0 += ctx->group)
-            if ((rc = enqueue_group32(ctx, dt, g0, std::min(ctx->group, gs[k + 1] - g0), nullptr, fork, joined)))
-                return rc;
         if (k >= 2) CK(cudaStreamWaitEvent(ctx->stream, ev_out[k - 2], 0));
-        q = 0;
-        for (int g = gs[k]; g < gs[k + 1]; g++, q += G) {
-            SlotDst<S> v{}, o{};
-            for (int c = 0; c < G; c++) {
-                const bool has = ctx->slot_tr[(size_t)g * G + c] >= 0;
-                v.p[c] = has ? out + (q + c) * per_tr : nullptr;
-                o.p[c] = (has && valuesold_out) ? out + (q + c) * per_tr + sN : nullptr;
-            }
-            const size_t go = (size_t)g * sN * G;
-            b32_unpack_group<S>(Lnew + go, G, sN, v, 1, 0, ctx->stream);
-            if (valuesold_out) {
-                // the new previous levels: the values the step started from (and, AB3, the level before)
+        if (valuesold_out) {
+            // the new previous levels are the values the step starts from (and, AB3, the level
+            // before): unpacked and copied out while the stage computes
+            q = 0;
+            for (int g = gs[k]; g < gs[k + 1]; g++, q += G) {
+                SlotDst<S> o{};
+                for (int c = 0; c < G; c++)
+                    o.p[c] = ctx->slot_tr[(size_t)g * G + c] >= 0 ? out + (q + c) * per_tr + sN : nullptr;
+                const size_t go = (size_t)g * sN * G;
                 b32_unpack_group<S>(L0 + go, G, sN, o, lv, 0, ctx->stream);
                 if (ab == 3) b32_unpack_group<S>(L1b + go, G, sN, o, 2, 1, ctx->stream);
             }
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(ev_comp[k], ctx->stream));
+            CK(cudaStreamWaitEvent(ctx->d2h, ev_comp[k], 0));
+            q = 0;
+            for (int g = gs[k]; g < gs[k + 1]; g++)
+                for (int c = 0; c < G; c++, q++) {
+                    const int t = ctx->slot_tr[(size_t)g * G + c];
+                    if (t >= 0)
+                        CK(cudaMemcpyAsync(valuesold_out[t], out + q * per_tr + sN, sizeof(S) * sN * lv,
+                                           cudaMemcpyDefault, ctx->d2h));
+                }
+        }
+        for (int g0 = gs[k]; g0 < gs[k + 1]; g0 += ctx->group)
+            if ((rc = enqueue_group32(ctx, dt, g0, std::min(ctx->group, gs[k + 1] - g0), nullptr, fork, joined)))
+                return rc;
+        q = 0;
+        for (int g = gs[k]; g < gs[k + 1]; g++, q += G) {
+            SlotDst<S> v{};
+            for (int c = 0; c < G; c++)
+                v.p[c] = ctx->slot_tr[(size_t)g * G + c] >= 0 ? out + (q + c) * per_tr : nullptr;
+            b32_unpack_group<S>(Lnew + (size_t)g * sN * G, G, sN, v, 1, 0, ctx->stream);
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev_comp[k], ctx->stream));
@@ -2274,9 +2311,6 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
                 const int t = ctx->slot_tr[(size_t)g * G + c];
                 if (t < 0) continue;
                 CK(cudaMemcpyAsync(values_out[t], out + q * per_tr, sizeof(S) * sN, cudaMemcpyDefault, ctx->d2h));
-                if (valuesold_out)
-                    CK(cudaMemcpyAsync(valuesold_out[t], out + q * per_tr + sN, sizeof(S) * sN * lv, cudaMemcpyDefault,
-                                       ctx->d2h));
             }
         CK(cudaEventRecord(ev_out[k], ctx->d2h));
     }
@@ -2285,9 +2319,8 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
     // the context's stream follows the copies out, so later calls see a quiet context
     CK(cudaEventRecord(ctx->ev_forcing, ctx->d2h));
     CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_forcing, 0));
-    if ((rc = wait_stream(ctx, -1))) return rc;
     unsigned st = 0;
-    CK(cudaMemcpy(&st, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    if ((rc = wait_status(ctx, &st))) return rc;
     if (st) {
         CK(cudaMemset(ctx->status, 0, sizeof(unsigned)));
         ctx->err = st & FESOM_STATUS_NAN ? "NaN in the tracer step" : "FCT limiter needed more than round-off clamping";

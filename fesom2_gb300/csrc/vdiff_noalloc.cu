@@ -16,21 +16,19 @@
 // start at zero.  A status word beside it records columns whose level bounds the
 // kernel refused (it is cleared at the start of every call).  All calls share both:
 // calls that overlap on the GPU (different streams, or different host threads) race
-// on them.  A call waits, with a time limit, for its kernel and reads the status word
-// back, so it returns only when the values are final.
+// on them.  A call waits, with a time limit, for its kernel and the status word, so it returns only when the values are final.
 //
 // The column solve is the one k_vdiff<double> runs (vdiff_column.cuh), built with
 // --fmad=false in both places, so the results equal those of fesom_gpu_vdiff_impl bit
 // for bit.
 #include <cuda_runtime.h>
 
-#include <chrono>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
-#include <thread>
 
 #include "../../include/fesom_gpu.h"
+#include "host_wait.h"
 #include "vdiff_column.cuh"
 
 namespace {
@@ -53,9 +51,13 @@ std::mutex g_mu;
 struct DevState {
     double *scratch = nullptr;
     unsigned *status = nullptr;
+    unsigned *h_status = nullptr;  // in g_host_status
     cudaEvent_t done = nullptr;
 };
 DevState g_dev[kMaxDevices];
+// the status words' host copies: static memory, page-locked at first use
+alignas(4096) unsigned g_host_status[1024];
+bool g_host_locked = false;
 
 void set_err(char *errbuf, int32_t errlen, const char *msg) {
     if (errbuf && errlen > 0) {
@@ -165,6 +167,15 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
                 set_err(errbuf, errlen, cudaGetErrorString(e));
                 return FESOM_ERR_CUDA;
             }
+            if (!g_host_locked) {
+                e = cudaHostRegister(g_host_status, sizeof g_host_status, cudaHostRegisterPortable);
+                if (e != cudaSuccess) {
+                    set_err(errbuf, errlen, cudaGetErrorString(e));
+                    return FESOM_ERR_CUDA;
+                }
+                g_host_locked = true;
+            }
+            d.h_status = g_host_status + dev;
             d.status = (unsigned *)q;
             d.scratch = (double *)p;
         }
@@ -191,34 +202,24 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
             st.scratch, st.status);
     }
     e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(st.h_status, st.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaEventRecord(st.done, s);
     if (e != cudaSuccess) {
         set_err(errbuf, errlen, cudaGetErrorString(e));
         return FESOM_ERR_CUDA;
     }
-    // wait, with a time limit, for the kernel, then read its status word
-    const auto t0 = std::chrono::steady_clock::now();
-    for (;;) {
-        e = cudaEventQuery(st.done);
-        if (e == cudaSuccess) break;
-        if (e != cudaErrorNotReady) {
-            set_err(errbuf, errlen, cudaGetErrorString(e));
-            return FESOM_ERR_CUDA;
-        }
-        const auto ms =
-            std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
-        if (ms > kWaitLimitMs) {
-            set_err(errbuf, errlen, "fesom_gpu_vdiff_impl_noalloc: the solve did not finish within the time limit");
-            return FESOM_ERR_TIMEOUT;
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(ms < 10 ? 20 : 500));
+    // wait, with a time limit, for the kernel and its status word
+    e = fesom::wait_event(st.done, kWaitLimitMs);
+    if (e == cudaErrorNotReady) {
+        set_err(errbuf, errlen, "fesom_gpu_vdiff_impl_noalloc: the solve did not finish within the time limit");
+        return FESOM_ERR_TIMEOUT;
     }
-    unsigned bits = 0;
-    e = cudaMemcpy(&bits, st.status, sizeof(unsigned), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         set_err(errbuf, errlen, cudaGetErrorString(e));
         return FESOM_ERR_CUDA;
     }
+    const unsigned bits = *st.h_status;
     if (bits & FESOM_STATUS_INDEX) {
         set_err(errbuf, errlen,
                 "fesom_gpu_vdiff_impl_noalloc: a column outside 1 <= ulevels_nod2D, nlevels_nod2D <= nl with at least "
