@@ -157,11 +157,35 @@ __global__ void k_f2d(const float *in, double *out, size_t n) {
         out[i] = (double)in[i];
 }
 
+// whether the n elements from p on are this device's memory, from the first to the last, and aligned: a
+// kernel then reads or writes the caller's array as it is, and copies to and from it need no staging.
+// Anything else (host memory, another device's, an array that ends too early) takes the copies, with
+// their errors.
+template <typename S>
+bool on_device(const S *p, size_t n) {
+    int dev = -1;
+    if (!p || !n || (uintptr_t)p % sizeof(S) || cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (const char *q : {(const char *)p, (const char *)(p + n) - 1}) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+            cudaGetLastError();  // no memory of CUDA's: not an error here
+            return false;
+        }
+        if (a.type != cudaMemoryTypeDevice || a.device != dev) return false;
+    }
+    return true;
+}
+
 // host FP64 -> device array of the context precision (chunked through the stage buffer)
 int put(fesom_gpu_ctx *ctx, void *dst, const double *src, size_t n) {
     if (!src) return FESOM_OK;
     if (ctx->prec == FESOM_PREC_FP64) {
         CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDefault, ctx->stream));
+        return FESOM_OK;
+    }
+    if (on_device(src, n)) {
+        k_d2f<<<(int)std::min<size_t>((n + 255) / 256, 152 * 32), 256, 0, ctx->stream>>>(src, (float *)dst, n);
+        CK(cudaGetLastError());
         return FESOM_OK;
     }
     for (size_t off = 0; off < n; off += ctx->stage_n) {
@@ -192,11 +216,16 @@ int get(fesom_gpu_ctx *ctx, double *dst, const void *src, size_t n) {
 static int nblk(size_t m) { return (int)std::min<size_t>((m + 255) / 256, 152 * 32); }
 
 // One tracer's column-major array (host or device; FP64 or FP32) into / out of its slot of a
-// group field of the FP32 form, through the stage buffer (chunks of stage_n doubles or
-// 2 stage_n floats).  `count` entries; pair: AB3's interleaved valuesold(2, level, node) into
+// group field of the FP32 form: straight where the array is in device memory, else through the
+// stage buffer (chunks of stage_n doubles or 2 stage_n floats).  `count` entries; pair: AB3's interleaved valuesold(2, level, node) into
 // / out of the group fields g1 (k = 1) and g2 (k = 2).
 int put_slot(fesom_gpu_ctx *ctx, float *grpf, int c, const double *src, size_t count) {
     if (!src) return FESOM_OK;
+    if (on_device(src, count)) {
+        b32_put_slot(src, grpf, ctx->gw, c, count, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     for (size_t off = 0; off < count; off += ctx->stage_n) {
         const size_t m = std::min(ctx->stage_n, count - off);
         CK(cudaMemcpyAsync(ctx->stage, src + off, m * sizeof(double), cudaMemcpyDefault, ctx->stream));
@@ -207,6 +236,11 @@ int put_slot(fesom_gpu_ctx *ctx, float *grpf, int c, const double *src, size_t c
 }
 int put_slot_f(fesom_gpu_ctx *ctx, float *grpf, int c, const float *src, size_t count) {
     if (!src) return FESOM_OK;
+    if (on_device(src, count)) {
+        b32_put_slot_f(src, grpf, ctx->gw, c, count, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     float *st = (float *)ctx->stage;
     const size_t ch = 2 * ctx->stage_n;
     for (size_t off = 0; off < count; off += ch) {
@@ -219,6 +253,11 @@ int put_slot_f(fesom_gpu_ctx *ctx, float *grpf, int c, const float *src, size_t 
 }
 int get_slot(fesom_gpu_ctx *ctx, double *dst, const float *grpf, int c, size_t count) {
     if (!dst) return FESOM_OK;
+    if (on_device(dst, count)) {
+        b32_get_slot(grpf, ctx->gw, c, count, dst, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     for (size_t off = 0; off < count; off += ctx->stage_n) {
         const size_t m = std::min(ctx->stage_n, count - off);
         b32_get_slot(grpf + off * ctx->gw, ctx->gw, c, m, ctx->stage, ctx->stream);
@@ -229,6 +268,11 @@ int get_slot(fesom_gpu_ctx *ctx, double *dst, const float *grpf, int c, size_t c
 }
 int get_slot_f(fesom_gpu_ctx *ctx, float *dst, const float *grpf, int c, size_t count) {
     if (!dst) return FESOM_OK;
+    if (on_device(dst, count)) {
+        b32_get_slot_f(grpf, ctx->gw, c, count, dst, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     float *st = (float *)ctx->stage;
     const size_t ch = 2 * ctx->stage_n;
     for (size_t off = 0; off < count; off += ch) {
@@ -241,6 +285,11 @@ int get_slot_f(fesom_gpu_ctx *ctx, float *dst, const float *grpf, int c, size_t 
 }
 int put_slot_pair(fesom_gpu_ctx *ctx, float *g1, float *g2, int c, const double *src, size_t count) {
     if (!src) return FESOM_OK;
+    if (on_device(src, 2 * count)) {
+        b32_put_slot_pair(src, g1, g2, ctx->gw, c, count, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     const size_t ch = ctx->stage_n / 2;
     for (size_t off = 0; off < count; off += ch) {
         const size_t m = std::min(ch, count - off);
@@ -252,6 +301,11 @@ int put_slot_pair(fesom_gpu_ctx *ctx, float *g1, float *g2, int c, const double 
 }
 int put_slot_pair_f(fesom_gpu_ctx *ctx, float *g1, float *g2, int c, const float *src, size_t count) {
     if (!src) return FESOM_OK;
+    if (on_device(src, 2 * count)) {
+        b32_put_slot_pair_f(src, g1, g2, ctx->gw, c, count, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     float *st = (float *)ctx->stage;
     const size_t ch = ctx->stage_n;
     for (size_t off = 0; off < count; off += ch) {
@@ -264,6 +318,11 @@ int put_slot_pair_f(fesom_gpu_ctx *ctx, float *g1, float *g2, int c, const float
 }
 int get_slot_pair(fesom_gpu_ctx *ctx, double *dst, const float *g1, const float *g2, int c, size_t count) {
     if (!dst) return FESOM_OK;
+    if (on_device(dst, 2 * count)) {
+        b32_get_slot_pair(g1, g2, ctx->gw, c, count, dst, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     const size_t ch = ctx->stage_n / 2;
     for (size_t off = 0; off < count; off += ch) {
         const size_t m = std::min(ch, count - off);
@@ -275,6 +334,11 @@ int get_slot_pair(fesom_gpu_ctx *ctx, double *dst, const float *g1, const float 
 }
 int get_slot_pair_f(fesom_gpu_ctx *ctx, float *dst, const float *g1, const float *g2, int c, size_t count) {
     if (!dst) return FESOM_OK;
+    if (on_device(dst, 2 * count)) {
+        b32_get_slot_pair_f(g1, g2, ctx->gw, c, count, dst, ctx->stream);
+        CK(cudaGetLastError());
+        return FESOM_OK;
+    }
     float *st = (float *)ctx->stage;
     const size_t ch = ctx->stage_n;
     for (size_t off = 0; off < count; off += ch) {
@@ -1437,6 +1501,31 @@ int fesom_gpu_forcing_upload_f32(fesom_gpu_ctx *ctx, const float *uv, const floa
     if (ctx->prec != FESOM_PREC_FP32) { ctx->err = "FP32 buffers need a FESOM_PREC_FP32 context"; return FESOM_ERR_STATE; }
     if (!ctx->state_ready) { ctx->err = "call fesom_gpu_state_setup first"; return FESOM_ERR_STATE; }
     const size_t sNI = (size_t)ctx->nl * ctx->N2;
+    // arrays in device memory: one launch for all of them
+    if (ctx->ngr * ctx->gw <= kForcingSlots && on_device(uv, 2 * (size_t)ctx->L1 * ctx->T2) && on_device(w, sNI) &&
+        on_device(we, sNI) && on_device(Kv, sNI) && (!wi || on_device(wi, sNI)) &&
+        (!bc_surf || on_device(bc_surf, (size_t)ctx->N2 * ctx->ntr))) {
+        ForcingCopy f{};
+        f.src[0] = uv; f.dst[0] = (float *)ctx->uv; f.n[0] = 2 * (size_t)ctx->L1 * ctx->T2;
+        f.src[1] = w; f.dst[1] = (float *)ctx->w; f.n[1] = sNI;
+        if (we == w) {
+            f.dst1b = (float *)ctx->we;  // one array given as w and w_e is read once
+        } else {
+            f.src[2] = we; f.dst[2] = (float *)ctx->we; f.n[2] = sNI;
+        }
+        f.src[3] = Kv; f.dst[3] = (float *)ctx->Kv; f.n[3] = sNI;
+        if (wi) { f.src[4] = wi; f.dst[4] = (float *)ctx->wi; f.n[4] = sNI; }
+        f.bc = bc_surf;
+        f.bc_dst = (float *)ctx->bc;
+        f.N2 = ctx->N2;
+        f.G = ctx->gw;
+        f.ngr = ctx->ngr;
+        for (int k = 0; k < ctx->ngr * ctx->gw; k++) f.slot_tr[k] = (short)ctx->slot_tr[k];
+        b32_forcing(f, ctx->stream);
+        CK(cudaGetLastError());
+        ctx->forcing_ready = true;
+        return FESOM_OK;
+    }
     CK(cudaMemcpyAsync(ctx->uv, uv, 4 * 2 * (size_t)ctx->L1 * ctx->T2, cudaMemcpyDefault, ctx->stream));
     CK(cudaMemcpyAsync(ctx->w, w, 4 * sNI, cudaMemcpyDefault, ctx->stream));
     CK(cudaMemcpyAsync(ctx->we, we, 4 * sNI, cudaMemcpyDefault, ctx->stream));

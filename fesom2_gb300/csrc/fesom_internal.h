@@ -202,6 +202,20 @@ void b32_put_slot_pair(const double *src, float *g1, float *g2, int G, int c, si
 void b32_put_slot_pair_f(const float *src, float *g1, float *g2, int G, int c, size_t count, cudaStream_t);
 void b32_get_slot_pair(const float *g1, const float *g2, int G, int c, size_t count, double *dst, cudaStream_t);
 void b32_get_slot_pair_f(const float *g1, const float *g2, int G, int c, size_t count, float *dst, cudaStream_t);
+// a step's FP32 forcing from the caller's device arrays into the context's, in one launch: up to five
+// plain copies (src null: none; dst1b: a second copy of array 1) and the surface flux of every tracer
+// into its slot of the group layout (zeros in empty slots, or everywhere with bc null)
+constexpr int kForcingSlots = 256;
+struct ForcingCopy {
+    const float *src[5];
+    float *dst[5], *dst1b;
+    size_t n[5];
+    const float *bc;
+    float *bc_dst;
+    int N2, G, ngr;
+    short slot_tr[kForcingSlots];
+};
+void b32_forcing(const ForcingCopy &, cudaStream_t);
 // a whole group at once: G staged column-major arrays (FP64 or FP32; p[c] of slot c, null:
 // zeros) into / out of one group field, full G-float entries; element i of slot c is
 // p[c][i * stride + off]
