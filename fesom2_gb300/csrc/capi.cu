@@ -88,7 +88,7 @@ struct fesom_gpu_ctx {
     // second stream: the tracer-independent vertical-diffusion factors run beside the
     // advection stages and join before the update
     cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_items = nullptr;
     // host-array step with overlapped transfers: copy-in and copy-out streams, an event per
     // tracer group for "resident" and "computed"
     cudaStream_t h2d = nullptr, d2h = nullptr;
@@ -736,6 +736,7 @@ int alloc_state32(fesom_gpu_ctx *ctx, int ab) {
         CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ctx->ev_items, cudaEventDisableTiming));
         CK(cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking));
         CK(cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&ctx->ev_forcing, cudaEventDisableTiming));
@@ -916,7 +917,6 @@ int enqueue_shared32(fesom_gpu_ctx *ctx, double dt, StageTimer *tm, bool &fork, 
     DForcing<float> f = forcing_view<float>(ctx, 0);
     bool any_vd = false;
     for (int t = 0; t < ctx->ntr; t++) any_vd |= ctx->cfgs[t].i_vert_diff != 0;
-    STAGE(8, b32_vflux(ctx->tp, g, f, ctx->VF, ctx->stream));
     if (redi_on(ctx) && any_vd) {
         // Redi: the factors of the implicit solve use K33 = Kv + Kd s^2
         STAGE(9, b32_k33(ctx->tp, g, (const float *)ctx->Kv, (const float *)ctx->Ki, (const float *)ctx->slope,
@@ -930,17 +930,31 @@ int enqueue_shared32(fesom_gpu_ctx *ctx, double dt, StageTimer *tm, bool &fork, 
         if (kv_ready) CK(cudaStreamWaitEvent(ctx->side, kv_ready, 0));
         b32_vfactors(ctx->tp, g, f, dt, ctx->vfac, ctx->side);
         CK(cudaEventRecord(ctx->ev_join, ctx->side));
-    } else if (any_vd) {
-        STAGE(9, b32_vfactors(ctx->tp, g, f, dt, ctx->vfac, ctx->stream));
     }
+    STAGE(8, b32_vflux(ctx->tp, g, f, ctx->VF, ctx->stream));
+    if (any_vd && !fork) STAGE(9, b32_vfactors(ctx->tp, g, f, dt, ctx->vfac, ctx->stream));
     return FESOM_OK;
 }
 
 // the stages of groups [g0, g0 + ng); `joined` records that the stream already waited for
 // the factors of the side stream
-int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *tm, bool fork, bool &joined) {
+//
+// The node-mean edge-layers (few blocks, each a long chain of gathers) run on the side stream beside the
+// LO and edge stages, from the volume fluxes on, and join before the bounds: 2.8 % of a step on the
+// seamount channel of 640k nodes and 1.4 % on the sphere of 7 subdivisions against their own place
+// between the edge stage and the bounds, nothing on 2.9k nodes.  In line where the side stream may be waiting for a copy (items_side
+// false), in a profiled step, and where the edge stage takes several launches.
+int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *tm, bool fork, bool &joined,
+                    bool items_side = true) {
     const DGeom<float> &g = ctx->g32;
     B32View B = view32(ctx, g0, ng);
+    const bool beside = items_side && fork && !tm && ctx->mw.n_items && stage_group(ctx, 1, ng) == ng;
+    if (beside) {
+        CK(cudaEventRecord(ctx->ev_items, ctx->stream));
+        CK(cudaStreamWaitEvent(ctx->side, ctx->ev_items, 0));
+        b32_ho_nodemean(ctx->tp, B, ctx->mw, ctx->VF, ctx->side);
+        CK(cudaEventRecord(ctx->ev_items, ctx->side));
+    }
     DForcing<float> fg = forcing_view<float>(ctx, 0);
     const bool any_fct = B.fct != 0;
     if (redi_on(ctx)) B.slope = (const float *)ctx->slope;
@@ -958,9 +972,12 @@ int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *t
     if (ctx->wsplit && any_fct) STAGE(10, b32_lo_impl(ctx->tp, g, fg, B, dt, ctx->scratch, ctx->stream));
     {
         const int sg = stage_group(ctx, 1, ng);
-        for (int s0 = 0; s0 < ng; s0 += sg)
-            STAGE(2, b32_ho(ctx->tp, g, sub32(B, s0, std::min(sg, ng - s0)), ctx->mw, ctx->VF, ctx->shape[1],
-                            ctx->stream));
+        for (int s0 = 0; s0 < ng; s0 += sg) {
+            const B32View Bs = sub32(B, s0, std::min(sg, ng - s0));
+            STAGE(2, b32_ho(ctx->tp, g, Bs, ctx->mw, ctx->VF, ctx->shape[1], ctx->stream));
+            if (!beside && ctx->mw.n_items) STAGE(2, b32_ho_nodemean(ctx->tp, Bs, ctx->mw, ctx->VF, ctx->stream));
+        }
+        if (beside) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_items, 0));
     }
     // diff_tracers_ale from the values before the update; the increment waits in Tnew (the
     // oldest level, read by lo_ad and ho only) for the update to add it after the limiter
@@ -1255,6 +1272,7 @@ int fesom_gpu_finalize(fesom_gpu_ctx *ctx) {
     if (ctx->ev_wait) cudaEventDestroy(ctx->ev_wait);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+    if (ctx->ev_items) cudaEventDestroy(ctx->ev_items);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->ev_forcing) cudaEventDestroy(ctx->ev_forcing);
     if (ctx->ev_vel) cudaEventDestroy(ctx->ev_vel);
@@ -2381,7 +2399,7 @@ int step_host(fesom_gpu_ctx *ctx, double dt, const S *uv, const S *w, const S *w
                 }
         }
         for (int g0 = gs[k]; g0 < gs[k + 1]; g0 += ctx->group)
-            if ((rc = enqueue_group32(ctx, dt, g0, std::min(ctx->group, gs[k + 1] - g0), nullptr, fork, joined)))
+            if ((rc = enqueue_group32(ctx, dt, g0, std::min(ctx->group, gs[k + 1] - g0), nullptr, fork, joined, !late)))
                 return rc;
         q = 0;
         for (int g = gs[k]; g < gs[k + 1]; g++, q += G) {

@@ -2241,16 +2241,17 @@ static void ho_g(const DTopo &tp, const B32View &B, const MusclW &mw, const floa
     (void)sh;
     const int t = tile_size(tp.E2, 0);
     k32_ho<G><<<(tp.E2 + t - 1) / t, kTileThreads, 0, s>>>(tp, B, mw, VF, t);
-    if (mw.n_items) {
-        int blocks = (mw.n_items + 255) / 256;
-        if (blocks > 152 * 8) blocks = 152 * 8;
-        k32_ho_nodemean<G><<<blocks, 256, 0, s>>>(tp, B, mw, VF);
-    }
 }
 void b32_ho(const DTopo &tp, const DGeom<float> &, const B32View &B, const MusclW &mw, const float *VF,
             const LaunchShape &sh, cudaStream_t s) {
     if (B.G == 4) ho_g<4>(tp, B, mw, VF, sh, s);
     else ho_g<2>(tp, B, mw, VF, sh, s);
+}
+void b32_ho_nodemean(const DTopo &tp, const B32View &B, const MusclW &mw, const float *VF, cudaStream_t s) {
+    if (!mw.n_items) return;
+    const int blocks = std::min((mw.n_items + 255) / 256, 152 * 8);
+    if (B.G == 4) k32_ho_nodemean<4><<<blocks, 256, 0, s>>>(tp, B, mw, VF);
+    else k32_ho_nodemean<2><<<blocks, 256, 0, s>>>(tp, B, mw, VF);
 }
 void b32_bounds(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, const LaunchShape &sh,
                 cudaStream_t s) {
