@@ -237,8 +237,10 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
                     ad = upwind64(t1, t2, vf) - flo;
                 } else {
                     const double *txy = tr.trxy + t * tr.sT;
-                    if (c.ph == 0.0 && !vbad && !nonfinite64(t1) && !nonfinite64(t2) &&
-                        !grad_bad(tp, txy, !means, neg ? E.up : E.dn, neg ? E.n1 : E.n2, nz)) {
+                    // short: the upwind reconstruction alone, while everything it leaves out is finite
+                    bool full = c.ph != 0.0 || vbad || nonfinite64(t1) || nonfinite64(t2) ||
+                                grad_bad(tp, txy, !means, neg ? E.up : E.dn, neg ? E.n1 : E.n2, nz);
+                    if (!full) {
                         double2 gr;
                         if (means) node_mean_grad(tp, g, txy, neg ? E.n2 : E.n1, nz, gr.x, gr.y);
                         else gr = reinterpret_cast<const double2 *>(txy)[ix1(nz, neg ? E.dn : E.up, L1)];
@@ -247,10 +249,11 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
                         if (c.hor == 0 && (neg ? E.nbl2 : E.nbl1) < nz) q = q * 0.0;
                         const double Tm = (neg ? t2 : t1) + (neg ? -q : q);
                         ad = -(Tm * vf) - flo;
-                    } else {
+                        full = nonfinite64(Tm);  // adv_ph (Tm1 + Tm2) is then 0 * inf
+                    }
+                    if (full)
                         ad = edge_ho_full(tp, g, txy, c, !means, E.up, E.dn, E.n1, E.n2, nz, t1, t2, vf, E.ca, E.cb,
                                           E.nbl1 >= nz, E.nbl2 >= nz, flo);
-                    }
                 }
             }
             if (c.lim) tr.FLO[t * tr.sE + ke] = flo;

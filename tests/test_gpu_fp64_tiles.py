@@ -100,3 +100,31 @@ def test_element_lists_beside_the_edges_bitwise():
     wet = (lev >= mesh.ulevels_nod2D[:, None]) & (lev <= mesh.nlevels_nod2D[:, None] - 1)
     assert np.array_equal(dh[wet], om.work["del_ttf_advhoriz"][wet])
     assert np.array_equal(dv[wet], om.work["del_ttf_advvert"][wet])
+
+
+@pytest.mark.parametrize("hor,ver,lim,ph,pv", [("MUSCL", "QR4C", "FCT", 0.0, 1.0), ("MFCT", "CDIFF", "FCT", 0.0, 1.0),
+                                               ("UPW1", "UPW1", "FCT", 0.0, 1.0), ("MUSCL", "QR4C", "NON", 0.3, 0.4),
+                                               ("MFCT", "QR4C", "FCT", 0.0, 0.7)])
+@pytest.mark.parametrize("bad", [(np.nan,), (np.inf, -np.inf), (np.nan, np.inf), (1e300, -1e300),
+                                 (1e-310, -1e-310, 0.0)], ids=["nan", "inf", "mixed", "huge", "tiny"])
+def test_values_outside_the_normal_range_bitwise(hor, ver, lim, ph, pv, bad):
+    """Not-a-number, infinite, huge and denormal values reach the same results through the short
+    expressions (a product that drops out, integer maxima, quotients by reciprocals) as in the oracle."""
+    mesh = M.sphere_mesh(4, M.stretched_zbar(33, 5.0, 250.0), seed=9)
+    f = O.ensure_f64(M.make_forcing(mesh, "sphere", seed=3, dt=600.0))
+    rng = np.random.default_rng(5)
+    T = np.array(M.make_tracers(mesh, "sphere", ntr=1, seed=4)[0], copy=True)
+    T *= 1.0 + 0.02 * rng.standard_normal(T.shape)
+    TAB = np.ascontiguousarray(T * (1.0 + 1e-3 * rng.standard_normal(T.shape)))
+    lev = np.arange(1, mesh.nl)[None, :]
+    wet = (lev >= mesh.ulevels_nod2D[:, None]) & (lev <= mesh.nlevels_nod2D[:, None] - 1)
+    idx = np.argwhere(wet)
+    for q, (n, k) in enumerate(idx[rng.choice(len(idx), 12, replace=False)]):
+        (T if q % 2 else TAB)[n, k] = bad[q % len(bad)]
+    om, cfg = O.OracleMesh(mesh), O.cfg_struct(hor, ver, lim, ph=ph, pv=pv)
+    om.init_tracers_AB(cfg, T.copy(), np.zeros_like(T), T.copy())
+    om.do_oce_adv_tra(f, cfg, T, TAB)
+    ctx = G.Context(mesh, G.PREC_FP64)
+    dh, dv = ctx.adv_tra(f, G.tra_cfg(hor, ver, lim, ph, pv), T, TAB)
+    assert np.array_equal(dh[wet], om.work["del_ttf_advhoriz"][wet], equal_nan=True)
+    assert np.array_equal(dv[wet], om.work["del_ttf_advvert"][wet], equal_nan=True)
