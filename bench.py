@@ -63,10 +63,10 @@ def parse():
     p.add_argument("--no-config5", action="store_true", help="skip the configuration-5 sub-run of the default line")
     p.add_argument("--width", type=int, default=0, help="FP32 tracer-group width (0: automatic, 2, 4)")
     p.add_argument("--stage-tr", default="", help="tracers per launch of lo_ad,ho,bounds,update (e.g. 8,0,8,8)")
-    p.add_argument("--shape", default="", help="blocks per SM of lo_ad,ho,bounds,update (0: one warp per unit)")
+    p.add_argument("--shape", default="", help="blocks per SM of lo_ad,ho,bounds,update (0: one block per tile)")
     p.add_argument("--variant", default="",
-                   help="kernel variant of lo_ad,ho,bounds,update (0 registers, 1 staged; update +2: the "
-                        "vertical diffusion as its own kernel)")
+                   help="kernel variant of lo_ad,ho,bounds,update (update 2: the vertical diffusion as its own "
+                        "kernel; bit 0 selects nothing)")
     return p.parse_args()
 
 

@@ -1,7 +1,7 @@
 // fp64_stages.cuh -- the advection stages of the FP64 form.
 //
-// All of these kernels are bound by the FP64 pipe (84-87 % busy before and after; DRAM under
-// 10 %), so they are built to issue as few FP64 warp instructions as possible for the
+// All of these kernels are bound by the FP64 unit (72-98 % of its one warp instruction in 19 cycles per
+// SM; DRAM under 10 %), so they are built to issue as few FP64 warp instructions as possible for the
 // reference's bits:
 //   * comparisons, maxima, absolute values and selections run on integers (fp64_arith.cuh);
 //   * v + |v| and v - |v| are 2v or 0: an upwind sum T1 (v + |v|) + T2 (v - |v|) is one product of
@@ -96,9 +96,8 @@ k_trxy(DTopo tp, DGeom<double> g, DTracers<double> tr, int tile) {
 // downwind one enters as 0 times a finite number); adv_ph /= 0, or a value or gradient at either
 // end that is not finite, takes the full expression.
 // Bound by FP64 issue.  FP64 instructions per edge-layer (FCT, MUSCL): 13 per tracer and 10
-// shared by the tracers, against about 70 per tracer.  A step of the sphere of 7 subdivisions
-// with 48 levels and 2 tracers: 17.5 ms with k_ab, k_trxy and k_edge_flux at 5.5 ms before, 14.1
-// ms with the three at 2.1 ms.
+// shared by the tracers, against about 70 per tracer: 4.84 -> 1.46 ms on the sphere of 7 subdivisions,
+// 48 levels, 2 tracers (1.70 before the node means were set aside and the registers bounded).
 // ===========================================================================
 // whether the gradient of node's reconstruction at nz (triangle el, or the node mean) is not finite
 __device__ __forceinline__ bool grad_bad(const DTopo &tp, const double *txy, bool tri, int el, int node, int nz) {
@@ -276,7 +275,8 @@ k_edge_flux(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, 
 // (T(nz-1) - T(nz)) / (Z(nz-1) - Z(nz)) of every interface once into shared memory, then the
 // layers, which read both neighbours' (the quotient was formed three times, the flux twice).
 // Every centred or surface flux is -(0.5 (A + B) W area) - fin with A, B chosen per interface;
-// the factor 0.5 is exact, so it is applied in the last, fused operation.
+// the factor 0.5 is exact, so it is applied in the last, fused operation.  51.8 -> 18.2 M FP64 warp
+// instructions on the sphere of 7 subdivisions, 48 levels, 2 tracers: 3.09 -> 1.11 ms.
 // ===========================================================================
 // the upwind flux of adv_tra_ver_upw1 through interface nz above layer nz (top: the surface)
 __device__ __forceinline__ double ver_upw64(double T0, double Tu, double W, double ar, bool top) {
@@ -381,7 +381,7 @@ k_node_lo(DTopo tp, DGeom<double> g, DForcing<double> f, DTracers<double> tr, do
 // edge is wet (each wet element is the wet side of two of the node's edges), plus -bignumber
 // where an element of the node is dry: 7 values instead of 18.  Maxima run on integer keys in
 // shared memory; only the sums and quotients are FP64 instructions (about 45 per node-layer and
-// tracer, 165 in two kernels before).  A mesh whose edges do not cover its elements' sides, or a
+// tracer, 165 in two kernels before; 4.17 -> 0.74 ms on the sphere of 7 subdivisions, 2 tracers).  A mesh whose edges do not cover its elements' sides, or a
 // value that is not a number, takes the elements themselves with the FP64 comparisons.
 // ===========================================================================
 // max / min over the elements of node n at layer nz in the order of the reference's loop
@@ -524,7 +524,8 @@ k_bounds_rpm(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int tile
 // update of diff_tracers_ale (src/oce_ale_tracer.F90:319-321, 743-754).
 // The limited edge flux is formed at each end node from R+/R- of both ends; a limited interface
 // flux once, in a first pass over the tile.  About 60 FP64 instructions per node-layer and
-// tracer (118 before: six of its divisions are by areasvol, at 4 instead of 8 each).
+// tracer (118 before: six of its divisions are by areasvol, at 4 instead of 8 each): 2.96 -> 1.23 ms on
+// the sphere of 7 subdivisions, 48 levels, 2 tracers, at the FP64 unit's rate.
 // ===========================================================================
 static __global__ void __launch_bounds__(kTileThreads)
 k_update(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int mode, int tile) {

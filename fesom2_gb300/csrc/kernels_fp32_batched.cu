@@ -18,8 +18,8 @@
 //   k32_bounds       per node: FCT bounds (max/min of LO and T over the node's
 //                    neighbours and the adjacent layers) and R+/R- (oce_adv_tra_fct.F90)
 //   k32_update       per node: limited fluxes, flux divergence, T* update, written to
-//                    the buffer of the oldest time level; then, by default, the same warp
-//                    runs the node's implicit vertical diffusion (k32_vdiff's column solve)
+//                    the buffer of the oldest time level; then, by default, the same block
+//                    runs its columns' implicit vertical diffusion (k32_vdiff's column solve)
 //   k32_vdiff        per node: the implicit vertical diffusion as two warp scans of
 //                    affine maps over the column (forward and back substitution with
 //                    the factors of k32_vfactors); its own launch only when asked for
@@ -42,19 +42,15 @@
 // edge's direction (edges(1,e) -> edges(2,e)) and added at one end and subtracted at the
 // other, so both ends use the same bits (the upwind LO flux is recomputed at each end by the
 // same expression; the antidiffusive flux is stored once per edge-layer and its limiter
-// factor min(R+, R-) is the same seen from either end); a vertical flux is one value shuffled
-// between the two layers it joins.  With hnode = hnode_new the LO solution is T plus the flux
+// factor min(R+, R-) is the same seen from either end); a vertical flux is one value, or the same
+// expression, at the two layers it joins.  With hnode = hnode_new the LO solution is T plus the flux
 // divergence (no rescaling of T that would round every value of the column).
 //
-// Mapping of the node stages: one warp per node for all groups of the launch.  The lanes
-// cover a chunk of the node's column (one level per lane); consecutive chunks overlap by the
-// halo levels each stage needs (the level above/below comes from the neighbouring lane
-// through a shuffle), and the halo lanes compute but do not store.  The last chunk of a
-// column, when its levels fill at most half a warp, carries several groups side by side in
-// lane segments.  The node's edge list, the neighbour offsets and the tracer-independent
-// geometry of a chunk sit in registers and serve every group.  Blocks of eight warps take
-// consecutive nodes (the node order is spatially local), so the neighbour columns a block
-// gathers are mostly shared between its warps.
+// Mapping: tiles (tile.cuh).  The node stages take blocks of consecutive whole columns, a layer per
+// thread, the layers above and below through shared memory; the edge stages take blocks of 4 or 8
+// edges whose wet levels are dealt to the threads.  Every warp but a tile's last is full, nothing is
+// computed twice, and a layer's neighbour offsets and tracer-independent geometry serve every group.
+// Tiles are consecutive in the node (edge) order, which is spatially local.
 //
 // No atomics on values: each edge flux is written once and every node sum is a gather.  The
 // Adams-Bashforth shift is a rotation of the time-level buffers (no copy).
@@ -123,6 +119,8 @@ __device__ __forceinline__ float sh_dn(float v, int d) { return __shfl_down_sync
 // ---------------------------------------------------------------------------
 // k32_vflux: volume flux of every edge-layer (shared by all tracers)
 // ---------------------------------------------------------------------------
+// A tile of edges.  Bound by issue (52 %) and the gathers of two elements: 95 -> 63 us on the sphere of
+// 7 subdivisions, 48 levels, against a warp per edge.
 struct EdgeV {
     int el1, el2, nl1, nu1, nl2, nu2;
     float dX1, dY1, dX2, dY2;
@@ -291,37 +289,19 @@ __global__ void __launch_bounds__(kTB) k32_vfactors(DTopo tp, DGeom<float> g, DF
         vfactors_col(tp, g, f, dt, vf, n, threadIdx.x & 31);
 }
 
-// chunk ch of a column, HU halo levels above and HD below the stored levels
+// chunk ch of a column over a warp's lanes, HU halo levels above and HD below the stored levels
 template <int HU, int HD>
 struct Chunk {
     static constexpr int OUT = 32 - HU - HD;
     int nz;
-    int q = 0;  // segment of the lane (packed chunks): its group is the pass's first plus q
     bool lvl, out;
     __device__ __forceinline__ Chunk(int nzmin, int nzmax, int ch, int lane) {
         nz = nzmin - HU + OUT * ch + lane;
         lvl = nz >= nzmin && nz <= nzmax - 1;
         out = lvl && lane >= HU && lane < 32 - HD;
     }
-    // the last chunk of a column in P segments of W = (its levels + HU + HD) lanes, one
-    // tracer group per segment: segment q holds the lanes [q W, (q + 1) W), laid out as a whole
-    // chunk, so the vertical shuffles of a stored lane stay inside its segment
-    __device__ __forceinline__ Chunk(int nzmin, int nzmax, int ch, int lane, int W, int P) {
-        q = lane / W;
-        const int l = lane - q * W;
-        nz = nzmin - HU + OUT * ch + l;
-        lvl = q < P && nz >= nzmin && nz <= nzmax - 1;
-        out = lvl && l >= HU && l < W - HD;
-    }
     static __device__ __forceinline__ int count(int nzmin, int nzmax) { return (nzmax - nzmin + OUT - 1) / OUT; }
-    // segments of the last chunk: its width, and how many fit a warp (1: not packed)
-    static __device__ __forceinline__ int last_width(int nzmin, int nzmax) {
-        const int nl = nzmax - nzmin;
-        return nl - OUT * (count(nzmin, nzmax) - 1) + HU + HD;
-    }
 };
-
-
 
 // ---------------------------------------------------------------------------
 // entries of G floats
@@ -570,6 +550,10 @@ __device__ __forceinline__ bool slot_wet(const int4 &q, int nz) { return nz >= (
 // edges(2,e)) is rn(rn(T_n p) + rn(T_m q)) with (p, q) = (-v+, -v-) at edges(1,e) and (v-, v+) at
 // edges(2,e): the same two products and the same sum as at the other end, so the two ends add
 // exactly opposite values.
+//
+// Bound by the latency of its gathers (issue 43 %, 32 warps per SM).  A warp per node and chunk, its
+// gathers staged by cp.async: 307 us on the sphere of 7 subdivisions, 48 levels, T and S, this form
+// 165; with 24 tracers on the sphere of 8, 70 levels, 4.4 -> 3.6 ms.
 __device__ __forceinline__ void edge_share(float v, bool own, float &p, float &q) {
     const float vp = fmaxf(v, 0.f), vm = fminf(v, 0.f);
     p = own ? -vp : vm;
@@ -746,7 +730,7 @@ __device__ __forceinline__ float2 ho_minus_lo2(int hor, int ab, float2 q1, float
 // ---------------------------------------------------------------------------
 // k32_ho: high-order minus low-order flux of every edge-layer
 // ---------------------------------------------------------------------------
-// One warp per edge, the lanes over the edge's levels [nu12, nl12].  MUSCL / MFCT
+// A tile of edges over their levels [nu12, nl12].  MUSCL / MFCT
 // (adv_tra_hor_muscl / _mfct, oce_adv_tra_hor.F90:261-834) on the AB values with the
 // gradients of fill_up_dn_grad (oce_muscl_adv.F90:356-525); UPW1 (:64-257).  The LO
 // flux is the upwind flux of the current values (oce_adv_tra_driver.F90:131-190).
@@ -758,8 +742,9 @@ __device__ __forceinline__ float2 ho_minus_lo2(int hor, int ab, float2 q1, float
 // other edge-layers (under one percent of an ocean mesh's) take the node means in
 // k32_ho_nodemean.
 //
-// A pass covers 32 levels of the edge; the last pass, when its levels fill at most half a
-// warp, carries P groups side by side in segments of W lanes (PACK).
+// Bound by the latency of ten gathers per edge-layer and group.  A warp per edge took 237 us on the
+// sphere of 7 subdivisions, 48 levels, T and S, this form 132; 4.6 -> 4.0 ms with 24 tracers on the
+// sphere of 8, 70 levels.
 // the group's high-minus-low fluxes of one edge-layer from its gathered entries
 template <int G>
 __device__ __forceinline__ Vec<G> ho_group(const B32View &B, int gq, int hor, const Vec<G> &T1, const Vec<G> &T2,
@@ -920,9 +905,11 @@ __global__ void __launch_bounds__(256) k32_ho_nodemean(DTopo tp, B32View B, Musc
 // ---------------------------------------------------------------------------
 // k32_bounds: FCT bounds and R+ / R- (FCT groups only)
 // ---------------------------------------------------------------------------
-// One chunk of a node's column for the FCT groups of the launch.  PACK: the column's last
-// chunk with P groups side by side in segments of W lanes; otherwise one group at a time
-// over the whole warp.
+// FCT bounds (max / min of LO and T over the node, its neighbours and the adjacent layers) and R+ / R-
+// of the FCT groups.  320 bytes from L2 per layer and group of 4, at 9 TB/s: what bounds it with several
+// groups, the latency of the gathers with one.  Sphere of 7 subdivisions, T and S: 220 -> 152 us against
+// a warp per node; 24 tracers on the sphere of 8: 5.1 -> 5.5 ms, where the barrier per group costs more
+// than the full lanes give.
 template <int G>
 using BoundsBuf = Vec<G>[2][2][kNT];  // [buffer][max, min][thread]
 
@@ -1204,6 +1191,9 @@ __device__ __forceinline__ void vdiff_unit(const DTopo &tp, const B32View &B, co
 // ---------------------------------------------------------------------------
 // k32_update: limited update, T*
 // ---------------------------------------------------------------------------
+// 440 bytes from L2 per layer and group of 4 (R+ and R- of six neighbours, six edge fluxes), at 9 TB/s
+// with several groups; latency with one.  Sphere of 7 subdivisions, T and S, with the diffusion: 331 ->
+// 231 us against a warp per node; 24 tracers on the sphere of 8: 7.2 -> 7.2 ms.
 template <int G>
 using UpdateBuf = Vec<G>[2][kNT];  // [buffer][thread]: limited interface fluxes
 

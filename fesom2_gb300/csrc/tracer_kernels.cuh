@@ -4,15 +4,17 @@
 // reference's FP64 arithmetic in the reference's evaluation order, so the results
 // match the serial Fortran loops bit for bit.  The FP32 form has its own kernels
 // (kernels_fp32_batched.cu) and takes only the content sums from here
-// (kernels_fp32.cu).
+// (kernels_fp32.cu).  The advection stages and the column solve of the step
+// are in fp64_stages.cuh and vdiff_column.cuh; here are the vertical PPM flux, the
+// diffusion and Redi kernels, the split velocity's solve and the column solve of
+// columns too deep for shared memory.
 //
 // Mapping: edge and node kernels run one warp per entity with the lanes over
 // the levels of the column (the reference's arrays are level-contiguous, so
-// every lane load is coalesced).  Node sums are gathers over the node's
-// ascending edge list instead of the reference's edge scatters: the terms are
-// added in the same order, without atomics, so sums are deterministic.  The
-// tridiagonal solve runs one thread per column (GB300's FP64 pipe is narrow;
-// a full warp of columns keeps every lane busy).
+// every lane load is coalesced); solves run one thread per column.  Node sums
+// are gathers over the node's ascending edge list instead of the reference's
+// edge scatters: the terms are added in the same order, without atomics, so
+// sums are deterministic.
 #pragma once
 #include <cuda_runtime.h>
 

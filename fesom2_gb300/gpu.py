@@ -327,13 +327,13 @@ class Context:
 
     def set_launch_shape(self, stage: int, blocks_per_sm: int):
         """FP32 form: at most blocks_per_sm x 152 blocks for stage 0 lo_ad, 1 ho, 2 bounds, 3 update
-        (0: one warp per node or edge)."""
+        (0: one block per tile)."""
         self._chk(self.L.fesom_gpu_set_launch_shape(self.h, int(stage), int(blocks_per_sm)))
 
     def set_stage_variant(self, stage: int, variant: int):
-        """FP32 form: kernel variant of stage 0 lo_ad, 1 ho, 2 bounds, 3 update (bit 0 clear: gathers
-        in registers, set: staged in shared memory; stage 3, bit 1: the implicit vertical diffusion
-        as its own kernel instead of the update's per-node epilogue)."""
+        """FP32 form: kernel variant of stage 0 lo_ad, 1 ho, 2 bounds, 3 update (stage 3, bit 1: the
+        implicit vertical diffusion as its own kernel instead of the update's epilogue; bit 0 is kept
+        and reported but selects nothing)."""
         self._chk(self.L.fesom_gpu_set_stage_variant(self.h, int(stage), int(variant)))
 
     def autotune(self, dt: float, steps: int = 2) -> dict:
