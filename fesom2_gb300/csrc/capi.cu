@@ -829,6 +829,18 @@ B32View sub32(const B32View &B, int s0, int ns) {
     return v;
 }
 
+// Whether the implicit vertical diffusion is its own launch after the update: as set, else where the
+// mesh is deep.  As the update's epilogue it saves writing the advected column and reading it again, but
+// takes a warp per column, and a tile of 256 layers then holds few columns for its 8 warps.  The line is
+// at 56 layers with groups of 4 slots, above 64 (three levels to a lane) with groups of 2.  Sphere of 7
+// subdivisions, partial-cell bottom, ms per call, epilogue / own launch: 8 tracers 2.89 / 2.93 (40 layers),
+// 3.87 / 3.86 (55), 4.13 / 4.11 (60), 4.83 / 4.76 (70), 7.71 / 7.36 (110); 2 tracers 2.05 / 2.06 (60), 2.40 / 2.37
+// (70), 3.80 / 3.62 (110); 24 tracers on 8 subdivisions, 70 layers: 44.54 / 44.02.
+inline bool vdiff_alone(const fesom_gpu_ctx *ctx) {
+    const int v = ctx->shape[3].vsep;
+    return v < 0 ? ctx->L1 >= (ctx->gw == 4 ? 56 : 65) : v > 0;
+}
+
 // groups per launch of node stage k of a launch group of ng groups (stage_tr in tracers)
 inline int stage_group(const fesom_gpu_ctx *ctx, int k, int ng) {
     const int t = ctx->stage_tr[k];
@@ -988,9 +1000,8 @@ int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *t
         for (int s0 = 0; s0 < ng; s0 += bg)
             STAGE(4, b32_bounds(ctx->tp, g, sub32(B, s0, std::min(bg, ng - s0)), dt, ctx->shape[2], ctx->stream));
     }
-    // the implicit vertical diffusion: the epilogue of each node of the update (default), or its
-    // own launch after it
-    const bool vd = (B.ivd & ~B.wimpl) != 0, vfuse = vd && !ctx->shape[3].vsep;
+    // the implicit vertical diffusion: the epilogue of the update's tiles, or its own launch after it
+    const bool vd = (B.ivd & ~B.wimpl) != 0, vfuse = vd && !vdiff_alone(ctx);
     if (vd && fork && !joined) {
         CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
         joined = true;
@@ -1032,7 +1043,7 @@ int launches_per_step(fesom_gpu_ctx *ctx) {
             // edge-layers); vdiff
             auto passes = [&](int k) { return (ng + stage_group(ctx, k, ng) - 1) / stage_group(ctx, k, ng); };
             n += passes(0) + passes(3) + (B.fct ? passes(2) : 0) + (B.diff ? 1 : 0) +
-                 passes(1) * (ctx->mw.n_items ? 2 : 1) + (((B.ivd & ~B.wimpl) && ctx->shape[3].vsep) ? 1 : 0) +
+                 passes(1) * (ctx->mw.n_items ? 2 : 1) + (((B.ivd & ~B.wimpl) && vdiff_alone(ctx)) ? 1 : 0) +
                  (ctx->Ki ? 1 : 0) +
                  (B.ppm ? 1 : 0) + ((ctx->wsplit && B.fct) ? 1 : 0) + (B.wimpl ? 1 : 0);
         }
@@ -1935,6 +1946,7 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
         if (!(rc = time_setting(ctx, dt, steps, e0, e1, &ms)) && ms < best_ms) { best = start; best_ms = ms; }
         ncand++;
     }
+    if (best.shape[3].vsep < 0) best.shape[3].vsep = vdiff_alone(ctx);
     // coordinate descent over the stages: kernel variant, blocks per SM, tracers per launch; a
     // candidate replaces the best when it is faster by more than 1 % (timing noise)
     const int ntr_slots = ctx->ngr * ctx->gw;
@@ -1947,7 +1959,7 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
             for (int b : bps)
                 for (int q = 0; q < ntrs && !rc; q++) {
                     TuneSetting c = best;
-                    c.shape[k].vsep = v != 0;
+                    if (k == 3) c.shape[k].vsep = v;
                     c.shape[k].blocks_per_sm = b;
                     c.stage_tr[k] = q ? 8 : 0;
                     if (c == best) continue;
@@ -1973,7 +1985,7 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
     for (int k = 0; k < 4; k++) {
         res->stage_tracers[k] = best.stage_tr[k];
         res->blocks_per_sm[k] = best.shape[k].blocks_per_sm;
-        res->variant[k] = best.shape[k].variant | (best.shape[k].vsep ? 2 : 0);
+        res->variant[k] = best.shape[k].variant | (best.shape[k].vsep > 0 ? 2 : 0);
     }
     return FESOM_OK;
 }

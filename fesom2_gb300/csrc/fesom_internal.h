@@ -165,7 +165,7 @@ void b32_vfactors(const DTopo &, const DGeom<float> &, const DForcing<float> &, 
 struct LaunchShape {
     int blocks_per_sm = 0;
     int variant = 0;      // bit 0 of fesom_gpu_set_stage_variant (kept and reported; one kernel per stage)
-    bool vsep = false;    // the update stage: the implicit vertical diffusion as its own kernel
+    int vsep = -1;        // the update stage: the implicit vertical diffusion as its own kernel (0, 1; -1: by the depth)
 };
 void b32_lo_ad(const DTopo &, const DGeom<float> &, const DForcing<float> &, const B32View &, const float *VF,
                double dt, const LaunchShape &, cudaStream_t);

@@ -332,8 +332,8 @@ class Context:
 
     def set_stage_variant(self, stage: int, variant: int):
         """FP32 form: kernel variant of stage 0 lo_ad, 1 ho, 2 bounds, 3 update (stage 3, bit 1: the
-        implicit vertical diffusion as its own kernel instead of the update's epilogue; bit 0 is kept
-        and reported but selects nothing)."""
+        implicit vertical diffusion as its own kernel instead of the update's epilogue, until set the
+        faster one for the mesh's depth; bit 0 is kept and reported but selects nothing)."""
         self._chk(self.L.fesom_gpu_set_stage_variant(self.h, int(stage), int(variant)))
 
     def autotune(self, dt: float, steps: int = 2) -> dict:

@@ -312,9 +312,9 @@ int fesom_gpu_set_launch_shape(fesom_gpu_ctx *ctx, int32_t stage, int32_t blocks
 /* Performance setting of the FP32 form: kernel variant of stage 0 (lo_ad), 1 (the edge fluxes),
  * 2 (bounds) or 3 (update).  Bit 0 is kept and reported but selects nothing: each stage has one
  * kernel.  Stage 3 only, bit 1 (values 2, 3): the implicit vertical diffusion runs as its own
- * kernel after the update; clear (the default), the block that has updated a tile of nodes
- * diffuses its columns in the same launch.  Results do not change.  Defaults: lo_ad 1, the
- * others 0. */
+ * kernel after the update; clear, the block that has updated a tile of nodes diffuses its columns
+ * in the same launch; until it is set, the one that is faster for the mesh's depth.  Results do
+ * not change.  Defaults of bit 0: lo_ad 1, the others 0. */
 int fesom_gpu_set_stage_variant(fesom_gpu_ctx *ctx, int32_t stage, int32_t variant);
 /* Autotuner of the FP32 form's launch settings (results do not change): times the step of the
  * context's own state under the library defaults, then by coordinate descent over the four node/edge
