@@ -99,10 +99,10 @@ def algorithmic_bytes(counts, ntr, s, vdiff_fused=False):
 # (sphere of 7 subdivisions, 12 tracers in one launch per stage as in the full workload; inputs
 # far above L2); the traffic of a full-size launch is this figure times the tracer-DOF it
 # processes
-MEASURED_DRAM_B_PER_TRACER_DOF = {"update": 43.58, "bounds": 37.86, "edge_flux": 23.85, "lo_ad": 21.60,
-                                  "vdiff": 9.35}
+MEASURED_DRAM_B_PER_TRACER_DOF = {"update": 37.77, "bounds": 36.16, "edge_flux": 23.85, "lo_ad": 21.66,
+                                  "vdiff": 9.36}
 # the update without the diffusion epilogue (the vertical diffusion as its own kernel, "vdiff")
-MEASURED_DRAM_B_PER_TRACER_DOF_UPDATE_ALONE = 39.88
+MEASURED_DRAM_B_PER_TRACER_DOF_UPDATE_ALONE = 35.96
 
 
 def stage_bytes(counts, ntr, s, ab=2, form="fp32", vdiff_fused=False):
