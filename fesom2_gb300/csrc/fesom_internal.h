@@ -130,7 +130,7 @@ struct B32View {
     // null: Redi off
     const float *slope;
 };
-// Node degree bound of the FP32 form (the node's edge list is staged per warp)
+// Node degree bound of the FP32 form (a tile's edge lists sit in shared memory)
 constexpr int kMaxDeg = 16;
 // Per-edge MUSCL/MFCT reconstruction data of the FP32 form, precomputed at init:
 // un / dn = nodes of the up (of edges(1,e)) and down (of edges(2,e)) triangle, the edge

@@ -18,11 +18,11 @@
 //   k32_bounds       per node: FCT bounds (max/min of LO and T over the node's
 //                    neighbours and the adjacent layers) and R+/R- (oce_adv_tra_fct.F90)
 //   k32_update       per node: limited fluxes, flux divergence, T* update, written to
-//                    the buffer of the oldest time level; then, by default, the same block
-//                    runs its columns' implicit vertical diffusion (k32_vdiff's column solve)
+//                    the buffer of the oldest time level; then, in shallow meshes, the
+//                    same block runs its columns' implicit vertical diffusion (k32_vdiff's solve)
 //   k32_vdiff        per node: the implicit vertical diffusion as two warp scans of
 //                    affine maps over the column (forward and back substitution with
-//                    the factors of k32_vfactors); its own launch only when asked for
+//                    the factors of k32_vfactors); its own launch in deep meshes or as set
 //   k32_vppm, k32_lo_impl, k32_vdiff_w, k32_hdiff, k32_diff
 //                    the optional parts: PPM vertical fluxes, the split vertical
 //                    velocity, horizontal and explicit vertical diffusion
