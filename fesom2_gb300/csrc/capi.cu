@@ -2529,7 +2529,7 @@ struct fesom_gpu_batch {
     double d_dt = -1.0;
     MultiIdx ix_et{}, ix_n{}, ix_nt{}, ix_it{};  // edge tiles, nodes, node tiles, node-mean items
     int maxL1 = 0;
-    bool any_vd = false, any_fct = false, any_hd = false, any_diff = false;
+    bool any_vd = false, any_fct = false, any_hd = false, any_hd_own = false, any_diff = false;
     bool any_ws = false, any_ppm = false, any_lo_impl = false, any_wimpl = false;
     cudaGraphExec_t gexec[3] = {nullptr, nullptr, nullptr};
     double g_dt[3] = {0.0, 0.0, 0.0};
@@ -2588,7 +2588,7 @@ void enqueue_batch_step(fesom_gpu_batch *b, cudaStream_t s) {
     if (b->any_ppm) bm32_vppm(I, b->ix_n, s);
     if (b->any_lo_impl) bm32_lo_impl(I, b->ix_n, s);
     bm32_ho(I, b->ix_et, b->ix_it, s);
-    if (b->any_hd) bm32_hdiff(I, b->ix_et, s);
+    if (b->any_hd) bm32_hdiff(I, b->ix_et, b->any_hd_own, s);
     if (b->any_diff) bm32_diff(I, b->ix_nt, s);
     if (b->any_fct) bm32_bounds(I, b->ix_nt, s);
     // (the implicit vertical diffusion runs inside the update, per tile)
@@ -2638,6 +2638,7 @@ int fesom_gpu_batch_create(fesom_gpu_ctx *const *ctxs, int32_t n, fesom_gpu_batc
             b->any_diff |= c->cfgs[t].i_vert_diff == 0;
         }
         b->any_hd |= c->Ki != nullptr;
+        b->any_hd_own |= c->Ki != nullptr && !c->tp.ring_ok;
         b->any_diff |= c->Ki != nullptr;
         b->maxL1 = std::max(b->maxL1, c->L1);
         b->inst.push_back(c);
@@ -2713,7 +2714,7 @@ int fesom_gpu_batch_launches_per_step(fesom_gpu_batch *b, int32_t *launches) {
     // vflux, vfactors (the diffusion itself runs inside the update), lo_ad and update (+ bounds),
     // diff, ho (+ its node-mean items), the optional stages
     int n = 1 + (b->any_vd ? 1 : 0) + 2 + (b->any_fct ? 1 : 0) + (b->any_diff ? 1 : 0) + 1 +
-            (b->ix_it.start[b->ix_it.n] ? 1 : 0) + (b->any_hd ? 1 : 0) + (b->any_ppm ? 1 : 0) +
+            (b->ix_it.start[b->ix_it.n] ? 1 : 0) + (b->any_hd ? 1 : 0) + (b->any_hd_own ? 1 : 0) + (b->any_ppm ? 1 : 0) +
             (b->any_lo_impl ? 1 : 0) + (b->any_wimpl ? 1 : 0);
     *launches = n;
     return FESOM_OK;

@@ -262,7 +262,8 @@ void bm32_vdiff_w(const Inst32 *, const MultiIdx &nodes, cudaStream_t);
 void bm32_ho(const Inst32 *, const MultiIdx &edge_tiles, const MultiIdx &items, cudaStream_t);
 void bm32_bounds(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 void bm32_update(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
-void bm32_hdiff(const Inst32 *, const MultiIdx &edge_tiles, cudaStream_t);
+// own: some instance's edges name elements without their ends (a second launch for those)
+void bm32_hdiff(const Inst32 *, const MultiIdx &edge_tiles, bool own, cudaStream_t);
 void bm32_diff(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 
 // reciprocals of a divisor array for DGeom::rav / rhn (kernels_fp64.cu)

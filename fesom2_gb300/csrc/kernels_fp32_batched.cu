@@ -1614,6 +1614,9 @@ __global__ void __launch_bounds__(128) k32_vdiff_w(DTopo tp, DGeom<float> g, DFo
 // nodes, the layers next to both ends) per edge-layer and group where gradients of two elements and
 // vertical differences took 12, and a third of the arithmetic.  Latency of the gathers bounds it: 1.10
 // -> 0.39 ms on the sphere of 7 subdivisions, 47 layers, 7 tracers with Redi.
+//
+// That holds where an edge's elements contain both its ends.  OWN: meshes whose edge_tri names some other
+// element (ring_ok is 0): each element's gradient from its own three nodes, 6 + 6 gathers.
 struct EdgeD {
     int ia, ib, xa, xb, l1, l2;          // first entries of the columns of both ends, the elements' third nodes, the elements
     int nl1, ul1, nl2, ul2;              // levels of the elements
@@ -1630,7 +1633,7 @@ __device__ __forceinline__ float2 gs_at(const DTopo &tp, const DGeom<float> &g, 
 }
 
 // tile ti of `tile` edges
-template <int G>
+template <int G, bool OWN>
 __device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &g, const B32View &B, int ti, int tile,
                                            Tile &S, EdgeD *Ed) {
     const int L1 = tp.L1, e0 = ti * tile;
@@ -1642,37 +1645,43 @@ __device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &
             EdgeD &E = Ed[j];
             const int n1 = tp.e_n1[e], n2 = tp.e_n2[e], el1 = tp.e_t1[e], el2 = tp.e_t2[e];
             const float4 d = reinterpret_cast<const float4 *>(g.ecd)[e];
-            auto third = [&](int el) { return tp.t_n[3 * el] + tp.t_n[3 * el + 1] + tp.t_n[3 * el + 2] - n1 - n2; };
-            const int x1 = third(el1);
-            const float2 b1 = gs_at(tp, g, el1, n2), c1 = gs_at(tp, g, el1, x1);
             E.ia = n1 * L1;
             E.ib = n2 * L1;
-            E.xa = x1 * L1;
             E.l1 = el1 * L1;
             E.nl1 = tp.t_nlev[el1] - 1;
             E.ul1 = tp.t_ulev[el1];
             E.dX1 = d.x;
             E.dY1 = d.y;
-            E.w1b = d.y * b1.x - d.x * b1.y;
-            E.w1x = d.y * c1.x - d.x * c1.y;
-            E.xb = E.l2 = 0;
+            E.l2 = 0;
             E.nl2 = E.ul2 = 0;
-            E.dX2 = E.dY2 = E.w2b = E.w2x = E.w3b = E.w3x = E.w3y = 0.f;
+            E.dX2 = E.dY2 = 0.f;
             if (el2 >= 0) {
-                const int x2 = third(el2);
-                const float2 b2 = gs_at(tp, g, el2, n2), c2 = gs_at(tp, g, el2, x2);
-                const float X = d.z - d.x, Y = d.w - d.y;
-                E.xb = x2 * L1;
                 E.l2 = el2 * L1;
                 E.nl2 = tp.t_nlev[el2] - 1;
                 E.ul2 = tp.t_ulev[el2];
                 E.dX2 = d.z;
                 E.dY2 = d.w;
-                E.w2b = d.z * b2.y - d.w * b2.x;
-                E.w2x = d.z * c2.y - d.w * c2.x;
-                E.w3b = 0.5f * (X * (b1.y + b2.y) - Y * (b1.x + b2.x));
-                E.w3x = 0.5f * (X * c1.y - Y * c1.x);
-                E.w3y = 0.5f * (X * c2.y - Y * c2.x);
+            }
+            if (!OWN) {
+                auto third = [&](int el) { return tp.t_n[3 * el] + tp.t_n[3 * el + 1] + tp.t_n[3 * el + 2] - n1 - n2; };
+                const int x1 = third(el1);
+                const float2 b1 = gs_at(tp, g, el1, n2), c1 = gs_at(tp, g, el1, x1);
+                E.xa = x1 * L1;
+                E.w1b = d.y * b1.x - d.x * b1.y;
+                E.w1x = d.y * c1.x - d.x * c1.y;
+                E.xb = 0;
+                E.w2b = E.w2x = E.w3b = E.w3x = E.w3y = 0.f;
+                if (el2 >= 0) {
+                    const int x2 = third(el2);
+                    const float2 b2 = gs_at(tp, g, el2, n2), c2 = gs_at(tp, g, el2, x2);
+                    const float X = d.z - d.x, Y = d.w - d.y;
+                    E.xb = x2 * L1;
+                    E.w2b = d.z * b2.y - d.w * b2.x;
+                    E.w2x = d.z * c2.y - d.w * c2.x;
+                    E.w3b = 0.5f * (X * (b1.y + b2.y) - Y * (b1.x + b2.x));
+                    E.w3x = 0.5f * (X * c1.y - Y * c1.x);
+                    E.w3y = 0.5f * (X * c2.y - Y * c2.x);
+                }
             }
             E.top1 = tp.n_ulev[n1];
             E.bot1 = tp.n_nlev[n1];
@@ -1698,8 +1707,9 @@ __device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &
         // the flux is Kh h (weights . (T - T1) + dY S_x Tz - dX S_y Tz)
         const float h = !seg ? 0.f : 0.5f * (B.Ki[i1] + B.Ki[i2]) *
                         (seg == 3 ? 0.5f * (g.helem[E.l1 + k] + g.helem[E.l2 + k]) : g.helem[(u2 ? E.l2 : E.l1) + k]);
-        const float wb = h * (seg == 3 ? E.w3b : u1 ? E.w1b : u2 ? E.w2b : 0.f);
-        const float wx = u1 ? h * (seg == 3 ? E.w3x : E.w1x) : 0.f, wy = u2 ? h * (seg == 3 ? E.w3y : E.w2x) : 0.f;
+        const float wb = OWN ? 0.f : h * (seg == 3 ? E.w3b : u1 ? E.w1b : u2 ? E.w2b : 0.f);
+        const float wx = u1 && !OWN ? h * (seg == 3 ? E.w3x : E.w1x) : 0.f,
+                    wy = u2 && !OWN ? h * (seg == 3 ? E.w3y : E.w2x) : 0.f;
         // Redi: weights of the differences to the layers above and below at both ends (0 at the
         // columns' ends)
         float a1 = 0.f, b1 = 0.f, a2 = 0.f, b2 = 0.f;
@@ -1719,16 +1729,32 @@ __device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &
         for (int gq = 0; gq < B.ng; gq++) {
             const float *__restrict__ T = grp<G>(B.T, gq, B.sN);
             const Vec<G> T1 = vld<G>(T, i1), T2 = vld<G>(T, i2);
-            const Vec<G> Tx = vldc<G>(u1, T, E.xa + k), Ty = vldc<G>(u2, T, E.xb + k);
+            const Vec<G> Tx = vldc<G>(u1 && !OWN, T, E.xa + k), Ty = vldc<G>(u2 && !OWN, T, E.xb + k);
             const Vec<G> m1 = vldc<G>(t1, T, i1 - 1), p1 = vldc<G>(d1, T, i1 + 1);
             const Vec<G> m2 = vldc<G>(t2, T, i2 - 1), p2 = vldc<G>(d2, T, i2 + 1);
             Vec<G> out;
+            if (OWN) {
+                out = vfill<G>(0.f);
+#pragma unroll 1
+                for (int q = 0; q < 6; q++) {
+                    if (!(q < 3 ? u1 : u2)) continue;
+                    const int el = (q < 3 ? E.l1 : E.l2) / L1, v = q < 3 ? q : q - 3;
+                    // weights of the element's d/dx and d/dy: the cross vectors of its segment, the mean of
+                    // both elements' gradients in segment C
+                    const float cx = seg == 3 ? 0.5f * (E.dY1 - E.dY2) : q < 3 ? E.dY1 : -E.dY2;
+                    const float cy = seg == 3 ? 0.5f * (E.dX2 - E.dX1) : q < 3 ? -E.dX1 : E.dX2;
+                    const float w = h * (cx * g.gs[6 * (size_t)el + v] + cy * g.gs[6 * (size_t)el + 3 + v]);
+                    const Vec<G> t = vld<G>(T, tp.t_n[3 * el + v] * L1 + k);
+#pragma unroll
+                    for (int c = 0; c < G; c++) out.c[c] += w * (t.c[c] - T1.c[c]);
+                }
+            }
 #pragma unroll
             for (int c = 0; c < G; c++) {
                 const float x1 = T1.c[c], x2 = T2.c[c];
-                float f = wb * (x2 - x1);
-                if (u1) f += wx * (Tx.c[c] - x1);
-                if (u2) f += wy * (Ty.c[c] - x1);
+                float f = OWN ? out.c[c] : wb * (x2 - x1);
+                if (!OWN && u1) f += wx * (Tx.c[c] - x1);
+                if (!OWN && u2) f += wy * (Ty.c[c] - x1);
                 if (redi) {
                     f += a1 * (m1.c[c] - x1) + b1 * (x1 - p1.c[c]);
                     f += a2 * (m2.c[c] - x2) + b2 * (x2 - p2.c[c]);
@@ -1740,11 +1766,11 @@ __device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &
     }
 }
 
-template <int G>
+template <int G, bool OWN>
 __global__ void __launch_bounds__(kTileThreads, MinB<G>::hdiff) k32_hdiff(DTopo tp, DGeom<float> g, B32View B, int tile) {
     __shared__ Tile S;
     __shared__ EdgeD Ed[kTileMax];
-    hdiff_tile<G>(tp, g, B, blockIdx.x, tile, S, Ed);
+    hdiff_tile<G, OWN>(tp, g, B, blockIdx.x, tile, S, Ed);
 }
 
 // k32_diff: the diffusion increment to T* of every group in the diff mask, parked in Tnew:
@@ -2170,12 +2196,15 @@ __global__ void __launch_bounds__(128) k32m_vdiff_w(const Inst32 *__restrict__ I
     else vdiff_w_column<2>(I[i].tp, I[i].g, I[i].f, I[i].B, I[i].dtd, I[i].scratch, u - ix.start[i]);
 }
 
+// the instances whose ring_ok is !OWN
+template <bool OWN>
 __global__ void __launch_bounds__(kTileThreads, MinB<4>::hdiff) k32m_hdiff(const Inst32 *__restrict__ I, MultiIdx ix) {
     __shared__ Tile S;
     __shared__ EdgeD Ed[kTileMax];
     const int i = find_inst(ix, blockIdx.x), ti = blockIdx.x - ix.start[i];
-    if (I[i].B.G == 4) hdiff_tile<4>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
-    else hdiff_tile<2>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
+    if ((I[i].tp.ring_ok != 0) == OWN) return;
+    if (I[i].B.G == 4) hdiff_tile<4, OWN>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
+    else hdiff_tile<2, OWN>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
 }
 __global__ void __launch_bounds__(kNT, MinB<4>::diff) k32m_diff(const Inst32 *__restrict__ I, MultiIdx ix) {
     __shared__ NodeTile S;
@@ -2337,8 +2366,13 @@ void b32_k33(const DTopo &tp, const DGeom<float> &g, const float *Kv, const floa
 
 void b32_hdiff(const DTopo &tp, const DGeom<float> &g, const B32View &B, cudaStream_t s) {
     const int t = tile_size(tp.E2, 0), nb = (tp.E2 + t - 1) / t;
-    if (B.G == 4) k32_hdiff<4><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
-    else k32_hdiff<2><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+    if (B.G == 4) {
+        if (tp.ring_ok) k32_hdiff<4, false><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+        else k32_hdiff<4, true><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+    } else {
+        if (tp.ring_ok) k32_hdiff<2, false><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+        else k32_hdiff<2, true><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+    }
 }
 void b32_diff(const DTopo &tp, const DGeom<float> &g, const B32View &B, double dt, cudaStream_t s) {
     if (B.G == 4) k32_diff<4><<<tp.n_nt, kNT, 0, s>>>(tp, g, B, (float)dt);
@@ -2438,9 +2472,11 @@ void bm32_update(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
     if (u) k32m_update<<<u, kNT, 0, s>>>(I, ix);
 }
-void bm32_hdiff(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
+void bm32_hdiff(const Inst32 *I, const MultiIdx &ix, bool own, cudaStream_t s) {
     const int u = ix.start[ix.n];
-    if (u) k32m_hdiff<<<u, kTileThreads, 0, s>>>(I, ix);
+    if (!u) return;
+    k32m_hdiff<false><<<u, kTileThreads, 0, s>>>(I, ix);
+    if (own) k32m_hdiff<true><<<u, kTileThreads, 0, s>>>(I, ix);
 }
 void bm32_diff(const Inst32 *I, const MultiIdx &ix, cudaStream_t s) {
     const int u = ix.start[ix.n];
