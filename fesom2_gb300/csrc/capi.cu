@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/fesom_gpu.h"
+#include "device_array.h"
 #include "fesom_internal.h"
 #include "host_wait.h"
 #include "mesh_prep.h"
@@ -155,25 +156,6 @@ __global__ void k_d2f(const double *in, float *out, size_t n) {
 __global__ void k_f2d(const float *in, double *out, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = (double)in[i];
-}
-
-// whether the n elements from p on are this device's memory, from the first to the last, and aligned: a
-// kernel then reads or writes the caller's array as it is, and copies to and from it need no staging.
-// Anything else (host memory, another device's, an array that ends too early) takes the copies, with
-// their errors.
-template <typename S>
-bool on_device(const S *p, size_t n) {
-    int dev = -1;
-    if (!p || !n || (uintptr_t)p % sizeof(S) || cudaGetDevice(&dev) != cudaSuccess) return false;
-    for (const char *q : {(const char *)p, (const char *)(p + n) - 1}) {
-        cudaPointerAttributes a{};
-        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
-            cudaGetLastError();  // no memory of CUDA's: not an error here
-            return false;
-        }
-        if (a.type != cudaMemoryTypeDevice || a.device != dev) return false;
-    }
-    return true;
 }
 
 // host FP64 -> device array of the context precision (chunked through the stage buffer)
