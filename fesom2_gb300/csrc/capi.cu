@@ -818,9 +818,10 @@ B32View sub32(const B32View &B, int s0, int ns) {
 // subdivisions, partial-cell bottom, ms per call, epilogue / own launch: 8 tracers 2.89 / 2.93 (40 layers),
 // 3.87 / 3.86 (55), 4.13 / 4.11 (60), 4.83 / 4.76 (70), 7.71 / 7.36 (110); 2 tracers 2.05 / 2.06 (60), 2.40 / 2.37
 // (70), 3.80 / 3.62 (110); 24 tracers on 8 subdivisions, 70 layers: 44.54 / 44.02.
+inline bool vdiff_deep(const fesom_gpu_ctx *ctx) { return ctx->L1 >= (ctx->gw == 4 ? 56 : 65); }
 inline bool vdiff_alone(const fesom_gpu_ctx *ctx) {
     const int v = ctx->shape[3].vsep;
-    return v < 0 ? ctx->L1 >= (ctx->gw == 4 ? 56 : 65) : v > 0;
+    return v < 0 ? vdiff_deep(ctx) : v > 0;
 }
 
 // groups per launch of node stage k of a launch group of ng groups (stage_tr in tracers)
@@ -1849,18 +1850,6 @@ int fesom_gpu_set_stage_tracers(fesom_gpu_ctx *ctx, int32_t stage, int32_t trace
 
 // ---- autotuning of the FP32 form's launch settings (results do not change) -----------------
 namespace {
-struct TuneSetting {
-    int stage_tr[4];
-    LaunchShape shape[4];
-    bool operator==(const TuneSetting &o) const {
-        for (int k = 0; k < 4; k++)
-            if (stage_tr[k] != o.stage_tr[k] || shape[k].blocks_per_sm != o.shape[k].blocks_per_sm ||
-                shape[k].variant != o.shape[k].variant || shape[k].vsep != o.shape[k].vsep)
-                return false;
-        return true;
-    }
-};
-
 TuneSetting get_setting(const fesom_gpu_ctx *ctx) {
     TuneSetting t;
     for (int k = 0; k < 4; k++) {
@@ -1913,45 +1902,15 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     const TuneSetting start = get_setting(ctx);
-    TuneSetting def{};
-    def.shape[0].variant = 1;  // the library defaults
-    int ncand = 0;
-    float def_ms = 0.f, best_ms = 0.f;
-    put_setting(ctx, def);
-    rc = time_setting(ctx, dt, steps, e0, e1, &def_ms);
-    TuneSetting best = def;
-    best_ms = def_ms;
-    ncand = 1;
-    if (!rc && !(start == def)) {
-        float ms = 0.f;
-        put_setting(ctx, start);
-        if (!(rc = time_setting(ctx, dt, steps, e0, e1, &ms)) && ms < best_ms) { best = start; best_ms = ms; }
-        ncand++;
-    }
-    if (best.shape[3].vsep < 0) best.shape[3].vsep = vdiff_alone(ctx);
-    // coordinate descent over the stages: kernel variant, blocks per SM, tracers per launch; a
-    // candidate replaces the best when it is faster by more than 1 % (timing noise)
-    const int ntr_slots = ctx->ngr * ctx->gw;
-    const int bps[] = {0, 2, 4};
-    for (int k = 0; k < 4 && !rc; k++) {
-        // the update: also with the vertical diffusion as its own launch
-        const int nvar = k == 3 ? 2 : 1;
-        const int ntrs = (k >= 2 && ntr_slots > 8) ? 2 : 1;
-        for (int v = 0; v < nvar && !rc; v++)
-            for (int b : bps)
-                for (int q = 0; q < ntrs && !rc; q++) {
-                    TuneSetting c = best;
-                    if (k == 3) c.shape[k].vsep = v;
-                    c.shape[k].blocks_per_sm = b;
-                    c.stage_tr[k] = q ? 8 : 0;
-                    if (c == best) continue;
-                    float ms = 0.f;
-                    put_setting(ctx, c);
-                    if ((rc = time_setting(ctx, dt, steps, e0, e1, &ms))) break;
-                    ncand++;
-                    if (ms < 0.99f * best_ms) { best = c; best_ms = ms; }
-                }
-    }
+    TuneOutcome tuned{};
+    rc = tune_search(
+        start, vdiff_deep(ctx), ctx->ngr * ctx->gw,
+        [&](const TuneSetting &c, float *ms) {
+            put_setting(ctx, c);
+            return time_setting(ctx, dt, steps, e0, e1, ms);
+        },
+        tuned);
+    const TuneSetting &best = tuned.best;
     put_setting(ctx, rc ? start : best);
     for (int k = 0; k < nlev; k++)
         cudaMemcpyAsync(ctx->Bf[k], (char *)backup + lev * k, lev, cudaMemcpyDeviceToDevice, ctx->stream);
@@ -1961,9 +1920,9 @@ int fesom_gpu_autotune(fesom_gpu_ctx *ctx, double dt, int32_t steps, fesom_tune_
     cudaEventDestroy(e1);
     dfree(ctx, backup);
     if (rc) return rc;
-    res->default_ms = def_ms;
-    res->tuned_ms = best_ms;
-    res->candidates = ncand;
+    res->default_ms = tuned.def_ms;
+    res->tuned_ms = tuned.best_ms;
+    res->candidates = tuned.candidates;
     for (int k = 0; k < 4; k++) {
         res->stage_tracers[k] = best.stage_tr[k];
         res->blocks_per_sm[k] = best.shape[k].blocks_per_sm;

@@ -13,6 +13,8 @@
 
 #include <cuda_runtime.h>
 
+#include "tune.h"
+
 namespace fesom {
 
 constexpr double kREarth = 6367500.0;  // src/oce_modules.F90:29
@@ -160,13 +162,6 @@ bool b32_fct_clamp();
 void b32_vflux(const DTopo &, const DGeom<float> &, const DForcing<float> &, float *VF, cudaStream_t);
 void b32_vfactors(const DTopo &, const DGeom<float> &, const DForcing<float> &, double dt, const VFactors &,
                   cudaStream_t);
-// launch shape of the node stages (the autotuner's choices): at most `blocks_per_sm` x 152 blocks
-// looping over the tiles (0: one block per tile)
-struct LaunchShape {
-    int blocks_per_sm = 0;
-    int variant = 0;      // bit 0 of fesom_gpu_set_stage_variant (kept and reported; one kernel per stage)
-    int vsep = -1;        // the update stage: the implicit vertical diffusion as its own kernel (0, 1; -1: by the depth)
-};
 void b32_lo_ad(const DTopo &, const DGeom<float> &, const DForcing<float> &, const B32View &, const float *VF,
                double dt, const LaunchShape &, cudaStream_t);
 void b32_ho(const DTopo &, const DGeom<float> &, const B32View &, const MusclW &, const float *VF,
