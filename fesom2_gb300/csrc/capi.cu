@@ -969,7 +969,7 @@ int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *t
         const int sg = stage_group(ctx, 1, ng);
         for (int s0 = 0; s0 < ng; s0 += sg) {
             const B32View Bs = sub32(B, s0, std::min(sg, ng - s0));
-            STAGE(2, b32_ho(ctx->tp, g, Bs, ctx->mw, ctx->VF, ctx->shape[1], ctx->stream));
+            STAGE(2, b32_ho(ctx->tp, g, Bs, ctx->mw, ctx->VF, ctx->stream));
             if (!beside && ctx->mw.n_items) STAGE(2, b32_ho_nodemean(ctx->tp, Bs, ctx->mw, ctx->VF, ctx->stream));
         }
         if (beside) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_items, 0));

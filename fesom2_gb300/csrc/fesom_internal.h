@@ -164,8 +164,7 @@ void b32_vfactors(const DTopo &, const DGeom<float> &, const DForcing<float> &, 
                   cudaStream_t);
 void b32_lo_ad(const DTopo &, const DGeom<float> &, const DForcing<float> &, const B32View &, const float *VF,
                double dt, const LaunchShape &, cudaStream_t);
-void b32_ho(const DTopo &, const DGeom<float> &, const B32View &, const MusclW &, const float *VF,
-            const LaunchShape &, cudaStream_t);
+void b32_ho(const DTopo &, const DGeom<float> &, const B32View &, const MusclW &, const float *VF, cudaStream_t);
 // the edge-layers of the node-mean gradients, which b32_ho leaves out
 void b32_ho_nodemean(const DTopo &, const B32View &, const MusclW &, const float *VF, cudaStream_t);
 void b32_bounds(const DTopo &, const DGeom<float> &, const B32View &, double dt, const LaunchShape &, cudaStream_t);

@@ -2255,16 +2255,14 @@ void b32_lo_ad(const DTopo &tp, const DGeom<float> &g, const DForcing<float> &f,
     }
 }
 template <int G>
-static void ho_g(const DTopo &tp, const B32View &B, const MusclW &mw, const float *VF, const LaunchShape &sh,
-                 cudaStream_t s) {
-    (void)sh;
+static void ho_g(const DTopo &tp, const B32View &B, const MusclW &mw, const float *VF, cudaStream_t s) {
     const int t = tile_size(tp.E2, 0);
     k32_ho<G><<<(tp.E2 + t - 1) / t, kTileThreads, 0, s>>>(tp, B, mw, VF, t);
 }
 void b32_ho(const DTopo &tp, const DGeom<float> &, const B32View &B, const MusclW &mw, const float *VF,
-            const LaunchShape &sh, cudaStream_t s) {
-    if (B.G == 4) ho_g<4>(tp, B, mw, VF, sh, s);
-    else ho_g<2>(tp, B, mw, VF, sh, s);
+            cudaStream_t s) {
+    if (B.G == 4) ho_g<4>(tp, B, mw, VF, s);
+    else ho_g<2>(tp, B, mw, VF, s);
 }
 void b32_ho_nodemean(const DTopo &tp, const B32View &B, const MusclW &mw, const float *VF, cudaStream_t s) {
     if (!mw.n_items) return;

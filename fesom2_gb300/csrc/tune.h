@@ -14,10 +14,11 @@ struct LaunchShape {
 struct TuneSetting {
     int stage_tr[4];
     LaunchShape shape[4];
-    bool operator==(const TuneSetting &o) const {
+    // whether both launch the same programs: bit 0 of a variant and the edge stage's blocks per SM select nothing
+    bool same_launches(const TuneSetting &o) const {
         for (int k = 0; k < 4; k++)
-            if (stage_tr[k] != o.stage_tr[k] || shape[k].blocks_per_sm != o.shape[k].blocks_per_sm ||
-                shape[k].variant != o.shape[k].variant || shape[k].vsep != o.shape[k].vsep)
+            if (stage_tr[k] != o.stage_tr[k] || (k != 1 && shape[k].blocks_per_sm != o.shape[k].blocks_per_sm) ||
+                (k == 3 && shape[k].vsep != o.shape[k].vsep))
                 return false;
         return true;
     }
@@ -33,11 +34,13 @@ struct TuneOutcome {
 // stages: the place of the vertical diffusion, blocks per SM, tracers per launch (with more than 8 slots).  A
 // candidate replaces the best when it is faster by more than 1 % (timing noise).  own_launch: where the
 // mesh's depth puts the diffusion while nothing is set; every setting that is timed names its place, so
-// the best is one that was timed.  time(setting, &ms) returns an error code; the first one ends the search.
+// the best is one that was timed.  No two candidates launch the same programs, and what selects nothing
+// stays as it was set.  time(setting, &ms) returns an error code; the first one ends the search.
 template <class Time>
 int tune_search(TuneSetting start, bool own_launch, int slots, Time &&time, TuneOutcome &out) {
-    TuneSetting def{};
-    def.shape[0].variant = 1;  // the library defaults
+    TuneSetting def{};  // the library defaults
+    for (int k = 0; k < 4; k++) def.shape[k].variant = start.shape[k].variant;
+    def.shape[1].blocks_per_sm = start.shape[1].blocks_per_sm;
     def.shape[3].vsep = own_launch;
     if (start.shape[3].vsep < 0) start.shape[3].vsep = own_launch;
     out = TuneOutcome{def, 0.f, 0.f, 0};
@@ -53,7 +56,7 @@ int tune_search(TuneSetting start, bool own_launch, int slots, Time &&time, Tune
             out.best_ms = ms;
         }
     };
-    if (!rc && !(start == def)) attempt(start, 1.f);
+    if (!rc && !start.same_launches(def)) attempt(start, 1.f);
     const int bps[] = {0, 2, 4};
     for (int k = 0; k < 4 && !rc; k++) {
         // the update: also with the vertical diffusion as its own launch
@@ -64,9 +67,9 @@ int tune_search(TuneSetting start, bool own_launch, int slots, Time &&time, Tune
                 for (int q = 0; q < ntrs && !rc; q++) {
                     TuneSetting c = out.best;
                     if (k == 3) c.shape[k].vsep = v;
-                    c.shape[k].blocks_per_sm = b;
+                    if (k != 1) c.shape[k].blocks_per_sm = b;
                     c.stage_tr[k] = q ? 8 : 0;
-                    if (!(c == out.best)) attempt(c, 0.99f);
+                    if (!c.same_launches(out.best)) attempt(c, 0.99f);
                 }
     }
     return rc;

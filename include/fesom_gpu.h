@@ -317,7 +317,7 @@ int fesom_gpu_set_launch_shape(fesom_gpu_ctx *ctx, int32_t stage, int32_t blocks
  * not change.  Defaults of bit 0: lo_ad 1, the others 0. */
 int fesom_gpu_set_stage_variant(fesom_gpu_ctx *ctx, int32_t stage, int32_t variant);
 /* Autotuner of the FP32 form's launch settings (results do not change): times the step of the
- * context's own state under the library defaults, then by coordinate descent over the four node/edge
+ * context's own state under the library defaults, then by coordinate descent over the three node
  * stages under blocks per SM (0, 2, 4), the place of the diffusion and, for bounds and update with more
  * than 8 tracer slots, 8 tracers per launch; a candidate is kept when it is more than 1 % faster.
  * Each candidate runs one untimed and `steps` timed steps (CUDA events on the context's stream).

@@ -12,6 +12,13 @@ static int bad = 0;
 static void check(bool ok, const char *what, int seed) {
     if (!ok) { std::printf("%s (%d)\n", what, seed); bad++; }
 }
+// the same launches: bit 0 of a variant and the edge stage's blocks per SM select nothing
+static bool same(const TuneSetting &a, const TuneSetting &b) {
+    bool r = a.shape[3].vsep == b.shape[3].vsep;
+    for (int k = 0; k < 4; k++)
+        r = r && a.stage_tr[k] == b.stage_tr[k] && (k == 1 || a.shape[k].blocks_per_sm == b.shape[k].blocks_per_sm);
+    return r;
+}
 static TuneSetting defaults() {
     TuneSetting t{};
     t.shape[0].variant = 1;
@@ -40,7 +47,7 @@ int main() {
                 TuneOutcome out{};
                 check(tune_search(start, own != 0, 12, time, out) == 0, "error", seed);
                 bool found = false;
-                for (const Timed &t : timed) found = found || (t.c == out.best && t.ms == out.best_ms);
+                for (const Timed &t : timed) found = found || (same(t.c, out.best) && t.ms == out.best_ms);
                 check(found, "the best was not timed, or took another time", seed);
                 check(out.best.shape[3].vsep == own, "the slower place of the diffusion was kept", seed);
                 check(out.def_ms == timed[0].ms && out.candidates == (int)timed.size(), "counts", seed);
@@ -57,3 +64,40 @@ int main() {
 
 def test_the_result_is_a_setting_that_was_timed(tmp_path):
     host_cpp.run(tmp_path, PLACE)
+
+
+INERT = COMMON + r"""
+int main() {
+    for (int seed = 0; seed < 60; seed++) {
+        TuneSetting start = defaults();
+        start.shape[3].vsep = -1;
+        start.shape[1].blocks_per_sm = seed % 3 ? 4 : 0;  // selects nothing
+        start.shape[2].variant = seed % 2;                // selects nothing
+        if (seed % 5 == 4) start.stage_tr[1] = 8;         // does
+        std::vector<Timed> timed;
+        unsigned r = 99u * seed + 1;
+        TuneSetting best{};  // the one a candidate is measured against
+        float best_ms = 0.f;
+        auto time = [&](const TuneSetting &c, float *ms) {
+            r = r * 1664525u + 1013904223u;
+            *ms = 10.f + 3.f * ((r >> 8) / 16777216.f);
+            if (!timed.empty()) check(!same(c, best), "the program of the best was timed again", seed);
+            const float margin = timed.size() == 1 && seed % 5 == 4 ? 1.f : 0.99f;  // the start's own settings
+            timed.push_back({c, *ms});
+            if (timed.size() == 1 || *ms < margin * best_ms) { best = c; best_ms = *ms; }
+            return 0;
+        };
+        TuneOutcome out{};
+        tune_search(start, false, 12, time, out);
+        check(same(best, out.best) && best_ms == out.best_ms, "another best", seed);
+        check(out.best.shape[1].blocks_per_sm == start.shape[1].blocks_per_sm, "the edge stage's blocks were tuned", seed);
+        for (int k = 0; k < 4; k++)
+            check(out.best.shape[k].variant == start.shape[k].variant, "a variant's bit 0 was changed", seed);
+    }
+    return bad;
+}
+"""
+
+
+def test_no_program_is_timed_against_itself(tmp_path):
+    host_cpp.run(tmp_path, INERT)
