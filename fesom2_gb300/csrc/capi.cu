@@ -50,7 +50,7 @@ struct fesom_gpu_ctx {
     double *scratch = nullptr, *partials = nullptr, *content_out = nullptr;
     int content_blocks = 0;
     unsigned *status = nullptr;
-    unsigned *h_status = nullptr;  // page-locked copy of the status word
+    unsigned *h_status = nullptr;  // page-locked copy of the status word (null: none to be had)
     cudaEvent_t ev_wait = nullptr;
     bool forcing_ready = false;
     bool state_ready = false;
@@ -1072,9 +1072,11 @@ int wait_stream(fesom_gpu_ctx *ctx, int timeout_ms) {
 
 // the same, with the status word read behind the stream's work
 int wait_status(fesom_gpu_ctx *ctx, unsigned *st) {
-    CK(cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    if (ctx->h_status)
+        CK(cudaMemcpyAsync(ctx->h_status, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     const int rc = wait_stream(ctx, -1);
-    *st = *ctx->h_status;
+    if (ctx->h_status) *st = *ctx->h_status;
+    else if (!rc) CK(cudaMemcpy(st, ctx->status, sizeof(unsigned), cudaMemcpyDeviceToHost));
     return rc;
 }
 
@@ -1232,7 +1234,10 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
     if ((rc = dalloc(ctx, (void **)&ctx->content_out, sizeof(double) * ctx->max_tr))) return rc;
     if ((rc = dalloc(ctx, (void **)&ctx->status, sizeof(unsigned)))) return rc;
     CK(cudaMemset(ctx->status, 0, sizeof(unsigned)));
-    CK(cudaHostAlloc((void **)&ctx->h_status, sizeof(unsigned), cudaHostAllocDefault));
+    if (cudaHostAlloc((void **)&ctx->h_status, sizeof(unsigned), cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->h_status = nullptr;
+    }
     CK(cudaDeviceSynchronize());
     return FESOM_OK;
 }

@@ -53,13 +53,14 @@ std::mutex g_mu;
 struct DevState {
     double *scratch = nullptr;
     unsigned *status = nullptr;
-    unsigned *h_status = nullptr;  // in g_host_status
+    unsigned *h_status = nullptr;  // in g_host_status, null where that is not page-locked
     cudaEvent_t done = nullptr;
 };
 DevState g_dev[kMaxDevices];
-// the status words' host copies: static memory, page-locked at first use
+// the status words' host copies: static memory, page-locked at first use.  A caller may have no page-locked
+// memory to give: the status word is then read by a blocking copy behind the wait
 alignas(4096) unsigned g_host_status[1024];
-bool g_host_locked = false;
+bool g_host_tried = false, g_host_locked = false;
 
 void set_err(char *errbuf, int32_t errlen, const char *msg) {
     if (errbuf && errlen > 0) {
@@ -169,15 +170,13 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
                 set_err(errbuf, errlen, cudaGetErrorString(e));
                 return FESOM_ERR_CUDA;
             }
-            if (!g_host_locked) {
-                e = cudaHostRegister(g_host_status, sizeof g_host_status, cudaHostRegisterPortable);
-                if (e != cudaSuccess) {
-                    set_err(errbuf, errlen, cudaGetErrorString(e));
-                    return FESOM_ERR_CUDA;
-                }
-                g_host_locked = true;
+            if (!g_host_tried) {
+                g_host_tried = true;
+                g_host_locked =
+                    cudaHostRegister(g_host_status, sizeof g_host_status, cudaHostRegisterPortable) == cudaSuccess;
+                if (!g_host_locked) cudaGetLastError();
             }
-            d.h_status = g_host_status + dev;
+            d.h_status = g_host_locked ? g_host_status + dev : nullptr;
             d.status = (unsigned *)q;
             d.scratch = (double *)p;
         }
@@ -204,7 +203,7 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
             st.scratch, st.status);
     }
     e = cudaGetLastError();
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && st.h_status)
         e = cudaMemcpyAsync(st.h_status, st.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaEventRecord(st.done, s);
     if (e != cudaSuccess) {
@@ -221,7 +220,16 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
         set_err(errbuf, errlen, cudaGetErrorString(e));
         return FESOM_ERR_CUDA;
     }
-    const unsigned bits = *st.h_status;
+    unsigned bits = 0;
+    if (st.h_status) {
+        bits = *st.h_status;
+    } else {
+        e = cudaMemcpy(&bits, st.status, sizeof bits, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) {
+            set_err(errbuf, errlen, cudaGetErrorString(e));
+            return FESOM_ERR_CUDA;
+        }
+    }
     if (bits & FESOM_STATUS_INDEX) {
         set_err(errbuf, errlen,
                 "fesom_gpu_vdiff_impl_noalloc: a column outside 1 <= ulevels_nod2D, nlevels_nod2D <= nl with at least "
