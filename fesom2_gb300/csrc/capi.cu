@@ -937,21 +937,25 @@ int enqueue_shared32(fesom_gpu_ctx *ctx, double dt, StageTimer *tm, bool &fork, 
 // The node-mean edge-layers (few blocks, each a long chain of gathers) run on the side stream beside the
 // LO and edge stages, from the volume fluxes on, and join before the bounds: 2.8 % of a step on the
 // seamount channel of 640k nodes and 1.4 % on the sphere of 7 subdivisions against their own place
-// between the edge stage and the bounds, nothing on 2.9k nodes.  In line where the side stream may be waiting for a copy (items_side
+// between the edge stage and the bounds, nothing on 2.9k nodes.  With the split velocity they start behind
+// its column kernel.  In line where the side stream may be waiting for a copy (items_side
 // false), in a profiled step, and where the edge stage takes several launches.
 int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *tm, bool fork, bool &joined,
                     bool items_side = true) {
     const DGeom<float> &g = ctx->g32;
     B32View B = view32(ctx, g0, ng);
     const bool beside = items_side && fork && !tm && ctx->mw.n_items && stage_group(ctx, 1, ng) == ng;
-    if (beside) {
+    const bool any_fct = B.fct != 0, lo_impl = ctx->wsplit && any_fct;
+    auto fork_items = [&]() -> int {
         CK(cudaEventRecord(ctx->ev_items, ctx->stream));
         CK(cudaStreamWaitEvent(ctx->side, ctx->ev_items, 0));
         b32_ho_nodemean(ctx->tp, B, ctx->mw, ctx->VF, ctx->side);
         CK(cudaEventRecord(ctx->ev_items, ctx->side));
-    }
+        return FESOM_OK;
+    };
+    int rc;
+    if (beside && !lo_impl && (rc = fork_items())) return rc;
     DForcing<float> fg = forcing_view<float>(ctx, 0);
-    const bool any_fct = B.fct != 0;
     if (redi_on(ctx)) B.slope = (const float *)ctx->slope;
     // the implicit solve with the w_i terms diffuses with K33 under Redi
     DForcing<float> fk = fg;
@@ -963,8 +967,17 @@ int enqueue_group32(fesom_gpu_ctx *ctx, double dt, int g0, int ng, StageTimer *t
                                 ctx->stream));
     }
     if (B.ppm) STAGE(10, b32_vppm(ctx->tp, g, fg, B, dt, ctx->stream));
-    // split vertical velocity: w_i advects the LO values implicitly (oce_adv_tra_driver.F90:323-334)
-    if (ctx->wsplit && any_fct) STAGE(10, b32_lo_impl(ctx->tp, g, fg, B, dt, ctx->scratch, ctx->stream));
+    // split vertical velocity: w_i advects the LO values implicitly (oce_adv_tra_driver.F90:323-334).
+    // Nothing runs beside it: it is a wave or less of long FP64 columns, and other blocks on the chip crowd
+    // its own onto some of the SMs (28k columns of 47 layers, T and S: 1404 us a step for 800)
+    if (lo_impl) {
+        if (fork && !joined) {
+            CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
+            joined = true;
+        }
+        STAGE(10, b32_lo_impl(ctx->tp, g, fg, B, dt, ctx->scratch, ctx->stream));
+        if (beside && (rc = fork_items())) return rc;
+    }
     {
         const int sg = stage_group(ctx, 1, ng);
         for (int s0 = 0; s0 < ng; s0 += sg) {
