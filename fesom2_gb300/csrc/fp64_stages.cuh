@@ -692,14 +692,14 @@ void Launch<double>::update(const DTopo &tp, const DGeom<double> &g, DTracers<do
 template <>
 void Launch<double>::vdiff(const DTopo &tp, const DGeom<double> &g, const DForcing<double> &f, DTracers<double> &tr,
                            double dt, double *scratch, cudaStream_t s) {
-    if (vtile_smem(tp.L1, kVCols, 1) > kVSmemMax) {
+    if (vtile_smem(tp.L1, kVCols, 1) > kVSmemMax || vdiff_by_column(tp.N2, tp.L1)) {
         k_vdiff<double><<<(tp.N2 + 127) / 128, 128, 0, s>>>(tp, g, f, tr, dt, scratch);
         return;
     }
     // as many tracers at a time as share the coefficients with two blocks resident per SM
     int nt = std::min(tr.ntr, 4);
     while (nt > 1 && vtile_smem(tp.L1, kVCols, nt) > kVSmemMax / 2) nt--;
-    const int cols = vtile_cols(tp.N2, nt);
+    const int cols = vtile_cols(tp.N2, nt, tp.L1);
     const VArgs P{tp.N2, tp.nl,      cols, tp.n_nlev, tp.n_ulev, g.zbar_n_bot, g.hnode_new,
                   g.area, g.areasvol, f.Kv, f.wi,      g.rav,     dt};
     const int nb = (tp.N2 + cols - 1) / cols;

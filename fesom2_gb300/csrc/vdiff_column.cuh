@@ -4,7 +4,8 @@
 // the same bits.
 //
 // Two mappings with the same bits: a tile of columns in shared memory (vdiff_tile), and one thread
-// per column over a scratch in device memory for columns too deep for it.  Scratch entry k of a column (Z_n, the Thomas factors cp and tp)
+// per column over a scratch in device memory for columns too deep for it and for many deep ones
+// (vdiff_by_column).  Scratch entry k of a column (Z_n, the Thomas factors cp and tp)
 // sits at p[k * st]: level-major over the columns of a launch, so the threads of a warp
 // touch consecutive addresses at every level.
 #pragma once
@@ -121,7 +122,7 @@ __device__ __forceinline__ void vdiff_col_solve(const ColScratch &s, int nzmin, 
 // ---------------------------------------------------------------------------
 // A thread per column (above) reads every array with the stride of a column (32 lines per warp
 // load) and runs one chain of five divisions per level.  Here only the recurrences run a lane per
-// column; coefficients and right-hand sides are formed by all 128 threads, the wet levels of the
+// column; coefficients and right-hand sides are formed by all 256 threads, the wet levels of the
 // tile dealt out one after another (coalesced, full warps), and up to 4 tracers share the
 // coefficients and the pivots.
 //
@@ -135,24 +136,39 @@ __device__ __forceinline__ void vdiff_col_solve(const ColScratch &s, int nzmin, 
 // holds (217 layers) take the thread per column.
 constexpr int kVCols = 32, kVThreads = 256, kVChunk = 8;
 constexpr size_t kVSmemMax = 224 * 1024;
+constexpr size_t kVSmemHalf = 115200;  // two blocks of it, their VTile and 1 KB reserved for each fill an SM's 228 KB
 __host__ __device__ constexpr size_t vtile_smem(int L1, int cols, int nt) {
     return (size_t)(3 + nt) * L1 * (cols | 1) * sizeof(double);
 }
 // columns per tile: the recurrences cost an SM 12 + 13 nt FP64 instructions per level and tile, the
 // rest 29 + 9 nt per 32 columns and level; the widest tile unless a narrower one shares the tiles
-// out better over the 152 SMs (2.9k columns: 20, one tile on each of 146 SMs)
-inline int vtile_cols(int n, int nt) {
+// out better over the 152 SMs (2.9k columns: 20, one tile on each of 146 SMs).  A tile that leaves no room for
+// a second one on its SM (32 columns from 110 layers on) has nobody to run while its recurrences do: 1.65
+// times the time per tile, where an SM gets several (78k columns of 120 layers: 2192 us with 32 columns, 1319
+// with 29)
+inline int vtile_cols(int n, int nt, int L1) {
     int best = kVCols;
     double cost = 0.0;
     for (int c = kVCols; c >= 8; c--) {
         const int waves = ((n + c - 1) / c + 151) / 152;
-        const double x = waves * (12.0 + 13.0 * nt + (29.0 + 9.0 * nt) * c / 32.0);
+        const bool alone = waves > 1 && vtile_smem(L1, c, nt) > kVSmemHalf;
+        const double x = waves * (12.0 + 13.0 * nt + (29.0 + 9.0 * nt) * c / 32.0) * (alone ? 1.65 : 1.0);
         if (c == kVCols || x < 0.98 * cost) {
             best = c;
             cost = x;
         }
     }
     return best;
+}
+
+// whether a thread per column is the faster mapping for columns that a tile would hold: deep tiles are narrow
+// (17 columns at 200 layers), so their recurrences, a lane per column, cost more of the FP64 unit, and with
+// enough columns a thread per column keeps it as busy where every column starts on a 32-byte sector.  Tile /
+// thread per column, us: 78k columns of 144 layers 1748 / 1781, 148: 1881 / 1824, 200: 2951 / 2467; 29k
+// of 156: 807 / 807, 160: 811 / 827, 172: 975 / 889; 22k of 216: 973 / 1117; off the sector, 78k of 201:
+// 2970 / 3510
+inline bool vdiff_by_column(int n, int L1) {
+    return L1 % 4 == 0 && n >= 26000 && L1 >= (n >= 60000 ? 148 : 160);
 }
 
 struct VArgs {

@@ -191,7 +191,7 @@ extern "C" int fesom_gpu_vdiff_impl_noalloc(int32_t nod2D, int32_t nl, const int
     // columns that fit a tile's shared memory leave the scratch alone (19.6k columns of 47 layers: the
     // kernel takes 127 us against 217 with a thread per column, of which the FP64 unit needs 113)
     if (fesom::vtile_smem(nl - 1, fesom::kVCols, 1) <= fesom::kVSmemMax) {
-        const int cols = fesom::vtile_cols(nod2D, 1);
+        const int cols = fesom::vtile_cols(nod2D, 1, nl - 1);
         const fesom::VArgs P{nod2D,     nl,   cols, nlevels_nod2D, ulevels_nod2D, zbar_n_bot, hnode_new, area,
                              areasvol, Kv,   nullptr, nullptr,     dt};
         k_vdiff_noalloc_tile<<<(nod2D + cols - 1) / cols, fesom::kVThreads, fesom::vtile_smem(nl - 1, cols, 1), s>>>(
