@@ -1196,6 +1196,13 @@ int fesom_gpu_init(const fesom_mesh_desc *mesh, int32_t precision, int32_t max_t
         (rc = upload_int(ctx, &tp.ne_ptr, h.ne_ptr)) || (rc = upload_int(ctx, &tp.ne_idx, h.ne_idx)) ||
         (rc = upload_int(ctx, &tp.nie_ptr, h.nie_ptr)) || (rc = upload_int(ctx, &tp.nie_idx, h.nie_idx)))
         return rc;
+    tp.grad_zero = 1;
+    for (size_t el = 0; el < (size_t)ctx->T2 && precision == FESOM_PREC_FP32; el++)
+        for (const double *w = mesh->gradient_sca + 6 * el; w < mesh->gradient_sca + 6 * el + 6; w += 3) {
+            const double top = std::max({std::fabs(w[0]), std::fabs(w[1]), std::fabs(w[2])});
+            // 2^-22: weights rounded to FP32 add up to no more; not a number: no
+            if (!(std::fabs(w[0] + w[1] + w[2]) <= 0x1p-22 * top)) tp.grad_zero = 0;
+        }
     // tiles of consecutive nodes for the FP32 node kernels
     tp.n_nt = 0;
     tp.nt_ptr = nullptr;
@@ -2597,7 +2604,7 @@ int fesom_gpu_batch_create(fesom_gpu_ctx *const *ctxs, int32_t n, fesom_gpu_batc
             b->any_diff |= c->cfgs[t].i_vert_diff == 0;
         }
         b->any_hd |= c->Ki != nullptr;
-        b->any_hd_own |= c->Ki != nullptr && !c->tp.ring_ok;
+        b->any_hd_own |= c->Ki != nullptr && !c->tp.diff_by_edges();
         b->any_diff |= c->Ki != nullptr;
         b->maxL1 = std::max(b->maxL1, c->L1);
         b->inst.push_back(c);

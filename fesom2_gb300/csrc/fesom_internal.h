@@ -38,6 +38,10 @@ struct DTopo {
     const int *nt_ptr;
     // every element lies on exactly three edges and in the element lists of exactly its three nodes
     int ring_ok;
+    // FP32 form: every element's gradient weights (gradient_sca) add up to zero, to the rounding of FP32
+    int grad_zero;
+    // whether the FP32 diffusion may take a gradient as weights of differences over a node's edges
+    __host__ __device__ bool diff_by_edges() const { return ring_ok && grad_zero; }
 };
 
 template <typename R>
@@ -256,7 +260,7 @@ void bm32_vdiff_w(const Inst32 *, const MultiIdx &nodes, cudaStream_t);
 void bm32_ho(const Inst32 *, const MultiIdx &edge_tiles, const MultiIdx &items, cudaStream_t);
 void bm32_bounds(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 void bm32_update(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
-// own: some instance's edges name elements without their ends (a second launch for those)
+// own: some instance takes its elements' own nodes (not diff_by_edges; a second launch for those)
 void bm32_hdiff(const Inst32 *, const MultiIdx &edge_tiles, bool own, cudaStream_t);
 void bm32_diff(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 

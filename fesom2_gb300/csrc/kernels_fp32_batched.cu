@@ -1615,8 +1615,9 @@ __global__ void __launch_bounds__(128) k32_vdiff_w(DTopo tp, DGeom<float> g, DFo
 // vertical differences took 12, and a third of the arithmetic.  Latency of the gathers bounds it: 1.10
 // -> 0.39 ms on the sphere of 7 subdivisions, 47 layers, 7 tracers with Redi.
 //
-// That holds where an edge's elements contain both its ends.  OWN: meshes whose edge_tri names some other
-// element (ring_ok is 0): each element's gradient from its own three nodes, 6 + 6 gathers.
+// That holds where an edge's elements contain both its ends and an element's weights add up to zero.  OWN:
+// meshes whose edge_tri names some other element or whose weights do not (not diff_by_edges): each
+// element's gradient from its own three nodes, 6 + 6 gathers.
 struct EdgeD {
     int ia, ib, xa, xb, l1, l2;          // first entries of the columns of both ends, the elements' third nodes, the elements
     int nl1, ul1, nl2, ul2;              // levels of the elements
@@ -1746,7 +1747,7 @@ __device__ __forceinline__ void hdiff_tile(const DTopo &tp, const DGeom<float> &
                     const float w = h * (cx * g.gs[6 * (size_t)el + v] + cy * g.gs[6 * (size_t)el + 3 + v]);
                     const Vec<G> t = vld<G>(T, tp.t_n[3 * el + v] * L1 + k);
 #pragma unroll
-                    for (int c = 0; c < G; c++) out.c[c] += w * (t.c[c] - T1.c[c]);
+                    for (int c = 0; c < G; c++) out.c[c] += w * (tp.grad_zero ? t.c[c] - T1.c[c] : t.c[c]);
                 }
             }
 #pragma unroll
@@ -1788,7 +1789,8 @@ __global__ void __launch_bounds__(kTileThreads, MinB<G>::hdiff) k32_hdiff(DTopo 
 // With the weights below, 6 gathers of T per group instead of 18: 0.68 -> 0.41 ms on the sphere of 7
 // subdivisions, 47 layers, 7 tracers with Redi.
 //
-// Redi: the node gradient's weights per edge slot.  The gradients of the node's elements sum over
+// Redi: the node gradient's weights per edge slot (diff_by_edges; else the elements themselves).  The
+// gradients of the node's elements sum over
 // the neighbours: with weights of a triangle that add up to zero, sum_el ea grad T = sum_m w_m
 // (T_m - T_n), where w_m joins the node's two elements at edge (n, m), each where it is wet.
 struct DiffSlots {
@@ -1904,7 +1906,7 @@ __device__ __forceinline__ void diff_tile(const DTopo &tp, const DGeom<float> &g
             }
         }
         if (B.slope) {
-            if (!tp.ring_ok && k.on) {  // edges that do not cover the elements' sides: the elements themselves
+            if (!tp.diff_by_edges() && k.on) {  // the elements themselves
                 p = vfill<G>(0.f);
                 for (int kk = tp.nie_ptr[k.n]; kk < tp.nie_ptr[k.n + 1]; kk++) {
                     const int el = tp.nie_idx[kk];
@@ -1914,7 +1916,7 @@ __device__ __forceinline__ void diff_tile(const DTopo &tp, const DGeom<float> &g
                         const Vec<G> t = vld<G>(T, tp.t_n[3 * el + m] * tp.L1 + nz - 1);
                         const float w = (sx * g.gs[6 * (size_t)el + m] + sy * g.gs[6 * (size_t)el + 3 + m]) * ea;
 #pragma unroll
-                        for (int c = 0; c < G; c++) p.c[c] += w * (t.c[c] - Tn.c[c]);
+                        for (int c = 0; c < G; c++) p.c[c] += w * (tp.grad_zero ? t.c[c] - Tn.c[c] : t.c[c]);
                     }
                 }
             }
@@ -1941,7 +1943,7 @@ __global__ void __launch_bounds__(kNT, MinB<G>::diff) k32_diff(DTopo tp, DGeom<f
     __shared__ DiffSlots D;
     __shared__ DiffBuf<G> X;
     node_tile_load(tp, blockIdx.x, S);
-    if (B.slope && tp.ring_ok) diff_slots_load(tp, g, S, D);
+    if (B.slope && tp.diff_by_edges()) diff_slots_load(tp, g, S, D);
     diff_tile<G>(tp, g, B, dt, S, D, X);
 }
 
@@ -2196,13 +2198,13 @@ __global__ void __launch_bounds__(128) k32m_vdiff_w(const Inst32 *__restrict__ I
     else vdiff_w_column<2>(I[i].tp, I[i].g, I[i].f, I[i].B, I[i].dtd, I[i].scratch, u - ix.start[i]);
 }
 
-// the instances whose ring_ok is !OWN
+// the instances that take their elements' own nodes (OWN), or those that do not
 template <bool OWN>
 __global__ void __launch_bounds__(kTileThreads, MinB<4>::hdiff) k32m_hdiff(const Inst32 *__restrict__ I, MultiIdx ix) {
     __shared__ Tile S;
     __shared__ EdgeD Ed[kTileMax];
     const int i = find_inst(ix, blockIdx.x), ti = blockIdx.x - ix.start[i];
-    if ((I[i].tp.ring_ok != 0) == OWN) return;
+    if (I[i].tp.diff_by_edges() == OWN) return;
     if (I[i].B.G == 4) hdiff_tile<4, OWN>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
     else hdiff_tile<2, OWN>(I[i].tp, I[i].g, I[i].B, ti, kTileMax, S, Ed);
 }
@@ -2217,7 +2219,7 @@ __global__ void __launch_bounds__(kNT, MinB<4>::diff) k32m_diff(const Inst32 *__
     const Inst32 &d = I[i];
     if (!d.B.diff) return;
     node_tile_load(d.tp, blockIdx.x - ix.start[i], S);
-    if (d.B.slope && d.tp.ring_ok) diff_slots_load(d.tp, d.g, S, D);
+    if (d.B.slope && d.tp.diff_by_edges()) diff_slots_load(d.tp, d.g, S, D);
     if (d.B.G == 4) diff_tile<4>(d.tp, d.g, d.B, d.dt, S, D, U.X4);
     else diff_tile<2>(d.tp, d.g, d.B, d.dt, S, D, U.X2);
 }
@@ -2365,10 +2367,10 @@ void b32_k33(const DTopo &tp, const DGeom<float> &g, const float *Kv, const floa
 void b32_hdiff(const DTopo &tp, const DGeom<float> &g, const B32View &B, cudaStream_t s) {
     const int t = tile_size(tp.E2, 0), nb = (tp.E2 + t - 1) / t;
     if (B.G == 4) {
-        if (tp.ring_ok) k32_hdiff<4, false><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+        if (tp.diff_by_edges()) k32_hdiff<4, false><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
         else k32_hdiff<4, true><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
     } else {
-        if (tp.ring_ok) k32_hdiff<2, false><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
+        if (tp.diff_by_edges()) k32_hdiff<2, false><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
         else k32_hdiff<2, true><<<nb, kTileThreads, 0, s>>>(tp, g, B, t);
     }
 }
