@@ -264,9 +264,9 @@ void bm32_update(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 void bm32_hdiff(const Inst32 *, const MultiIdx &edge_tiles, bool own, cudaStream_t);
 void bm32_diff(const Inst32 *, const MultiIdx &node_tiles, cudaStream_t);
 
-// reciprocals of a divisor array for DGeom::rav / rhn (kernels_fp64.cu)
 // shared-memory limits of the FP64 kernels, once per context (kernels_fp64.cu)
 cudaError_t fp64_prepare();
+// reciprocals of a divisor array for DGeom::rav / rhn (kernels_fp64.cu)
 void recip_table(const double *y, double2 *out, size_t n, cudaStream_t);
 
 // tail of the tracer loop (kernels_tail.cu): one tracer's decay, relaxation and clamp

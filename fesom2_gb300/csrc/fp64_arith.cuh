@@ -3,8 +3,8 @@
 //
 // sm_103a issues one FP64 warp instruction per SM every 19 cycles (measured over
 // the stages of the form; one warp alone, every 64), so a compare, a maximum or a select done
-// in integer instructions costs next to nothing beside one FP64 add, and a division (8 FP64
-// instructions) is the most expensive operation of the form.  Everything here returns the bits of
+// in integer instructions costs next to nothing beside one FP64 add, and a division (the time of 9
+// FP64 instructions) is the most expensive operation of the form.  Everything here returns the bits of
 // the plain expression it replaces (zeros may differ in sign; quotients below 2^-600 take the
 // plain division).
 #pragma once
@@ -57,7 +57,7 @@ __device__ __forceinline__ double div_edge64(double x, double y, bool y_mid) {
 // RN(x / y) with r = recip64(y): x (h + l) is within a rounding of x/y (a faithful quotient), the
 // remainder x - y q is then exact and q + (x - y q) h rounds correctly (P. Markstein, Computation
 // of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).
-// 4 FP64 instructions instead of 8.
+// 4 FP64 instructions instead of 9.
 __device__ __forceinline__ double sdiv64(double x, double y, double2 r) {
     double q = __fma_rn(x, r.x, __dmul_rn(x, r.y));
     q = __fma_rn(__fma_rn(-y, q, x), r.x, q);

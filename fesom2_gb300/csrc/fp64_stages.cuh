@@ -7,7 +7,7 @@
 //   * v + |v| and v - |v| are 2v or 0: an upwind sum T1 (v + |v|) + T2 (v - |v|) is one product of
 //     the upwind value, and 0.5 * (T * 2v) is T * v; both only while the operand that drops out
 //     is finite (0 * inf is a NaN the reference would produce), else the full expression;
-//   * divisions by shared or constant divisors take 3 or 4 instructions instead of 8;
+//   * divisions by shared or constant divisors take 3 or 4 instructions instead of 9;
 //   * the wet levels of a tile of entities are dealt to the threads one after another (Tile), so
 //     every warp but a tile's last is full.  A warp per column left 27 to 50 % of the lanes idle
 //     (47 layers are 32 + 15 lanes), and an FP64 instruction costs its 19 cycles however many
@@ -524,7 +524,7 @@ k_bounds_rpm(DTopo tp, DGeom<double> g, DTracers<double> tr, double dt, int tile
 // update of diff_tracers_ale (src/oce_ale_tracer.F90:319-321, 743-754).
 // The limited edge flux is formed at each end node from R+/R- of both ends; a limited interface
 // flux once, in a first pass over the tile.  About 60 FP64 instructions per node-layer and
-// tracer (118 before: six of its divisions are by areasvol, at 4 instead of 8 each): 2.96 -> 1.23 ms on
+// tracer (118 before: six of its divisions are by areasvol, at 4 instead of 9 each): 2.96 -> 1.23 ms on
 // the sphere of 7 subdivisions, 48 levels, 2 tracers, at the FP64 unit's rate.
 // ===========================================================================
 static __global__ void __launch_bounds__(kTileThreads)

@@ -105,9 +105,8 @@ struct MinB {
 __device__ __forceinline__ size_t i1(int nz, int n, int L1) { return (size_t)n * L1 + (nz - 1); }
 
 // FP32 quotients of the node stages (geometry factors, limiter ratios): the fast division
-// (2 ulp) instead of the correctly rounded one; far inside the FP32 form's 1e-5, and the FCT
-// clamp into the stored bounds keeps every result inside its bounds whatever the last bits
-// of R+/R-
+// (2 ulp) instead of the correctly rounded one; far inside the FP32 form's 1e-5.  A limited value
+// may pass its bounds by the last bits of R+/R- (a build with the FCT clamp holds it inside them)
 __device__ __forceinline__ float qdiv(float a, float b) { return __fdividef(a, b); }
 
 }  // namespace
@@ -906,10 +905,11 @@ __global__ void __launch_bounds__(256) k32_ho_nodemean(DTopo tp, B32View B, Musc
 // k32_bounds: FCT bounds and R+ / R- (FCT groups only)
 // ---------------------------------------------------------------------------
 // FCT bounds (max / min of LO and T over the node, its neighbours and the adjacent layers) and R+ / R-
-// of the FCT groups.  320 bytes from L2 per layer and group of 4, at 9 TB/s: what bounds it with several
-// groups, the latency of the gathers with one.  Sphere of 7 subdivisions, T and S: 220 -> 152 us against
-// a warp per node; 24 tracers on the sphere of 8: 5.1 -> 5.5 ms, where the barrier per group costs more
-// than the full lanes give.
+// of the FCT groups.  Bound by the latency of its gathers, 320 bytes per layer and group of 4: 7.8 warps
+// a scheduler at 64 registers issue in 50 % of the cycles, and of the rest most wait for loads; L2 at
+// 36 % of its rate, DRAM at 42 % (12 tracers, 70 layers).  Sphere of 7 subdivisions, T and S: 220 -> 152
+// us against a warp per node; 24 tracers on the sphere of 8: 5.1 -> 5.5 ms, where the barrier per group
+// costs more than the full lanes give.
 template <int G>
 using BoundsBuf = Vec<G>[2][2][kNT];  // [buffer][max, min][thread]
 
@@ -1191,9 +1191,10 @@ __device__ __forceinline__ void vdiff_unit(const DTopo &tp, const B32View &B, co
 // ---------------------------------------------------------------------------
 // k32_update: limited update, T*
 // ---------------------------------------------------------------------------
-// 440 bytes from L2 per layer and group of 4 (R+ and R- of six neighbours, six edge fluxes), at 9 TB/s
-// with several groups; latency with one.  Sphere of 7 subdivisions, T and S, with the diffusion: 331 ->
-// 231 us against a warp per node; 24 tracers on the sphere of 8: 7.2 -> 7.2 ms.
+// Bound by the latency of its gathers, 440 bytes per layer and group of 4 (R+ and R- of six neighbours,
+// six edge fluxes): issue 38 % with 5.9 warps a scheduler at 80 registers, L2 at 30 % of its rate, DRAM
+// at 42 % (12 tracers, 70 layers).  Sphere of 7 subdivisions, T and S, with the diffusion: 331 -> 231 us
+// against a warp per node; 24 tracers on the sphere of 8: 7.2 -> 7.2 ms.
 template <int G>
 using UpdateBuf = Vec<G>[2][kNT];  // [buffer][thread]: limited interface fluxes
 

@@ -133,7 +133,7 @@ __device__ __forceinline__ void vdiff_col_solve(const ColScratch &s, int nzmin, 
 //
 // Entry (level, column) of a shared array sits at level * pad + column with an odd pad: both a lane
 // per column and a lane per level touch different banks.  Deeper columns than the shared memory
-// holds (217 layers) take the thread per column.
+// holds (217 layers), and many deep ones (vdiff_by_column), take the thread per column.
 constexpr int kVCols = 32, kVThreads = 256, kVChunk = 8;
 constexpr size_t kVSmemMax = 224 * 1024;
 constexpr size_t kVSmemHalf = 115200;  // two blocks of it, their VTile and 1 KB reserved for each fill an SM's 228 KB
