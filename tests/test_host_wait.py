@@ -27,8 +27,15 @@ int main() {
     check(wait_event(nullptr, 30) == cudaErrorNotReady, "the limit ends it");
     const auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
     check(ms >= 30 && ms < 2000, "the limit's time");
-    // 5 ms of spinning, then sleeps: one yield in 500 us (fewer where this process has to wait for a core)
-    check(yields >= 1 && yields <= 12, "the spin's yields");
+    // 5 ms of spinning, then sleeps: one yield in 500 us (fewer where this process has to wait for a core, so
+    // a wait without one is tried again)
+    long most = yields;
+    for (int k = 0; k < 20 && !most; k++) {
+        reset(1l << 60, cudaSuccess);
+        wait_event(nullptr, 10);
+        most = yields;
+    }
+    check(most >= 1 && most <= 12, "the spin's yields");
     return bad;
 }
 """
